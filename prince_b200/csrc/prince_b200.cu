@@ -634,10 +634,11 @@ __global__ void k_eval_exp(const double* __restrict__ x, double* __restrict__ y,
 //
 // Per step, two launches (stage 1 and 2) over the rows; short rows get a warp,
 // rows with more than kLongRow coupling entries a whole CTA.  The per-row
-// factors of a step (kappa, eD, phi1, phi2) are computed once per row by the
-// stage-2 launch of the previous step (k_prep for the first step) into a
-// buffer pair indexed by the step's parity, so the column tiles of the batched
-// kernel never recompute them.
+// factors of a step (kappa, eD, phi1, phi2) depend on z alone: k_prep computes
+// them for a run of steps in one launch (kPrepRows rows x steps), so that the
+// serial double-double exp of a row is never on a step's critical path.  One
+// launch per step (as part of the stage-2 kernels and a kernel of its own) cost
+// 5 us of latency each; a run of 16 steps of the A <= 56 network takes 15 us.
 // ---------------------------------------------------------------------------
 struct StepParams {
   int64_t n;
@@ -678,11 +679,13 @@ struct StepParams {
   int n_src;
   const int* src_ptr;
   const double* coeff;
-  // per-row step factors, [2][n] each (parity of the step)
-  double* eD;
-  double* phi1;
-  double* phi2;
-  double* kap;
+  // per-row factors of this step (n each), inside the run of steps of `rf`
+  const double* eD;
+  const double* phi1;
+  const double* phi2;
+  const double* kap;
+  double* rf;               // [steps][4][n] eD, phi1, phi2, kappa of a run of steps
+  int64_t rf_k0;            // step of rf's first entry
   // states
   const double* src;  // stage 1: x ; stage 2: a
   const double* x;    // stage 1: x
@@ -705,10 +708,10 @@ struct StepParams {
   int ctiles;               // column tiles per long row in `counter`
   // recording for the adjoint (all null in a plain solve)
   double inv_scale;         // 1 / photon scale
-  double* dsig;             // [2][n] d(d)/d(scale)
-  double* dphi1;            // [2][n] phi1'(h d)
-  double* dphi2;            // [2][n] phi2'(h d)
-  double* rec_rf;           // [rec_len][4][n]: eD, phi1, phi2, kappa of each recorded step
+  const double* dsig;       // n: d(d)/d(scale) of this step
+  const double* dphi1;      // n: phi1'(h d)
+  const double* dphi2;      // n: phi2'(h d)
+  double* dsf;              // [steps][3][n] of the three, for the run of steps from prep_k0
   double* rec_P;            // [rec_len][n x ld]
   double* rec_Q;            // [rec_len][n x ld]
   double* rec_sx;           // n x ld: S x of the current step (stage 1 -> stage 2)
@@ -728,7 +731,9 @@ struct StepParams {
   int slab_maxq;            // quads of the largest bin (shared-memory sizing)
   int slab_maxp;            // row quartets of a bin
   const int* slab_rowslot;  // [n] quartet slot of each bin-local row (-1: other rows)
-  double* slab_fac;         // [2][3][slab_nslots] eD, phi1, phi2 of the bin-local rows in quartet-slot order
+  const double* slab_fac;   // [3][slab_nslots] eD, phi1, phi2 of the bin-local rows of this step in quartet-slot order
+  double* sfac;             // [steps][3][slab_nslots] for the run of steps from prep_k0, or null
+  int64_t prep_k0;          // first step of the run of steps of sfac and dsf
   int64_t slab_nslots;
   const int* fd_cnt;        // per bin: FD stencil entries, row offsets and values
   const int* fd_off;
@@ -818,58 +823,78 @@ __device__ __forceinline__ void row_prep(const StepParams& p, int64_t step, int6
   if (s.decay) d = __dadd_rn(d, __dmul_rn(p.l_diag[r], s.dl));
   double e, f1, f2;
   phi_of(s.h, d, e, f1, f2);
-  const size_t o = (size_t)(step & 1) * p.n + r;
-  p.eD[o] = e;
-  p.phi1[o] = f1;
-  p.phi2[o] = f2;
-  p.kap[o] = k;
-  if (p.slab_rowslot) {  // k_slab stages the factors of a bin's rows as three contiguous runs
+  double* rf = p.rf + (size_t)(step - p.rf_k0) * 4 * p.n + r;
+  rf[0] = e;
+  rf[p.n] = f1;
+  rf[2 * p.n] = f2;
+  rf[3 * p.n] = k;
+  if (p.sfac) {  // k_slab stages the factors of a bin's rows as three contiguous runs
     const int sl = p.slab_rowslot[r];
     if (sl >= 0) {
-      double* fc = p.slab_fac + (size_t)(step & 1) * 3 * p.slab_nslots + sl;
+      double* fc = p.sfac + (size_t)(step - p.prep_k0) * 3 * p.slab_nslots + sl;
       fc[0] = e;
       fc[p.slab_nslots] = f1;
       fc[2 * p.slab_nslots] = f2;
     }
   }
-  if (p.dsig) {  // derivatives with respect to the photon scale (adjoint record pass)
+  if (p.dsf) {  // derivatives with respect to the photon scale (adjoint record pass)
     const double md = p.m_diag[(size_t)s.w * p.n + r] * p.inv_scale;
     double ds = md;
     if (s.kap && s.pair) ds += (p.kp[(size_t)s.w * p.n + r] * p.inv_scale) * p.d_diag[r];
     ds *= s.dl;
     double d1, d2;
     dphi_of(s.h * d, e, f1, f2, d1, d2);
-    p.dsig[o] = ds;
-    p.dphi1[o] = d1;
-    p.dphi2[o] = d2;
-  }
-  if (p.rec_rf) {
-    const int64_t j = step - p.rec_k0;
-    if (j >= 0 && j < p.rec_len) {
-      double* rf = p.rec_rf + (size_t)j * 4 * p.n;
-      rf[r] = e;
-      rf[p.n + r] = f1;
-      rf[2 * p.n + r] = f2;
-      rf[3 * p.n + r] = k;
-    }
+    double* g = p.dsf + (size_t)(step - p.prep_k0) * 3 * p.n + r;
+    g[0] = ds;
+    g[p.n] = d1;
+    g[2 * p.n] = d2;
   }
 }
 
-__global__ void k_prep(StepParams p) {
+// The row factors of the steps prep_k0 .. prep_k0 + gridDim.y - 1.
+__global__ void __launch_bounds__(128) k_prep(StepParams p) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < p.n) row_prep(p, p.step, r);
+  if (r < p.n) row_prep(p, p.prep_k0 + blockIdx.y, r);
+}
+
+constexpr int64_t kPrepRows = 1 << 19;  // rows x steps of one k_prep launch (about 30 MB of factors)
+// Steps whose factors one launch prepares.
+constexpr int64_t kPrepMaxSteps = 1024;
+inline int64_t prep_steps(int64_t n) {
+  return std::max<int64_t>(4, std::min<int64_t>(kPrepMaxSteps, kPrepRows / std::max<int64_t>(n, 1)));
+}
+
+// Prepares the steps [k0, k0 + count) (the factors land at steps k0 - rf_k0 .. of p.rf).
+void launch_prep(StepParams& p, int64_t k0, int64_t count, cudaStream_t st) {
+  p.prep_k0 = k0;
+  k_prep<<<dim3(blocks_for(p.n, 128), (unsigned)count), 128, 0, st>>>(p);
+}
+
+// Points the per-step factor pointers at step k of the prepared run.
+void set_step_factors(StepParams& p, int64_t k) {
+  p.eD = p.rf + (size_t)(k - p.rf_k0) * 4 * p.n;
+  p.phi1 = p.eD + p.n;
+  p.phi2 = p.eD + 2 * p.n;
+  p.kap = p.eD + 3 * p.n;
+  if (p.sfac) p.slab_fac = p.sfac + (size_t)(k - p.prep_k0) * 3 * p.slab_nslots;
+  if (p.dsf) {
+    p.dsig = p.dsf + (size_t)(k - p.prep_k0) * 3 * p.n;
+    p.dphi1 = p.dsig + p.n;
+    p.dphi2 = p.dsig + 2 * p.n;
+  }
 }
 
 // ---------------------------------------------------------------------------
 // Scratch of pb_integrate_const_noalloc: one file-scope device array (every
 // GPU that loads the library holds it until exit).  Layout, in bytes from the
-// start: a and F(x) (n doubles each), the row factors (8 n doubles), the
+// start: a and F(x) (n doubles each), the row factors of two steps (8 n doubles), the
 // per-step h and dl/dz (s doubles each), the window index (s ints), the row
 // list (n ints), an all-zero row pointer (n + 1 int64) and a 256-byte status
 // block (the CSR check's flag), for n = the state limit and s = the step limit.
 // ---------------------------------------------------------------------------
 constexpr int64_t kNaMaxStates = PB_NOALLOC_MAX_STATES;
 constexpr int64_t kNaMaxSteps = PB_NOALLOC_MAX_STEPS;
+constexpr int kNaPrepSteps = 2;  // steps whose row factors fit the scratch
 constexpr size_t kNaBytes = (size_t)kNaMaxStates * 10 * sizeof(double) + (size_t)kNaMaxSteps * 2 * sizeof(double) +
                             (size_t)kNaMaxSteps * sizeof(int) + (size_t)kNaMaxStates * sizeof(int) +
                             (size_t)(kNaMaxStates + 1) * sizeof(int64_t) + 256;
@@ -923,7 +948,7 @@ __device__ __forceinline__ double inj_at(const StepParams& p, const StepScalars&
 // CSR order without contraction, as the host sparse products do.
 __device__ __forceinline__ double finish_F(const StepParams& p, const StepScalars& s, int64_t r,
                                            int k, const double* __restrict__ v, double sM) {
-  const double* kap = p.kap + (size_t)(p.step & 1) * p.n;
+  const double* kap = p.kap;
   double out = sM;
   if (s.kap) {
     double sD = 0.0;
@@ -964,7 +989,7 @@ __device__ __forceinline__ double scale_deriv_apply(const StepParams& p, const S
 template <int STAGE>
 __device__ __forceinline__ void record(const StepParams& p, const StepScalars& s, int64_t r, int k, double sM,
                                        double F) {
-  const size_t o = (size_t)(p.step & 1) * p.n + r;
+  const int64_t o = r;
   const size_t idx = (size_t)r * p.ld + k;
   const int64_t j = p.step - p.rec_k0;
   if (j < 0 || j >= p.rec_len) return;
@@ -984,7 +1009,7 @@ __device__ __forceinline__ void record(const StepParams& p, const StepScalars& s
 template <int STAGE>
 __device__ __forceinline__ void row_epilogue(const StepParams& p, const StepScalars& s, int64_t r,
                                              int k, double sM) {
-  const size_t o = (size_t)(p.step & 1) * p.n + r;
+  const int64_t o = r;
   const size_t idx = (size_t)r * p.ld + k;
   const double F = finish_F(p, s, r, k, p.src, sM);
   if (p.rec_P) record<STAGE>(p, s, r, k, sM, F);
@@ -998,11 +1023,6 @@ __device__ __forceinline__ void row_epilogue(const StepParams& p, const StepScal
     const double dF = __dmul_rn(__dadd_rn(F, -p.f[idx]), s.h);
     p.xout[idx] = __dadd_rn(p.a[idx], __dmul_rn(dF, p.phi2[o]));
   }
-}
-
-// stage 2 of step k prepares the row factors of step k + 1 (one thread per row)
-__device__ __forceinline__ void prep_next(const StepParams& p, int64_t r) {
-  if (p.step + 1 < p.n_steps) row_prep(p, p.step + 1, r);
 }
 
 // Long rows are cut into segments of at most kSegLen coupling entries.  A warp
@@ -1043,7 +1063,6 @@ __global__ void __launch_bounds__(256) k_step_plain(StepParams p) {
       for (int64_t j = p.m_indptr[r]; j < j1; ++j) acc = __dadd_rn(acc, __dmul_rn(mv[j], v[p.m_indices[j]]));
     }
     row_epilogue<STAGE>(p, s, r, 0, acc);
-    if (STAGE == 2) prep_next(p, r);
     return;
   }
   const int seg = (blockIdx.x - p.nsb) * (blockDim.x >> 5) + wid;
@@ -1061,7 +1080,6 @@ __global__ void __launch_bounds__(256) k_step_plain(StepParams p) {
     for (int q = 0; q < ns; ++q) t += __ldcg(p.partial + s0 + q);
     const int64_t r = p.lr_row[lr];
     row_epilogue<STAGE>(p, s, r, 0, t);
-    if (STAGE == 2) prep_next(p, r);
   }
 }
 
@@ -1106,7 +1124,6 @@ __global__ void __launch_bounds__(256) k_step_multi(StepParams p) {
     const double acc = s.photohad ? gather_sum(mv, p.m_indices, v, p.ld, kk, p.m_indptr[r], p.m_indptr[r + 1], lane)
                                   : 0.0;
     if (active) row_epilogue<STAGE>(p, s, r, k, acc);
-    if (STAGE == 2 && blockIdx.y == 0 && lane == 0) prep_next(p, r);
     return;
   }
   const int seg = (blockIdx.x - p.nsb) * (blockDim.x >> 5) + wid;
@@ -1120,7 +1137,6 @@ __global__ void __launch_bounds__(256) k_step_multi(StepParams p) {
   for (int q = 0; q < ns; ++q) t = __dadd_rn(t, __ldcg(p.partial + (size_t)(s0 + q) * p.ld + blockIdx.y * kColTile + lane));
   const int64_t r = p.lr_row[lr];
   if (active) row_epilogue<STAGE>(p, s, r, k, t);
-  if (STAGE == 2 && blockIdx.y == 0 && lane == 0) prep_next(p, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -1211,14 +1227,13 @@ __global__ void __launch_bounds__(256) k_fd(StepParams p) {
   double* vb = fsm;                  // d x 32
   double* kb = fsm + d * kColTile;   // d
   double* kpb = kb + d;              // d: kappa_pair of the window (recording only)
-  const size_t o0 = (size_t)(p.step & 1) * p.n;
   const double* __restrict__ v = p.src + (size_t)sp * d * ld + blockIdx.y * kColTile;
   for (int t = threadIdx.x; t < d * (kColTile / 2); t += blockDim.x) {
     const int e = t / (kColTile / 2), c = 2 * (t - e * (kColTile / 2));
     cp_async16(vb + e * kColTile + c, v + (size_t)e * ld + c);
   }
   cp_async_commit();
-  for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[o0 + (size_t)sp * d + e];
+  for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[(size_t)sp * d + e];
   const double* kpw = p.fdkp ? p.kp + (size_t)p.win[p.step] * p.n + (size_t)sp * d : nullptr;
   if (kpw)
     for (int e = threadIdx.x; e < d; e += blockDim.x) kpb[e] = kpw[e];
@@ -1259,7 +1274,6 @@ __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
   double* wt = vb + (size_t)d * kColTile;        // d x kFdDenseW
   double* kb = wt + (size_t)d * kFdDenseW;       // d
   double* kpb = kb + d;                          // d: kappa_pair of the window (KP)
-  const size_t o0 = (size_t)(p.step & 1) * p.n + (size_t)sp * d;
   const double* __restrict__ v = p.src + (size_t)sp * d * ld + blockIdx.y * kColTile;
   for (int t = threadIdx.x; t < d * (kColTile / 2); t += blockDim.x) {
     const int e = t / (kColTile / 2), c = 2 * (t - e * (kColTile / 2));
@@ -1267,7 +1281,7 @@ __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
   }
   for (int t = threadIdx.x; t < d * (kFdDenseW / 2); t += blockDim.x) cp_async16(wt + 2 * t, p.fd_dense + 2 * t);
   cp_async_commit();
-  for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[o0 + e];
+  for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[(size_t)sp * d + e];
   if (KP)
     for (int e = threadIdx.x; e < d; e += blockDim.x) kpb[e] = p.kp[(size_t)p.step_w * p.n + (size_t)sp * d + e];
   cp_async_wait<0>();
@@ -1312,7 +1326,7 @@ __device__ __forceinline__ void record_blocked(const StepParams& p, const StepSc
                                                double sM, double F, double own, double fprev) {
   const int64_t j = p.step - p.rec_k0;
   if (j < 0 || j >= p.rec_len) return;
-  const size_t o = (size_t)(p.step & 1) * p.n + r;
+  const int64_t o = r;
   const size_t idx = (size_t)r * p.ld + k;
   const size_t ro = (size_t)j * p.n * p.ld + idx;
   const double h = s.h, ds = p.dsig[o];
@@ -1429,7 +1443,6 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   const int colA = col0 + 2 * j;  // this lane's columns colA, colA + 1 (< ld)
   const bool actA = colA < p.ncols, actB = colA + 1 < p.ncols;
   const StepScalars s = load_scalars(p, p.step);
-  const size_t o0 = (size_t)(p.step & 1) * p.n;
   const int ld = p.ld, d = p.d;
   SlabSmem L(sm, p.nsp, p.slab_maxq, p.slab_maxp);
   const int qb = p.slab_qbase[e], nqb = p.slab_qbase[e + 1] - qb;
@@ -1437,7 +1450,7 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   const int fs = kSlabRows * p.slab_maxp;  // stride of the three row-factor arrays
   unsigned long long* stage_bar = L.bar;
   const double* mv = p.slab_vals + (size_t)p.step_w * p.slab_stride + (size_t)qb * 4;
-  const double* fc = p.slab_fac + (size_t)(p.step & 1) * 3 * p.slab_nslots + (size_t)kSlabRows * gb0;
+  const double* fc = p.slab_fac + (size_t)kSlabRows * gb0;
   if (p.tmap_src) {  // TMA: the slab as tensor boxes, the rest as bulk copies, one barrier
     if (threadIdx.x == 0) mbar_init(stage_bar, 1);
     __syncthreads();
@@ -1502,8 +1515,8 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
         if (need_f) fxr[U] = *reinterpret_cast<const double2*>(p.f + r_ * ld + colA);                    \
         if (s.inj) slr[U] = p.inj_slot[r_];                                                              \
         if (rec_on) {                                                                                    \
-          rds[U] = p.dsig[o0 + r_];                                                                      \
-          rd12[U] = STAGE == 1 ? p.dphi1[o0 + r_] : p.dphi2[o0 + r_];                                    \
+          rds[U] = p.dsig[r_];                                                                           \
+          rd12[U] = STAGE == 1 ? p.dphi1[r_] : p.dphi2[r_];                                              \
           rkp[U] = (s.kap && s.pair) ? *reinterpret_cast<const double2*>(p.fdkp + r_ * ld + colA) : z2;  \
           rsx[U] = STAGE == 2 ? *reinterpret_cast<const double2*>(p.rec_sx + r_ * ld + colA) : z2;       \
         }                                                                                                \
@@ -1637,15 +1650,6 @@ SlabKernel slab_kernel(int stage, bool rec, int pre) {
     case 3: return slab_kernel_p<3>(stage, rec);
     default: return slab_kernel_p<2>(stage, rec);
   }
-}
-
-// Stage 2: the row factors of the next step for the bin-local rows (one
-// thread per row; the band rows are prepared by k_band_finish).
-__global__ void k_slab_prep(StepParams p) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)p.n_slab_spec * p.d) return;
-  const int i = (int)(t / p.d), e = (int)(t - (int64_t)i * p.d);
-  prep_next(p, (int64_t)p.slab_spec[i] * p.d + e);
 }
 
 // Band partial sums.  CTA = (64-column block, mother-species group, pair of
@@ -1815,7 +1819,7 @@ __global__ void __launch_bounds__(256) k_band_finish(StepParams p) {
     }
     out = __dmul_rn(out, s.dl);
     if (s.inj) out = __dadd_rn(out, inj_at(p, s, r, col));
-    const size_t o = (size_t)(p.step & 1) * p.n + r;
+    const int64_t o = r;
     if (p.rec_P) record_blocked<STAGE>(p, s, r, col, t, out, p.x[idx], STAGE == 2 ? p.f[idx] : 0.0);
     if (STAGE == 1) {
       p.a[idx] = __dadd_rn(__dmul_rn(p.eD[o], p.x[idx]), __dmul_rn(__dmul_rn(p.phi1[o], out), s.h));
@@ -1825,7 +1829,6 @@ __global__ void __launch_bounds__(256) k_band_finish(StepParams p) {
       p.xout[idx] = __dadd_rn(p.a[idx], __dmul_rn(dF, p.phi2[o]));
     }
   }
-  if (STAGE == 2 && blockIdx.y == 0 && lane == 0) prep_next(p, r);
 }
 
 // Band partial sums with TMA staging (8 warps; the same tiles and arithmetic
@@ -2945,6 +2948,12 @@ void csr_transpose(int64_t n, int64_t nnz, const int64_t* ip, const int32_t* ix,
 }
 
 
+// Whether a solve with K columns runs the bin-blocked kernels.
+bool use_blocked(const pb_context* c, int K) {
+  const int64_t ld = ((K + kColTile - 1) / kColTile) * kColTile;
+  return c->blocked_ok && c->fd_tab_ok && c->batched_mode == 1 && K > 1 && c->n * ld < ((int64_t)1 << 31);
+}
+
 // Step parameters of a solve on the context's device buffers.
 void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flags, bool pair, bool inj, int64_t S,
                       int ctiles) {
@@ -2988,10 +2997,7 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.a = c->A.as<double>();
   p.f = c->F.as<double>();
   p.n_steps = S;
-  p.eD = c->rowf.as<double>();
-  p.phi1 = p.eD + 2 * n;
-  p.phi2 = p.eD + 4 * n;
-  p.kap = p.eD + 6 * n;
+  p.rf = c->rowf.as<double>();
   p.rows = c->short_rows.as<int>();
   p.nrows = (int)c->h_short_rows.size();
   p.nsb = (int)blocks_for(p.nrows, K == 1 ? 256 : 8);   // thread per row (K = 1) or warp per row
@@ -3017,8 +3023,8 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.slab_stride = c->slab_nent;
   p.slab_maxq = c->slab_maxbin;
   p.slab_maxp = (c->n_slab_spec + kSlabRows - 1) / kSlabRows;
-  p.slab_rowslot = c->blocked_ok ? c->slab_rowslot.as<int>() : nullptr;
-  p.slab_fac = c->slab_fac.as<double>();
+  p.slab_rowslot = c->slab_rowslot.as<int>();
+  p.sfac = use_blocked(c, K) ? c->slab_fac.as<double>() : nullptr;
   p.slab_nslots = c->slab_nslots;
   p.fd_cnt = c->fd_cnt.as<int>();
   p.fd_off = c->fd_off.as<int>();
@@ -3143,12 +3149,6 @@ const CUtensorMap* stage_tmap_band(const pb_context* c, int stage) {
                                                           : nullptr;
 }
 
-// Whether a solve with K columns runs the bin-blocked kernels.
-bool use_blocked(const pb_context* c, int K) {
-  const int64_t ld = ((K + kColTile - 1) / kColTile) * kColTile;
-  return c->blocked_ok && c->fd_tab_ok && c->batched_mode == 1 && K > 1 && c->n * ld < ((int64_t)1 << 31);
-}
-
 // One stage of the bin-blocked path: k_band on the second stream, k_fd then
 // k_slab on the launching stream, then k_band_finish (and the next step's row
 // factors of the bin-local rows after stage 2).
@@ -3217,10 +3217,6 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   const dim3 sg(p.d, (unsigned)blocks_for(p.ncols, kSlabCols));
   slab_kernel(STAGE, p.rec_P != nullptr, c->slab_pre)<<<sg, kSlabWarps * 32, c->slab_smem, st>>>(p);
   ++launches;
-  if (STAGE == 2 && p.step + 1 < p.n_steps) {
-    k_slab_prep<<<blocks_for((int64_t)p.n_slab_spec * p.d, 256), 256, 0, st>>>(p);
-    ++launches;
-  }
   if (c->n_tail > 0) {  // tail rows (another grid): the general row kernel, a warp per row
     if (c->tail_wait) {  // the previous step's EM hook (on its own stream) writes the tail rows
       cudaStreamWaitEvent(st, c->ev_hook_done, 0);
@@ -3312,7 +3308,8 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
   double* X = c->X.as<double>();
   const size_t sbytes = (size_t)n * p.ld * sizeof(double);
   int64_t launches = 0;
-  bool prepared = false;
+  int64_t prepared = -1;  // end of the run of steps whose row factors are ready
+  const bool record = p.rec_P != nullptr;  // the factors of the segment stay in p.rf for the sweep
   const bool em = c->have_em && (p.flags & PB_EM_CASCADE);
   // With the EM rows as the tail of the bin-blocked layout, a step's EM hook
   // (it reads the nuclei and writes only the EM rows) runs on stream3 beside
@@ -3333,11 +3330,14 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
     p.step_w = c->h_win[k];
     p.ncols = n_active[k];
     if (p.ncols == 0) continue;
-    if (!prepared) {  // row factors of the first active step; later steps get them from stage 2
-      k_prep<<<blocks_for(n, 256), 256, 0, st>>>(p);
+    if (k >= prepared) {
+      const int64_t count = std::min<int64_t>(prep_steps(n), k1 - k);
+      if (!record) p.rf_k0 = k;
+      launch_prep(p, k, count, st);
       ++launches;
-      prepared = true;
+      prepared = k + count;
     }
+    set_step_factors(p, k);
     const bool blocked = use_blocked(c, K) && (!p.rec_P || p.fdkp || !(p.flags & PB_PAIRPROD));
     const bool overlap = em && blocked && c->n_tail > 0;
     if (!overlap) join_hook();
@@ -3380,6 +3380,24 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
   }
   join_hook();
   return launches;
+}
+
+// All steps of a constant operator (one column), state x in place.
+void const_steps(StepParams& p, int64_t per_prep, double* x, cudaStream_t st) {
+  p.x = x;
+  p.xout = x;
+  for (int64_t k = 0; k < p.n_steps; ++k) {
+    if (k % per_prep == 0) {
+      p.rf_k0 = k;
+      launch_prep(p, k, std::min(per_prep, p.n_steps - k), st);
+    }
+    set_step_factors(p, k);
+    p.step = k;
+    p.src = x;
+    k_step_plain<1><<<blocks_for(p.n, 256), 256, 0, st>>>(p);
+    p.src = p.a;
+    k_step_plain<2><<<blocks_for(p.n, 256), 256, 0, st>>>(p);
+  }
 }
 
 }  // namespace
@@ -4093,8 +4111,9 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   if ((rc = upload(c, c->slab_wrp, wrp.data(), wrp.size()))) return rc;
   if ((rc = upload(c, c->slab_rowslot, rowslot.data(), rowslot.size()))) return rc;
   c->slab_nslots = (int64_t)squart.size();
-  PB_CUDA(c, c->slab_fac.ensure((size_t)2 * 3 * c->slab_nslots * sizeof(double)));
-  PB_CUDA(c, cudaMemsetAsync(c->slab_fac.p, 0, (size_t)2 * 3 * c->slab_nslots * sizeof(double), c->stream));
+  const size_t fac_bytes = (size_t)prep_steps(n) * 3 * c->slab_nslots * sizeof(double);
+  PB_CUDA(c, c->slab_fac.ensure(fac_bytes));
+  PB_CUDA(c, cudaMemsetAsync(c->slab_fac.p, 0, fac_bytes, c->stream));  // slots without a row stay zero
   if ((rc = upload(c, c->slab_slot, sslot.data(), sslot.size()))) return rc;
   PB_CUDA(c, cudaStreamSynchronize(c->stream));
   std::vector<const void*> slab_fns;
@@ -4261,6 +4280,9 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   p.err = c->d_err.as<int>();
   cudaStream_t st = c->stream;
+  p.rf_k0 = step;
+  launch_prep(p, step, 1, st);
+  set_step_factors(p, step);
   const bool photohad = (flags & PB_PHOTOHAD) != 0, kap = (flags & PB_PARTIAL_DIFF) != 0;
   const unsigned tiles = (unsigned)blocks_for(p.ncols, kColTile);
   const BandInstance bi = (c->band_warps == 8 && p.tmap_band) ? band_kernel_tma(c->band_RT, c->band_J)
@@ -4780,7 +4802,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
     PB_CUDA(c, c->em_wbuf.ensure((size_t)c->em_ncr * ld * sizeof(double)));
     for (DBuf* b : {&c->em_es, &c->em_lep, &c->em_y}) PB_CUDA(c, b->ensure((size_t)c->em_n * ld * sizeof(double)));
   }
-  PB_CUDA(c, c->rowf.ensure((size_t)8 * n * sizeof(double)));
+  PB_CUDA(c, c->rowf.ensure((size_t)prep_steps(n) * 4 * n * sizeof(double)));
   const int ctiles = ld / (K == 1 ? 1 : kColTile);
   const int nlong_rows = (int)c->h_long_rows.size();
   PB_CUDA(c, c->seg_mb.ensure((size_t)std::max(c->n_seg, 1) * sizeof(int64_t)));
@@ -5112,7 +5134,7 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
   PB_CUDA(c, c->mu.ensure(sb));
   PB_CUDA(c, c->rec_rf.ensure((size_t)CK * 4 * n * sizeof(double)));
   PB_CUDA(c, c->rec_sx.ensure(sb));
-  PB_CUDA(c, c->dsig.ensure((size_t)6 * n * sizeof(double)));
+  PB_CUDA(c, c->dsig.ensure((size_t)prep_steps(n) * 3 * n * sizeof(double)));
   if (want_scale) {
     PB_CUDA(c, c->rec_P.ensure((size_t)CK * sb));
     PB_CUDA(c, c->rec_Q.ensure((size_t)CK * sb));
@@ -5148,12 +5170,10 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
   const int ctiles = ld / (K == 1 ? 1 : kColTile);
   fill_step_params(c, p, K, ld, flags, pair, inj, S, ctiles);
   p.inv_scale = 1.0 / a->photon_scale;
-  p.rec_rf = c->rec_rf.as<double>();
+  p.rf = c->rec_rf.as<double>();
   p.rec_sx = c->rec_sx.as<double>();
   if (want_scale) {
-    p.dsig = c->dsig.as<double>();
-    p.dphi1 = p.dsig + 2 * n;
-    p.dphi2 = p.dsig + 4 * n;
+    p.dsf = c->dsig.as<double>();
     p.rec_P = c->rec_P.as<double>();
     p.rec_Q = c->rec_Q.as<double>();
     if (use_blocked(c, K) && pair) {  // the bin-blocked record pass needs D_off (kappa_pair v)
@@ -5190,19 +5210,15 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
     int64_t kf = k0;
     while (kf < k1 && a->n_active[kf] == 0) ++kf;
     if (kf == k1) continue;  // no active column in this segment
-    p.rec_k0 = k0;
+    p.rec_k0 = p.rf_k0 = k0;
     p.rec_len = (int)(k1 - k0);
     if (want_scale) {  // the sensitivities P, Q need the states: recompute the segment from its checkpoint
       PB_CUDA(c, cudaMemcpyAsync(c->X.p, c->ckpt.as<double>() + (size_t)sg * n * ld, sb, cudaMemcpyDeviceToDevice, st));
       PB_CUDA(c, cudaMemsetAsync(c->counter.p, 0, (size_t)std::max<size_t>(c->h_long_rows.size(), 1) * ctiles * sizeof(int), st));
       launch_steps(c, p, K, a->n_active, k0, k1, st, nullptr, 0);
     } else {  // the operator factors depend on z alone: record them without recomputing the states
-      for (int64_t k = kf; k < k1; ++k) {
-        if (a->n_active[k] == 0) continue;
-        p.step = k;
-        p.step_w = c->h_win[k];
-        k_prep<<<blocks_for(n, 256), 256, 0, st>>>(p);
-      }
+      p.sfac = nullptr;
+      for (int64_t k = kf; k < k1; k += kPrepMaxSteps) launch_prep(p, k, std::min<int64_t>(kPrepMaxSteps, k1 - k), st);
     }
     if (blockedT) {
       for (int64_t k = k1 - 1; k >= kf; --k) {
@@ -5455,7 +5471,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
     return rc;
   }
   if (A.ensure((size_t)n * sizeof(double)) != cudaSuccess || F.ensure((size_t)n * sizeof(double)) != cudaSuccess ||
-      rowf.ensure((size_t)8 * n * sizeof(double)) != cudaSuccess) {
+      rowf.ensure((size_t)prep_steps(n) * 4 * n * sizeof(double)) != cudaSuccess) {
     cleanup();
     return fail(c, PB_ERR_CUDA, "pb_integrate_const: allocation failed");
   }
@@ -5481,21 +5497,8 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   p.nrows = (int)n;
   p.nsb = (int)blocks_for(n, 256);
   p.n_steps = n_steps;
-  p.eD = rowf.as<double>();
-  p.phi1 = p.eD + 2 * n;
-  p.phi2 = p.eD + 4 * n;
-  p.kap = p.eD + 6 * n;
-  p.step = 0;
-  if (n_steps > 0) k_prep<<<blocks_for(n, 256), 256, 0, st>>>(p);
-  for (int64_t k = 0; k < n_steps; ++k) {
-    p.step = k;
-    p.x = X.as<double>();
-    p.xout = X.as<double>();
-    p.src = X.as<double>();
-    k_step_plain<1><<<blocks_for(n, 256), 256, 0, st>>>(p);
-    p.src = A.as<double>();
-    k_step_plain<2><<<blocks_for(n, 256), 256, 0, st>>>(p);
-  }
+  p.rf = rowf.as<double>();
+  const_steps(p, prep_steps(n), X.as<double>(), st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(state, X.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -5593,21 +5596,8 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
   p.nrows = (int)n;
   p.nsb = (int)blocks_for(n, 256);
   p.n_steps = n_steps;
-  p.eD = rowf;
-  p.phi1 = rowf + 2 * n;
-  p.phi2 = rowf + 4 * n;
-  p.kap = rowf + 6 * n;
-  p.step = 0;
-  if (n_steps > 0) k_prep<<<blocks_for(n, 256), 256, 0, st>>>(p);
-  for (int64_t k = 0; k < n_steps; ++k) {
-    p.step = k;
-    p.x = state;
-    p.xout = state;
-    p.src = state;
-    k_step_plain<1><<<blocks_for(n, 256), 256, 0, st>>>(p);
-    p.src = a;
-    k_step_plain<2><<<blocks_for(n, 256), 256, 0, st>>>(p);
-  }
+  p.rf = rowf;
+  const_steps(p, kNaPrepSteps, state, st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(c, PB_ERR_CUDA, "pb_integrate_const_noalloc: %s", cudaGetErrorString(e));
