@@ -33,7 +33,9 @@ struct BGemm {
   double* C;
   int M, N, K, lda, ldb, ldc;
   long long sA, sB, sC;
-  int accumulate;
+  const double* Cin;    // added to the product (laid out as C), or null
+  const StepScal* sc;   // a step's scalars: N = its active columns, A = that of its window (stride sW), or null
+  long long sW;
 };
 
 constexpr int kGn = 32, kGk = 16;
@@ -46,9 +48,15 @@ __global__ void __launch_bounds__(WM * 64) k_bgemm(BGemm g) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int wm = wid % WM, wn = wid / WM;
   const int m0 = blockIdx.y * kGm, n0 = blockIdx.x * kGn;
+  if (g.sc) {
+    g.N = g.sc->ncols;
+    if (n0 >= g.N) return;
+    g.A += g.sW * g.sc->w;
+  }
   const double* __restrict__ A = g.A + (size_t)blockIdx.z * g.sA;
   const double* __restrict__ B = g.B + (size_t)blockIdx.z * g.sB;
-  double* __restrict__ C = g.C + (size_t)blockIdx.z * g.sC;
+  const double* Ci = g.Cin ? g.Cin + (size_t)blockIdx.z * g.sC : nullptr;
+  double* C = g.C + (size_t)blockIdx.z * g.sC;
   double acc[2][2][2];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
@@ -88,20 +96,30 @@ __global__ void __launch_bounds__(WM * 64) k_bgemm(BGemm g) {
       for (int h = 0; h < 2; ++h) {
         const int col = n0 + wn * 16 + ni * 8 + (lane & 3) * 2 + h;
         if (col >= g.N) continue;
-        double* out = C + (size_t)row * g.ldc + col;
-        *out = g.accumulate ? __dadd_rn(*out, acc[mi][ni][h]) : acc[mi][ni][h];
+        const size_t o = (size_t)row * g.ldc + col;
+        C[o] = Ci ? __dadd_rn(Ci[o], acc[mi][ni][h]) : acc[mi][ni][h];
       }
     }
 }
 
+void launch_bgemm(cudaStream_t st, const BGemm& g, int batch) {
+  const long long ctas64 = (long long)((g.N + kGn - 1) / kGn) * ((g.M + 63) / 64) * batch;
+  if (ctas64 < 256)
+    k_bgemm<2><<<dim3((g.N + kGn - 1) / kGn, (g.M + 31) / 32, batch), 128, 0, st>>>(g);
+  else
+    k_bgemm<4><<<dim3((g.N + kGn - 1) / kGn, (g.M + 63) / 64, batch), 256, 0, st>>>(g);
+}
+
 void bgemm(cudaStream_t st, const double* A, const double* B, double* C, int M, int N, int K, int lda, int ldb,
            int ldc, long long sA, long long sB, long long sC, int batch, bool accumulate) {
-  BGemm g{A, B, C, M, N, K, lda, ldb, ldc, sA, sB, sC, accumulate ? 1 : 0};
-  const long long ctas64 = (long long)((N + kGn - 1) / kGn) * ((M + 63) / 64) * batch;
-  if (ctas64 < 256)
-    k_bgemm<2><<<dim3((N + kGn - 1) / kGn, (M + 31) / 32, batch), 128, 0, st>>>(g);
-  else
-    k_bgemm<4><<<dim3((N + kGn - 1) / kGn, (M + 63) / 64, batch), 256, 0, st>>>(g);
+  launch_bgemm(st, BGemm{A, B, C, M, N, K, lda, ldb, ldc, sA, sB, sC, accumulate ? C : nullptr, nullptr, 0}, batch);
+}
+
+// C = A_w B (+ Cin) on a step's active columns: A (M x K) of the step's window
+// at A + w sW, B and C with leading dimension ld; `cols` bounds the grid.
+void bgemm_step(cudaStream_t st, const StepScal* sc, const double* A, long long sW, const double* B, const double* Cin,
+                double* C, int M, int cols, int K, int ld) {
+  launch_bgemm(st, BGemm{A, B, C, M, cols, K, K, ld, ld, 0, 0, 0, Cin, sc, sW}, 1);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,7 +1,7 @@
 // prince_b200 -- B200-native ETD2 propagation core (sm_100a).
 //
 // One solve of the transport equation dn/dz = L(z) n + b(z) runs entirely on the
-// device, in one CUDA graph:
+// device:
 //
 //   1. photon matrix   PT[w][j] = s * n_gamma(E_ph[j], z_w)          (all windows)
 //   2. pair-loss rate  kp[w][r] = scale[r] * trapz_xi(...)            (all windows)
@@ -51,6 +51,15 @@ constexpr int kMaxBhSpecies = 3072;  // charged nuclei of the hook's pair weight
 
 thread_local std::string g_error;
 
+// The scalars of one redshift step, read on the device, so that a captured run
+// of steps can be replayed for any schedule.
+struct __align__(16) StepScal {
+  double h, dl, hc, finj;
+  long long step;
+  int w;        // rate window
+  int ncols;    // active columns
+};
+
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------
@@ -79,6 +88,12 @@ struct DBuf {
 
 constexpr long long kWaitTries = 1ll << 24;  // polls of a bounded wait (well above any staging time)
 constexpr int kSlabPreDefault = 2;           // k_slab's default prefetch depth (row quartets)
+struct StepGraph {  // a captured run of steps and the parameters it was captured for
+  std::vector<uint64_t> key;
+  cudaGraphExec_t exec = nullptr;
+  int64_t launches = 0;
+  uint64_t used = 0;
+};
 struct pb_context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -123,13 +138,14 @@ struct pb_context {
 
   // per-solve workspace
   DBuf PT, zwin, rs, kp, keep, pos, dest, m_indptr, m_indices, m_vals, m_diag;
-  DBuf s_h, s_dldz, s_hc, s_finj, s_win, s_coeff;
+  DBuf s_scal, s_finj, s_coeff;     // step scalars; the adjoint's gradients read finj alone
+  DBuf s_run;                       // scalars of the run of steps a captured graph is replayed for
   DBuf X, A, F, rowf;
   DBuf scan_tmp;
   size_t scan_tmp_bytes = 0;
   int32_t last_W = 0;
   bool have_solution = false;
-  std::vector<int32_t> h_win;   // window of each step of the current solve (host copy)
+  std::vector<StepScal> h_scal;  // step scalars of the current solve (host copy)
   std::vector<int32_t> h_nact;  // active columns of each step of the last solve (host copy)
   int64_t band_nnz = 0, slab_nnz = 0;  // coupling entries of the band rows and the bin-local rows
 
@@ -200,7 +216,7 @@ struct pb_context {
   int64_t em_g = -1, em_m = -1, em_p = -1;
   DBuf em_bh_off, em_bh_A, em_invE, em_dE, em_Tg, em_Te, em_R, em_wbuf, em_es, em_lep, em_y;
   DBuf em_TgT, em_TeT, em_RT;       // per-window transposes (adjoint)
-  std::vector<double> em_dl;
+  DBuf em_dlw;                      // dl_step per window
 
   // transposed constant operators (adjoint)
   DBuf dt_indptr, dt_indices, dt_vals, lt_indptr, lt_indices, lt_vals;
@@ -213,10 +229,9 @@ struct pb_context {
   uint32_t last_flags = 0;
   double last_scale = 1.0;
 
-  // CUDA graph of the last solve's device work and the shape it was captured for
-  cudaGraphExec_t graph_exec = nullptr, graph_exec2 = nullptr;
-  std::vector<uint64_t> graph_key;
-  int64_t graph_launches = 0;
+  // captured runs of steps
+  std::vector<StepGraph> step_graphs;
+  uint64_t graph_clock = 0;
 
   // timing
   float last_solve_ms = 0.f, last_device_ms = 0.f, last_steps_ms = 0.f;
@@ -643,20 +658,14 @@ __global__ void k_eval_exp(const double* __restrict__ x, double* __restrict__ y,
 struct StepParams {
   int64_t n;
   int ld;            // leading dimension of the (n x ld) state buffers
-  int ncols;         // active columns this step
-  int64_t step;
-  int step_w;        // rate window of this step (k_slab's entry values), set with step
+  int hcols;         // host side: columns the launch grids cover (at least sc->ncols)
+  const StepScal* sc;  // the step's scalars
   const CUtensorMap* tmap_src;  // k_slab: tensor map of src for the TMA staging, or null (cp.async staging)
   const CUtensorMap* tmap_band;  // k_band_tma: tensor map of src as (64 columns x d bins) boxes, or null
   long long wait_tries;         // k_slab: polls of the staging wait before it gives up (the drain keeps kWaitTries)
   int* err;          // set to a nonzero code when a bounded wait gives up
   int64_t n_steps;
   uint32_t flags;
-  const double* h;
-  const double* dldz;
-  const double* hc;
-  const double* finj;
-  const int* win;
   // operator
   const int64_t* m_indptr;
   const int* m_indices;
@@ -752,17 +761,20 @@ struct StepParams {
 
 struct StepScalars {
   double h, dl, hc, finj;
-  int w;
+  int64_t step;
+  int w, ncols;
   bool kap, adia, pair, photohad, inj, decay;
 };
 
-__device__ __forceinline__ StepScalars load_scalars(const StepParams& p, int64_t step) {
+__device__ __forceinline__ StepScalars load_scalars(const StepParams& p, const StepScal* sc) {
   StepScalars s;
-  s.h = p.h[step];
-  s.dl = p.dldz[step];
-  s.hc = p.hc[step];
-  s.finj = p.finj[step];
-  s.w = p.win[step];
+  s.h = sc->h;
+  s.dl = sc->dl;
+  s.hc = sc->hc;
+  s.finj = sc->finj;
+  s.step = sc->step;
+  s.w = sc->w;
+  s.ncols = sc->ncols;
   s.kap = (p.flags & PB_PARTIAL_DIFF) != 0;
   s.adia = (p.flags & PB_ADIABATIC) != 0;
   s.pair = (p.flags & PB_PAIRPROD) != 0 && p.kp != nullptr;
@@ -814,7 +826,7 @@ __device__ __forceinline__ void dphi_of(double w, double e, double f1, double f2
 // kappa (propagation.py:1393-1401) and d = dldz (M_diag + kappa D_diag [+ Lambda_diag])
 // (propagation.py:1408-1422) of row r at `step`, then its phi factors.
 __device__ __forceinline__ void row_prep(const StepParams& p, int64_t step, int64_t r) {
-  const StepScalars s = load_scalars(p, step);
+  const StepScalars s = load_scalars(p, p.sc + (step - p.prep_k0));
   double k = 0.0;
   if (s.adia) k = __dmul_rn(s.hc, p.E[r]);
   if (s.pair) k = __dadd_rn(k, p.kp[(size_t)s.w * p.n + r]);
@@ -851,7 +863,7 @@ __device__ __forceinline__ void row_prep(const StepParams& p, int64_t step, int6
   }
 }
 
-// The row factors of the steps prep_k0 .. prep_k0 + gridDim.y - 1.
+// The row factors of the steps prep_k0 .. prep_k0 + gridDim.y - 1 (p.sc: the first one's scalars).
 __global__ void __launch_bounds__(128) k_prep(StepParams p) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < p.n) row_prep(p, p.prep_k0 + blockIdx.y, r);
@@ -859,14 +871,16 @@ __global__ void __launch_bounds__(128) k_prep(StepParams p) {
 
 constexpr int64_t kPrepRows = 1 << 19;  // rows x steps of one k_prep launch (about 30 MB of factors)
 // Steps whose factors one launch prepares.
+constexpr int64_t kGraphSteps = 16;     // steps of a captured run
 constexpr int64_t kPrepMaxSteps = 1024;
 inline int64_t prep_steps(int64_t n) {
   return std::max<int64_t>(4, std::min<int64_t>(kPrepMaxSteps, kPrepRows / std::max<int64_t>(n, 1)));
 }
 
 // Prepares the steps [k0, k0 + count) (the factors land at steps k0 - rf_k0 .. of p.rf).
-void launch_prep(StepParams& p, int64_t k0, int64_t count, cudaStream_t st) {
+void launch_prep(StepParams& p, const StepScal* scal, int64_t k0, int64_t count, cudaStream_t st) {
   p.prep_k0 = k0;
+  p.sc = scal + k0;
   k_prep<<<dim3(blocks_for(p.n, 128), (unsigned)count), 128, 0, st>>>(p);
 }
 
@@ -887,16 +901,15 @@ void set_step_factors(StepParams& p, int64_t k) {
 // ---------------------------------------------------------------------------
 // Scratch of pb_integrate_const_noalloc: one file-scope device array (every
 // GPU that loads the library holds it until exit).  Layout, in bytes from the
-// start: a and F(x) (n doubles each), the row factors of two steps (8 n doubles), the
-// per-step h and dl/dz (s doubles each), the window index (s ints), the row
-// list (n ints), an all-zero row pointer (n + 1 int64) and a 256-byte status
+// start: a and F(x) (n doubles each), the row factors of two steps
+// (8 n doubles), the step scalars (s of them), the row list (n ints), an all-zero row pointer (n + 1 int64) and a 256-byte status
 // block (the CSR check's flag), for n = the state limit and s = the step limit.
 // ---------------------------------------------------------------------------
 constexpr int64_t kNaMaxStates = PB_NOALLOC_MAX_STATES;
 constexpr int64_t kNaMaxSteps = PB_NOALLOC_MAX_STEPS;
 constexpr int kNaPrepSteps = 2;  // steps whose row factors fit the scratch
-constexpr size_t kNaBytes = (size_t)kNaMaxStates * 10 * sizeof(double) + (size_t)kNaMaxSteps * 2 * sizeof(double) +
-                            (size_t)kNaMaxSteps * sizeof(int) + (size_t)kNaMaxStates * sizeof(int) +
+constexpr size_t kNaBytes = (size_t)kNaMaxStates * 10 * sizeof(double) + (size_t)kNaMaxSteps * sizeof(StepScal) +
+                            (size_t)kNaMaxStates * sizeof(int) +
                             (size_t)(kNaMaxStates + 1) * sizeof(int64_t) + 256;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
@@ -917,14 +930,11 @@ __global__ void k_noalloc_check_csr(int64_t n, int64_t nnz, const int64_t* __res
   }
 }
 
-__global__ void k_noalloc_fill(int64_t n, int64_t n_steps, const double* __restrict__ z, double* __restrict__ h,
-                               double* __restrict__ ones, int* __restrict__ win, int* __restrict__ rows,
-                               int64_t* __restrict__ zero_indptr) {
+__global__ void k_noalloc_fill(int64_t n, int64_t n_steps, const double* __restrict__ z, StepScal* __restrict__ sc,
+                               int* __restrict__ rows, int64_t* __restrict__ zero_indptr) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_steps) {
-    h[i] = __dadd_rn(z[i + 1], -z[i]);
-    ones[i] = 1.0;
-    win[i] = 0;
+    sc[i] = StepScal{__dadd_rn(z[i + 1], -z[i]), 1.0, 1.0, 1.0, i, 0, 1};
   }
   if (i < n) rows[i] = (int)i;
   if (i <= n) zero_indptr[i] = 0;
@@ -936,7 +946,7 @@ __device__ __forceinline__ double inj_at(const StepParams& p, const StepScalars&
   if (slot < 0) return 0.0;
   const int s0 = p.src_ptr[k], s1 = p.src_ptr[k + 1];
   if (s0 == s1) return 0.0;
-  const double* c = p.coeff + (size_t)p.step * p.n_src;
+  const double* c = p.coeff + (size_t)s.step * p.n_src;
   const double* g = p.G + (size_t)slot * p.n_src;
   double acc = __dmul_rn(c[s0], g[s0]);
   for (int q = s0 + 1; q < s1; ++q) acc = __dadd_rn(acc, __dmul_rn(c[q], g[q]));
@@ -991,7 +1001,7 @@ __device__ __forceinline__ void record(const StepParams& p, const StepScalars& s
                                        double F) {
   const int64_t o = r;
   const size_t idx = (size_t)r * p.ld + k;
-  const int64_t j = p.step - p.rec_k0;
+  const int64_t j = s.step - p.rec_k0;
   if (j < 0 || j >= p.rec_len) return;
   const size_t ro = (size_t)j * p.n * p.ld + idx;
   const double h = s.h, ds = p.dsig[o];
@@ -1048,7 +1058,7 @@ __device__ __forceinline__ bool last_of_row(const StepParams& p, int lr, int til
 // [nsb, ...): a warp per long-row segment.
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_step_plain(StepParams p) {
-  const StepScalars s = load_scalars(p, p.step);
+  const StepScalars s = load_scalars(p, p.sc);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double* __restrict__ v = p.src;
   const double* __restrict__ mv = p.m_vals + (size_t)s.w * p.m_wstride;
@@ -1110,10 +1120,11 @@ __device__ __forceinline__ double gather_sum(const double* __restrict__ mv, cons
 // [0, nsb): a warp per short row; blocks [nsb, ...): a warp per long-row segment.
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_step_multi(StepParams p) {
-  const StepScalars s = load_scalars(p, p.step);
+  const StepScalars s = load_scalars(p, p.sc);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if ((int)blockIdx.y * kColTile >= s.ncols) return;
   const int k = blockIdx.y * kColTile + lane;
-  const bool active = k < p.ncols;
+  const bool active = k < s.ncols;
   const int kk = active ? k : 0;
   const double* __restrict__ v = p.src;
   const double* __restrict__ mv = p.m_vals + (size_t)s.w * p.m_wstride;
@@ -1221,6 +1232,7 @@ constexpr int kErrStagingWait = 1;           // err code: a k_slab CTA's staging
 // with zero weights on the row itself).
 __global__ void __launch_bounds__(256) k_fd(StepParams p) {
   extern __shared__ double fsm[];
+  if ((int)blockIdx.y * kColTile >= p.sc->ncols) return;
   const int sp = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int d = p.d, ld = p.ld;
   const int col = blockIdx.y * kColTile + lane;  // < ld
@@ -1234,7 +1246,7 @@ __global__ void __launch_bounds__(256) k_fd(StepParams p) {
   }
   cp_async_commit();
   for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[(size_t)sp * d + e];
-  const double* kpw = p.fdkp ? p.kp + (size_t)p.win[p.step] * p.n + (size_t)sp * d : nullptr;
+  const double* kpw = p.fdkp ? p.kp + (size_t)p.sc->w * p.n + (size_t)sp * d : nullptr;
   if (kpw)
     for (int e = threadIdx.x; e < d; e += blockDim.x) kpb[e] = kpw[e];
   cp_async_wait<0>();
@@ -1267,6 +1279,7 @@ __global__ void __launch_bounds__(256) k_fd(StepParams p) {
 template <bool KP>
 __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
   extern __shared__ double fsm[];
+  if ((int)blockIdx.y * kColTile >= p.sc->ncols) return;
   const int sp = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int d = p.d, ld = p.ld;
   const int col = blockIdx.y * kColTile + lane;  // < ld
@@ -1283,7 +1296,7 @@ __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
   cp_async_commit();
   for (int e = threadIdx.x; e < d; e += blockDim.x) kb[e] = p.kap[(size_t)sp * d + e];
   if (KP)
-    for (int e = threadIdx.x; e < d; e += blockDim.x) kpb[e] = p.kp[(size_t)p.step_w * p.n + (size_t)sp * d + e];
+    for (int e = threadIdx.x; e < d; e += blockDim.x) kpb[e] = p.kp[(size_t)p.sc->w * p.n + (size_t)sp * d + e];
   cp_async_wait<0>();
   __syncthreads();
   constexpr int U = kFdChunk + 2 * kFdHalo;
@@ -1324,7 +1337,7 @@ __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
 template <int STAGE>
 __device__ __forceinline__ void record_blocked(const StepParams& p, const StepScalars& s, int64_t r, int k,
                                                double sM, double F, double own, double fprev) {
-  const int64_t j = p.step - p.rec_k0;
+  const int64_t j = s.step - p.rec_k0;
   if (j < 0 || j >= p.rec_len) return;
   const int64_t o = r;
   const size_t idx = (size_t)r * p.ld + k;
@@ -1354,7 +1367,7 @@ __device__ __forceinline__ void record_pre(const StepParams& p, const StepScalar
                                            double F, double own, double fprev, const RecIn& in) {
   if (!in.on) return;
   const size_t idx = (size_t)r * p.ld + k;
-  const size_t ro = (size_t)(p.step - p.rec_k0) * p.n * p.ld + idx;
+  const size_t ro = (size_t)(s.step - p.rec_k0) * p.n * p.ld + idx;
   const double h = s.h, ds = in.ds;
   double S = s.photohad ? sM : 0.0;
   if (s.kap && s.pair) S += in.kp;
@@ -1409,8 +1422,8 @@ __device__ __forceinline__ double2 dadd2(double2 a, double2 b) {
   return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
 }
 // The injection of one column (rows of injected species only).
-__device__ __forceinline__ double slab_inj(const StepParams& p, int slot, int src0, int src1) {
-  const double* cf = p.coeff + (size_t)p.step * p.n_src;
+__device__ __forceinline__ double slab_inj(const StepParams& p, int64_t step, int slot, int src0, int src1) {
+  const double* cf = p.coeff + (size_t)step * p.n_src;
   const double* g = p.G + (size_t)slot * p.n_src;
   double a = __dmul_rn(cf[src0], g[src0]);
   for (int q = src0 + 1; q < src1; ++q) a = __dadd_rn(a, __dmul_rn(cf[q], g[q]));
@@ -1441,15 +1454,16 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   const int g = lane >> 3, j = lane & 7;
   const int col0 = blockIdx.y * kSlabCols;
   const int colA = col0 + 2 * j;  // this lane's columns colA, colA + 1 (< ld)
-  const bool actA = colA < p.ncols, actB = colA + 1 < p.ncols;
-  const StepScalars s = load_scalars(p, p.step);
+  const StepScalars s = load_scalars(p, p.sc);
+  if (col0 >= s.ncols) return;
+  const bool actA = colA < s.ncols, actB = colA + 1 < s.ncols;
   const int ld = p.ld, d = p.d;
   SlabSmem L(sm, p.nsp, p.slab_maxq, p.slab_maxp);
   const int qb = p.slab_qbase[e], nqb = p.slab_qbase[e + 1] - qb;
   const int gb0 = p.slab_wrp[e * (kSlabWarps + 1)], ngb = p.slab_wrp[e * (kSlabWarps + 1) + kSlabWarps] - gb0;
   const int fs = kSlabRows * p.slab_maxp;  // stride of the three row-factor arrays
   unsigned long long* stage_bar = L.bar;
-  const double* mv = p.slab_vals + (size_t)p.step_w * p.slab_stride + (size_t)qb * 4;
+  const double* mv = p.slab_vals + (size_t)s.w * p.slab_stride + (size_t)qb * 4;
   const double* fc = p.slab_fac + (size_t)kSlabRows * gb0;
   if (p.tmap_src) {  // TMA: the slab as tensor boxes, the rest as bulk copies, one barrier
     if (threadIdx.x == 0) mbar_init(stage_bar, 1);
@@ -1496,7 +1510,7 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   double2 fdr[PRE], fxr[PRE];
   int slr[PRE];
   // record pass: dsigma and phi1' / phi2' of the row, D_off (kappa_pair v) and S x of (row, column)
-  const int64_t rj = p.step - p.rec_k0;
+  const int64_t rj = s.step - p.rec_k0;
   const bool rec_on = REC && rj >= 0 && rj < p.rec_len;
   double rds[PRE], rd12[PRE];
   double2 rkp[PRE], rsx[PRE];
@@ -1596,8 +1610,8 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
         out.x = __dmul_rn(out.x, s.dl);
         out.y = __dmul_rn(out.y, s.dl);
         if (slr[u] >= 0) {  // injection (rows of injected species only)
-          if (srcA1 > srcA0) out.x = __dadd_rn(out.x, __dmul_rn(s.finj, slab_inj(p, slr[u], srcA0, srcA1)));
-          if (actB && srcB1 > srcA1) out.y = __dadd_rn(out.y, __dmul_rn(s.finj, slab_inj(p, slr[u], srcA1, srcB1)));
+          if (srcA1 > srcA0) out.x = __dadd_rn(out.x, __dmul_rn(s.finj, slab_inj(p, s.step, slr[u], srcA0, srcA1)));
+          if (actB && srcB1 > srcA1) out.y = __dadd_rn(out.y, __dmul_rn(s.finj, slab_inj(p, s.step, slr[u], srcA1, srcB1)));
         }
         const double2 own = *reinterpret_cast<const double2*>(L.slab + sp * kSlabCols + 2 * j);
         const int slot = kSlabRows * (pi - gb0) + g;
@@ -1668,11 +1682,13 @@ __global__ void __launch_bounds__(NW * 32, 1) k_band(StepParams p) {
   constexpr int AH = RT * J * 32;        // one band species of it
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c0 = blockIdx.x * (NW * 8) + wid * 8;
-  const bool wact = c0 < p.ncols;  // c0 + 7 < ld: ld is a multiple of 32
+  const int ncols = p.sc->ncols;
+  if ((int)blockIdx.x * (NW * 8) >= ncols) return;
+  const bool wact = c0 < ncols;  // c0 + 7 < ld: ld is a multiple of 32
   const int pair = blockIdx.z, g = blockIdx.y;
   const int s0 = g * p.spg, s1 = min(p.nsp, s0 + p.spg);
   const int d = p.d, ld = p.ld;
-  const int w = p.win[p.step];
+  const int w = p.sc->w;
   const double* __restrict__ A = p.band_vals + (size_t)w * p.band_stride;
   const int npairs = gridDim.z;
   double* As = sm;  // [2][ABLK]
@@ -1797,14 +1813,14 @@ size_t band_smem_bytes() {
 // with the FD term from fdbuf.
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_band_finish(StepParams p) {
-  const StepScalars s = load_scalars(p, p.step);
+  const StepScalars s = load_scalars(p, p.sc);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int rb = blockIdx.x * (blockDim.x >> 5) + wid;
   if (rb >= p.nb * p.d) return;
   const int b = rb / p.d, e = rb - b * p.d;
   const int64_t r = (int64_t)p.band_spec[b] * p.d + e;
   const int col = blockIdx.y * kColTile + lane;
-  if (col < p.ncols) {
+  if (col < s.ncols) {
     double t = 0.0;
     for (int g = 0; g < p.ngroups; ++g)
       t = __dadd_rn(t, p.band_part[((size_t)(g * p.nb + b) * p.d + e) * p.ld + col]);
@@ -1847,11 +1863,13 @@ __global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
   constexpr int XS = 8 * RT * 64;        // X of one species: bins x 64 columns
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int cb = blockIdx.x * 64, c0 = cb + wid * 8;
-  const bool wact = c0 < p.ncols;  // c0 + 7 < ld: ld is a multiple of 32
+  const int ncols = p.sc->ncols;
+  if ((int)blockIdx.x * 64 >= ncols) return;
+  const bool wact = c0 < ncols;  // c0 + 7 < ld: ld is a multiple of 32
   const int pair = blockIdx.z, g = blockIdx.y;
   const int s0 = g * p.spg, s1 = min(p.nsp, s0 + p.spg);
   const int d = p.d, ld = p.ld;
-  const int w = p.win[p.step];
+  const int w = p.sc->w;
   const double* __restrict__ A = p.band_vals + (size_t)w * p.band_stride;
   const int npairs = gridDim.z;
   double* As = sm;             // [2][ABLK]
@@ -2018,16 +2036,17 @@ namespace {
 struct EmParams {
   int64_t n;
   int ld;
-  int ncols;
+  int hcols;                      // host side: columns the launch grids cover
+  const StepScal* sc;             // the step's window and active columns
   int n_em, n_cr, n_bh;
   int64_t g_off, em_off, ep_off;  // block offsets of gamma, e-, e+ (e+- may be -1)
   const int64_t* bh_off;          // block offset of each charged nucleus
   const double* bh_A;
   const double* invE;             // 1 / E on the nucleon grid
   const double* dE;               // gradient of E
-  const double* kp;               // kappa_pair of the window (n)
-  double dl_step;
-  const double* Tg;               // n_em x n_em
+  const double* kp;               // kappa_pair, W x n
+  const double* dl;               // dl_step of every window
+  const double* Tg;               // per window: n_em x n_em
   const double* Te;               // n_em x n_em
   const double* R;                // n_em x n_cr
   double* X;
@@ -2035,7 +2054,7 @@ struct EmParams {
   double* es;                     // n_em x ld: R w (forward) or Te^T lam_gamma (adjoint)
   double* lep;                    // n_em x ld: e- + e+ with the pairs (forward)
   double* y;                      // n_em x ld: the new gamma rows (forward) or Tg^T lam_gamma (adjoint)
-  const double* TgT;              // transposes of the window's matrices (adjoint)
+  const double* TgT;              // transposes of the windows' matrices (adjoint)
   const double* TeT;
   const double* RT;               // n_cr x n_em
 };
@@ -2043,8 +2062,9 @@ struct EmParams {
 // l = (e- + es) + (e+ + es) with es = R w, then e+- <- 0 (the lepton half of the hook).
 __global__ void k_em_lep(EmParams e) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)e.n_em * e.ncols) return;
-  const int j = (int)(t / e.ncols), k = (int)(t % e.ncols);
+  if (t >= (int64_t)e.n_em * e.hcols) return;
+  const int j = (int)(t / e.hcols), k = (int)(t % e.hcols);
+  if (k >= e.sc->ncols) return;
   const double es = e.es[(size_t)j * e.ld + k];
   double l = 0.0;
   if (e.em_off >= 0) {
@@ -2063,8 +2083,9 @@ __global__ void k_em_lep(EmParams e) {
 // Adjoint lepton rows: lam_e+- <- Te^T lam_gamma (e.es), and lw = n_lep R^T (that) is a GEMM after.
 __global__ void k_em_lepT(EmParams e) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)e.n_em * e.ncols) return;
-  const int j = (int)(t / e.ncols), k = (int)(t % e.ncols);
+  if (t >= (int64_t)e.n_em * e.hcols) return;
+  const int j = (int)(t / e.hcols), k = (int)(t % e.hcols);
+  if (k >= e.sc->ncols) return;
   const double m = e.es[(size_t)j * e.ld + k];
   if (e.em_off >= 0) e.X[(size_t)(e.em_off + j) * e.ld + k] = m;
   if (e.ep_off >= 0) e.X[(size_t)(e.ep_off + j) * e.ld + k] = m;
@@ -2073,8 +2094,9 @@ __global__ void k_em_lepT(EmParams e) {
 // Scales the first n_cr x ncols block of e.w by s (the lepton count of the adjoint pair weights).
 __global__ void k_em_scale_w(EmParams e, double s) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)e.n_cr * e.ncols) return;
-  const int i = (int)(t / e.ncols), k = (int)(t % e.ncols);
+  if (t >= (int64_t)e.n_cr * e.hcols) return;
+  const int i = (int)(t / e.hcols), k = (int)(t % e.hcols);
+  if (k >= e.sc->ncols) return;
   e.w[(size_t)i * e.ld + k] *= s;
 }
 
@@ -2092,6 +2114,10 @@ constexpr int kEmWBatch = 8;
 template <int V>
 __global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
   extern __shared__ unsigned char em_w_smem[];
+  const int ncols = e.sc->ncols, w = e.sc->w;
+  if ((int)blockIdx.y * (32 * V) >= ncols) return;
+  const double* __restrict__ kp = e.kp + (size_t)w * e.n;
+  const double dl_step = e.dl[w];
   int64_t* soff = reinterpret_cast<int64_t*>(em_w_smem);
   double* sA = reinterpret_cast<double*>(soff + e.n_bh);
   for (int t = threadIdx.x; t < e.n_bh; t += blockDim.x) {
@@ -2103,7 +2129,7 @@ __global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
   const int i = blockIdx.x * 8 + wid;
   if (i >= e.n_cr) return;
   const int k = blockIdx.y * (32 * V) + V * lane;  // columns k .. k + V - 1
-  const bool active = k < e.ncols;
+  const bool active = k < ncols;
   const int kk = active ? k : 0;
   const double ie = e.invE[i], de = e.dE[i];
   double acc[V];
@@ -2127,14 +2153,14 @@ __global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
         } else {
           xv[u][0] = __ldg(src);
         }
-        kv[u] = __ldg(e.kp + row);
+        kv[u] = __ldg(kp + row);
       }
     }
 #pragma unroll
     for (int u = 0; u < kEmWBatch; ++u) {
       const int s = s0 + u;
       if (s < e.n_bh) {
-        const double cw = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(sA[s], kv[u]), e.dl_step), ie), de);
+        const double cw = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(sA[s], kv[u]), dl_step), ie), de);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const double t = __dmul_rn(cw, xv[u][v]);
@@ -2145,12 +2171,14 @@ __global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
   }
 #pragma unroll
   for (int v = 0; v < V; ++v)
-    if (k + v < e.ncols) e.w[(size_t)i * e.ld + k + v] = acc[v];
+    if (k + v < ncols) e.w[(size_t)i * e.ld + k + v] = acc[v];
 }
 
 // Adjoint of the pair weights: X[s, i][k] += cw_si lw[i][k] (e.X = lam, e.w = lw).
 __global__ void __launch_bounds__(256) k_em_wT(EmParams e) {
   extern __shared__ unsigned char em_w_smem[];
+  const int w = e.sc->w;
+  const double* __restrict__ kp = e.kp + (size_t)w * e.n;
   int64_t* soff = reinterpret_cast<int64_t*>(em_w_smem);
   double* sA = reinterpret_cast<double*>(soff + e.n_bh);
   for (int t = threadIdx.x; t < e.n_bh; t += blockDim.x) {
@@ -2162,8 +2190,8 @@ __global__ void __launch_bounds__(256) k_em_wT(EmParams e) {
   const int i = blockIdx.x * 8 + wid;
   if (i >= e.n_cr) return;
   const int k = blockIdx.y * 32 + lane;
-  if (k >= e.ncols) return;
-  const double l = e.w[(size_t)i * e.ld + k] * e.dl_step * e.invE[i] * e.dE[i];
+  if (k >= e.sc->ncols) return;
+  const double l = e.w[(size_t)i * e.ld + k] * e.dl[w] * e.invE[i] * e.dE[i];
   for (int s0 = 0; s0 < e.n_bh; s0 += kEmWBatch) {
     double xv[kEmWBatch], kv[kEmWBatch];
 #pragma unroll
@@ -2171,7 +2199,7 @@ __global__ void __launch_bounds__(256) k_em_wT(EmParams e) {
       if (s0 + u < e.n_bh) {
         const int64_t row = soff[s0 + u] + i;
         xv[u] = e.X[(size_t)row * e.ld + k];
-        kv[u] = __ldg(e.kp + row);
+        kv[u] = __ldg(kp + row);
       }
 #pragma unroll
     for (int u = 0; u < kEmWBatch; ++u)
@@ -2187,34 +2215,34 @@ __global__ void __launch_bounds__(256) k_em_wT(EmParams e) {
 //   y = Tg gamma + Te l, gamma <- y.
 void em_hook_forward(const EmParams& e, cudaStream_t st) {
   const size_t wsm = (size_t)e.n_bh * (sizeof(int64_t) + sizeof(double));
+  const long long nn = (long long)e.n_em * e.n_em, nr = (long long)e.n_em * e.n_cr;
   if (e.ld % 2 == 0)
-    k_em_w<2><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.ncols, 64)), 256, wsm, st>>>(e);
+    k_em_w<2><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.hcols, 64)), 256, wsm, st>>>(e);
   else
-    k_em_w<1><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.ncols, 32)), 256, wsm, st>>>(e);
-  bgemm(st, e.R, e.w, e.es, e.n_em, e.ncols, e.n_cr, e.n_cr, e.ld, e.ld, 0, 0, 0, 1, false);
-  k_em_lep<<<(unsigned)blocks_for((int64_t)e.n_em * e.ncols, 256), 256, 0, st>>>(e);
+    k_em_w<1><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.hcols, 32)), 256, wsm, st>>>(e);
+  bgemm_step(st, e.sc, e.R, nr, e.w, nullptr, e.es, e.n_em, e.hcols, e.n_cr, e.ld);
+  k_em_lep<<<(unsigned)blocks_for((int64_t)e.n_em * e.hcols, 256), 256, 0, st>>>(e);
   double* gam = e.X + (size_t)e.g_off * e.ld;
-  bgemm(st, e.Tg, gam, e.y, e.n_em, e.ncols, e.n_em, e.n_em, e.ld, e.ld, 0, 0, 0, 1, false);
-  bgemm(st, e.Te, e.lep, e.y, e.n_em, e.ncols, e.n_em, e.n_em, e.ld, e.ld, 0, 0, 0, 1, true);
-  cudaMemcpy2DAsync(gam, (size_t)e.ld * sizeof(double), e.y, (size_t)e.ld * sizeof(double),
-                    (size_t)e.ncols * sizeof(double), (size_t)e.n_em, cudaMemcpyDeviceToDevice, st);
+  bgemm_step(st, e.sc, e.Tg, nn, gam, nullptr, e.y, e.n_em, e.hcols, e.n_em, e.ld);
+  bgemm_step(st, e.sc, e.Te, nn, e.lep, e.y, gam, e.n_em, e.hcols, e.n_em, e.ld);
 }
 
 // Its transpose on lam (e.X): mu = Te^T lam_gamma, lam_gamma <- Tg^T lam_gamma,
 // lam_e+- <- mu, lam_nuclei += cw (n_lep R^T mu) (k_em_wT).
 void em_hook_adjoint(const EmParams& e, cudaStream_t st) {
   double* gam = e.X + (size_t)e.g_off * e.ld;
-  bgemm(st, e.TeT, gam, e.es, e.n_em, e.ncols, e.n_em, e.n_em, e.ld, e.ld, 0, 0, 0, 1, false);
-  bgemm(st, e.TgT, gam, e.y, e.n_em, e.ncols, e.n_em, e.n_em, e.ld, e.ld, 0, 0, 0, 1, false);
+  const long long nn = (long long)e.n_em * e.n_em, nr = (long long)e.n_em * e.n_cr;
+  bgemm_step(st, e.sc, e.TeT, nn, gam, nullptr, e.es, e.n_em, e.hcols, e.n_em, e.ld);
+  bgemm_step(st, e.sc, e.TgT, nn, gam, nullptr, e.y, e.n_em, e.hcols, e.n_em, e.ld);
   cudaMemcpy2DAsync(gam, (size_t)e.ld * sizeof(double), e.y, (size_t)e.ld * sizeof(double),
-                    (size_t)e.ncols * sizeof(double), (size_t)e.n_em, cudaMemcpyDeviceToDevice, st);
-  k_em_lepT<<<(unsigned)blocks_for((int64_t)e.n_em * e.ncols, 256), 256, 0, st>>>(e);
-  bgemm(st, e.RT, e.es, e.w, e.n_cr, e.ncols, e.n_em, e.n_em, e.ld, e.ld, 0, 0, 0, 1, false);
+                    (size_t)e.hcols * sizeof(double), (size_t)e.n_em, cudaMemcpyDeviceToDevice, st);
+  k_em_lepT<<<(unsigned)blocks_for((int64_t)e.n_em * e.hcols, 256), 256, 0, st>>>(e);
+  bgemm_step(st, e.sc, e.RT, nr, e.es, nullptr, e.w, e.n_cr, e.hcols, e.n_em, e.ld);
   const double nl = (double)((e.em_off >= 0) + (e.ep_off >= 0));
   if (nl != 1.0)
-    k_em_scale_w<<<(unsigned)blocks_for((int64_t)e.n_cr * e.ncols, 256), 256, 0, st>>>(e, nl);
+    k_em_scale_w<<<(unsigned)blocks_for((int64_t)e.n_cr * e.hcols, 256), 256, 0, st>>>(e, nl);
   const size_t wsm = (size_t)e.n_bh * (sizeof(int64_t) + sizeof(double));
-  k_em_wT<<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.ncols, 32)), 256, wsm, st>>>(e);
+  k_em_wT<<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.hcols, 32)), 256, wsm, st>>>(e);
 }
 
 
@@ -2884,7 +2912,7 @@ int set_device(pb_context* c) {
 
 FieldDesc field_desc(const pb_context* c, double scale) {
   FieldDesc f;
-  memset(&f, 0, sizeof(f));  // padding bytes take part in the graph key
+  memset(&f, 0, sizeof(f));
   f.n = c->n_comp;
   for (int i = 0; i < 8; ++i) {
     f.kind[i] = i < c->n_comp ? c->comp_kind[i] : 0;
@@ -2901,18 +2929,18 @@ FieldDesc field_desc(const pb_context* c, double scale) {
   return f;
 }
 
-// Buffers the forward solve reads or writes (the two captured graphs point into these).
+// Buffers the forward solve reads or writes.
 std::vector<DBuf*> solve_buffers(pb_context* c) {
   return {&c->cpl_indptr, &c->cpl_indices, &c->cpl_row, &c->cpl_is_diag, &c->short_rows, &c->long_rows, &c->kernel,
           &c->eph, &c->d_indptr, &c->d_indices, &c->d_vals, &c->d_diag, &c->adia_E, &c->pair_scale, &c->pair_bin,
           &c->xi, &c->phi_xi2, &c->pair_pg, &c->l_diag, &c->l_indptr, &c->l_indices, &c->l_vals, &c->inj_slot,
           &c->inj_G, &c->src_ptr, &c->PT, &c->zwin, &c->rs, &c->kp, &c->keep, &c->pos, &c->dest, &c->m_indptr,
-          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_h, &c->s_dldz, &c->s_hc, &c->s_finj, &c->s_win, &c->s_coeff,
+          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_scal, &c->s_finj, &c->s_coeff, &c->s_run,
           &c->X, &c->A, &c->F, &c->rowf, &c->scan_tmp, &c->seg_cb, &c->seg_ce, &c->seg_lr, &c->lr_seg0, &c->lr_nseg,
           &c->seg_mb, &c->seg_me, &c->partial, &c->counter, &c->dt_indptr, &c->dt_indices, &c->dt_vals,
           &c->lt_indptr, &c->lt_indices, &c->lt_vals, &c->inj_rows, &c->src_col_d, &c->ckpt,
           &c->em_bh_off, &c->em_bh_A, &c->em_invE, &c->em_dE, &c->em_Tg, &c->em_Te, &c->em_R, &c->em_wbuf,
-          &c->em_es, &c->em_lep, &c->em_y, &c->em_TgT, &c->em_TeT, &c->em_RT,
+          &c->em_es, &c->em_lep, &c->em_y, &c->em_TgT, &c->em_TeT, &c->em_RT, &c->em_dlw,
           &c->band_slot, &c->band_spec, &c->slab_spec, &c->band_vals, &c->band_part, &c->slab_rp,
           &c->slab_sidx, &c->slab_slot, &c->slab_vals, &c->slab_quart, &c->slab_wrp, &c->slab_rowslot, &c->slab_fac, &c->fd_cnt, &c->fd_off, &c->fd_val, &c->fd_dense, &c->fdT_dense, &c->fdbuf,
           &c->bandT_slot, &c->slabT_rp, &c->slabT_offs, &c->slabT_slot, &c->fdT_cnt, &c->fdT_off, &c->fdT_val,
@@ -2965,11 +2993,6 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.wait_tries = c->staging_wait_tries;
   if (!pair) p.flags &= ~PB_PAIRPROD;
   if (!inj) p.flags &= ~PB_INJECTION;
-  p.h = c->s_h.as<double>();
-  p.dldz = c->s_dldz.as<double>();
-  p.hc = c->s_hc.as<double>();
-  p.finj = c->s_finj.as<double>();
-  p.win = c->s_win.as<int>();
   p.m_indptr = c->m_indptr.as<int64_t>();
   p.m_indices = c->m_indices.as<int>();
   p.m_vals = c->m_vals.as<double>();
@@ -3157,7 +3180,7 @@ const CUtensorMap* stage_tmap_band(const pb_context* c, int stage) {
 // at least one wave of the SMs (a CTA per SM); with nw = 4 they stay within one
 // wave, so that each SM holds at most one k_band CTA beside its k_slab CTA.
 int band_grid(const pb_context* c, StepParams& p, int nw) {
-  const int cblocks = (int)blocks_for(p.ncols, 8 * nw);
+  const int cblocks = (int)blocks_for(p.hcols, 8 * nw);
   const int per = cblocks * std::max(c->band_npairs, 1);
   int G;
   if (nw == 4) {
@@ -3206,7 +3229,7 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
     cudaEventRecord(c->ev_join, c->stream2);
     ++launches;
   }
-  const unsigned tiles = (unsigned)blocks_for(p.ncols, kColTile);
+  const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
   if (kap) {
     const size_t fsmem = (size_t)p.d * (kColTile + kFdDenseW + 2) * sizeof(double);
     if (c->fd_dense_ok && p.fdkp) k_fd_dense<true><<<dim3(p.nsp, tiles), 256, fsmem, st>>>(p);
@@ -3214,7 +3237,7 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
     else k_fd<<<dim3(p.nsp, tiles), 256, (size_t)p.d * (kColTile + 2) * sizeof(double), st>>>(p);
     ++launches;
   }
-  const dim3 sg(p.d, (unsigned)blocks_for(p.ncols, kSlabCols));
+  const dim3 sg(p.d, (unsigned)blocks_for(p.hcols, kSlabCols));
   slab_kernel(STAGE, p.rec_P != nullptr, c->slab_pre)<<<sg, kSlabWarps * 32, c->slab_smem, st>>>(p);
   ++launches;
   if (c->n_tail > 0) {  // tail rows (another grid): the general row kernel, a warp per row
@@ -3265,12 +3288,14 @@ void launch_adj_blocked(pb_context* c, AdjBlk& q, cudaStream_t st) {
   k_slabT<STAGE><<<dim3(q.d, (unsigned)blocks_for(q.ncols, kSlabCols)), kSlabTWarps * 32, c->slabT_smem, st>>>(q);
 }
 
-// The EM hook's operands for window w on the n x ld buffer X (a state, or the adjoint's lam).
-EmParams em_params(const pb_context* c, int w, int ld, int ncols, double* X) {
+// The EM hook's operands for the step sc on the n x ld buffer X (a state, or the adjoint's lam).
+EmParams em_params(const pb_context* c, const StepScal* sc, int ld, int hcols, double* X) {
   EmParams e;
+  memset(&e, 0, sizeof(e));
   e.n = c->n;
   e.ld = ld;
-  e.ncols = ncols;
+  e.hcols = hcols;
+  e.sc = sc;
   e.n_em = c->em_n;
   e.n_cr = c->em_ncr;
   e.n_bh = c->em_nbh;
@@ -3281,118 +3306,226 @@ EmParams em_params(const pb_context* c, int w, int ld, int ncols, double* X) {
   e.bh_A = c->em_bh_A.as<double>();
   e.invE = c->em_invE.as<double>();
   e.dE = c->em_dE.as<double>();
-  e.kp = c->kp.as<double>() + (size_t)w * c->n;
-  e.dl_step = c->em_dl[w];
-  e.Tg = c->em_Tg.as<double>() + (size_t)w * c->em_n * c->em_n;
-  e.Te = c->em_Te.as<double>() + (size_t)w * c->em_n * c->em_n;
-  e.R = c->em_R.as<double>() + (size_t)w * c->em_n * c->em_ncr;
+  e.kp = c->kp.as<double>();
+  e.dl = c->em_dlw.as<double>();
+  e.Tg = c->em_Tg.as<double>();
+  e.Te = c->em_Te.as<double>();
+  e.R = c->em_R.as<double>();
   e.X = X;
   e.w = c->em_wbuf.as<double>();
   e.es = c->em_es.as<double>();
   e.lep = c->em_lep.as<double>();
   e.y = c->em_y.as<double>();
-  e.TgT = c->em_TgT.as<double>() + (size_t)w * c->em_n * c->em_n;
-  e.TeT = c->em_TeT.as<double>() + (size_t)w * c->em_n * c->em_n;
-  e.RT = c->em_RT.as<double>() + (size_t)w * c->em_n * c->em_ncr;
+  e.TgT = c->em_TgT.as<double>();
+  e.TeT = c->em_TeT.as<double>();
+  e.RT = c->em_RT.as<double>();
   return e;
 }
 
-
-// Enqueue the ETD2 steps [k0, k1) on `st`.  Columns [0, n_active[k]) are
-// advanced at step k; a step without active columns is skipped (every column
-// is still exactly zero).  With `ckpt`, the state before every step k with
-// k % every == 0 is copied to checkpoint k / every.  Returns the kernel count.
-int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_active, int64_t k0, int64_t k1,
-                     cudaStream_t st, double* ckpt, int every) {
-  const int64_t n = c->n;
+// One ETD2 step (both stages and the EM hook) on `st`; sc: its scalars on the
+// device, p.hcols: the columns the grids cover.  hook_pending: the previous
+// step's EM hook is still running on stream3.  Returns the kernel count.
+int64_t launch_step(pb_context* c, StepParams& p, int K, const StepScal* sc, bool& hook_pending, cudaStream_t st) {
   double* X = c->X.as<double>();
-  const size_t sbytes = (size_t)n * p.ld * sizeof(double);
   int64_t launches = 0;
-  int64_t prepared = -1;  // end of the run of steps whose row factors are ready
-  const bool record = p.rec_P != nullptr;  // the factors of the segment stay in p.rf for the sweep
   const bool em = c->have_em && (p.flags & PB_EM_CASCADE);
+  p.sc = sc;
+  const bool blocked = use_blocked(c, K) && (!p.rec_P || p.fdkp || !(p.flags & PB_PAIRPROD));
+  const bool overlap = em && blocked && c->n_tail > 0;
   // With the EM rows as the tail of the bin-blocked layout, a step's EM hook
   // (it reads the nuclei and writes only the EM rows) runs on stream3 beside
   // the next step's first stage; that stage's tail kernel, and everything
   // after it on the launching stream, waits for it.
-  bool hook_pending = false;
-  auto join_hook = [&]() {
-    if (hook_pending) cudaStreamWaitEvent(st, c->ev_hook_done, 0);
+  if (!overlap && hook_pending) {
+    cudaStreamWaitEvent(st, c->ev_hook_done, 0);
     hook_pending = false;
-    c->tail_wait = false;
+  }
+  c->tail_wait = hook_pending;
+  for (int stage = 1; stage <= 2; ++stage) {
+    p.src = stage == 1 ? X : c->A.as<double>();
+    p.x = X;
+    p.xout = X;
+    p.tmap_src = blocked ? stage_tmap(c, stage) : nullptr;
+    p.tmap_band = blocked ? stage_tmap_band(c, stage) : nullptr;
+    p.err = c->d_err.as<int>();
+    if (blocked) {
+      launches += stage == 1 ? launch_blocked_stage<1>(c, p, st) : launch_blocked_stage<2>(c, p, st);
+      continue;
+    }
+    const unsigned tiles = K == 1 ? 1u : blocks_for(p.hcols, kColTile);
+    dim3 grid((unsigned)p.nsb + blocks_for(p.nseg, 8), tiles);
+    if (K == 1) {
+      if (stage == 1) k_step_plain<1><<<grid, 256, 0, st>>>(p); else k_step_plain<2><<<grid, 256, 0, st>>>(p);
+    } else {
+      if (stage == 1) k_step_multi<1><<<grid, 256, 0, st>>>(p); else k_step_multi<2><<<grid, 256, 0, st>>>(p);
+    }
+    ++launches;
+  }
+  if (c->tail_wait) cudaStreamWaitEvent(st, c->ev_hook_done, 0);  // no tail launch consumed the wait
+  c->tail_wait = false;
+  hook_pending = false;
+  if (em) {
+    const EmParams e = em_params(c, sc, p.ld, p.hcols, X);
+    if (overlap) {
+      cudaEventRecord(c->ev_hook_fork, st);
+      cudaStreamWaitEvent(c->stream3, c->ev_hook_fork, 0);
+      em_hook_forward(e, c->stream3);
+      cudaEventRecord(c->ev_hook_done, c->stream3);
+      hook_pending = true;
+    } else {
+      em_hook_forward(e, st);
+    }
+    launches += 5;
+  }
+  return launches;
+}
+
+void join_hook(pb_context* c, bool& hook_pending, cudaStream_t st) {
+  if (hook_pending) cudaStreamWaitEvent(st, c->ev_hook_done, 0);
+  hook_pending = false;
+}
+
+constexpr size_t kMaxStepGraphs = 24;
+constexpr int kGraphCols = 64;  // column granularity of a captured run's grids
+
+// The captured run of `G` steps on the context's step-scalar buffer s_run for
+// up to `cols` active columns, or null when it cannot be captured.  The steps
+// read their scalars (step size, window, active columns) on the device, so a
+// run serves every schedule, every set of points and every part of a solve; a
+// whole solve captured as one graph cost 25 us per node, 230 ms for the 9,000
+// nodes of 1,000 batched steps, whenever the points and so the active columns
+// changed.  At most kMaxStepGraphs are kept, the least recently used go.
+StepGraph* step_graph(pb_context* c, StepParams p, int K, int G, int cols, cudaStream_t st) {
+  p.sc = nullptr;
+  p.hcols = cols;
+  p.prep_k0 = p.rf_k0 = 0;
+  p.eD = p.phi1 = p.phi2 = p.kap = p.slab_fac = nullptr;
+  p.src = p.x = nullptr;
+  p.xout = nullptr;
+  p.tmap_src = p.tmap_band = nullptr;
+  p.err = nullptr;
+  p.ngroups = p.spg = 0;
+  p.n_steps = 0;
+  std::vector<uint64_t> key;
+  auto put_bytes = [&](const void* q, size_t bytes) {
+    const size_t w0 = key.size();
+    key.resize(w0 + (bytes + 7) / 8, 0);
+    memcpy(key.data() + w0, q, bytes);
   };
-  for (int64_t k = k0; k < k1; ++k) {
-    if (ckpt && every > 0 && k % every == 0) {
-      join_hook();
+  put_bytes(&p, sizeof(p));
+  const EmParams e = em_params(c, nullptr, p.ld, cols, nullptr);
+  put_bytes(&e, sizeof(e));
+  for (uint64_t v : {(uint64_t)K, (uint64_t)G, (uint64_t)use_blocked(c, K), (uint64_t)c->tma_ok, (uint64_t)c->tma_band_ok,
+                     (uint64_t)c->band_tma_fits, (uint64_t)c->band_warps, (uint64_t)c->slab_pre, (uint64_t)c->band_RT,
+                     (uint64_t)c->band_J, (uint64_t)c->band_npairs, (uint64_t)c->slab_smem, (uint64_t)c->n_tail,
+                     (uint64_t)(uintptr_t)c->tail_rows.p, (uint64_t)c->fd_dense_ok, (uint64_t)c->have_em,
+                     (uint64_t)(uintptr_t)c->X.p, (uint64_t)(uintptr_t)c->tmaps.p, (uint64_t)(uintptr_t)c->d_err.p,
+                     (uint64_t)(uintptr_t)c->s_run.p})
+    key.push_back(v);
+  ++c->graph_clock;
+  for (StepGraph& g : c->step_graphs)
+    if (g.key == key) {
+      g.used = c->graph_clock;
+      return &g;
+    }
+  if (c->step_graphs.size() >= kMaxStepGraphs) {
+    auto old = std::min_element(c->step_graphs.begin(), c->step_graphs.end(),
+                                [](const StepGraph& a, const StepGraph& b) { return a.used < b.used; });
+    cudaGraphExecDestroy(old->exec);
+    c->step_graphs.erase(old);
+  }
+  StepGraph g;
+  const StepScal* run = c->s_run.as<StepScal>();
+  if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
+  bool hook = false;
+  for (int j = 0; j < G; ++j) {
+    set_step_factors(p, j);
+    g.launches += launch_step(c, p, K, run + j, hook, st);
+  }
+  join_hook(c, hook, st);
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) {
+    if (graph) cudaGraphDestroy(graph);
+    return nullptr;
+  }
+  cudaGraphDestroy(graph);
+  g.key = std::move(key);
+  g.used = c->graph_clock;
+  c->step_graphs.push_back(std::move(g));
+  return &c->step_graphs.back();
+}
+
+// Enqueue the ETD2 steps [k0, k1) on `st`.  Columns [0, n_active[k]) are
+// advanced at step k; a step without active columns is skipped (every column
+// is still exactly zero).  With `ckpt`, the state before every step k with
+// k % every == 0 is copied to checkpoint k / every.  Runs of steps between
+// checkpoints replay a captured graph; what is left, and the record pass, is
+// launched step by step.  Returns the kernel count, or -1 on a failure.
+int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_active, int64_t k0, int64_t k1,
+                     cudaStream_t st, double* ckpt, int every) {
+  const int64_t n = c->n;
+  double* X = c->X.as<double>();
+  const StepScal* scal = c->s_scal.as<StepScal>();
+  const size_t sbytes = (size_t)n * p.ld * sizeof(double);
+  int64_t launches = 0;
+  int64_t prepared = -1;  // end of the run of steps whose row factors are ready
+  const bool record = p.rec_P != nullptr;  // the factors of the segment stay in p.rf for the sweep
+  const int G = (int)std::min<int64_t>(kGraphSteps, prep_steps(n));
+  static const bool no_graph = getenv("PRINCE_B200_NO_GRAPH") != nullptr;
+  bool hook_pending = false;
+  for (int64_t k = k0; k < k1;) {
+    const bool copy = ckpt && every > 0;
+    if (copy && k % every == 0) {
+      join_hook(c, hook_pending, st);
       cudaMemcpyAsync(ckpt + (size_t)(k / every) * n * p.ld, X, sbytes, cudaMemcpyDeviceToDevice, st);
     }
-    p.step = k;
-    p.step_w = c->h_win[k];
-    p.ncols = n_active[k];
-    if (p.ncols == 0) continue;
+    if (n_active[k] == 0) {
+      ++k;
+      continue;
+    }
+    const int64_t stop = copy ? std::min<int64_t>(k1, (k / every + 1) * every) : k1;  // the next checkpoint
+    if (!no_graph && !record && k >= prepared && stop - k >= G) {
+      join_hook(c, hook_pending, st);
+      int cols = 0;
+      for (int64_t q = k; q < k + G; ++q) cols = std::max(cols, n_active[q]);
+      cols = K == 1 ? 1 : std::min((cols + kGraphCols - 1) / kGraphCols * kGraphCols, p.ld);
+      StepGraph* g = step_graph(c, p, K, G, cols, st);
+      if (!g) return -1;
+      p.rf_k0 = k;
+      launch_prep(p, scal, k, G, st);
+      cudaMemcpyAsync(c->s_run.p, scal + k, G * sizeof(StepScal), cudaMemcpyDeviceToDevice, st);
+      if (cudaGraphLaunch(g->exec, st) != cudaSuccess) return -1;
+      launches += 1 + g->launches;
+      k += G;
+      continue;
+    }
     if (k >= prepared) {
-      const int64_t count = std::min<int64_t>(prep_steps(n), k1 - k);
+      const int64_t count = std::min<int64_t>(prep_steps(n), (stop - k >= G ? k1 : stop) - k);
       if (!record) p.rf_k0 = k;
-      launch_prep(p, k, count, st);
+      launch_prep(p, scal, k, count, st);
       ++launches;
       prepared = k + count;
     }
     set_step_factors(p, k);
-    const bool blocked = use_blocked(c, K) && (!p.rec_P || p.fdkp || !(p.flags & PB_PAIRPROD));
-    const bool overlap = em && blocked && c->n_tail > 0;
-    if (!overlap) join_hook();
-    c->tail_wait = hook_pending;
-    for (int stage = 1; stage <= 2; ++stage) {
-      p.src = stage == 1 ? X : c->A.as<double>();
-      p.x = X;
-      p.xout = X;
-      p.tmap_src = blocked ? stage_tmap(c, stage) : nullptr;
-      p.tmap_band = blocked ? stage_tmap_band(c, stage) : nullptr;
-      p.err = c->d_err.as<int>();
-      if (blocked) {
-        launches += stage == 1 ? launch_blocked_stage<1>(c, p, st) : launch_blocked_stage<2>(c, p, st);
-        continue;
-      }
-      const unsigned tiles = K == 1 ? 1u : blocks_for(p.ncols, kColTile);
-      dim3 grid((unsigned)p.nsb + blocks_for(p.nseg, 8), tiles);
-      if (K == 1) {
-        if (stage == 1) k_step_plain<1><<<grid, 256, 0, st>>>(p); else k_step_plain<2><<<grid, 256, 0, st>>>(p);
-      } else {
-        if (stage == 1) k_step_multi<1><<<grid, 256, 0, st>>>(p); else k_step_multi<2><<<grid, 256, 0, st>>>(p);
-      }
-      ++launches;
-    }
-    if (c->tail_wait) join_hook();  // no tail launch consumed the wait
-    hook_pending = false;
-    if (em) {
-      const EmParams e = em_params(c, c->h_win[k], p.ld, p.ncols, X);
-      if (overlap) {
-        cudaEventRecord(c->ev_hook_fork, st);
-        cudaStreamWaitEvent(c->stream3, c->ev_hook_fork, 0);
-        em_hook_forward(e, c->stream3);
-        cudaEventRecord(c->ev_hook_done, c->stream3);
-        hook_pending = true;
-      } else {
-        em_hook_forward(e, st);
-      }
-      launches += 5;
-    }
+    p.hcols = n_active[k];
+    launches += launch_step(c, p, K, scal + k, hook_pending, st);
+    ++k;
   }
-  join_hook();
+  join_hook(c, hook_pending, st);
   return launches;
 }
 
 // All steps of a constant operator (one column), state x in place.
-void const_steps(StepParams& p, int64_t per_prep, double* x, cudaStream_t st) {
+void const_steps(StepParams& p, const StepScal* scal, int64_t per_prep, double* x, cudaStream_t st) {
   p.x = x;
   p.xout = x;
   for (int64_t k = 0; k < p.n_steps; ++k) {
     if (k % per_prep == 0) {
       p.rf_k0 = k;
-      launch_prep(p, k, std::min(per_prep, p.n_steps - k), st);
+      launch_prep(p, scal, k, std::min(per_prep, p.n_steps - k), st);
     }
     set_step_factors(p, k);
-    p.step = k;
+    p.sc = scal + k;
     p.src = x;
     k_step_plain<1><<<blocks_for(p.n, 256), 256, 0, st>>>(p);
     p.src = p.a;
@@ -3460,8 +3593,7 @@ void pb_destroy(pb_context* c) {
   if (c->stream2) cudaStreamSynchronize(c->stream2);
   if (c->stream3) cudaStreamSynchronize(c->stream3);
   for (DBuf* b : all_buffers(c)) b->release();
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph_exec2) cudaGraphExecDestroy(c->graph_exec2);
+  for (StepGraph& g : c->step_graphs) cudaGraphExecDestroy(g.exec);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   cudaEventDestroy(c->ev2);
@@ -4269,9 +4401,7 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   StepParams p;
   memset(&p, 0, sizeof(p));
   fill_step_params(c, p, K, ld, flags, pair, inj, c->last_S, ld / kColTile);
-  p.step = step;
-  p.step_w = c->h_win[step];
-  p.ncols = c->h_nact[step];
+  p.hcols = c->h_nact[step];
   p.src = stage == 1 ? c->X.as<double>() : c->A.as<double>();
   p.x = c->X.as<double>();
   p.xout = c->X.as<double>();
@@ -4281,10 +4411,10 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   p.err = c->d_err.as<int>();
   cudaStream_t st = c->stream;
   p.rf_k0 = step;
-  launch_prep(p, step, 1, st);
+  launch_prep(p, c->s_scal.as<StepScal>(), step, 1, st);
   set_step_factors(p, step);
   const bool photohad = (flags & PB_PHOTOHAD) != 0, kap = (flags & PB_PARTIAL_DIFF) != 0;
-  const unsigned tiles = (unsigned)blocks_for(p.ncols, kColTile);
+  const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
   const BandInstance bi = (c->band_warps == 8 && p.tmap_band) ? band_kernel_tma(c->band_RT, c->band_J)
                                                               : band_kernel(c->band_RT, c->band_J, c->band_warps);
   const int cblocks = band_grid(c, p, bi.warps);
@@ -4301,7 +4431,7 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
         else k_fd<<<dim3(p.nsp, tiles), 256, (size_t)p.d * (kColTile + 2) * sizeof(double), st>>>(p);
       }
       if (kk == 1) {
-        const dim3 sg(p.d, (unsigned)blocks_for(p.ncols, kSlabCols));
+        const dim3 sg(p.d, (unsigned)blocks_for(p.hcols, kSlabCols));
         slab_kernel(stage, false, c->slab_pre)<<<sg, kSlabWarps * 32, c->slab_smem, st>>>(p);
       }
       if (kk == 2) bi.fn<<<dim3(cblocks, p.ngroups, c->band_npairs), bi.warps * 32, bi.smem, st>>>(p);
@@ -4465,8 +4595,8 @@ int pb_set_em_windows(pb_context* c, int32_t n_windows, const double* Tg, const 
     if ((rc = upload(c, c->em_TeT, te.data(), te.size()))) return rc;
     if ((rc = upload(c, c->em_RT, rt.data(), rt.size()))) return rc;
   }
+  if ((rc = upload(c, c->em_dlw, dl_step, (size_t)n_windows))) return rc;
   PB_CUDA(c, cudaStreamSynchronize(c->stream));
-  c->em_dl.assign(dl_step, dl_step + n_windows);
   c->em_W = n_windows;
   return PB_OK;
 }
@@ -4764,7 +4894,6 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
     if (a->n_active[k] < 0 || a->n_active[k] > K) return fail(c, PB_ERR_ARG, "pb_solve: n_active out of range");
   }
   if ((int64_t)W * c->n >= ((int64_t)1 << 40)) return fail(c, PB_ERR_ARG, "pb_solve: too many windows");
-  c->h_win.assign(a->window, a->window + S);
   c->h_nact.assign(a->n_active, a->n_active + S);
   int rc = set_device(c);
   if (rc) return rc;
@@ -4775,11 +4904,11 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   // ---- per-solve uploads -------------------------------------------------
   if ((rc = upload(c, c->zwin, a->z_window, (size_t)W))) return rc;
   if (S > 0) {
-    if ((rc = upload(c, c->s_h, a->h, (size_t)S))) return rc;
-    if ((rc = upload(c, c->s_dldz, a->dldz, (size_t)S))) return rc;
-    if ((rc = upload(c, c->s_hc, a->hc, (size_t)S))) return rc;
+    c->h_scal.resize((size_t)S);
+    for (int64_t k = 0; k < S; ++k)
+      c->h_scal[k] = StepScal{a->h[k], a->dldz[k], a->hc[k], a->finj[k], k, a->window[k], a->n_active[k]};
+    if ((rc = upload(c, c->s_scal, c->h_scal.data(), (size_t)S))) return rc;
     if ((rc = upload(c, c->s_finj, a->finj, (size_t)S))) return rc;
-    if ((rc = upload(c, c->s_win, a->window, (size_t)S))) return rc;
     if (inj && (rc = upload(c, c->s_coeff, a->coeff, (size_t)S * c->n_src))) return rc;
   }
   PB_CUDA(c, c->PT.ensure((size_t)W * c->dph * sizeof(double)));
@@ -4853,9 +4982,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   }
   const FieldDesc fd = field_desc(c, a->photon_scale);
   int64_t launches = 0;
-  // Everything from here to the end of the last step is enqueued by `enqueue`:
-  // directly, or under stream capture into a CUDA graph that is replayed while
-  // the solve's shape and buffers stay the same.
+  // The per-solve operator set-up is enqueued by `enqueue`, the steps by launch_steps.
   StepParams p;
   memset(&p, 0, sizeof(p));
   auto enqueue = [&](int64_t& launches) -> int {
@@ -4920,74 +5047,18 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   fill_step_params(c, p, K, ld, flags, pair, inj, S, ctiles);
     return PB_OK;
   };
-  auto enqueue_steps = [&](int64_t& launches) -> int {
-  const int CK = a->ckpt_every;
-  launches += launch_steps(c, p, K, a->n_active, 0, S, st, CK > 0 ? c->ckpt.as<double>() : nullptr, CK);
-  PB_CUDA(c, cudaGetLastError());
-    return PB_OK;
-  };
-
-  std::vector<uint64_t> key;
-  {
-    auto put = [&](uint64_t v) { key.push_back(v); };
-    put((uint64_t)S); put((uint64_t)W); put((uint64_t)K); put((uint64_t)ld); put(flags); put(inj); put(R);
-    put((uint64_t)c->n_seg); put((uint64_t)c->h_short_rows.size()); put((uint64_t)c->n_cr_bins);
-    put((uint64_t)a->ckpt_every);
-    put((uint64_t)blocked);
-    put((uint64_t)(blocked && c->tma_ok));
-    put((uint64_t)c->staging_wait_tries);
-    put((uint64_t)c->band_warps);
-    put((uint64_t)c->slab_pre);
-    put((uint64_t)c->band_RT); put((uint64_t)c->band_J); put((uint64_t)c->band_nb); put((uint64_t)c->lay_d);
-    put((uint64_t)c->slab_nent);
-    put((uint64_t)c->em_W);
-    for (double v : c->em_dl) { uint64_t b; memcpy(&b, &v, 8); put(b); }
-    const unsigned char* fb = reinterpret_cast<const unsigned char*>(&fd);
-    for (size_t i = 0; i < sizeof(fd); i += 8) { uint64_t w = 0; memcpy(&w, fb + i, std::min<size_t>(8, sizeof(fd) - i)); put(w); }
-    for (const DBuf* b : solve_buffers(c)) put((uint64_t)(uintptr_t)b->p);  // adjoint scratch is not in the graphs
-    for (int64_t k = 0; k < S; ++k) put((uint64_t)a->n_active[k]);
+  PB_CUDA(c, cudaEventRecord(c->ev0, st));
+  if ((rc = enqueue(launches))) return rc;
+  PB_CUDA(c, cudaEventRecord(c->ev2, st));
+  if (S > 0) {
+    PB_CUDA(c, c->s_run.ensure(kGraphSteps * sizeof(StepScal)));
+    const int64_t l = launch_steps(c, p, K, a->n_active, 0, S, st, a->ckpt_every > 0 ? c->ckpt.as<double>() : nullptr,
+                                   a->ckpt_every);
+    PB_CUDA(c, cudaGetLastError());
+    if (l < 0) return fail(c, PB_ERR_CUDA, "pb_solve: capturing or launching a run of steps failed");
+    launches += l;
   }
-  // Two graphs -- the per-solve operator set-up and the step loop -- with the
-  // timing events recorded on the stream between them.
-  static const bool no_graph = getenv("PRINCE_B200_NO_GRAPH") != nullptr;
-  if (no_graph) {
-    PB_CUDA(c, cudaEventRecord(c->ev0, st));
-    if ((rc = enqueue(launches))) return rc;
-    PB_CUDA(c, cudaEventRecord(c->ev2, st));
-    if ((rc = enqueue_steps(launches))) return rc;
-    PB_CUDA(c, cudaEventRecord(c->ev3, st));
-  } else {
-    if (!c->graph_exec || !c->graph_exec2 || c->graph_key != key) {
-      for (cudaGraphExec_t* ge : {&c->graph_exec, &c->graph_exec2})
-        if (*ge) {
-          cudaGraphExecDestroy(*ge);
-          *ge = nullptr;
-        }
-      int64_t l1 = 0, l2 = 0;
-      for (int part = 0; part < 2; ++part) {
-        PB_CUDA(c, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const int rc2 = part == 0 ? enqueue(l1) : enqueue_steps(l2);
-        cudaGraph_t g = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(st, &g);
-        if (rc2) {
-          if (g) cudaGraphDestroy(g);
-          return rc2;
-        }
-        PB_CUDA(c, e);
-        const cudaError_t ei = cudaGraphInstantiate(part == 0 ? &c->graph_exec : &c->graph_exec2, g, 0);
-        cudaGraphDestroy(g);
-        PB_CUDA(c, ei);
-      }
-      c->graph_key = key;
-      c->graph_launches = l1 + l2;
-    }
-    PB_CUDA(c, cudaEventRecord(c->ev0, st));
-    PB_CUDA(c, cudaGraphLaunch(c->graph_exec, st));
-    PB_CUDA(c, cudaEventRecord(c->ev2, st));
-    PB_CUDA(c, cudaGraphLaunch(c->graph_exec2, st));
-    PB_CUDA(c, cudaEventRecord(c->ev3, st));
-    launches = c->graph_launches;
-  }
+  PB_CUDA(c, cudaEventRecord(c->ev3, st));
   const cudaMemcpyKind out_kind = a->state_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const bool ocols = a->out_cols && K > 1;
   if (ocols || rmap) {  // rows and columns in the caller's order, gathered on the device, then one copy
@@ -5021,7 +5092,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
 // The tile parameters of the bin-blocked stage, searched on the live operator:
 // every (band-tile CTA warps, k_slab prefetch depth, k_slab staging) candidate
 // runs the caller's (short) solve `reps` times and is scored by its fastest
-// step loop (CUDA events around the step graph); the fastest candidate stays
+// step loop (CUDA events around the steps); the fastest candidate stays
 // set on the context.  Only the batched bin-blocked path has choices.
 int pb_autotune(pb_context* c, const pb_solve_args* a, int32_t reps, int32_t max_out, pb_tune_choice* out,
                 int32_t* n_out) {
@@ -5041,7 +5112,7 @@ int pb_autotune(pb_context* c, const pb_solve_args* a, int32_t reps, int32_t max
     c->slab_pre = cand[i].slab_prefetch;
     c->tma_mode = cand[i].tma_staging;
     double t = 1e300;
-    for (int r = 0; r < reps + 1; ++r) {  // the first run captures the candidate's graph
+    for (int r = 0; r < reps + 1; ++r) {  // the first run captures the candidate's run of steps
       const int rc = pb_solve(c, a);
       if (rc) {
         c->band_warps = keep_bw;
@@ -5218,7 +5289,7 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
       launch_steps(c, p, K, a->n_active, k0, k1, st, nullptr, 0);
     } else {  // the operator factors depend on z alone: record them without recomputing the states
       p.sfac = nullptr;
-      for (int64_t k = kf; k < k1; k += kPrepMaxSteps) launch_prep(p, k, std::min<int64_t>(kPrepMaxSteps, k1 - k), st);
+      for (int64_t k = kf; k < k1; k += kPrepMaxSteps) launch_prep(p, c->s_scal.as<StepScal>(), k, std::min<int64_t>(kPrepMaxSteps, k1 - k), st);
     }
     if (blockedT) {
       for (int64_t k = k1 - 1; k >= kf; --k) {
@@ -5270,7 +5341,7 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
           q.inj_slot = c->inj_slot.as<int>();
           q.gb_inj = c->gb_inj.as<double>() + (size_t)k * n_inj * ld;
         }
-        if (em) em_hook_adjoint(em_params(c, a->window[k], ld, q.ncols, lam), st);  // the hook after step k
+        if (em) em_hook_adjoint(em_params(c, c->s_scal.as<StepScal>() + k, ld, q.ncols, lam), st);  // the hook after step k
         if (k == k1 - 1 || em)  // v1 of the segment's last step; later steps get it from stage 2
           k_adj_v1<<<dim3(blocks_for(n, 8), blocks_for(q.ncols, kColTile)), 256, 0, st>>>(
               q.rf + 2 * n, lam, n, ld, q.ncols, c->vbuf.as<double>());
@@ -5359,7 +5430,7 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
         q.inj_slot = c->inj_slot.as<int>();
         q.gb_inj = c->gb_inj.as<double>() + (size_t)k * n_inj * ld;
       }
-      if (em) em_hook_adjoint(em_params(c, a->window[k], ld, q.ncols, lam), st);  // the hook after step k
+      if (em) em_hook_adjoint(em_params(c, c->s_scal.as<StepScal>() + k, ld, q.ncols, lam), st);  // the hook after step k
       dim3 grid(blocks_for(n, 8), K == 1 ? 1u : blocks_for(q.ncols, kColTile));
       k_adj<1><<<grid, 256, 0, st>>>(q);
       k_adj<2><<<grid, 256, 0, st>>>(q);
@@ -5454,18 +5525,17 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   cudaStream_t st = c->stream;
   // A constant operator is one window with M_off = L_off, M_diag = d, dl/dz = 1
   // and no losses or injection.
-  DBuf ip, ix, iv, dg, hs, ones, zero_i, X, A, F, rows, rowf;
+  DBuf ip, ix, iv, dg, hs, X, A, F, rows, rowf;
   auto cleanup = [&]() {
-    for (DBuf* b : {&ip, &ix, &iv, &dg, &hs, &ones, &zero_i, &X, &A, &F, &rows, &rowf}) b->release();
+    for (DBuf* b : {&ip, &ix, &iv, &dg, &hs, &X, &A, &F, &rows, &rowf}) b->release();
   };
-  std::vector<double> hv((size_t)std::max<int64_t>(n_steps, 1)), one((size_t)std::max<int64_t>(n_steps, 1), 1.0);
-  for (int64_t k = 0; k < n_steps; ++k) hv[k] = z_grid[k + 1] - z_grid[k];
-  std::vector<int> zi((size_t)std::max<int64_t>(n_steps, 1), 0), rl((size_t)n);
+  std::vector<StepScal> hv((size_t)std::max<int64_t>(n_steps, 1));
+  for (int64_t k = 0; k < n_steps; ++k) hv[k] = StepScal{z_grid[k + 1] - z_grid[k], 1.0, 1.0, 1.0, k, 0, 1};
+  std::vector<int> rl((size_t)n);
   for (int64_t i = 0; i < n; ++i) rl[i] = (int)i;
   if ((rc = upload(c, ip, indptr, (size_t)n + 1)) || (rc = upload(c, ix, indices, (size_t)nnz)) ||
       (rc = upload(c, iv, values, (size_t)nnz)) || (rc = upload(c, dg, d, (size_t)n)) ||
-      (rc = upload(c, hs, hv.data(), hv.size())) || (rc = upload(c, ones, one.data(), one.size())) ||
-      (rc = upload(c, zero_i, zi.data(), zi.size())) || (rc = upload(c, X, state, (size_t)n)) ||
+      (rc = upload(c, hs, hv.data(), hv.size())) || (rc = upload(c, X, state, (size_t)n)) ||
       (rc = upload(c, rows, rl.data(), rl.size()))) {
     cleanup();
     return rc;
@@ -5479,13 +5549,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   memset(&p, 0, sizeof(p));
   p.n = n;
   p.ld = 1;
-  p.ncols = 1;
   p.flags = PB_PHOTOHAD;
-  p.h = hs.as<double>();
-  p.dldz = ones.as<double>();
-  p.hc = ones.as<double>();
-  p.finj = ones.as<double>();
-  p.win = zero_i.as<int>();
   p.m_indptr = ip.as<int64_t>();
   p.m_indices = ix.as<int>();
   p.m_vals = iv.as<double>();
@@ -5498,7 +5562,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   p.nsb = (int)blocks_for(n, 256);
   p.n_steps = n_steps;
   p.rf = rowf.as<double>();
-  const_steps(p, prep_steps(n), X.as<double>(), st);
+  const_steps(p, hs.as<StepScal>(), prep_steps(n), X.as<double>(), st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(state, X.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -5547,10 +5611,8 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
   double* a = reinterpret_cast<double*>(base);
   double* f = a + kNaMaxStates;
   double* rowf = f + kNaMaxStates;
-  double* h = rowf + 8 * kNaMaxStates;
-  double* ones = h + kNaMaxSteps;
-  int* win = reinterpret_cast<int*>(ones + kNaMaxSteps);
-  int* rows = win + kNaMaxSteps;
+  StepScal* scal = reinterpret_cast<StepScal*>(rowf + 8 * kNaMaxStates);
+  int* rows = reinterpret_cast<int*>(scal + kNaMaxSteps);
   int64_t* zero_indptr = reinterpret_cast<int64_t*>(rows + kNaMaxStates);
   unsigned int* csr_flag = reinterpret_cast<unsigned int*>(zero_indptr + kNaMaxStates + 1);
   cudaStream_t st = c->stream;
@@ -5573,18 +5635,12 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
     if (bad & 2u) return fail(c, PB_ERR_ARG, "pb_integrate_const_noalloc: CSR column index outside [0, n)");
   }
   const int64_t fill = std::max<int64_t>(n + 1, n_steps);
-  k_noalloc_fill<<<blocks_for(fill, 256), 256, 0, st>>>(n, n_steps, z_grid, h, ones, win, rows, zero_indptr);
+  k_noalloc_fill<<<blocks_for(fill, 256), 256, 0, st>>>(n, n_steps, z_grid, scal, rows, zero_indptr);
   StepParams p;
   memset(&p, 0, sizeof(p));
   p.n = n;
   p.ld = 1;
-  p.ncols = 1;
   p.flags = PB_PHOTOHAD;
-  p.h = h;
-  p.dldz = ones;
-  p.hc = ones;
-  p.finj = ones;
-  p.win = win;
   p.m_indptr = nnz > 0 ? indptr : zero_indptr;
   p.m_indices = indices;
   p.m_vals = values;
@@ -5597,7 +5653,7 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
   p.nsb = (int)blocks_for(n, 256);
   p.n_steps = n_steps;
   p.rf = rowf;
-  const_steps(p, kNaPrepSteps, state, st);
+  const_steps(p, scal, kNaPrepSteps, state, st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(c, PB_ERR_CUDA, "pb_integrate_const_noalloc: %s", cudaGetErrorString(e));
