@@ -22,6 +22,7 @@
 // The data layout, the kernels and the launch structure are this project's own.
 
 #include <cuda.h>  // CUtensorMap (the encoder is reached through cudaGetDriverEntryPoint)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cub/cub.cuh>
 #include <math_constants.h>
@@ -183,6 +184,11 @@ struct pb_context {
   int64_t slabT_nent = 0;
   int32_t slabT_maxbin = 0;
   size_t slabT_smem = 0, bandT_smem = 0;
+  // small networks (k_small)
+  DBuf small_order;                 // rows by coupling entries, longest first
+  int32_t small_cap[4] = {0, 0, 0, 0};  // coupling entries of a CTA for clusters of 1, 2, 4, 8
+  int64_t fd_row_max = 0;           // off-diagonal FD entries of a row (at most)
+  bool small_off = false;           // the tuner measures the bin-blocked kernels
   int32_t batched_mode = 1;         // 0: general row kernels; 1: bin-blocked kernels when the layout allows
   int32_t tma_mode = 1;             // 1: k_slab stages by TMA when tensor maps can be encoded; 0: cp.async
   long long staging_wait_tries = kWaitTries;  // k_slab's first staging wait (PB_OPT_STAGING_WAIT_TRIES)
@@ -1148,6 +1154,253 @@ __global__ void __launch_bounds__(256) k_step_multi(StepParams p) {
   for (int q = 0; q < ns; ++q) t = __dadd_rn(t, __ldcg(p.partial + (size_t)(s0 + q) * p.ld + blockIdx.y * kColTile + lane));
   const int64_t r = p.lr_row[lr];
   if (active) row_epilogue<STAGE>(p, s, r, k, t);
+}
+
+// ---------------------------------------------------------------------------
+// Small networks: all steps of a solve in one launch.
+//
+// A cluster of CS CTAs owns CC state columns.  Its CTAs share the rows (row i
+// of the length order goes to CTA i mod CS) and hold their rows' coupling
+// entries of the current window, the loss stencil and every row of the
+// columns' x and a in shared memory; a stage's new values go to all CTAs of
+// the cluster through distributed shared memory, and one cluster barrier ends
+// the stage.  Columns are independent, so nothing else is exchanged: a step
+// costs two barriers instead of two to eight launches of 4 to 25 us each.  A
+// group of LPR lanes sums a row (entries j, j + LPR, ..., then a butterfly),
+// and its first CC lanes apply the stage update; the losses' terms add in CSR
+// order.  Bound by the shared-memory wavefronts of the entries (about 5 per 32
+// entries: value, index, gathered state) and the two barriers.
+// ---------------------------------------------------------------------------
+constexpr int kSmallRows = 1024;    // rows (one thread each loads the next step's factors)
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallFd = 4;         // off-diagonal stencil entries per row
+
+struct SmallArgs {
+  const int* order;   // rows by coupling entries, longest first
+  int K;              // columns
+  int count;          // steps, from p.sc and p.rf
+  int slots;          // rows of a CTA (at most)
+  int cap;            // coupling entries of a CTA (at most)
+  int lpr;            // lanes per row
+  double* X;
+};
+
+struct SmallSmem {
+  double *x, *a, *fac, *F, *b, *dval, *vals;
+  int *row, *inj, *beg, *len, *src;
+  unsigned short *dcol, *idx;
+  __host__ __device__ static size_t bytes(int n, int slots, int cap, int cc) {
+    return ((size_t)n * (2 * cc + 8) + (size_t)slots * (3 * cc + 4) + cap) * sizeof(double) +
+           ((size_t)4 * slots) * sizeof(int) + ((size_t)slots * kSmallFd + cap) * sizeof(unsigned short) + 16;
+  }
+  __device__ SmallSmem(double* base, int n, int slots, int cap, int cc) {
+    x = base;
+    a = x + n * cc;
+    fac = a + n * cc;       // [2][4][n] eD, phi1, phi2, kappa of this and the next step
+    F = fac + 8 * n;        // [slots][cc] F(x)
+    b = F + slots * cc;     // [2][slots][cc] injection of this and the next step
+    dval = b + 2 * slots * cc;
+    vals = dval + slots * kSmallFd;
+    row = reinterpret_cast<int*>(vals + cap);
+    inj = row + slots;
+    beg = inj + slots;
+    len = beg + slots;
+    dcol = reinterpret_cast<unsigned short*>(len + slots);
+    idx = dcol + slots * kSmallFd;
+  }
+};
+
+template <int CC>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallArgs q) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) double sm[];
+  __shared__ typename cub::BlockScan<int, kSmallThreads>::TempStorage scan;
+  cg::cluster_group cl = cg::this_cluster();
+  const int CS = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int n = (int)p.n, tid = threadIdx.x, lpr = q.lpr;
+  const int c0 = (blockIdx.x / CS) * CC;
+  SmallSmem L(sm, n, q.slots, q.cap, CC);
+  const bool photohad = (p.flags & PB_PHOTOHAD) != 0, kap = (p.flags & PB_PARTIAL_DIFF) != 0;
+  const bool inj = (p.flags & PB_INJECTION) != 0 && p.G != nullptr, decay = (p.flags & PB_DECAY) != 0 && p.l_diag;
+
+  // ---- rows, pattern, stencil, states -----------------------------------
+  int r0 = -1, l0 = 0;
+  if (tid < q.slots) {
+    const int i = tid * CS + rank;
+    r0 = i < n ? q.order[i] : -1;
+    l0 = (r0 >= 0 && photohad) ? (int)(p.m_indptr[r0 + 1] - p.m_indptr[r0]) : 0;
+  }
+  int b0;
+  cub::BlockScan<int, kSmallThreads>(scan).ExclusiveSum(l0, b0);
+  if (tid < q.slots) {
+    L.row[tid] = r0;
+    L.len[tid] = l0;
+    L.beg[tid] = b0;
+    L.inj[tid] = (inj && r0 >= 0) ? p.inj_slot[r0] : -1;
+    for (int t = 0; t < kSmallFd; ++t) {
+      L.dval[tid * kSmallFd + t] = 0.0;
+      L.dcol[tid * kSmallFd + t] = 0xffff;
+    }
+    if (kap && r0 >= 0) {
+      const int64_t j0 = p.d_indptr[r0];
+      for (int t = 0; t < (int)(p.d_indptr[r0 + 1] - j0); ++t) {
+        L.dval[tid * kSmallFd + t] = p.d_vals[j0 + t];
+        L.dcol[tid * kSmallFd + t] = (unsigned short)p.d_indices[j0 + t];
+      }
+    }
+  }
+  for (int t = tid; t < n * CC; t += kSmallThreads) {
+    const int r = t / CC, c = c0 + t % CC;
+    L.x[t] = c < q.K ? q.X[(size_t)r * p.ld + c] : 0.0;
+    L.a[t] = 0.0;
+  }
+  int k = 0;
+  while (k < q.count && p.sc[k].ncols <= c0) ++k;  // the cluster's columns are all still switched off
+  if (tid < n && k < q.count)
+    for (int f = 0; f < 4; ++f) L.fac[((k & 1) * 4 + f) * n + tid] = p.rf[((size_t)k * 4 + f) * n + tid];
+  __syncthreads();
+  const int grp = tid / lpr, ngrp = kSmallThreads / lpr, l = tid % lpr;
+  for (int sl = grp; sl < q.slots; sl += ngrp) {
+    const int len = L.len[sl], beg = L.beg[sl];
+    const int64_t m0 = len ? p.m_indptr[L.row[sl]] : 0;
+    for (int j = l; j < len; j += lpr) L.idx[beg + j] = (unsigned short)p.m_indices[m0 + j];
+  }
+  // this lane's column of the injection and its sources
+  const int col = c0 + l;
+  const bool mine = l < CC && col < q.K;
+  int s0 = 0, s1 = 0;
+  if (inj && mine) {
+    s0 = p.src_ptr[col];
+    s1 = p.src_ptr[col + 1];
+  }
+  auto injection = [&](int sl, const StepScal& sc) {
+    const double* cf = p.coeff + (size_t)sc.step * p.n_src;
+    const double* g = p.G + (size_t)L.inj[sl] * p.n_src;
+    double v = __dmul_rn(cf[s0], g[s0]);
+    for (int t = s0 + 1; t < s1; ++t) v = __dadd_rn(v, __dmul_rn(cf[t], g[t]));
+    return __dmul_rn(sc.finj, v);
+  };
+  if (k < q.count && s1 > s0) {
+    const StepScal sc = p.sc[k];
+    for (int sl = grp; sl < q.slots; sl += ngrp)
+      if (L.inj[sl] >= 0) L.b[((k & 1) * q.slots + sl) * CC + l] = injection(sl, sc);
+  }
+  cl.sync();
+
+  // ---- the steps -----------------------------------------------------------
+  StepScal sc = k < q.count ? p.sc[k] : StepScal{};
+  int w = -1;
+  for (; k < q.count; ++k) {
+    const int par = k & 1, nxt = par ^ 1;
+    const bool more = k + 1 < q.count;
+    // the next step's scalars and factors, stored before the step's last barrier
+    StepScal scn = more ? p.sc[k + 1] : sc;
+    double fn[4];
+    if (more && tid < n)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) fn[f] = p.rf[((size_t)(k + 1) * 4 + f) * n + tid];
+    if (sc.ncols > c0) {
+      if (photohad && sc.w != w) {  // a group reads only entries that its own lanes wrote
+        w = sc.w;
+        const double* mv = p.m_vals + (size_t)w * p.m_wstride;
+        for (int sl = grp; sl < q.slots; sl += ngrp) {
+          const int len = L.len[sl], beg = L.beg[sl];
+          const int64_t m0 = len ? p.m_indptr[L.row[sl]] : 0;
+          for (int j = l; j < len; j += lpr) L.vals[beg + j] = mv[m0 + j];
+        }
+      }
+      const bool on = mine && col < sc.ncols;
+      const double* eD = L.fac + (size_t)par * 4 * n;
+      const double* kp = eD + 3 * n;
+#pragma unroll 1
+      for (int stage = 1; stage <= 2; ++stage) {
+        const double* v = stage == 1 ? L.x : L.a;
+        for (int sb = 0; sb < q.slots; sb += ngrp) {  // the same trip count in every lane of a warp
+          const int sl = sb + grp;
+          const bool have = sl < q.slots && L.row[sl] >= 0;
+          const int len = have ? L.len[sl] : 0, beg = have ? L.beg[sl] : 0;
+          double acc[CC], acc2[CC];
+#pragma unroll
+          for (int c = 0; c < CC; ++c) acc[c] = acc2[c] = 0.0;
+          int j = l;
+          for (; j + lpr < len; j += 2 * lpr) {
+            const double m0 = L.vals[beg + j], m1 = L.vals[beg + j + lpr];
+            const double* v0 = v + L.idx[beg + j] * CC;
+            const double* v1 = v + L.idx[beg + j + lpr] * CC;
+#pragma unroll
+            for (int c = 0; c < CC; ++c) {
+              acc[c] = __fma_rn(m0, v0[c], acc[c]);
+              acc2[c] = __fma_rn(m1, v1[c], acc2[c]);
+            }
+          }
+          if (j < len) {
+            const double m0 = L.vals[beg + j];
+            const double* v0 = v + L.idx[beg + j] * CC;
+#pragma unroll
+            for (int c = 0; c < CC; ++c) acc[c] = __fma_rn(m0, v0[c], acc[c]);
+          }
+          __syncwarp();
+          double sM = 0.0;
+#pragma unroll
+          for (int c = 0; c < CC; ++c) {
+            double t = __dadd_rn(acc[c], acc2[c]);
+            for (int o = lpr >> 1; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+            if (l == c) sM = t;
+          }
+          if (have && on) {
+            const int r = L.row[sl];
+            double out = sM;
+            if (kap) {
+              double sD = 0.0;
+#pragma unroll
+              for (int t = 0; t < kSmallFd; ++t) {
+                const int cx = L.dcol[sl * kSmallFd + t];
+                if (cx != 0xffff)
+                  sD = __dadd_rn(sD, __dmul_rn(L.dval[sl * kSmallFd + t], __dmul_rn(kp[cx], v[cx * CC + l])));
+              }
+              out = __dadd_rn(out, sD);
+            }
+            if (decay) {
+              double sL = 0.0;
+              for (int64_t t = p.l_indptr[r]; t < p.l_indptr[r + 1]; ++t)
+                sL = __dadd_rn(sL, __dmul_rn(p.l_vals[t], v[p.l_indices[t] * CC + l]));
+              out = __dadd_rn(out, sL);
+            }
+            out = __dmul_rn(out, sc.dl);
+            if (s1 > s0 && L.inj[sl] >= 0) out = __dadd_rn(out, L.b[(par * q.slots + sl) * CC + l]);
+            double res;
+            double* dst;
+            if (stage == 1) {  // a = eD x + (phi1 F(x)) h
+              L.F[sl * CC + l] = out;
+              res = __dadd_rn(__dmul_rn(eD[r], v[r * CC + l]), __dmul_rn(__dmul_rn(eD[n + r], out), sc.h));
+              dst = L.a + r * CC + l;
+            } else {  // x = a + ((F(a) - F(x)) h) phi2
+              const double dF = __dmul_rn(__dadd_rn(out, -L.F[sl * CC + l]), sc.h);
+              res = __dadd_rn(v[r * CC + l], __dmul_rn(dF, eD[2 * n + r]));
+              dst = L.x + r * CC + l;
+            }
+            if (CS == 1) *dst = res;
+            else
+              for (int o = 0; o < CS; ++o) *cl.map_shared_rank(dst, o) = res;
+          }
+          __syncwarp();
+        }
+        if (stage == 1) cl.sync();
+      }
+    }
+    if (more) {
+      if (tid < n)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) L.fac[(nxt * 4 + f) * n + tid] = fn[f];
+      if (s1 > s0)
+        for (int sl = grp; sl < q.slots; sl += ngrp)
+          if (L.inj[sl] >= 0) L.b[(nxt * q.slots + sl) * CC + l] = injection(sl, scn);
+    }
+    cl.sync();
+    sc = scn;
+  }
+  for (int sl = grp; sl < q.slots; sl += ngrp)
+    if (mine && L.row[sl] >= 0) q.X[(size_t)L.row[sl] * p.ld + col] = L.x[L.row[sl] * CC + l];
 }
 
 // ---------------------------------------------------------------------------
@@ -2935,7 +3188,7 @@ std::vector<DBuf*> solve_buffers(pb_context* c) {
           &c->eph, &c->d_indptr, &c->d_indices, &c->d_vals, &c->d_diag, &c->adia_E, &c->pair_scale, &c->pair_bin,
           &c->xi, &c->phi_xi2, &c->pair_pg, &c->l_diag, &c->l_indptr, &c->l_indices, &c->l_vals, &c->inj_slot,
           &c->inj_G, &c->src_ptr, &c->PT, &c->zwin, &c->rs, &c->kp, &c->keep, &c->pos, &c->dest, &c->m_indptr,
-          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_scal, &c->s_finj, &c->s_coeff, &c->s_run,
+          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_scal, &c->s_finj, &c->s_coeff, &c->s_run, &c->small_order,
           &c->X, &c->A, &c->F, &c->rowf, &c->scan_tmp, &c->seg_cb, &c->seg_ce, &c->seg_lr, &c->lr_seg0, &c->lr_nseg,
           &c->seg_mb, &c->seg_me, &c->partial, &c->counter, &c->dt_indptr, &c->dt_indices, &c->dt_vals,
           &c->lt_indptr, &c->lt_indices, &c->lt_vals, &c->inj_rows, &c->src_col_d, &c->ckpt,
@@ -3385,6 +3638,90 @@ void join_hook(pb_context* c, bool& hook_pending, cudaStream_t st) {
   hook_pending = false;
 }
 
+// Whether a solve runs k_small, and how: one wave of clusters must hold all
+// columns (beyond it the bin-blocked kernels read the operator fewer times).
+// One column per cluster and the largest cluster that leaves the columns in
+// one wave, then more columns per CTA.  Measured on the light network
+// (384 rows, 12,792 entries, 1000 steps): see the launch code's figures.
+struct SmallPlan {
+  int cc = 0, cs = 0, slots = 0, cap = 0, lpr = 0;
+  size_t smem = 0;
+};
+const void* small_fn(int cc) {
+  return cc == 1 ? (const void*)k_small<1> : cc == 2 ? (const void*)k_small<2> : (const void*)k_small<4>;
+}
+SmallPlan small_plan(pb_context* c, int K, uint32_t flags, int ckpt_every) {
+  SmallPlan s;
+  if (c->small_off || c->n > kSmallRows || ckpt_every > 0 || (flags & PB_EM_CASCADE) || (K > 1 && c->batched_mode == 0) ||
+      c->fd_row_max > kSmallFd || c->small_order.p == nullptr)
+    return s;
+  const int n = (int)c->n;
+  for (int cc : {1, 2, 4})
+    for (int cs : {8, 4, 2, 1}) {
+      const int clusters = (K + cc - 1) / cc, slots = (n + cs - 1) / cs;
+      if (clusters * cs > c->num_sms) continue;
+      const int cap = c->small_cap[cs == 8 ? 3 : cs == 4 ? 2 : cs == 2 ? 1 : 0];
+      const size_t smem = SmallSmem::bytes(n, slots, cap, cc);
+      if (smem > 220 * 1024) continue;  // and the scan's static storage
+      int lpr = 8;
+      while (lpr < 32 && slots * lpr * 2 <= kSmallThreads) lpr *= 2;
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = cs;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.gridDim = dim3(clusters * cs);
+      cfg.blockDim = dim3(kSmallThreads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      if (cudaFuncSetAttribute(small_fn(cc), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) continue;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, small_fn(cc), &cfg) != cudaSuccess || fit < clusters) {
+        cudaGetLastError();
+        continue;
+      }
+      s.cc = cc;
+      s.cs = cs;
+      s.slots = slots;
+      s.cap = cap;
+      s.lpr = lpr;
+      s.smem = smem;
+      return s;
+    }
+  return s;
+}
+
+// Enqueue all S steps as k_small launches (one per run of prepared steps).
+// Returns the kernel count, or -1 on a failure.
+int64_t launch_small(pb_context* c, StepParams& p, const SmallPlan& pl, int K, int64_t S, cudaStream_t st) {
+  int64_t launches = 0;
+  p.sfac = nullptr;
+  for (int64_t k = 0; k < S; k += prep_steps(c->n)) {
+    const int64_t count = std::min(prep_steps(c->n), S - k);
+    p.rf_k0 = k;
+    launch_prep(p, c->s_scal.as<StepScal>(), k, count, st);
+    const SmallArgs q{c->small_order.as<int>(), K, (int)count, pl.slots, pl.cap, pl.lpr, c->X.as<double>()};
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = pl.cs;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((K + pl.cc - 1) / pl.cc * pl.cs);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = pl.smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = pl.cc == 1   ? cudaLaunchKernelEx(&cfg, k_small<1>, p, q)
+                          : pl.cc == 2 ? cudaLaunchKernelEx(&cfg, k_small<2>, p, q)
+                                       : cudaLaunchKernelEx(&cfg, k_small<4>, p, q);
+    if (e != cudaSuccess) return -1;
+    launches += 2;
+  }
+  return launches;
+}
+
 constexpr size_t kMaxStepGraphs = 24;
 constexpr int kGraphCols = 64;  // column granularity of a captured run's grids
 
@@ -3663,6 +4000,20 @@ int pb_set_coupling(pb_context* c, int64_t n, int64_t R, const int64_t* indptr, 
   if ((rc = upload(c, c->seg_lr, slr.data(), slr.size()))) return rc;
   if ((rc = upload(c, c->lr_seg0, l0.data(), l0.size()))) return rc;
   if ((rc = upload(c, c->lr_nseg, ln.data(), ln.size()))) return rc;
+  if (n <= kSmallRows) {
+    std::vector<int32_t> order((size_t)n);
+    for (int64_t i = 0; i < n; ++i) order[i] = (int32_t)i;
+    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+      return indptr[a + 1] - indptr[a] > indptr[b + 1] - indptr[b];
+    });
+    for (int v = 0; v < 4; ++v) {
+      std::vector<int64_t> sum((size_t)1 << v, 0);
+      for (int64_t i = 0; i < n; ++i) sum[i % sum.size()] += indptr[order[i] + 1] - indptr[order[i]];
+      c->small_cap[v] = (int32_t)(*std::max_element(sum.begin(), sum.end()) + 3) / 4 * 4;
+    }
+    if ((rc = upload(c, c->small_order, order.data(), order.size()))) return rc;
+    PB_CUDA(c, cudaStreamSynchronize(c->stream));  // `order` goes out of scope
+  }
   PB_CUDA(c, cudaStreamSynchronize(c->stream));
   c->have_coupling = true;
   c->have_kernel = false;
@@ -3948,6 +4299,8 @@ int pb_set_fd_operator(pb_context* c, int64_t nnz, const int64_t* indptr, const 
   c->h_d_indptr.assign(indptr, indptr + c->n + 1);
   c->h_d_indices.assign(indices, indices + nnz);
   c->h_d_vals.assign(values, values + nnz);
+  c->fd_row_max = 0;
+  for (int64_t r = 0; r < c->n; ++r) c->fd_row_max = std::max(c->fd_row_max, indptr[r + 1] - indptr[r]);
   return build_fd_table(c);
 }
 
@@ -4390,7 +4743,7 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   if (!ms || reps < 1 || (stage != 1 && stage != 2)) return fail(c, PB_ERR_ARG, "pb_profile_stage: bad arguments");
   if (!c->have_solution) return fail(c, PB_ERR_STATE, "pb_profile_stage: run pb_solve first");
   const int K = c->last_K;
-  if (!use_blocked(c, K)) return fail(c, PB_ERR_STATE, "pb_profile_stage: the last solve did not run the bin-blocked kernels");
+  if (!use_blocked(c, K) || !c->last_blocked) return fail(c, PB_ERR_STATE, "pb_profile_stage: the last solve did not run the bin-blocked kernels");
   if (step < 0 || step >= c->last_S || c->h_nact[step] == 0) return fail(c, PB_ERR_ARG, "pb_profile_stage: step without active columns");
   int rc = set_device(c);
   if (rc) return rc;
@@ -4944,7 +5297,8 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
       if (a->out_cols[j] < 0 || a->out_cols[j] >= K) return fail(c, PB_ERR_ARG, "pb_solve: out_cols[%d] out of range", j);
   if (a->ckpt_every > 0)
     PB_CUDA(c, c->ckpt.ensure((size_t)((S + a->ckpt_every - 1) / a->ckpt_every + 1) * n * ld * sizeof(double)));
-  const bool blocked = use_blocked(c, K);
+  const SmallPlan small = small_plan(c, K, flags, a->ckpt_every);
+  const bool blocked = !small.cc && use_blocked(c, K);
   if (blocked) {
     PB_CUDA(c, c->slab_vals.ensure((size_t)W * std::max<int64_t>(c->slab_nent, 1) * sizeof(double)));
     PB_CUDA(c, c->fdbuf.ensure(sbytes));
@@ -5052,8 +5406,9 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   PB_CUDA(c, cudaEventRecord(c->ev2, st));
   if (S > 0) {
     PB_CUDA(c, c->s_run.ensure(kGraphSteps * sizeof(StepScal)));
-    const int64_t l = launch_steps(c, p, K, a->n_active, 0, S, st, a->ckpt_every > 0 ? c->ckpt.as<double>() : nullptr,
-                                   a->ckpt_every);
+    const int64_t l = small.cc ? launch_small(c, p, small, K, S, st)
+                               : launch_steps(c, p, K, a->n_active, 0, S, st,
+                                              a->ckpt_every > 0 ? c->ckpt.as<double>() : nullptr, a->ckpt_every);
     PB_CUDA(c, cudaGetLastError());
     if (l < 0) return fail(c, PB_ERR_CUDA, "pb_solve: capturing or launching a run of steps failed");
     launches += l;
@@ -5107,6 +5462,11 @@ int pb_autotune(pb_context* c, const pb_solve_args* a, int32_t reps, int32_t max
     for (int bw : {8, 4})
       for (int pre : {2, 1, 3}) cand.push_back(pb_tune_choice{bw, pre, tma, 0.0});
   int best = -1;
+  struct SmallOff {  // every candidate runs the bin-blocked kernels, whatever the solve's size
+    pb_context* c;
+    explicit SmallOff(pb_context* x) : c(x) { c->small_off = true; }
+    ~SmallOff() { c->small_off = false; }
+  } small_off(c);
   for (size_t i = 0; i < cand.size(); ++i) {
     c->band_warps = cand[i].band_warps;
     c->slab_pre = cand[i].slab_prefetch;

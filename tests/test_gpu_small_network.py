@@ -1,0 +1,44 @@
+"""Small networks: all steps of a solve in one launch (needs a B200).
+
+The light network (384 states) runs ``k_small`` for every batch that fits one
+wave of clusters: one or two columns per cluster of one to eight CTAs.  The
+batch sizes below are the edges of those choices, with columns switching on at
+different redshifts.  As for the full network's short-range batches, every bin
+must match the CPU oracle to 1e-10 of its local magnitude, and at most 1e-4 of
+the support may miss the strict per-bin 1e-10: bins at the zero crossings of
+the loss stencil's oscillations, which a relative 1e-15 of the oracle's own
+operator values moves by as much.
+"""
+
+import pytest
+
+from golden_io import local_scale_check
+from oracle import etd2_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+
+@pytest.fixture(scope="module")
+def light():
+    from workloads import light_run
+    return light_run()
+
+
+@pytest.mark.parametrize("K", [2, 17, 19, 38, 75, 149, 297])
+def test_small_network_batches_match_the_oracle(light, K):
+    from prince_b200 import _lib
+    from prince_b200.solvers import MultiRHSPropagationSolverETD2
+    from workloads import draw_points, point_source
+    run = light
+    srcs = [point_source(run, p) for p in draw_points(run, K, seed=K, z_range=(0.01, 0.06))]
+    m = MultiRHSPropagationSolverETD2(initial_z=0.05, final_z=0.0, prince_run=run, K=K)
+    for k, s in enumerate(srcs):
+        m[k].add_source_class(s)
+    m.solve(dz=1e-3)
+    # up to two columns per CTA fit one wave of 148; beyond that the bin-blocked kernels run
+    assert m._dev.ctx.info(_lib.PB_INFO_LAST_BLOCKED) == (1 if K > 2 * 148 else 0)
+    ref = O.OracleSolver(run, 0.05, 0.0, K=K, exp="cr").solve([[s] for s in srcs], dz=1e-3)
+    worst, above, total = local_scale_check(m.state, ref, [s.sl for s in run.spec_man.species_refs], tol=TOL)
+    assert worst <= TOL, (worst, above, total)
+    assert above <= 1e-4 * total, (above, total)
