@@ -186,7 +186,7 @@ struct pb_context {
   size_t slabT_smem = 0, bandT_smem = 0;
   // small networks (k_small)
   DBuf small_order;                 // rows by coupling entries, longest first
-  int32_t small_cap[4] = {0, 0, 0, 0};  // coupling entries of a CTA for clusters of 1, 2, 4, 8
+  std::vector<int32_t> small_len;   // their coupling entries
   int64_t fd_row_max = 0;           // off-diagonal FD entries of a row (at most)
   bool small_off = false;           // the tuner measures the bin-blocked kernels
   int32_t batched_mode = 1;         // 0: general row kernels; 1: bin-blocked kernels when the layout allows
@@ -1167,31 +1167,35 @@ __global__ void __launch_bounds__(256) k_step_multi(StepParams p) {
 // the stage.  Columns are independent, so nothing else is exchanged: a step
 // costs two barriers instead of two to eight launches of 4 to 25 us each.  A
 // group of LPR lanes sums a row (entries j, j + LPR, ..., then a butterfly),
-// and its first CC lanes apply the stage update; the losses' terms add in CSR
-// order.  Bound by the shared-memory wavefronts of the entries (about 5 per 32
-// entries: value, index, gathered state) and the two barriers.
+// and its first CC lanes apply the stage update; the losses' terms, a lane
+// each, add in CSR order.  Bound by latency: the chain of shared loads and
+// FP64 operations of a row and the two cluster barriers.  The light network
+// (384 rows, 12,792 entries), 1000 steps of one column: 12.6 / 9.0 / 6.2 /
+// 5.2 ms with clusters of 1 / 2 / 4 / 8 (52 ms with a launch per stage), hence
+// the largest cluster that leaves all columns in one wave; 4.1 ms with the
+// entries in warp blocks, four loads of a row in flight and 128 registers (of
+// a step's 9,300 clocks the two barriers take 3,500, the row sums 2,900).
 // ---------------------------------------------------------------------------
 constexpr int kSmallRows = 1024;    // rows (one thread each loads the next step's factors)
-constexpr int kSmallThreads = 1024;
+constexpr int kSmallLanes = 8;      // lanes per row
 constexpr int kSmallFd = 4;         // off-diagonal stencil entries per row
 
 struct SmallArgs {
   const int* order;   // rows by coupling entries, longest first
   int K;              // columns
   int count;          // steps, from p.sc and p.rf
-  int slots;          // rows of a CTA (at most)
-  int cap;            // coupling entries of a CTA (at most)
-  int lpr;            // lanes per row
+  int slots;          // rows of a CTA, padded to whole warps
+  int cap;            // entry places of a CTA (at most)
   double* X;
 };
 
 struct SmallSmem {
   double *x, *a, *fac, *F, *b, *dval, *vals;
-  int *row, *inj, *beg, *len, *src;
+  int *row, *inj, *beg, *len, *src, *it;  // beg, it: of the warp's rows; src: the row's first entry in M_off
   unsigned short *dcol, *idx;
   __host__ __device__ static size_t bytes(int n, int slots, int cap, int cc) {
     return ((size_t)n * (2 * cc + 8) + (size_t)slots * (3 * cc + 4) + cap) * sizeof(double) +
-           ((size_t)4 * slots) * sizeof(int) + ((size_t)slots * kSmallFd + cap) * sizeof(unsigned short) + 16;
+           ((size_t)6 * slots) * sizeof(int) + ((size_t)slots * kSmallFd + cap) * sizeof(unsigned short) + 16;
   }
   __device__ SmallSmem(double* base, int n, int slots, int cap, int cc) {
     x = base;
@@ -1205,19 +1209,22 @@ struct SmallSmem {
     inj = row + slots;
     beg = inj + slots;
     len = beg + slots;
-    dcol = reinterpret_cast<unsigned short*>(len + slots);
+    src = len + slots;
+    it = src + slots;
+    dcol = reinterpret_cast<unsigned short*>(it + slots);
     idx = dcol + slots * kSmallFd;
   }
 };
 
-template <int CC>
-__global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallArgs q) {
+template <int CC, int T>
+__global__ void __launch_bounds__(T, 1) k_small(StepParams p, SmallArgs q) {
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) double sm[];
-  __shared__ typename cub::BlockScan<int, kSmallThreads>::TempStorage scan;
+  __shared__ int warp_sum[32];
   cg::cluster_group cl = cg::this_cluster();
   const int CS = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int n = (int)p.n, tid = threadIdx.x, lpr = q.lpr;
+  constexpr int lpr = kSmallLanes, rpw = 32 / lpr;
+  const int n = (int)p.n, tid = threadIdx.x;
   const int c0 = (blockIdx.x / CS) * CC;
   SmallSmem L(sm, n, q.slots, q.cap, CC);
   const bool photohad = (p.flags & PB_PHOTOHAD) != 0, kap = (p.flags & PB_PARTIAL_DIFF) != 0;
@@ -1225,17 +1232,38 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
 
   // ---- rows, pattern, stencil, states -----------------------------------
   int r0 = -1, l0 = 0;
+  // The 32 / lpr rows of a warp's pass share an entry block: place (t, lane) is
+  // entry lane % lpr + t lpr of the lane's row, zero past its end, so that the
+  // lanes read consecutive places (rows stored one after another met four-way
+  // bank conflicts).
+  int m0 = 0;
   if (tid < q.slots) {
     const int i = tid * CS + rank;
     r0 = i < n ? q.order[i] : -1;
-    l0 = (r0 >= 0 && photohad) ? (int)(p.m_indptr[r0 + 1] - p.m_indptr[r0]) : 0;
+    if (r0 >= 0 && photohad) {
+      m0 = (int)p.m_indptr[r0];
+      l0 = (int)p.m_indptr[r0 + 1] - m0;
+    }
   }
-  int b0;
-  cub::BlockScan<int, kSmallThreads>(scan).ExclusiveSum(l0, b0);
+  int it = (l0 + lpr - 1) / lpr;  // passes of the warp's longest row
+#pragma unroll
+  for (int o = 1; o < rpw; o <<= 1) it = max(it, __shfl_xor_sync(0xffffffffu, it, o));
+  int b0 = tid % rpw == 0 ? 32 * it : 0;
+  const int own = b0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, b0, o);
+    if ((tid & 31) >= o) b0 += t;
+  }
+  if ((tid & 31) == 31) warp_sum[tid >> 5] = b0;
+  __syncthreads();
+  b0 -= own;
+  for (int o = 0; o < (tid >> 5); ++o) b0 += warp_sum[o];
   if (tid < q.slots) {
     L.row[tid] = r0;
     L.len[tid] = l0;
+    L.it[tid] = it;
     L.beg[tid] = b0;
+    L.src[tid] = m0;
     L.inj[tid] = (inj && r0 >= 0) ? p.inj_slot[r0] : -1;
     for (int t = 0; t < kSmallFd; ++t) {
       L.dval[tid * kSmallFd + t] = 0.0;
@@ -1249,7 +1277,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
       }
     }
   }
-  for (int t = tid; t < n * CC; t += kSmallThreads) {
+  for (int t = tid; t < n * CC; t += blockDim.x) {
     const int r = t / CC, c = c0 + t % CC;
     L.x[t] = c < q.K ? q.X[(size_t)r * p.ld + c] : 0.0;
     L.a[t] = 0.0;
@@ -1259,11 +1287,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
   if (tid < n && k < q.count)
     for (int f = 0; f < 4; ++f) L.fac[((k & 1) * 4 + f) * n + tid] = p.rf[((size_t)k * 4 + f) * n + tid];
   __syncthreads();
-  const int grp = tid / lpr, ngrp = kSmallThreads / lpr, l = tid % lpr;
+  // slots is a multiple of rpw and ngrp too: a warp's lanes share every trip count
+  const int grp = tid / lpr, ngrp = blockDim.x / lpr, l = tid % lpr, lane = tid & 31;
   for (int sl = grp; sl < q.slots; sl += ngrp) {
-    const int len = L.len[sl], beg = L.beg[sl];
-    const int64_t m0 = len ? p.m_indptr[L.row[sl]] : 0;
-    for (int j = l; j < len; j += lpr) L.idx[beg + j] = (unsigned short)p.m_indices[m0 + j];
+    const int len = L.len[sl], it = L.it[sl], src = L.src[sl];
+    unsigned short* id = L.idx + L.beg[sl - grp % rpw] + lane;
+    for (int t = 0; t < it; ++t)
+      id[32 * t] = (unsigned short)(l + t * lpr < len ? p.m_indices[src + l + t * lpr] : max(L.row[sl], 0));
   }
   // this lane's column of the injection and its sources
   const int col = c0 + l;
@@ -1304,9 +1334,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
         w = sc.w;
         const double* mv = p.m_vals + (size_t)w * p.m_wstride;
         for (int sl = grp; sl < q.slots; sl += ngrp) {
-          const int len = L.len[sl], beg = L.beg[sl];
-          const int64_t m0 = len ? p.m_indptr[L.row[sl]] : 0;
-          for (int j = l; j < len; j += lpr) L.vals[beg + j] = mv[m0 + j];
+          const int len = L.len[sl], it = L.it[sl];
+          const double* m = mv + L.src[sl] + l;
+          double* to = L.vals + L.beg[sl - grp % rpw] + lane;
+#pragma unroll 8
+          for (int t = 0; t < it; ++t) to[32 * t] = l + t * lpr < len ? m[t * lpr] : 0.0;
         }
       }
       const bool on = mine && col < sc.ncols;
@@ -1317,49 +1349,68 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
         const double* v = stage == 1 ? L.x : L.a;
         for (int sb = 0; sb < q.slots; sb += ngrp) {  // the same trip count in every lane of a warp
           const int sl = sb + grp;
-          const bool have = sl < q.slots && L.row[sl] >= 0;
-          const int len = have ? L.len[sl] : 0, beg = have ? L.beg[sl] : 0;
-          double acc[CC], acc2[CC];
+          if (sl >= q.slots) break;  // the whole warp
+          const bool have = L.row[sl] >= 0;
+          const int it = L.it[sl], beg = L.beg[sl - grp % rpw] + lane;
+          // the row's loss terms, a lane each (lanes 0 .. kSmallFd - 1)
+          double fd[CC];
 #pragma unroll
-          for (int c = 0; c < CC; ++c) acc[c] = acc2[c] = 0.0;
-          int j = l;
-          for (; j + lpr < len; j += 2 * lpr) {
-            const double m0 = L.vals[beg + j], m1 = L.vals[beg + j + lpr];
-            const double* v0 = v + L.idx[beg + j] * CC;
-            const double* v1 = v + L.idx[beg + j + lpr] * CC;
+          for (int c = 0; c < CC; ++c) fd[c] = 0.0;
+          const int dc = (have && l < kSmallFd) ? L.dcol[sl * kSmallFd + l] : 0xffff;
+          if (dc != 0xffff) {
+            const double dv = L.dval[sl * kSmallFd + l], kk = kp[dc];
+#pragma unroll
+            for (int c = 0; c < CC; ++c) fd[c] = __dmul_rn(dv, __dmul_rn(kk, v[dc * CC + c]));
+          }
+          double acc[CC];
+#pragma unroll
+          for (int c = 0; c < CC; ++c) acc[c] = 0.0;
+          const double* va = L.vals + beg;
+          const unsigned short* id = L.idx + beg;
+          int t = 0;
+          for (; t + 4 <= it; t += 4) {  // four independent load chains at a time
+            int ix[4];
+            double m[4], x[4][CC];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              ix[u] = id[32 * (t + u)] * CC;
+              m[u] = va[32 * (t + u)];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+              for (int c = 0; c < CC; ++c) x[u][c] = v[ix[u] + c];
 #pragma unroll
             for (int c = 0; c < CC; ++c) {
-              acc[c] = __fma_rn(m0, v0[c], acc[c]);
-              acc2[c] = __fma_rn(m1, v1[c], acc2[c]);
+              const double s0 = __fma_rn(m[1], x[1][c], __dmul_rn(m[0], x[0][c]));
+              const double s1 = __fma_rn(m[3], x[3][c], __dmul_rn(m[2], x[2][c]));
+              acc[c] = __dadd_rn(acc[c], __dadd_rn(s0, s1));
             }
           }
-          if (j < len) {
-            const double m0 = L.vals[beg + j];
-            const double* v0 = v + L.idx[beg + j] * CC;
+          for (; t < it; ++t) {
+            const double m = va[32 * t];
+            const double* vj = v + id[32 * t] * CC;
 #pragma unroll
-            for (int c = 0; c < CC; ++c) acc[c] = __fma_rn(m0, v0[c], acc[c]);
+            for (int c = 0; c < CC; ++c) acc[c] = __fma_rn(m, vj[c], acc[c]);
           }
           __syncwarp();
-          double sM = 0.0;
+          double sM = 0.0, sD = 0.0;
 #pragma unroll
           for (int c = 0; c < CC; ++c) {
-            double t = __dadd_rn(acc[c], acc2[c]);
+            double t = acc[c], d = __shfl_sync(0xffffffffu, fd[c], 0, lpr);
+#pragma unroll
+            for (int o = 1; o < kSmallFd; ++o) d = __dadd_rn(d, __shfl_sync(0xffffffffu, fd[c], o, lpr));  // CSR order
+#pragma unroll
             for (int o = lpr >> 1; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
-            if (l == c) sM = t;
+            if (l == c) {
+              sM = t;
+              sD = d;
+            }
           }
           if (have && on) {
             const int r = L.row[sl];
             double out = sM;
-            if (kap) {
-              double sD = 0.0;
-#pragma unroll
-              for (int t = 0; t < kSmallFd; ++t) {
-                const int cx = L.dcol[sl * kSmallFd + t];
-                if (cx != 0xffff)
-                  sD = __dadd_rn(sD, __dmul_rn(L.dval[sl * kSmallFd + t], __dmul_rn(kp[cx], v[cx * CC + l])));
-              }
-              out = __dadd_rn(out, sD);
-            }
+            if (kap) out = __dadd_rn(out, sD);
             if (decay) {
               double sL = 0.0;
               for (int64_t t = p.l_indptr[r]; t < p.l_indptr[r + 1]; ++t)
@@ -1379,9 +1430,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(StepParams p, SmallA
               res = __dadd_rn(v[r * CC + l], __dmul_rn(dF, eD[2 * n + r]));
               dst = L.x + r * CC + l;
             }
-            if (CS == 1) *dst = res;
-            else
-              for (int o = 0; o < CS; ++o) *cl.map_shared_rank(dst, o) = res;
+            if (CS == 1) {
+              *dst = res;
+            } else {
+#pragma unroll
+              for (int o = 0; o < 8; ++o)
+                if (o < CS) *cl.map_shared_rank(dst, o) = res;
+            }
           }
           __syncwarp();
         }
@@ -3641,14 +3696,18 @@ void join_hook(pb_context* c, bool& hook_pending, cudaStream_t st) {
 // Whether a solve runs k_small, and how: one wave of clusters must hold all
 // columns (beyond it the bin-blocked kernels read the operator fewer times).
 // One column per cluster and the largest cluster that leaves the columns in
-// one wave, then more columns per CTA.  Measured on the light network
-// (384 rows, 12,792 entries, 1000 steps): see the launch code's figures.
+// one wave, then more columns per CTA.
 struct SmallPlan {
-  int cc = 0, cs = 0, slots = 0, cap = 0, lpr = 0;
+  int cc = 0, cs = 0, slots = 0, cap = 0;
+  int threads = 0;
+  bool wide = false;
   size_t smem = 0;
 };
-const void* small_fn(int cc) {
-  return cc == 1 ? (const void*)k_small<1> : cc == 2 ? (const void*)k_small<2> : (const void*)k_small<4>;
+using SmallKernel = void (*)(StepParams, SmallArgs);
+// Up to 512 rows in CTAs of 512 threads (128 registers: at 64 the entry loop's pointers spill).
+SmallKernel small_fn(int cc, bool wide) {
+  if (wide) return cc == 1 ? k_small<1, 1024> : cc == 2 ? k_small<2, 1024> : k_small<4, 1024>;
+  return cc == 1 ? k_small<1, 512> : cc == 2 ? k_small<2, 512> : k_small<4, 512>;
 }
 SmallPlan small_plan(pb_context* c, int K, uint32_t flags, int ckpt_every) {
   SmallPlan s;
@@ -3658,26 +3717,36 @@ SmallPlan small_plan(pb_context* c, int K, uint32_t flags, int ckpt_every) {
   const int n = (int)c->n;
   for (int cc : {1, 2, 4})
     for (int cs : {8, 4, 2, 1}) {
-      const int clusters = (K + cc - 1) / cc, slots = (n + cs - 1) / cs;
+      const int clusters = (K + cc - 1) / cc;
+      int slots = (n + cs - 1) / cs;
       if (clusters * cs > c->num_sms) continue;
-      const int cap = c->small_cap[cs == 8 ? 3 : cs == 4 ? 2 : cs == 2 ? 1 : 0];
+      const int lpr = kSmallLanes, rpw = 32 / lpr;
+      slots = (slots + rpw - 1) / rpw * rpw;
+      int cap = 0;  // the largest CTA's entry places
+      for (int r = 0; r < cs; ++r) {
+        int sum = 0;
+        for (int sl = 0; sl < slots; sl += rpw)  // rows by length: the warp's first row is its longest
+          if (sl * cs + r < n) sum += 32 * ((c->small_len[sl * cs + r] + lpr - 1) / lpr);
+        cap = std::max(cap, sum);
+      }
       const size_t smem = SmallSmem::bytes(n, slots, cap, cc);
-      if (smem > 220 * 1024) continue;  // and the scan's static storage
-      int lpr = 8;
-      while (lpr < 32 && slots * lpr * 2 <= kSmallThreads) lpr *= 2;
+      if (smem > 224 * 1024) continue;
       cudaLaunchConfig_t cfg{};
       cudaLaunchAttribute at{};
       at.id = cudaLaunchAttributeClusterDimension;
       at.val.clusterDim.x = cs;
       at.val.clusterDim.y = at.val.clusterDim.z = 1;
       cfg.gridDim = dim3(clusters * cs);
-      cfg.blockDim = dim3(kSmallThreads);
+      const bool wide = n > 512;
+      const SmallKernel fn = small_fn(cc, wide);
+      const int threads = std::min(wide ? 1024 : 512, (std::max(slots * lpr, n) + 31) / 32 * 32);
+      cfg.blockDim = dim3(threads);
       cfg.dynamicSmemBytes = smem;
       cfg.attrs = &at;
       cfg.numAttrs = 1;
-      if (cudaFuncSetAttribute(small_fn(cc), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) continue;
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024) != cudaSuccess) continue;
       int fit = 0;
-      if (cudaOccupancyMaxActiveClusters(&fit, small_fn(cc), &cfg) != cudaSuccess || fit < clusters) {
+      if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess || fit < clusters) {
         cudaGetLastError();
         continue;
       }
@@ -3685,7 +3754,8 @@ SmallPlan small_plan(pb_context* c, int K, uint32_t flags, int ckpt_every) {
       s.cs = cs;
       s.slots = slots;
       s.cap = cap;
-      s.lpr = lpr;
+      s.threads = threads;
+      s.wide = wide;
       s.smem = smem;
       return s;
     }
@@ -3701,22 +3771,19 @@ int64_t launch_small(pb_context* c, StepParams& p, const SmallPlan& pl, int K, i
     const int64_t count = std::min(prep_steps(c->n), S - k);
     p.rf_k0 = k;
     launch_prep(p, c->s_scal.as<StepScal>(), k, count, st);
-    const SmallArgs q{c->small_order.as<int>(), K, (int)count, pl.slots, pl.cap, pl.lpr, c->X.as<double>()};
+    const SmallArgs q{c->small_order.as<int>(), K, (int)count, pl.slots, pl.cap, c->X.as<double>()};
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = pl.cs;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3((K + pl.cc - 1) / pl.cc * pl.cs);
-    cfg.blockDim = dim3(kSmallThreads);
+    cfg.blockDim = dim3(pl.threads);
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    const cudaError_t e = pl.cc == 1   ? cudaLaunchKernelEx(&cfg, k_small<1>, p, q)
-                          : pl.cc == 2 ? cudaLaunchKernelEx(&cfg, k_small<2>, p, q)
-                                       : cudaLaunchKernelEx(&cfg, k_small<4>, p, q);
-    if (e != cudaSuccess) return -1;
+    if (cudaLaunchKernelEx(&cfg, small_fn(pl.cc, pl.wide), p, q) != cudaSuccess) return -1;
     launches += 2;
   }
   return launches;
@@ -4006,11 +4073,8 @@ int pb_set_coupling(pb_context* c, int64_t n, int64_t R, const int64_t* indptr, 
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
       return indptr[a + 1] - indptr[a] > indptr[b + 1] - indptr[b];
     });
-    for (int v = 0; v < 4; ++v) {
-      std::vector<int64_t> sum((size_t)1 << v, 0);
-      for (int64_t i = 0; i < n; ++i) sum[i % sum.size()] += indptr[order[i] + 1] - indptr[order[i]];
-      c->small_cap[v] = (int32_t)(*std::max_element(sum.begin(), sum.end()) + 3) / 4 * 4;
-    }
+    c->small_len.resize((size_t)n);
+    for (int64_t i = 0; i < n; ++i) c->small_len[i] = (int32_t)(indptr[order[i] + 1] - indptr[order[i]]);
     if ((rc = upload(c, c->small_order, order.data(), order.size()))) return rc;
     PB_CUDA(c, cudaStreamSynchronize(c->stream));  // `order` goes out of scope
   }
