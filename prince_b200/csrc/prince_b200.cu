@@ -112,6 +112,8 @@ struct pb_context {
   DBuf cpl_indptr, cpl_indices, cpl_row, cpl_is_diag;
   std::vector<int32_t> h_short_rows, h_long_rows;
   DBuf short_rows, long_rows;
+  DBuf plain_rows;                  // all rows, in k_step_plain's order
+  int32_t n_plong = 0, n_pmid = 0;  // its CTA rows and warp rows
   // long-row segments over the coupling entries
   int32_t n_seg = 0;
   DBuf seg_cb, seg_ce, seg_lr, lr_seg0, lr_nseg, seg_mb, seg_me, partial, counter;
@@ -707,7 +709,9 @@ struct StepParams {
   double* a;          // stage 1 writes, stage 2 reads
   double* f;          // F(x): stage 1 writes, stage 2 reads
   double* xout;       // stage 2 writes
-  const int* rows;    // short rows
+  // one column: all rows, those of k_step_plain's CTAs, then of its warps, then the rest
+  int n_prows, n_plong, n_pmid, nb_pmid;
+  const int* rows;    // short rows (one column: all rows in k_step_plain's order)
   int nrows;
   int nsb;            // blocks of the launch that work on short rows
   // long rows: segments of at most kSegLen coupling entries
@@ -1059,44 +1063,152 @@ __device__ __forceinline__ bool last_of_row(const StepParams& p, int lr, int til
   return last;
 }
 
-// Single column.  Blocks [0, nsb): a thread per short row, summing the row in
-// CSR order without contraction (as the host CSR product does).  Blocks
-// [nsb, ...): a warp per long-row segment.
+// Single column.  Rows by their coupling entries: a CTA per row above
+// kPlainLong (the redistributed nucleons: up to 14,600 entries), a warp per row
+// above kPlainMid (the light fragments: 329), four lanes per shorter row, in
+// that order of blocks, so that the long rows start first and all blocks fit
+// about one wave.  A row's loss terms are a lane each (added in CSR order), and
+// everything the row's update reads is loaded ahead of the sum.  The bound is
+// the operator's 32 MB per stage from L2 and the latency of a row's dependent
+// loads.  Measured at the A <= 56 network per stage: a thread per short row and
+// 256-entry segments of the long rows with a ticket 16 / 21 us; eight lanes per
+// row with those segments 19 us (2,200 blocks in four waves); this split 9.7 us.
+// ---------------------------------------------------------------------------
+constexpr int kPlainLanes = 4;
+constexpr int kPlainThreads = 512;
+constexpr int kPlainLong = 1024, kPlainMid = 64;
+
+// The (CSR-ordered) loss sum of row r: D_off (kappa v), lanes of a group of kPlainLanes.
+__device__ __forceinline__ double plain_fd(const StepParams& p, int64_t r, bool have, int l, const double* __restrict__ v) {
+  double sD = 0.0;
+  const int64_t j0 = have ? p.d_indptr[r] : 0, j1 = have ? p.d_indptr[r + 1] : 0;
+  int64_t longest = j1 - j0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  for (int64_t b = 0; b < longest; b += kPlainLanes) {
+    double t = 0.0;
+    const int64_t j = j0 + b + l;
+    if (j < j1) {
+      const int c = p.d_indices[j];
+      t = __dmul_rn(p.d_vals[j], __dmul_rn(p.kap[c], v[c]));
+    }
+    const int cnt = (int)min((int64_t)kPlainLanes, longest - b);
+    for (int q = 0; q < cnt; ++q) sD = __dadd_rn(sD, __shfl_sync(0xffffffffu, t, q, kPlainLanes));
+  }
+  return sD;
+}
+
+// The stage update of row r from its coupling sum and loss sum (one lane).
 template <int STAGE>
-__global__ void __launch_bounds__(256) k_step_plain(StepParams p) {
+__device__ __forceinline__ void plain_update(const StepParams& p, const StepScalars& s, int64_t r, double sM, double sD,
+                                             double fa, double own, double fx) {
+  double out = sM;
+  if (s.kap) out = __dadd_rn(out, sD);
+  if (s.decay) {
+    double sL = 0.0;
+    for (int64_t j = p.l_indptr[r]; j < p.l_indptr[r + 1]; ++j)
+      sL = __dadd_rn(sL, __dmul_rn(p.l_vals[j], p.src[p.l_indices[j]]));
+    out = __dadd_rn(out, sL);
+  }
+  out = __dmul_rn(out, s.dl);
+  if (s.inj) out = __dadd_rn(out, inj_at(p, s, r, 0));
+  if (p.rec_P) record<STAGE>(p, s, r, 0, sM, out);
+  if (STAGE == 1) {  // a = eD x + (phi1 F(x)) h
+    p.a[r] = __dadd_rn(__dmul_rn(fa, own), __dmul_rn(__dmul_rn(fx, out), s.h));
+    p.f[r] = out;
+  } else {  // x = a + ((F(a) - F(x)) h) phi2
+    p.xout[r] = __dadd_rn(own, __dmul_rn(__dmul_rn(__dadd_rn(out, -fx), s.h), fa));
+  }
+}
+
+// One lane's share of the coupling entries j, j + STEP, ... < j1 of a row, U load chains in flight.
+template <int STEP, int U>
+__device__ __forceinline__ double plain_sum(const double* __restrict__ mv, const int* __restrict__ idx,
+                                            const double* __restrict__ v, int64_t j, int64_t j1) {
+  double acc = 0.0, acc1 = 0.0;
+  const int cnt = (int)(j1 - j);
+  mv += j;
+  idx += j;
+  for (int b = 0; b < cnt; b += U * STEP) {
+    int c[U];
+    double m[U], x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = b + u * STEP < cnt;
+      c[u] = in ? idx[b + u * STEP] : -1;
+      m[u] = in ? mv[b + u * STEP] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = c[u] >= 0 ? v[c[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; u += 2) {
+      acc = __fma_rn(m[u], x[u], acc);
+      acc1 = __fma_rn(m[u + 1], x[u + 1], acc1);
+    }
+  }
+  return __dadd_rn(acc, acc1);
+}
+
+template <int STAGE>
+__global__ void __launch_bounds__(kPlainThreads, 2) k_step_plain(StepParams p) {
+  __shared__ double red[kPlainThreads / 32];
   const StepScalars s = load_scalars(p, p.sc);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double* __restrict__ v = p.src;
   const double* __restrict__ mv = p.m_vals + (size_t)s.w * p.m_wstride;
-  if ((int)blockIdx.x < p.nsb) {
-    const int64_t ri = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (ri >= p.nrows) return;
-    const int64_t r = p.rows[ri];
-    double acc = 0.0;
-    if (s.photohad) {
-      const int64_t j1 = p.m_indptr[r + 1];
-#pragma unroll 4
-      for (int64_t j = p.m_indptr[r]; j < j1; ++j) acc = __dadd_rn(acc, __dmul_rn(mv[j], v[p.m_indices[j]]));
-    }
-    row_epilogue<STAGE>(p, s, r, 0, acc);
+  // own inputs of the update: stage 1 eD, x, phi1; stage 2 phi2, a, F(x)
+  auto inputs = [&](int64_t r, double& fa, double& own, double& fx) {
+    fa = STAGE == 1 ? p.eD[r] : p.phi2[r];
+    own = v[r];
+    fx = STAGE == 1 ? p.phi1[r] : p.f[r];
+  };
+  double fa = 0.0, own = 0.0, fx = 0.0, acc = 0.0;
+  if ((int)blockIdx.x < p.n_plong) {  // a CTA per row
+    const int64_t r = p.rows[blockIdx.x];
+    if (threadIdx.x == 0) inputs(r, fa, own, fx);
+    if (s.photohad) acc = plain_sum<kPlainThreads, 8>(mv, p.m_indices, v, p.m_indptr[r] + threadIdx.x, p.m_indptr[r + 1]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane == 0) red[wid] = acc;
+    double sD = 0.0;
+    if (wid == 0 && s.kap) sD = plain_fd(p, r, true, lane & (kPlainLanes - 1), v);
+    __syncthreads();
+    if (wid != 0) return;
+    acc = lane < kPlainThreads / 32 ? red[lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane == 0) plain_update<STAGE>(p, s, r, acc, sD, fa, own, fx);
     return;
   }
-  const int seg = (blockIdx.x - p.nsb) * (blockDim.x >> 5) + wid;
-  if (seg >= p.nseg) return;
-  double acc = 0.0;
-  if (s.photohad)
-    for (int64_t j = p.seg_mb[seg] + lane; j < p.seg_me[seg]; j += 32) acc += mv[j] * v[p.m_indices[j]];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) p.partial[seg] = acc;
-  const int lr = p.seg_lr[seg];
-  if (!last_of_row(p, lr, 0, lane)) return;
-  if (lane == 0) {
-    const int s0 = p.lr_seg0[lr], ns = p.lr_nseg[lr];
-    double t = 0.0;
-    for (int q = 0; q < ns; ++q) t += __ldcg(p.partial + s0 + q);
-    const int64_t r = p.lr_row[lr];
-    row_epilogue<STAGE>(p, s, r, 0, t);
+  if ((int)blockIdx.x < p.n_plong + p.nb_pmid) {  // a warp per row
+    const int ri = p.n_plong + ((int)blockIdx.x - p.n_plong) * (kPlainThreads / 32) + wid;
+    if (ri >= p.n_plong + p.n_pmid) return;
+    const int64_t r = p.rows[ri];
+    if (lane == 0) inputs(r, fa, own, fx);
+    if (s.photohad) acc = plain_sum<32, 8>(mv, p.m_indices, v, p.m_indptr[r] + lane, p.m_indptr[r + 1]);
+    const double sD = s.kap ? plain_fd(p, r, true, lane & (kPlainLanes - 1), v) : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane == 0) plain_update<STAGE>(p, s, r, acc, sD, fa, own, fx);
+    return;
   }
+  const int l = lane & (kPlainLanes - 1);
+  const int64_t ri = p.n_plong + p.n_pmid +
+                     ((int64_t)((int)blockIdx.x - p.n_plong - p.nb_pmid) * kPlainThreads + threadIdx.x) / kPlainLanes;
+  const bool have = ri < p.n_prows;
+  const int64_t r = have ? p.rows[ri] : 0;
+  if (have && l == 0) inputs(r, fa, own, fx);
+  if (s.photohad && have) acc = plain_sum<kPlainLanes, 4>(mv, p.m_indices, v, p.m_indptr[r] + l, p.m_indptr[r + 1]);
+  const double sD = s.kap ? plain_fd(p, r, have, l, v) : 0.0;
+#pragma unroll
+  for (int o = kPlainLanes >> 1; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+  if (have && l == 0) plain_update<STAGE>(p, s, r, acc, sD, fa, own, fx);
+}
+
+// Blocks of a k_step_plain launch over all rows.
+inline unsigned plain_blocks(const StepParams& p) {
+  return (unsigned)(p.n_plong + p.nb_pmid) +
+         blocks_for((int64_t)p.n_prows - p.n_plong - p.n_pmid, kPlainThreads / kPlainLanes);
 }
 
 // Sum of M_off[j] * v[col_j, kk] over j in [j0, j1) for one column per lane:
@@ -3243,7 +3355,7 @@ std::vector<DBuf*> solve_buffers(pb_context* c) {
           &c->eph, &c->d_indptr, &c->d_indices, &c->d_vals, &c->d_diag, &c->adia_E, &c->pair_scale, &c->pair_bin,
           &c->xi, &c->phi_xi2, &c->pair_pg, &c->l_diag, &c->l_indptr, &c->l_indices, &c->l_vals, &c->inj_slot,
           &c->inj_G, &c->src_ptr, &c->PT, &c->zwin, &c->rs, &c->kp, &c->keep, &c->pos, &c->dest, &c->m_indptr,
-          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_scal, &c->s_finj, &c->s_coeff, &c->s_run, &c->small_order,
+          &c->m_indices, &c->m_vals, &c->m_diag, &c->s_scal, &c->s_finj, &c->s_coeff, &c->s_run, &c->small_order, &c->plain_rows,
           &c->X, &c->A, &c->F, &c->rowf, &c->scan_tmp, &c->seg_cb, &c->seg_ce, &c->seg_lr, &c->lr_seg0, &c->lr_nseg,
           &c->seg_mb, &c->seg_me, &c->partial, &c->counter, &c->dt_indptr, &c->dt_indices, &c->dt_vals,
           &c->lt_indptr, &c->lt_indices, &c->lt_vals, &c->inj_rows, &c->src_col_d, &c->ckpt,
@@ -3329,9 +3441,13 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.f = c->F.as<double>();
   p.n_steps = S;
   p.rf = c->rowf.as<double>();
-  p.rows = c->short_rows.as<int>();
+  p.rows = K == 1 ? c->plain_rows.as<int>() : c->short_rows.as<int>();
+  p.n_prows = (int)n;
+  p.n_plong = c->n_plong;
+  p.n_pmid = c->n_pmid;
+  p.nb_pmid = (int)blocks_for(p.n_pmid, kPlainThreads / 32);
   p.nrows = (int)c->h_short_rows.size();
-  p.nsb = (int)blocks_for(p.nrows, K == 1 ? 256 : 8);   // thread per row (K = 1) or warp per row
+  p.nsb = (int)blocks_for(p.nrows, 8);  // a warp per row
   p.seg_lr = c->seg_lr.as<int>();
   p.seg_mb = c->seg_mb.as<int64_t>();
   p.seg_me = c->seg_me.as<int64_t>();
@@ -3660,10 +3776,10 @@ int64_t launch_step(pb_context* c, StepParams& p, int K, const StepScal* sc, boo
       launches += stage == 1 ? launch_blocked_stage<1>(c, p, st) : launch_blocked_stage<2>(c, p, st);
       continue;
     }
-    const unsigned tiles = K == 1 ? 1u : blocks_for(p.hcols, kColTile);
-    dim3 grid((unsigned)p.nsb + blocks_for(p.nseg, 8), tiles);
+    const dim3 grid((unsigned)p.nsb + blocks_for(p.nseg, 8), blocks_for(p.hcols, kColTile));
     if (K == 1) {
-      if (stage == 1) k_step_plain<1><<<grid, 256, 0, st>>>(p); else k_step_plain<2><<<grid, 256, 0, st>>>(p);
+      if (stage == 1) k_step_plain<1><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
+      else k_step_plain<2><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
     } else {
       if (stage == 1) k_step_multi<1><<<grid, 256, 0, st>>>(p); else k_step_multi<2><<<grid, 256, 0, st>>>(p);
     }
@@ -3931,9 +4047,9 @@ void const_steps(StepParams& p, const StepScal* scal, int64_t per_prep, double* 
     set_step_factors(p, k);
     p.sc = scal + k;
     p.src = x;
-    k_step_plain<1><<<blocks_for(p.n, 256), 256, 0, st>>>(p);
+    k_step_plain<1><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
     p.src = p.a;
-    k_step_plain<2><<<blocks_for(p.n, 256), 256, 0, st>>>(p);
+    k_step_plain<2><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
   }
 }
 
@@ -4067,6 +4183,19 @@ int pb_set_coupling(pb_context* c, int64_t n, int64_t R, const int64_t* indptr, 
   if ((rc = upload(c, c->seg_lr, slr.data(), slr.size()))) return rc;
   if ((rc = upload(c, c->lr_seg0, l0.data(), l0.size()))) return rc;
   if ((rc = upload(c, c->lr_nseg, ln.data(), ln.size()))) return rc;
+  {
+    std::vector<int32_t> rows;
+    rows.reserve((size_t)n);
+    auto len = [&](int64_t i) { return indptr[i + 1] - indptr[i]; };
+    for (int64_t i = 0; i < n; ++i) if (len(i) > kPlainLong) rows.push_back((int32_t)i);
+    c->n_plong = (int32_t)rows.size();
+    std::stable_sort(rows.begin(), rows.end(), [&](int32_t a, int32_t b) { return len(a) > len(b); });
+    for (int64_t i = 0; i < n; ++i) if (len(i) > kPlainMid && len(i) <= kPlainLong) rows.push_back((int32_t)i);
+    c->n_pmid = (int32_t)rows.size() - c->n_plong;
+    for (int64_t i = 0; i < n; ++i) if (len(i) <= kPlainMid) rows.push_back((int32_t)i);
+    if ((rc = upload(c, c->plain_rows, rows.data(), rows.size()))) return rc;
+    PB_CUDA(c, cudaStreamSynchronize(c->stream));  // `rows` goes out of scope
+  }
   if (n <= kSmallRows) {
     std::vector<int32_t> order((size_t)n);
     for (int64_t i = 0; i < n; ++i) order[i] = (int32_t)i;
@@ -5982,8 +6111,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   p.a = A.as<double>();
   p.f = F.as<double>();
   p.rows = rows.as<int>();
-  p.nrows = (int)n;
-  p.nsb = (int)blocks_for(n, 256);
+  p.n_prows = (int)n;
   p.n_steps = n_steps;
   p.rf = rowf.as<double>();
   const_steps(p, hs.as<StepScal>(), prep_steps(n), X.as<double>(), st);
@@ -6073,8 +6201,7 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
   p.a = a;
   p.f = f;
   p.rows = rows;
-  p.nrows = (int)n;
-  p.nsb = (int)blocks_for(n, 256);
+  p.n_prows = (int)n;
   p.n_steps = n_steps;
   p.rf = rowf;
   const_steps(p, scal, kNaPrepSteps, state, st);

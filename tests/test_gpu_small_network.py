@@ -42,3 +42,30 @@ def test_small_network_batches_match_the_oracle(light, K):
     worst, above, total = local_scale_check(m.state, ref, [s.sl for s in run.spec_man.species_refs], tol=TOL)
     assert worst <= TOL, (worst, above, total)
     assert above <= 1e-4 * total, (above, total)
+
+
+@pytest.mark.parametrize("K", [1, 3])
+def test_small_network_with_more_than_512_rows(K):
+    """576 states (96 bins): the 1024-thread CTAs, one and three columns."""
+    from prince_b200 import photonfields as pf, synth
+    from prince_b200.run import PriNCeRun
+    from prince_b200.solvers import MultiRHSPropagationSolverETD2, UHECRPropagationSolverETD2
+    from workloads import A56_GRID, A56_PHOTON, draw_points, point_source
+    model = synth.SyntheticPhotoNuclear(synth.light_network_species(), seed=1)
+    run = PriNCeRun(model, pf.CMBPhotonSpectrum(), cosmic_ray_grid=A56_GRID, photon_grid=A56_PHOTON)
+    assert run.dim_states == 576
+    srcs = [point_source(run, p) for p in draw_points(run, K, seed=K, z_range=(0.03, 0.05))]
+    if K == 1:
+        m = UHECRPropagationSolverETD2(initial_z=0.05, final_z=0.0, prince_run=run)
+        m.add_source_class(srcs[0])
+    else:
+        m = MultiRHSPropagationSolverETD2(initial_z=0.05, final_z=0.0, prince_run=run, K=K)
+        for k, s in enumerate(srcs):
+            m[k].add_source_class(s)
+    m.solve(dz=1e-3)
+    ref = O.OracleSolver(run, 0.05, 0.0, K=K, exp="cr").solve([[s] for s in srcs], dz=1e-3).reshape(576, K)
+    worst, above, total = local_scale_check(m.state.reshape(576, K), ref, [s.sl for s in run.spec_man.species_refs],
+                                            tol=TOL)
+    assert worst <= TOL, (worst, above, total)
+    assert above <= 1e-4 * total, (above, total)
+
