@@ -499,73 +499,162 @@ __device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double
                : "d"(a), "d"(b));
 }
 
-constexpr int kFoldBM = 64, kFoldBN = 64;
+// A persistent CTA keeps the photon vectors of its (up to 128) windows in
+// shared memory and walks tiles of 32 WM kernel rows, the next tile arriving by
+// cp.async while this one is multiplied (one buffer where two do not fit); the
+// entry's slots are loaded ahead of the products.  The tile's warps are WM x
+// WN, a warp 32 entries x 16 windows, WN just covering the windows.  Bound by
+// the FP64 tensor pipe for many windows (51 GFLOP = 1.4 ms at 37 TFLOP/s for
+// the A <= 56 network's 2.67M x 96 kernel and 100 windows), by the kernel's 2 GB
+// for few.  The former 64 x 64 tiles, one load phase and one product phase per
+// CTA with an integer division per element loaded, took 7.0 ms for 100 windows (no blocks);
+// this 2.8 ms.
+constexpr int kFoldMaxWN = 8;
 
-__global__ void __launch_bounds__(256) k_fold_gemm(const double* __restrict__ K, int64_t R, int dph,
-                                                   int kpad, const double* __restrict__ PT, int W,
-                                                   const int* __restrict__ dest,
-                                                   const int* __restrict__ diag_row,
-                                                   double* __restrict__ mv, int64_t mv_stride,
-                                                   double* __restrict__ md, int64_t n,
-                                                   const int* __restrict__ band_slot,
-                                                   double* __restrict__ band, int64_t band_stride,
-                                                   const int* __restrict__ slab_slot,
-                                                   double* __restrict__ slab, int64_t slab_stride) {
-  extern __shared__ double smem[];
-  const int lda = kpad + 4;  // +4 doubles: 8-row fragments spread over all banks
-  double* As = smem;
-  double* Bs = smem + kFoldBM * lda;
-  const int64_t r0 = (int64_t)blockIdx.x * kFoldBM;
-  const int w0 = blockIdx.y * kFoldBN;
-  for (int i = threadIdx.x; i < kFoldBM * kpad; i += blockDim.x) {
-    int rr = i / kpad, kk = i % kpad;
-    As[rr * lda + kk] = (r0 + rr < R && kk < dph) ? K[(size_t)(r0 + rr) * dph + kk] : 0.0;
-  }
-  for (int i = threadIdx.x; i < kFoldBN * kpad; i += blockDim.x) {
-    int ww = i / kpad, kk = i % kpad;
-    Bs[ww * lda + kk] = (w0 + ww < W && kk < dph) ? PT[(size_t)(w0 + ww) * dph + kk] : 0.0;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int wm = wid & 1, wn = wid >> 1;  // warp tile: 32 entries x 16 windows
-  const int g = lane >> 2, t = lane & 3;
-  double acc[4][2][2];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-  for (int k0 = 0; k0 < kpad; k0 += 4) {
-    double af[4], bf[2];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt) af[mt] = As[(wm * 32 + mt * 8 + g) * lda + k0 + t];
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) bf[nt] = Bs[(wn * 16 + nt * 8 + g) * lda + k0 + t];
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) dmma884(acc[mt][nt][0], acc[mt][nt][1], af[mt], bf[nt]);
-  }
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {
-    const int64_t r = r0 + wm * 32 + mt * 8 + g;
-    if (r >= R) continue;
-    const int de = dest[r];
-    const int dr = diag_row[r];
-    const int bs = (band_slot && de >= 0) ? band_slot[r] : -1;
-    const int ss = (slab_slot && de >= 0) ? slab_slot[r] : -1;
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int w = w0 + wn * 16 + nt * 8 + t * 2 + i;
-        if (w >= W) continue;
-        const double v = acc[mt][nt][i];
-        if (de >= 0) mv[(size_t)w * mv_stride + de] = v;
-        if (dr >= 0) md[(size_t)w * n + dr] = v;
-        if (bs >= 0) band[(size_t)w * band_stride + bs] = v;
-        if (ss >= 0) slab[(size_t)w * slab_stride + ss] = v;
+struct FoldArgs {
+  const double* K;
+  int64_t R;
+  int dph, kpad, W;
+  const double* PT;
+  const int *dest, *diag_row;
+  double* mv;
+  int64_t mv_stride;
+  double* md;
+  int64_t n;
+  const int* band_slot;
+  double* band;
+  int64_t band_stride;
+  const int* slab_slot;
+  double* slab;
+  int64_t slab_stride;
+  int wm, wn, stages;  // warps of the tile, buffers of kernel rows
+};
+
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+__global__ void __launch_bounds__(512, 1) k_fold_gemm(FoldArgs q) {
+  extern __shared__ __align__(16) double smem[];
+  const int lda = q.kpad + 4;  // +4 doubles: 8-row fragments spread over all banks
+  const int BM = 32 * q.wm, BN = 16 * q.wn, dph = q.dph;
+  double* Bs = smem;
+  double* As = smem + BN * lda;  // [stages][BM][lda]
+  const int w0 = blockIdx.y * BN;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  for (int ww = wid; ww < BN; ww += nwarps)
+    for (int kk = lane; kk < q.kpad; kk += 32)
+      Bs[ww * lda + kk] = (w0 + ww < q.W && kk < dph) ? q.PT[(size_t)(w0 + ww) * dph + kk] : 0.0;
+  for (int rr = wid; rr < q.stages * BM; rr += nwarps)  // columns past dph stay zero
+    for (int kk = dph + lane; kk < q.kpad; kk += 32) As[rr * lda + kk] = 0.0;
+  auto load = [&](int64_t tile, int buf) {  // a warp per kernel row
+    const int64_t r0 = tile * BM;
+    for (int rr = wid; rr < BM; rr += nwarps) {
+      if (r0 + rr >= q.R) break;
+      const double* src = q.K + (size_t)(r0 + rr) * dph;
+      double* dst = As + (size_t)(buf * BM + rr) * lda;
+      if (dph & 1) {
+        for (int kk = lane; kk < dph; kk += 32) cp_async8(dst + kk, src + kk);
+      } else {
+        for (int kk = 2 * lane; kk < dph; kk += 64) cp_async16(dst + kk, src + kk);
       }
+    }
+    cp_async_commit();
+  };
+  const int wm = wid % q.wm, wn = wid / q.wm;  // warp tile: 32 entries x 16 windows
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t ntiles = (q.R + BM - 1) / BM;
+  int64_t tile = blockIdx.x;
+  if (tile < ntiles) load(tile, 0);
+  for (int it = 0; tile < ntiles; tile += gridDim.x, ++it) {
+    const int buf = q.stages == 2 ? it & 1 : 0;
+    const int64_t next = tile + gridDim.x;
+    if (q.stages == 2 && next < ntiles) {
+      load(next, buf ^ 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    int de[4], dr[4], bs[4], ss[4];
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      const int64_t r = tile * BM + wm * 32 + mt * 8 + g;
+      const bool in = r < q.R;
+      de[mt] = in ? q.dest[r] : -1;
+      dr[mt] = in ? q.diag_row[r] : -1;
+      bs[mt] = (q.band_slot && in) ? q.band_slot[r] : -1;
+      ss[mt] = (q.slab_slot && in) ? q.slab_slot[r] : -1;
+    }
+    __syncthreads();
+    const double* A = As + (size_t)(buf * BM + wm * 32 + g) * lda + t;
+    const double* B = Bs + (wn * 16 + g) * lda + t;
+    double acc[4][2][2];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll 2
+    for (int k0 = 0; k0 < q.kpad; k0 += 4) {
+      double af[4], bf[2];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) af[mt] = A[mt * 8 * lda + k0];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) bf[nt] = B[nt * 8 * lda + k0];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) dmma884(acc[mt][nt][0], acc[mt][nt][1], af[mt], bf[nt]);
+    }
+    __syncthreads();  // every warp is done with this buffer before it is refilled
+    if (q.stages == 1 && next < ntiles) load(next, 0);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int w = w0 + wn * 16 + nt * 8 + t * 2 + i;
+          if (w >= q.W) continue;
+          const double v = acc[mt][nt][i];
+          if (de[mt] >= 0) {
+            q.mv[(size_t)w * q.mv_stride + de[mt]] = v;
+            if (bs[mt] >= 0) q.band[(size_t)w * q.band_stride + bs[mt]] = v;
+            if (ss[mt] >= 0) q.slab[(size_t)w * q.slab_stride + ss[mt]] = v;
+          }
+          if (dr[mt] >= 0) q.md[(size_t)w * q.n + dr[mt]] = v;
+        }
+    }
   }
+}
+
+// The fold's tile for W windows: as many warps of rows as keep the CTA within
+// 16 warps and two buffers within the shared memory (one for a long photon axis).
+struct FoldTile {
+  int wm, wn, stages;
+  size_t smem;
+};
+FoldTile fold_tile(int dph, int W) {
+  const int lda = (dph + 3) / 4 * 4 + 4;
+  FoldTile f;
+  f.wn = std::min(kFoldMaxWN, (W + 15) / 16);
+  for (f.stages = 2; f.stages >= 1; --f.stages)
+    for (f.wm = std::min(4, 16 / f.wn); f.wm >= 1; --f.wm) {
+      f.smem = (size_t)(16 * f.wn + f.stages * 32 * f.wm) * lda * sizeof(double);
+      if (f.smem <= 227 * 1024 && (f.wm >= 2 || f.stages == 1)) return f;
+    }
+  f.stages = 1;
+  f.wm = 1;
+  f.wn = std::min(f.wn, 4);  // kMaxPhoton bins: 96 rows of 204 doubles
+  f.smem = (size_t)(16 * f.wn + 32) * lda * sizeof(double);
+  return f;
 }
 
 // ---------------------------------------------------------------------------
@@ -1596,14 +1685,6 @@ constexpr int kFdHalo = 3;          // k_fd_dense: stencil offsets within +-kFdH
 constexpr int kFdDenseW = 8;        // dense weights per bin (2 kFdHalo + 1, padded to 16 bytes)
 constexpr int kFdChunk = 12;        // k_fd_dense: bins per warp pass
 constexpr int kMaxBandGroups = 64;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // mbarrier and bulk-copy helpers of the TMA staging (CTA-local barrier, no cluster)
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -4097,7 +4178,7 @@ int pb_create(int device, pb_context** out) {
     return fail(nullptr, PB_ERR_CUDA, "stream/event creation failed");
   }
   e = cudaFuncSetAttribute(k_fold_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (kFoldBM + kFoldBN) * (kMaxPhoton + 4) * (int)sizeof(double));
+                           227 * 1024);
   if (e != cudaSuccess) {
     pb_destroy(c);
     return fail(nullptr, PB_ERR_CUDA, "cudaFuncSetAttribute(k_fold_gemm): %s", cudaGetErrorString(e));
@@ -5572,13 +5653,15 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
                                                            c->seg_me.as<int64_t>());
       ++launches;
     }
-    const int kpad = (c->dph + 3) / 4 * 4;
-    const size_t smem = (size_t)(kFoldBM + kFoldBN) * (kpad + 4) * sizeof(double);
-    k_fold_gemm<<<dim3(blocks_for(R, kFoldBM), blocks_for(W, kFoldBN)), 256, smem, st>>>(
-        c->kernel.as<double>(), R, c->dph, kpad, c->PT.as<double>(), W, dest, diag_row, c->m_vals.as<double>(),
-        mstride, c->m_diag.as<double>(), n, blocked ? c->band_slot.as<int>() : nullptr,
-        blocked ? c->band_vals.as<double>() : nullptr, c->band_stride, blocked ? c->slab_slot.as<int>() : nullptr,
-        blocked ? c->slab_vals.as<double>() : nullptr, c->slab_nent);
+    const FoldTile ft = fold_tile(c->dph, W);
+    const FoldArgs fa{c->kernel.as<double>(), R, c->dph, (c->dph + 3) / 4 * 4, W, c->PT.as<double>(), dest, diag_row,
+                      c->m_vals.as<double>(), mstride, c->m_diag.as<double>(), n,
+                      blocked ? c->band_slot.as<int>() : nullptr, blocked ? c->band_vals.as<double>() : nullptr,
+                      c->band_stride, blocked ? c->slab_slot.as<int>() : nullptr,
+                      blocked ? c->slab_vals.as<double>() : nullptr, c->slab_nent, ft.wm, ft.wn, ft.stages};
+    const int64_t ftiles = (R + 32 * ft.wm - 1) / (32 * ft.wm);
+    const unsigned fcols = blocks_for(W, 16 * ft.wn);
+    k_fold_gemm<<<dim3((unsigned)std::min<int64_t>(ftiles, c->num_sms), fcols), 32 * ft.wm * ft.wn, ft.smem, st>>>(fa);
     launches += 5;
   } else {
     PB_CUDA(c, cudaMemsetAsync(c->m_indptr.p, 0, ((size_t)n + 1) * sizeof(int64_t), st));
