@@ -165,10 +165,10 @@ struct pb_context {
   int32_t band_npairs = 0;
   DBuf band_slot, band_spec, slab_spec, band_vals, band_part;
   // bin-local rows: coupling entries in bin-major order
-  DBuf slab_rp, slab_sidx, slab_slot, slab_vals, slab_quart, slab_wrp, slab_rowslot, slab_fac;
-  int64_t slab_nslots = 0;          // quartet slots over all bins (four per quartet)  // slab_rp: quad base per bin; slab_sidx: quads
-  int64_t slab_nent = 0;            // value slots per window (4 per quad)
-  int32_t slab_maxbin = 0;          // quads of the largest bin
+  DBuf slab_kbase, slab_ebase, slab_k, slab_g, slab_wrp, slab_slot, slab_vals, slab_rowslot, slab_fac;
+  int64_t slab_nslots = 0;          // group slots over all bins (eight per group)
+  int64_t slab_nent = 0;            // entries per window (every bin's count rounded up to even)
+  int32_t slab_maxe = 0, slab_maxk = 0, slab_maxg = 0;  // of the largest bin
   size_t slab_smem = 0, band_smem = 0;
   // FD stencil per bin (same in every species block): host copy of D and the table
   std::vector<int64_t> h_d_indptr;
@@ -752,6 +752,8 @@ __global__ void k_eval_exp(const double* __restrict__ x, double* __restrict__ y,
 // launch per step (as part of the stage-2 kernels and a kernel of its own) cost
 // 5 us of latency each; a run of 16 steps of the A <= 56 network takes 15 us.
 // ---------------------------------------------------------------------------
+struct SlabK;
+struct SlabG;
 struct StepParams {
   int64_t n;
   int ld;            // leading dimension of the (n x ld) state buffers
@@ -830,16 +832,16 @@ struct StepParams {
   int nsp;                  // species blocks
   const int* slab_spec;     // species whose coupling rows are bin-local
   int n_slab_spec;
-  const int* slab_qbase;    // [d + 1] first entry quad of each bin (even)
-  const unsigned long long* slab_q;  // per quad: byte offsets of the 4 entries' mother rows in k_slab's slab, 16 bits each
-  const int4* slab_quart;   // row quartets of k_slab's warps: species 0 | 1 << 16, 2 | 3 << 16 (0xffff: none), first quad, quads per row
-  const int* slab_wrp;      // [d][kSlabWarps + 1] first quartet of each warp of a bin's CTA
-  const double* slab_vals;  // [W][slab_stride] M_off values of the quads (4 per quad, zero padding)
+  const int* slab_kbase;    // [d + 1] first k-tile of each bin
+  const int* slab_ebase;    // [d + 1] first entry of each bin (even)
+  const SlabK* slab_k;      // k-tiles of k_slab
+  const SlabG* slab_g;      // row groups
+  const int* slab_wrp;      // [d][kSlabWarps + 1] first group of each warp of a bin's CTA
+  const double* slab_vals;  // [W][slab_stride] M_off values of the bin-local entries in k-tile order
   int64_t slab_stride;
-  int slab_maxq;            // quads of the largest bin (shared-memory sizing)
-  int slab_maxp;            // row quartets of a bin
-  const int* slab_rowslot;  // [n] quartet slot of each bin-local row (-1: other rows)
-  const double* slab_fac;   // [3][slab_nslots] eD, phi1, phi2 of the bin-local rows of this step in quartet-slot order
+  int slab_maxe, slab_maxk, slab_maxg;  // entries, k-tiles and groups of the largest bin (shared-memory sizing)
+  const int* slab_rowslot;  // [n] group slot of each bin-local row (-1: other rows)
+  const double* slab_fac;   // [3][slab_nslots] eD, phi1, phi2 of the bin-local rows of this step in group-slot order
   double* sfac;             // [steps][3][slab_nslots] for the run of steps from prep_k0, or null
   int64_t prep_k0;          // first step of the run of steps of sfac and dsf
   int64_t slab_nslots;
@@ -1855,70 +1857,62 @@ __device__ __forceinline__ void record_blocked(const StepParams& p, const StepSc
   }
 }
 
-// The record inputs of one (row, column), loaded by k_slab with the row's
-// other inputs ahead of its sum: the scale derivatives, the step factors, the
-// FD term with kappa_pair and (stage 2) the stage-1 S x.
-struct RecIn {
-  double ds, d12, f0, f1, kp, sx;
-  bool on;
+// The bin-local rows of one bin as DMMA tiles.  The rows are gathered in groups
+// of eight that share many mothers; a group multiplies its 8 x 4 k-tiles, each
+// over four mother species (any four: the B rows are gathered from the slab).
+// A k-tile's entries are stored without its zeros: `mask` has bit 4 g + kk set
+// where row g couples to mother kk, and the entries follow one another from
+// `base` in the order of those bits.
+struct __align__(16) SlabK {
+  unsigned mask;
+  unsigned base;           // byte offset of the first entry from the slab's start
+  unsigned short row[4];   // of the four mothers' slab rows r: 8 r + (r mod 8), the 16-byte chunk 0 with its swizzle
 };
-// record_blocked with preloaded inputs (same arithmetic)
-template <int STAGE>
-__device__ __forceinline__ void record_pre(const StepParams& p, const StepScalars& s, int64_t r, int k, double sM,
-                                           double F, double own, double fprev, const RecIn& in) {
-  if (!in.on) return;
-  const size_t idx = (size_t)r * p.ld + k;
-  const size_t ro = (size_t)(s.step - p.rec_k0) * p.n * p.ld + idx;
-  const double h = s.h, ds = in.ds;
-  double S = s.photohad ? sM : 0.0;
-  if (s.kap && s.pair) S += in.kp;
-  S = S * s.dl * p.inv_scale;
-  if (STAGE == 1) {
-    p.rec_sx[idx] = S;
-    p.rec_P[ro] = in.f0 * h * ds * own + h * h * in.d12 * ds * F + h * in.f1 * S;
-  } else {
-    p.rec_Q[ro] = h * h * in.d12 * ds * (F - fprev) + h * in.f0 * (S - in.sx);
-  }
-}
+struct __align__(16) SlabG {
+  unsigned short sp[8];    // species of the eight rows, 0xffff: none
+  int kt0, nkt;            // k-tiles, from the bin's first; an even count
+  int pad[2];
+};
 
-// k_slab's shared memory: the state slab of one bin (nsp x 16 columns), the
-// bin's entry values (4 per quad), mother-row byte offsets (4 x 16 bits per
-// quad), the row quartets of the bin and the row factors (eD, phi1, phi2) of
-// each quartet slot.  Every block starts on a 16-byte boundary (the quad count
-// of a bin is a multiple of 4).
+// k_slab's shared memory: the state slab of one bin (nsp x 16 columns, rows of
+// 128 bytes whose eight 16-byte chunks are permuted by the row's low three
+// bits, as the TMA 128-byte swizzle does), the bin's entries, k-tiles and row
+// groups, and the row factors (eD, phi1, phi2) of each group slot.  The slab
+// starts on a 1024-byte boundary (the swizzle's period).
 constexpr int kSlabCols = 16;       // state columns of a k_slab CTA
-constexpr int kSlabRows = 4;        // rows per warp: a quarter-warp per row, two columns per lane
-constexpr int kSlabWarps = 12;      // two CTAs per SM: 24 warps of 80 registers (loads in flight per warp)
+constexpr int kSlabRows = 8;        // rows of a group (a DMMA tile's)
+constexpr int kSlabWarps = 8;       // two CTAs per SM at 128 registers
 struct SlabSmem {
-  double* slab;
+  char* slab;
   double* vals;
-  unsigned long long* sidx;
-  int4* quart;
+  SlabK* ks;
+  SlabG* grp;
   double* fac;  // [3][kSlabRows maxg]
   unsigned long long* bar;  // the TMA staging barrier
-  // species rows of the slab, padded to whole TMA boxes of at most 256 species
+  // species rows of the slab, padded to whole TMA boxes of at most 256 species (multiples of the swizzle's 8 rows)
   __host__ __device__ static int nbox(int nsp) { return (nsp + 255) / 256; }
-  __host__ __device__ static int box_rows(int nsp) { return (nsp + nbox(nsp) - 1) / nbox(nsp); }
+  __host__ __device__ static int box_rows(int nsp) { return ((nsp + nbox(nsp) - 1) / nbox(nsp) + 7) / 8 * 8; }
   __host__ __device__ static int rows(int nsp) { return nbox(nsp) * box_rows(nsp); }
-  __host__ __device__ static size_t bytes(int nsp, int maxq, int maxg) {
-    return (size_t)rows(nsp) * kSlabCols * sizeof(double) +
-           (size_t)maxq * (4 * sizeof(double) + sizeof(unsigned long long)) +
-           (size_t)maxg * (sizeof(int4) + 3 * kSlabRows * sizeof(double)) + sizeof(unsigned long long);
+  __host__ __device__ static size_t bytes(int nsp, int maxe, int maxk, int maxg) {
+    return 1024 + (size_t)rows(nsp) * kSlabCols * sizeof(double) + (size_t)maxe * sizeof(double) +
+           (size_t)maxk * sizeof(SlabK) + (size_t)maxg * (sizeof(SlabG) + 3 * kSlabRows * sizeof(double)) +
+           sizeof(unsigned long long);
   }
-  __device__ SlabSmem(double* base, int nsp, int maxq, int maxg) {
-    slab = base;
-    vals = slab + (size_t)rows(nsp) * kSlabCols;
-    sidx = reinterpret_cast<unsigned long long*>(vals + (size_t)maxq * 4);
-    quart = reinterpret_cast<int4*>(sidx + maxq);
-    fac = reinterpret_cast<double*>(quart + maxg);
+  __device__ SlabSmem(void* base, int nsp, int maxe, int maxk, int maxg) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(base);
+    slab = static_cast<char*>(base) + ((1024u - (a & 1023u)) & 1023u);
+    vals = reinterpret_cast<double*>(slab + (size_t)rows(nsp) * kSlabCols * sizeof(double));
+    ks = reinterpret_cast<SlabK*>(vals + maxe);
+    grp = reinterpret_cast<SlabG*>(ks + maxk);
+    fac = reinterpret_cast<double*>(grp + maxg);
     bar = reinterpret_cast<unsigned long long*>(fac + 3 * kSlabRows * (size_t)maxg);
   }
 };
-
-// Species of row g of a quartet descriptor (0xffff: no row).
-__device__ __forceinline__ unsigned quart_species(const int4& qd, int g) {
-  return ((unsigned)(g < 2 ? qd.x : qd.y) >> (16 * (g & 1))) & 0xffffu;
+// The 16-byte chunk c (columns 2c, 2c + 1) of slab row r.
+__device__ __forceinline__ const double2& slab_chunk(const char* slab, unsigned r, unsigned c) {
+  return *reinterpret_cast<const double2*>(slab + r * 128u + ((c ^ (r & 7u)) << 4));
 }
+
 __device__ __forceinline__ double2 dadd2(double2 a, double2 b) {
   return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
 }
@@ -1930,58 +1924,139 @@ __device__ __forceinline__ double slab_inj(const StepParams& p, int64_t step, in
   for (int q = src0 + 1; q < src1; ++q) a = __dadd_rn(a, __dmul_rn(cf[q], g[q]));
   return a;
 }
+// Four adjacent columns of a row, as two 16-byte words; the store writes the first n columns.
+__device__ __forceinline__ void load4(const double* __restrict__ src, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(src), b = *reinterpret_cast<const double2*>(src + 2);
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+__device__ __forceinline__ void store4(double* dst, const double (&v)[4], int n) {
+  if (n >= 2) *reinterpret_cast<double2*>(dst) = make_double2(v[0], v[1]);
+  else dst[0] = v[0];
+  if (n == 4) *reinterpret_cast<double2*>(dst + 2) = make_double2(v[2], v[3]);
+  else if (n == 3) dst[2] = v[2];
+}
 
-// Bin-local rows.  CTA = (bin e, 16-column tile); a warp takes four rows at
-// a time (a quartet), a quarter-warp per row, and lane j of the quarter owns
-// columns col0 + 2j and col0 + 2j + 1.  The state slab of bin e, the bin's
-// entry quads, its quartets and their row factors (written in slot order by
-// the row preparation) arrive in shared memory by asynchronous copies; a
-// warp then walks its quartets (balanced over the warps when the layout is
-// built), sums each row from shared memory (four accumulators per column, one
-// per quad position, in the row's CSR order) and applies the stage update.
-// The four rows' quads interleave, so that one 16-byte value load and one
-// offset load serve four rows without bank conflicts, and a slab load of
-// 16 bytes per lane serves two columns; a quad's offsets are loaded one quad
-// ahead.  The row's FD term (fdbuf), F(x) in stage 2 and its injection slot
-// are loaded PREF quartets ahead into registers.  REC: the adjoint's record
-// pass (P / Q sensitivities); its row and (row, column) inputs are loaded with
-// the others, a quartet less ahead.  Offsets into the (n x ld) state buffers
-// are 32-bit (n ld < 2^31, checked at launch).
+// Shared loads at 32-bit addresses.
+__device__ __forceinline__ uint4 lds_u4(unsigned a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ double2 lds_d2(unsigned a) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ double lds_d(unsigned a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+
+// The k-tiles of one row group: C (8 rows x 16 columns) += A B on the FP64
+// tensor pipe, two k-tiles at a time (a group has an even count), their
+// descriptors loaded PREF - 1 pairs ahead (past a group's end: the next bytes
+// of shared memory, unused).  n-tile 0 holds the even columns and n-tile 1 the
+// odd ones (a lane's 16-byte B load is columns 2n and 2n + 1), so lane (g, t)
+// ends with columns 4t .. 4t + 3 of row g: acc0[0], acc1[0], acc0[1], acc1[1].
+template <int PREF>
+__device__ __forceinline__ void slab_tiles(unsigned ks, int nkt, unsigned slab, int lane, double (&acc0)[2],
+                                           double (&acc1)[2]) {
+  const unsigned bit = 1u << lane, below = bit - 1u;
+  const unsigned g = lane >> 2, pick = lane & 1 ? 0x4432u : 0x4410u;
+  const bool hi = lane & 2;
+  uint4 q[PREF][2];
+#pragma unroll
+  for (int f = 0; f < PREF - 1; ++f) {
+    q[f][0] = lds_u4(ks + 32 * f);
+    q[f][1] = lds_u4(ks + 32 * f + 16);
+  }
+  for (int k = 0; k < nkt; k += 2, ks += 32) {
+    q[PREF - 1][0] = lds_u4(ks + 32 * (PREF - 1));
+    q[PREF - 1][1] = lds_u4(ks + 32 * (PREF - 1) + 16);
+    double a[2];
+    double2 x[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint4 kd = q[0][u];
+      x[u] = lds_d2(slab + ((__byte_perm(hi ? kd.w : kd.z, 0, pick) ^ g) << 4));
+      a[u] = 0.0;
+      if (kd.x & bit) a[u] = lds_d(slab + kd.y + 8 * __popc(kd.x & below));
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      dmma884(acc0[0], acc0[1], a[u], x[u].x);
+      dmma884(acc1[0], acc1[1], a[u], x[u].y);
+    }
+#pragma unroll
+    for (int f = 0; f < PREF - 1; ++f) {
+      q[f][0] = q[f + 1][0];
+      q[f][1] = q[f + 1][1];
+    }
+  }
+}
+
+// Bin-local rows.  CTA = (bin e, 16-column tile); the state slab of bin e, the
+// bin's entries, k-tiles, row groups and row factors arrive in shared memory by
+// asynchronous copies; a warp then walks its row groups (balanced over the
+// warps when the layout is built), multiplies each on the FP64 tensor pipe and
+// applies the stage update to its eight rows, a lane four adjacent columns of a
+// row.  The rows' FD term (fdbuf), F(x) in stage 2 and injection slots are
+// loaded before the group's products.
+// REC: the adjoint's record pass (P / Q sensitivities).  A mother's state
+// multiplies the zeros of the rows that do not couple to it, so a non-finite
+// state of one species reaches the other rows of its tiles too.
+//
+// Bound by HBM by bytes.  One row per quarter-warp with the entries' states
+// gathered one by one was bound by shared-memory wavefronts (28M per launch at
+// K = 512, 84 per 16-column group of 16 entries); an 8 x 4 tile reads its four
+// mothers' rows once for eight daughters: at the A <= 56 network 458 k-tiles of
+// 35% fill per bin instead of 1,476 entry quads, 8 wavefronts and 8 tensor
+// clocks each.  Measured per launch at K = 512: 165 / 170 us before, 160 / 154 us
+// now; what is left is the latency of a CTA's phases (staging, products, update)
+// at two CTAs per SM: 2 x 12 warps, three teams of eight warps sharing the
+// tables, and entries read from L2 at four CTAs per SM were slower (163 / 170,
+// 170 / 189, 202 / 218 us).
 template <int STAGE, bool REC, int PREF>
 __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
-  extern __shared__ __align__(128) double sm[];  // TMA boxes land at 128-byte boundaries
+  extern __shared__ __align__(128) double sm[];
   const int e = blockIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int g = lane >> 3, j = lane & 7;
+  const int g = lane >> 2, t4 = lane & 3;
   const int col0 = blockIdx.y * kSlabCols;
-  const int colA = col0 + 2 * j;  // this lane's columns colA, colA + 1 (< ld)
+  const int colA = col0 + 4 * t4;  // this lane's columns colA .. colA + 3 (< ld)
   const StepScalars s = load_scalars(p, p.sc);
   if (col0 >= s.ncols) return;
-  const bool actA = colA < s.ncols, actB = colA + 1 < s.ncols;
+  const int nact = min(max(s.ncols - colA, 0), 4);
   const int ld = p.ld, d = p.d;
-  SlabSmem L(sm, p.nsp, p.slab_maxq, p.slab_maxp);
-  const int qb = p.slab_qbase[e], nqb = p.slab_qbase[e + 1] - qb;
+  SlabSmem L(sm, p.nsp, p.slab_maxe, p.slab_maxk, p.slab_maxg);
+  const int kb = p.slab_kbase[e], nk = p.slab_kbase[e + 1] - kb;
+  const int eb = p.slab_ebase[e], ne = p.slab_ebase[e + 1] - eb;
   const int gb0 = p.slab_wrp[e * (kSlabWarps + 1)], ngb = p.slab_wrp[e * (kSlabWarps + 1) + kSlabWarps] - gb0;
-  const int fs = kSlabRows * p.slab_maxp;  // stride of the three row-factor arrays
+  const int fs = kSlabRows * p.slab_maxg;  // stride of the three row-factor arrays
   unsigned long long* stage_bar = L.bar;
-  const double* mv = p.slab_vals + (size_t)s.w * p.slab_stride + (size_t)qb * 4;
+  const double* mv = p.slab_vals + (size_t)s.w * p.slab_stride + eb;
   const double* fc = p.slab_fac + (size_t)kSlabRows * gb0;
   if (p.tmap_src) {  // TMA: the slab as tensor boxes, the rest as bulk copies, one barrier
     if (threadIdx.x == 0) mbar_init(stage_bar, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
       const int nb = SlabSmem::nbox(p.nsp), br = SlabSmem::box_rows(p.nsp);
-      unsigned bytes = (unsigned)(nb * br * kSlabCols * sizeof(double)) + (unsigned)(ngb * sizeof(int4)) +
-                       (unsigned)(3 * kSlabRows * ngb * sizeof(double));
-      if (s.photohad) bytes += (unsigned)(nqb * (4 * sizeof(double) + sizeof(unsigned long long)));
+      unsigned bytes = (unsigned)(nb * br * kSlabCols * sizeof(double)) +
+                       (unsigned)(ngb * (sizeof(SlabG) + 3 * kSlabRows * sizeof(double)));
+      if (s.photohad) bytes += (unsigned)(ne * sizeof(double) + nk * sizeof(SlabK));
       mbar_expect_tx(stage_bar, bytes);
-      for (int b = 0; b < nb; ++b) tma_load_3d(L.slab + (size_t)b * br * kSlabCols, p.tmap_src, col0, e, b * br, stage_bar);
-      if (s.photohad && nqb > 0) {
-        bulk_load(L.vals, mv, (unsigned)(nqb * 4 * sizeof(double)), stage_bar);
-        bulk_load(L.sidx, p.slab_q + qb, (unsigned)(nqb * sizeof(unsigned long long)), stage_bar);
+      for (int b = 0; b < nb; ++b)
+        tma_load_3d(L.slab + (size_t)b * br * kSlabCols * sizeof(double), p.tmap_src, col0, e, b * br, stage_bar);
+      if (s.photohad && nk > 0) {
+        bulk_load(L.vals, mv, (unsigned)(ne * sizeof(double)), stage_bar);
+        bulk_load(L.ks, p.slab_k + kb, (unsigned)(nk * sizeof(SlabK)), stage_bar);
       }
       if (ngb > 0) {
-        bulk_load(L.quart, p.slab_quart + gb0, (unsigned)(ngb * sizeof(int4)), stage_bar);
+        bulk_load(L.grp, p.slab_g + gb0, (unsigned)(ngb * sizeof(SlabG)), stage_bar);
         for (int k = 0; k < 3; ++k)
           bulk_load(L.fac + k * fs, fc + (size_t)k * p.slab_nslots, (unsigned)(kSlabRows * ngb * sizeof(double)), stage_bar);
       }
@@ -1989,66 +2064,29 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   } else {
     const double* vs = p.src + (size_t)e * ld + col0;
     for (int t = threadIdx.x; t < p.nsp * (kSlabCols / 2); t += blockDim.x) {
-      const int q = t / (kSlabCols / 2), cc = 2 * (t - q * (kSlabCols / 2));
-      cp_async16(L.slab + q * kSlabCols + cc, vs + (size_t)q * d * ld + cc);
+      const int q = t / (kSlabCols / 2), cc = t - q * (kSlabCols / 2);
+      cp_async16(const_cast<double2*>(&slab_chunk(L.slab, q, cc)), vs + (size_t)q * d * ld + 2 * cc);
     }
     if (s.photohad) {
-      for (int t = threadIdx.x; t < 2 * nqb; t += blockDim.x) cp_async16(L.vals + 2 * t, mv + 2 * t);
-      const unsigned long long* mq = p.slab_q + qb;
-      for (int t = threadIdx.x; t < nqb / 2; t += blockDim.x) cp_async16(L.sidx + 2 * t, mq + 2 * t);
+      for (int t = threadIdx.x; t < ne / 2; t += blockDim.x) cp_async16(L.vals + 2 * t, mv + 2 * t);
+      for (int t = threadIdx.x; t < nk; t += blockDim.x) cp_async16(L.ks + t, p.slab_k + kb + t);
     }
-    for (int t = threadIdx.x; t < ngb; t += blockDim.x) cp_async16(L.quart + t, p.slab_quart + gb0 + t);
-    for (int t = threadIdx.x; t < 3 * 2 * ngb; t += blockDim.x) {  // kSlabRows ngb slots per factor, 16 bytes a copy
-      const int k = t / (2 * ngb), u = t - k * 2 * ngb;
+    for (int t = threadIdx.x; t < 2 * ngb; t += blockDim.x)  // two 16-byte halves per group
+      cp_async16(reinterpret_cast<char*>(L.grp) + 16 * t, reinterpret_cast<const char*>(p.slab_g + gb0) + 16 * t);
+    for (int t = threadIdx.x; t < 3 * (kSlabRows / 2) * ngb; t += blockDim.x) {  // kSlabRows ngb slots per factor
+      const int k = t / (kSlabRows / 2 * ngb), u = t - k * (kSlabRows / 2) * ngb;
       cp_async16(L.fac + k * fs + 2 * u, fc + (size_t)k * p.slab_nslots + 2 * u);
     }
     cp_async_commit();
   }
-  const int w0 = p.slab_wrp[e * (kSlabWarps + 1) + wid], w1 = p.slab_wrp[e * (kSlabWarps + 1) + wid + 1];
+  const int w0 = p.slab_wrp[e * (kSlabWarps + 1) + wid] - gb0, w1 = p.slab_wrp[e * (kSlabWarps + 1) + wid + 1] - gb0;
   const bool need_fd = s.kap, need_f = STAGE == 2;
-  constexpr int PRE = (REC && PREF > 1) ? PREF - 1 : PREF;  // the record inputs take registers too
-  const double2 z2 = make_double2(0.0, 0.0);
-  double2 fdr[PRE], fxr[PRE];
-  int slr[PRE];
-  // record pass: dsigma and phi1' / phi2' of the row, D_off (kappa_pair v) and S x of (row, column)
   const int64_t rj = s.step - p.rec_k0;
   const bool rec_on = REC && rj >= 0 && rj < p.rec_len;
-  double rds[PRE], rd12[PRE];
-  double2 rkp[PRE], rsx[PRE];
-  // the FD term, F(x) and injection slot of quartet pi's row g (staged: the
-  // quartet comes from shared memory; the first ones are read from global memory)
-#define PB_SLAB_LOAD(U, PI, QD)                                                                          \
-  do {                                                                                                   \
-    fdr[U] = z2;                                                                                         \
-    fxr[U] = z2;                                                                                         \
-    slr[U] = -1;                                                                                         \
-    if ((PI) < w1) {                                                                                     \
-      const unsigned sp_ = quart_species((QD), g);                                                       \
-      if (sp_ != 0xffffu) {                                                                              \
-        const int r_ = (int)sp_ * d + e;                                                                 \
-        if (need_fd) fdr[U] = *reinterpret_cast<const double2*>(p.fdbuf + r_ * ld + colA);               \
-        if (need_f) fxr[U] = *reinterpret_cast<const double2*>(p.f + r_ * ld + colA);                    \
-        if (s.inj) slr[U] = p.inj_slot[r_];                                                              \
-        if (rec_on) {                                                                                    \
-          rds[U] = p.dsig[r_];                                                                           \
-          rd12[U] = STAGE == 1 ? p.dphi1[r_] : p.dphi2[r_];                                              \
-          rkp[U] = (s.kap && s.pair) ? *reinterpret_cast<const double2*>(p.fdkp + r_ * ld + colA) : z2;  \
-          rsx[U] = STAGE == 2 ? *reinterpret_cast<const double2*>(p.rec_sx + r_ * ld + colA) : z2;       \
-        }                                                                                                \
-      }                                                                                                  \
-    }                                                                                                    \
-  } while (0)
+  int src[5] = {0, 0, 0, 0, 0};
+  if (s.inj && nact > 0)
 #pragma unroll
-  for (int u = 0; u < PRE; ++u) {
-    const int pi = w0 + u;
-    PB_SLAB_LOAD(u, pi, pi < w1 ? __ldg(p.slab_quart + pi) : make_int4(-1, -1, 0, 0));
-  }
-  int srcA0 = 0, srcA1 = 0, srcB1 = 0;
-  if (s.inj && actA) {
-    srcA0 = p.src_ptr[colA];
-    srcA1 = p.src_ptr[colA + 1];
-    if (actB) srcB1 = p.src_ptr[colA + 2];
-  }
+    for (int c = 0; c <= 4; ++c) src[c] = p.src_ptr[colA + min(c, nact)];
   if (p.tmap_src) {
     if (!mbar_wait_bounded(stage_bar, 0, p.wait_tries)) {  // the copies did not land: report and leave
       if (threadIdx.x == 0) atomicExch(p.err, kErrStagingWait);
@@ -2060,99 +2098,101 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
   }
   __syncthreads();
 
-  const char* slb = reinterpret_cast<const char*>(L.slab + 2 * j);
-  const double2* vq = reinterpret_cast<const double2*>(L.vals);
-  for (int pb = w0; pb < w1; pb += PRE) {
-#pragma unroll
-    for (int u = 0; u < PRE; ++u) {
-      const int pi = pb + u;
-      if (pi >= w1) break;
-      const int4 qd = L.quart[pi - gb0];
-      const unsigned spw = quart_species(qd, g);
-      double2 acc0 = z2, acc1 = z2, acc2 = z2, acc3 = z2;
-      if (s.photohad) {  // uniform over the warp: rows without entries walk zero quads
-        const int q1 = qd.z + kSlabRows * qd.w;
-        unsigned long long mn = qd.w > 0 ? L.sidx[qd.z + g] : 0ull;  // the offsets one quad ahead
-#pragma unroll 1
-        for (int q = qd.z + g; q < q1; q += kSlabRows) {
-          const unsigned long long m = mn;
-          if (q + kSlabRows < q1) mn = L.sidx[q + kSlabRows];
-          const double2 va = vq[2 * q], vb = vq[2 * q + 1];
-          const double2 x0 = *reinterpret_cast<const double2*>(slb + ((unsigned)m & 0xffffu));
-          const double2 x1 = *reinterpret_cast<const double2*>(slb + ((unsigned)(m >> 16) & 0xffffu));
-          const double2 x2 = *reinterpret_cast<const double2*>(slb + ((unsigned)(m >> 32) & 0xffffu));
-          const double2 x3 = *reinterpret_cast<const double2*>(slb + (unsigned)(m >> 48));
-          acc0.x = __fma_rn(va.x, x0.x, acc0.x);
-          acc0.y = __fma_rn(va.x, x0.y, acc0.y);
-          acc1.x = __fma_rn(va.y, x1.x, acc1.x);
-          acc1.y = __fma_rn(va.y, x1.y, acc1.y);
-          acc2.x = __fma_rn(vb.x, x2.x, acc2.x);
-          acc2.y = __fma_rn(vb.x, x2.y, acc2.y);
-          acc3.x = __fma_rn(vb.y, x3.x, acc3.x);
-          acc3.y = __fma_rn(vb.y, x3.y, acc3.y);
-        }
+  for (int gi = w0; gi < w1; ++gi) {
+    const SlabG* G = L.grp + gi;
+    const unsigned sp = G->sp[g];
+    const bool have = sp != 0xffffu && nact > 0;
+    const int r = have ? (int)sp * d + e : e;
+    const int ro = r * ld + colA;
+    double fd[4] = {0.0, 0.0, 0.0, 0.0}, fx[4] = {0.0, 0.0, 0.0, 0.0}, rkp[4] = {0.0, 0.0, 0.0, 0.0},
+           rsx[4] = {0.0, 0.0, 0.0, 0.0}, rds = 0.0, rd12 = 0.0;
+    int slot = -1;
+    if (have) {
+      if (need_fd) load4(p.fdbuf + ro, fd);
+      if (need_f) load4(p.f + ro, fx);
+      if (s.inj) slot = p.inj_slot[r];
+      if (rec_on) {
+        rds = p.dsig[r];
+        rd12 = STAGE == 1 ? p.dphi1[r] : p.dphi2[r];
+        if (s.kap && s.pair) load4(p.fdkp + ro, rkp);
+        if (STAGE == 2) load4(p.rec_sx + ro, rsx);
       }
-      if (spw != 0xffffu && actA) {
-        const int sp = (int)spw;
-        const int r = sp * d + e;
-        const double2 sM = dadd2(dadd2(acc0, acc1), dadd2(acc2, acc3));
-        double2 out = sM;
-        if (s.kap) out = dadd2(out, fdr[u]);
-        if (s.decay) {
-          double2 sL = z2;
-          for (int64_t jj = p.l_indptr[r]; jj < p.l_indptr[r + 1]; ++jj) {
-            const double lv = p.l_vals[jj];
-            const double2 xv = *reinterpret_cast<const double2*>(p.src + (size_t)p.l_indices[jj] * ld + colA);
-            sL.x = __dadd_rn(sL.x, __dmul_rn(lv, xv.x));
-            sL.y = __dadd_rn(sL.y, __dmul_rn(lv, xv.y));
-          }
-          out = dadd2(out, sL);
+    }
+    double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
+    if (s.photohad) slab_tiles<PREF>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, acc0, acc1);
+    if (have) {
+      const double sM[4] = {acc0[0], acc1[0], acc0[1], acc1[1]};
+      double own[4];
+      {
+        const double2 oa = slab_chunk(L.slab, sp, 2 * t4), ob = slab_chunk(L.slab, sp, 2 * t4 + 1);
+        own[0] = oa.x;
+        own[1] = oa.y;
+        own[2] = ob.x;
+        own[3] = ob.y;
+      }
+      double out[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) out[c] = s.kap ? __dadd_rn(sM[c], fd[c]) : sM[c];
+      if (s.decay) {
+        double sL[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int64_t jj = p.l_indptr[r]; jj < p.l_indptr[r + 1]; ++jj) {
+          const double lv = p.l_vals[jj];
+          double xv[4];
+          load4(p.src + (size_t)p.l_indices[jj] * ld + colA, xv);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sL[c] = __dadd_rn(sL[c], __dmul_rn(lv, xv[c]));
         }
-        out.x = __dmul_rn(out.x, s.dl);
-        out.y = __dmul_rn(out.y, s.dl);
-        if (slr[u] >= 0) {  // injection (rows of injected species only)
-          if (srcA1 > srcA0) out.x = __dadd_rn(out.x, __dmul_rn(s.finj, slab_inj(p, s.step, slr[u], srcA0, srcA1)));
-          if (actB && srcB1 > srcA1) out.y = __dadd_rn(out.y, __dmul_rn(s.finj, slab_inj(p, s.step, slr[u], srcA1, srcB1)));
-        }
-        const double2 own = *reinterpret_cast<const double2*>(L.slab + sp * kSlabCols + 2 * j);
-        const int slot = kSlabRows * (pi - gb0) + g;
-        const int ro = r * ld + colA;
-        if (rec_on) {
-          const double f0 = STAGE == 1 ? L.fac[slot] : L.fac[2 * fs + slot], f1 = L.fac[fs + slot];
-          record_pre<STAGE>(p, s, r, colA, sM.x, out.x, own.x, fxr[u].x, RecIn{rds[u], rd12[u], f0, f1, rkp[u].x, rsx[u].x, true});
-          if (actB)
-            record_pre<STAGE>(p, s, r, colA + 1, sM.y, out.y, own.y, fxr[u].y,
-                              RecIn{rds[u], rd12[u], f0, f1, rkp[u].y, rsx[u].y, true});
+#pragma unroll
+        for (int c = 0; c < 4; ++c) out[c] = __dadd_rn(out[c], sL[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        out[c] = __dmul_rn(out[c], s.dl);
+        // injection (rows of injected species only)
+        if (slot >= 0 && src[c + 1] > src[c])
+          out[c] = __dadd_rn(out[c], __dmul_rn(s.finj, slab_inj(p, s.step, slot, src[c], src[c + 1])));
+      }
+      const int fslot = kSlabRows * gi + g;
+      if (rec_on) {
+        const double f0 = STAGE == 1 ? L.fac[fslot] : L.fac[2 * fs + fslot], f1 = L.fac[fs + fslot];
+        const size_t rr = (size_t)rj * p.n * ld + ro;
+        double S[4], PQ[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          S[c] = s.photohad ? sM[c] : 0.0;
+          if (s.kap && s.pair) S[c] += rkp[c];
+          S[c] = S[c] * s.dl * p.inv_scale;
+          PQ[c] = STAGE == 1 ? f0 * s.h * rds * own[c] + s.h * s.h * rd12 * rds * out[c] + s.h * f1 * S[c]
+                             : s.h * s.h * rd12 * rds * (out[c] - fx[c]) + s.h * f0 * (S[c] - rsx[c]);
         }
         if (STAGE == 1) {
-          // a = eD x + (phi1 F(x)) h
-          const double eD = L.fac[slot], p1 = L.fac[fs + slot];
-          const double2 av = make_double2(__dadd_rn(__dmul_rn(eD, own.x), __dmul_rn(__dmul_rn(p1, out.x), s.h)),
-                                          __dadd_rn(__dmul_rn(eD, own.y), __dmul_rn(__dmul_rn(p1, out.y), s.h)));
-          if (actB) {
-            *reinterpret_cast<double2*>(p.a + ro) = av;
-            *reinterpret_cast<double2*>(p.f + ro) = out;
-          } else {
-            p.a[ro] = av.x;
-            p.f[ro] = out.x;
-          }
+          store4(p.rec_sx + ro, S, nact);
+          store4(p.rec_P + rr, PQ, nact);
         } else {
-          // x = a + ((F(a) - F(x)) h) phi2
-          const double p2 = L.fac[2 * fs + slot];
-          const double2 xv = make_double2(__dadd_rn(own.x, __dmul_rn(__dmul_rn(__dadd_rn(out.x, -fxr[u].x), s.h), p2)),
-                                          __dadd_rn(own.y, __dmul_rn(__dmul_rn(__dadd_rn(out.y, -fxr[u].y), s.h), p2)));
-          if (actB) *reinterpret_cast<double2*>(p.xout + ro) = xv;
-          else p.xout[ro] = xv.x;
+          store4(p.rec_Q + rr, PQ, nact);
         }
       }
-      const int pn = pi + PRE;
-      PB_SLAB_LOAD(u, pn, pn < w1 ? L.quart[pn - gb0] : make_int4(-1, -1, 0, 0));
+      double res[4];
+      if (STAGE == 1) {  // a = eD x + (phi1 F(x)) h
+        const double eD = L.fac[fslot], p1 = L.fac[fs + fslot];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          res[c] = __dadd_rn(__dmul_rn(eD, own[c]), __dmul_rn(__dmul_rn(p1, out[c]), s.h));
+        store4(p.a + ro, res, nact);
+        store4(p.f + ro, out, nact);
+      } else {  // x = a + ((F(a) - F(x)) h) phi2
+        const double p2 = L.fac[2 * fs + fslot];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          res[c] = __dadd_rn(own[c], __dmul_rn(__dmul_rn(__dadd_rn(out[c], -fx[c]), s.h), p2));
+        store4(p.xout + ro, res, nact);
+      }
     }
+    __syncwarp();
   }
-#undef PB_SLAB_LOAD
 }
 
-// k_slab instance for (stage, record pass, prefetch depth in quartets).
+// k_slab instance for (stage, record pass, prefetch depth).
 using SlabKernel = void (*)(StepParams);
 template <int PREF>
 SlabKernel slab_kernel_p(int stage, bool rec) {
@@ -3442,8 +3482,8 @@ std::vector<DBuf*> solve_buffers(pb_context* c) {
           &c->lt_indptr, &c->lt_indices, &c->lt_vals, &c->inj_rows, &c->src_col_d, &c->ckpt,
           &c->em_bh_off, &c->em_bh_A, &c->em_invE, &c->em_dE, &c->em_Tg, &c->em_Te, &c->em_R, &c->em_wbuf,
           &c->em_es, &c->em_lep, &c->em_y, &c->em_TgT, &c->em_TeT, &c->em_RT, &c->em_dlw,
-          &c->band_slot, &c->band_spec, &c->slab_spec, &c->band_vals, &c->band_part, &c->slab_rp,
-          &c->slab_sidx, &c->slab_slot, &c->slab_vals, &c->slab_quart, &c->slab_wrp, &c->slab_rowslot, &c->slab_fac, &c->fd_cnt, &c->fd_off, &c->fd_val, &c->fd_dense, &c->fdT_dense, &c->fdbuf,
+          &c->band_slot, &c->band_spec, &c->slab_spec, &c->band_vals, &c->band_part, &c->slab_kbase,
+          &c->slab_ebase, &c->slab_k, &c->slab_g, &c->slab_slot, &c->slab_vals, &c->slab_wrp, &c->slab_rowslot, &c->slab_fac, &c->fd_cnt, &c->fd_off, &c->fd_val, &c->fd_dense, &c->fdT_dense, &c->fdbuf,
           &c->bandT_slot, &c->slabT_rp, &c->slabT_offs, &c->slabT_slot, &c->fdT_cnt, &c->fdT_off, &c->fdT_val,
           &c->slabT_pairs, &c->slabT_wrp, &c->tmaps, &c->d_err, &c->tab_z, &c->tab_le, &c->tab_v};
 }
@@ -3543,14 +3583,16 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.nsp = c->lay_nsp;
   p.slab_spec = c->slab_spec.as<int>();
   p.n_slab_spec = c->n_slab_spec;
-  p.slab_qbase = c->slab_rp.as<int>();
-  p.slab_q = c->slab_sidx.as<unsigned long long>();
-  p.slab_quart = c->slab_quart.as<int4>();
+  p.slab_kbase = c->slab_kbase.as<int>();
+  p.slab_ebase = c->slab_ebase.as<int>();
+  p.slab_k = c->slab_k.as<SlabK>();
+  p.slab_g = c->slab_g.as<SlabG>();
   p.slab_wrp = c->slab_wrp.as<int>();
   p.slab_vals = c->slab_vals.as<double>();
   p.slab_stride = c->slab_nent;
-  p.slab_maxq = c->slab_maxbin;
-  p.slab_maxp = (c->n_slab_spec + kSlabRows - 1) / kSlabRows;
+  p.slab_maxe = c->slab_maxe;
+  p.slab_maxk = c->slab_maxk;
+  p.slab_maxg = c->slab_maxg;
   p.slab_rowslot = c->slab_rowslot.as<int>();
   p.sfac = use_blocked(c, K) ? c->slab_fac.as<double>() : nullptr;
   p.slab_nslots = c->slab_nslots;
@@ -3610,7 +3652,7 @@ int ensure_tmaps(pb_context* c, bool blocked, int ld) {
                                band ? 1u : (cuuint32_t)SlabSmem::box_rows(nsp)};
     const cuuint32_t es[3] = {1u, 1u, 1u};
     if (enc(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, k % 2 == 0 ? c->X.p : c->A.p, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, band ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
       if (!band) return PB_OK;
       band_ok = false;
@@ -4133,6 +4175,189 @@ void const_steps(StepParams& p, const StepScal* scal, int64_t per_prep, double* 
     k_step_plain<2><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
   }
 }
+
+// Rows of one bin as groups of eight with shared columns, and each group's
+// columns as k-tiles of four (SlabG, SlabK), bin by bin.  Rows with many columns
+// go together (longest first); then a group starts with the first row left and
+// takes, seven times, the row that adds the fewest new columns.  A k-tile takes
+// its columns from the four classes of ((column / 2) mod 4) where it can: the
+// slab rows of distinct classes lie in distinct shared-memory banks.  A bin with
+// the previous bin's columns keeps its groups.
+struct SlabTiles {
+  struct Row {
+    int32_t sp;
+    std::vector<std::pair<int32_t, int64_t>> ent;  // (column, entry), in CSR order
+  };
+  struct Group {
+    std::vector<int> rows;      // indices into the bin's rows
+    std::vector<int32_t> cols;  // in k-tile order, four per tile (-1: none)
+    bool pad = false;           // the last tile holds no entries
+  };
+  int d, nsp, nwarps;
+  unsigned entry_offset;        // of the bin's entries from the slab's start in shared memory
+  std::vector<int32_t> kbase, ebase, wrp;
+  std::vector<SlabK> ks;
+  std::vector<SlabG> gs;
+  int64_t nent = 0;
+  int32_t maxe = 0, maxk = 0, maxg = 0;
+  std::vector<std::vector<int32_t>> last_cols;
+  std::vector<Group> groups;
+
+  SlabTiles(int d_, int nsp_, int nwarps_)
+      : d(d_), nsp(nsp_), nwarps(nwarps_), entry_offset((unsigned)SlabSmem::rows(nsp_) * kSlabCols * sizeof(double)) {}
+
+  void make_groups(const std::vector<Row>& rows) {
+    groups.clear();
+    const int n = (int)rows.size(), words = (nsp + 63) / 64;
+    std::vector<std::vector<uint64_t>> bits((size_t)n, std::vector<uint64_t>((size_t)words, 0));
+    for (int i = 0; i < n; ++i)
+      for (const auto& q : rows[i].ent) bits[i][q.first / 64] |= 1ull << (q.first % 64);
+    std::vector<char> used((size_t)n, 0);
+    std::vector<int> heavy;
+    for (int i = 0; i < n; ++i)
+      if ((int)rows[i].ent.size() > 48) heavy.push_back(i);
+    std::stable_sort(heavy.begin(), heavy.end(), [&](int a, int b) { return rows[a].ent.size() > rows[b].ent.size(); });
+    size_t next_heavy = 0;
+    int first = 0, left = n;
+    while (left > 0) {
+      Group gr;
+      std::vector<uint64_t> u((size_t)words, 0);
+      auto take = [&](int i) {
+        gr.rows.push_back(i);
+        used[i] = 1;
+        --left;
+        for (int w = 0; w < words; ++w) u[w] |= bits[i][w];
+      };
+      if (next_heavy < heavy.size()) {
+        while (next_heavy < heavy.size() && gr.rows.size() < (size_t)kSlabRows) take(heavy[next_heavy++]);
+      } else {
+        while (used[first]) ++first;
+        take(first);
+      }
+      while (gr.rows.size() < (size_t)kSlabRows && left > 0) {
+        int best = -1, add = 0, share = 0;
+        for (int i = 0; i < n; ++i) {
+          if (used[i]) continue;
+          int a = 0, b = 0;
+          for (int w = 0; w < words; ++w) {
+            a += __builtin_popcountll(bits[i][w] & ~u[w]);
+            b += __builtin_popcountll(bits[i][w] & u[w]);
+          }
+          if (best < 0 || a < add || (a == add && b > share)) {
+            best = i;
+            add = a;
+            share = b;
+          }
+        }
+        take(best);
+      }
+      std::vector<std::vector<int32_t>> cls(4);
+      for (int m = 0; m < nsp; ++m)
+        if (u[m / 64] >> (m % 64) & 1) cls[(m >> 1) & 3].push_back(m);
+      size_t rest = cls[0].size() + cls[1].size() + cls[2].size() + cls[3].size();
+      while (rest > 0) {
+        int order[4] = {0, 1, 2, 3};
+        std::stable_sort(order, order + 4, [&](int a, int b) { return cls[a].size() > cls[b].size(); });
+        int got = 0;
+        for (int pass = 0; got < 4 && pass < 4; ++pass)
+          for (int q = 0; q < 4 && got < 4; ++q) {
+            auto& v = cls[order[q]];
+            if (v.empty()) continue;
+            gr.cols.push_back(v.back());
+            v.pop_back();
+            ++got;
+            --rest;
+          }
+        for (; got < 4; ++got) gr.cols.push_back(-1);
+      }
+      if (gr.cols.size() % 8) {  // an even number of k-tiles: one more without entries, on the first tile's first row
+        const int32_t m = gr.cols[0];
+        gr.cols.push_back(m);
+        for (int q = 0; q < 3; ++q) gr.cols.push_back(-1);
+        gr.pad = true;
+      }
+      groups.push_back(std::move(gr));
+    }
+  }
+
+  // Adds bin kbase.size(): `slot[entry]` gets each entry's place, `row_slot(sp, s)` each row's group slot.
+  template <class F>
+  void add_bin(const std::vector<Row>& rows, std::vector<int32_t>& slot, F row_slot) {
+    std::vector<std::vector<int32_t>> cols(rows.size());
+    for (size_t i = 0; i < rows.size(); ++i)
+      for (const auto& q : rows[i].ent) cols[i].push_back(q.first);
+    if (kbase.empty() || cols != last_cols) {
+      make_groups(rows);
+      last_cols = std::move(cols);
+    }
+    const int kb = (int)ks.size(), gb = (int)gs.size();
+    kbase.push_back(kb);
+    ebase.push_back((int32_t)nent);
+    // groups over the warps, the longest first to the least loaded
+    std::vector<int> order(groups.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return groups[a].cols.size() > groups[b].cols.size(); });
+    std::vector<std::vector<int>> wl((size_t)nwarps);
+    std::vector<int64_t> load((size_t)nwarps, 0);
+    for (int i : order) {
+      const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      wl[w].push_back(i);
+      load[w] += (int64_t)groups[i].cols.size() / 4 + 4;  // the update costs about four k-tiles
+    }
+    unsigned ent = 0;
+    std::vector<std::vector<int64_t>> at((size_t)kSlabRows, std::vector<int64_t>((size_t)nsp, -1));
+    for (int w = 0; w < nwarps; ++w) {
+      wrp.push_back((int32_t)gs.size());
+      for (int i : wl[w]) {
+        const Group& gr = groups[i];
+        SlabG G;
+        memset(&G, 0, sizeof(G));
+        G.kt0 = (int)ks.size() - kb;
+        G.nkt = (int)gr.cols.size() / 4;
+        for (int g = 0; g < kSlabRows; ++g) {
+          G.sp[g] = g < (int)gr.rows.size() ? (unsigned short)rows[gr.rows[g]].sp : 0xffff;
+          if (g >= (int)gr.rows.size()) continue;
+          row_slot(rows[gr.rows[g]].sp, (int32_t)(gs.size() * kSlabRows + g));
+          for (const auto& q : rows[gr.rows[g]].ent) at[g][q.first] = q.second;
+        }
+        for (int k = 0; k < G.nkt; ++k) {
+          SlabK K;
+          memset(&K, 0, sizeof(K));
+          K.base = entry_offset + ent * (unsigned)sizeof(double);
+          for (int kk = 0; kk < 4; ++kk) {
+            const int m = gr.cols[4 * k + kk] >= 0 ? gr.cols[4 * k + kk] : gr.cols[4 * k];
+            K.row[kk] = (unsigned short)(8 * m + (m & 7));
+          }
+          for (int g = 0; g < (int)gr.rows.size(); ++g)
+            for (int kk = 0; kk < 4; ++kk) {
+              const int m = gr.cols[4 * k + kk];
+              if (m < 0 || at[g][m] < 0 || (gr.pad && k == G.nkt - 1)) continue;
+              K.mask |= 1u << (4 * g + kk);
+              slot[at[g][m]] = (int32_t)(nent + ent);
+              ++ent;
+            }
+          ks.push_back(K);
+        }
+        for (int g = 0; g < (int)gr.rows.size(); ++g)
+          for (const auto& q : rows[gr.rows[g]].ent) at[g][q.first] = -1;
+        gs.push_back(G);
+      }
+    }
+    wrp.push_back((int32_t)gs.size());
+    ent += ent & 1;  // bulk copies are multiples of 16 bytes
+    nent += ent;
+    maxe = std::max(maxe, (int32_t)ent);
+    maxk = std::max(maxk, (int32_t)ks.size() - kb);
+    maxg = std::max(maxg, (int32_t)gs.size() - gb);
+  }
+
+  void finish() {
+    kbase.push_back((int32_t)ks.size());
+    ebase.push_back((int32_t)nent);
+    if (ks.empty()) ks.push_back(SlabK{});
+    if (gs.empty()) gs.push_back(SlabG{});
+  }
+};
 
 }  // namespace
 
@@ -4759,91 +4984,32 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   int RT = 0, J = 0;
   for (int v : kBandRT) if (!RT && v >= RTr) RT = v;
   for (int v : kBandJ) if (!J && v >= Jr) J = v;
-  // bin-local rows, per bin: rows ordered by entry quads (longest first) and
-  // grouped in quartets, a quarter-warp of k_slab per row; quartets spread
-  // over k_slab's warps longest-processing-time first.  Each row's entries in
-  // CSR order in quads of 4; zero values pad the row's last quad and the row
-  // up to the longest row of its quartet.  The quads of a quartet's four rows
-  // interleave (row g's quad t at q0 + 4 t + g), so that the four rows' entry
-  // loads fall into distinct shared-memory banks; every bin and quartet starts
-  // on a multiple of 4 quads.
+  // bin-local rows, per bin, as DMMA row groups and k-tiles (SlabTiles)
   int64_t band_nnz = 0, slab_nnz = 0;
-  std::vector<int32_t> qbase((size_t)d + 1, 0), wrp((size_t)d * (kSlabWarps + 1), 0), squart;
-  std::vector<unsigned long long> squad;
   std::vector<int32_t> sslot((size_t)std::max<int64_t>(R, 1), -1), rowslot((size_t)n, -1);
-  int32_t maxbin = 0;
-  // 16-bit slab byte offsets and 16-bit species (0xffff marks an empty quartet row)
-  bool quads_fit = (size_t)nsp * kSlabCols * sizeof(double) <= (1 << 16) && nsp < 0xffff;
+  SlabTiles tiles(d, nsp, kSlabWarps);
   {
-    std::vector<int32_t> nq(nss), order(nss);
-    std::vector<std::vector<int32_t>> wl(kSlabWarps);
-    std::vector<int64_t> load(kSlabWarps);
+    std::vector<SlabTiles::Row> rows((size_t)nss);
     for (int e = 0; e < d; ++e) {
-      qbase[e] = (int32_t)squad.size();
       for (int i = 0; i < nss; ++i) {
         const int64_t r = (int64_t)sspec[i] * d + e;
-        int64_t cnt = 0;
-        for (int64_t j = ip[r]; j < ip[r + 1]; ++j) cnt += ix[j] != r;
-        nq[i] = (int32_t)((cnt + 3) / 4);
-        order[i] = i;
+        rows[i].sp = sspec[i];
+        rows[i].ent.clear();
+        for (int64_t j = ip[r]; j < ip[r + 1]; ++j)
+          if (ix[j] != r) rows[i].ent.push_back({ix[j] / d, j});
+        slab_nnz += (int64_t)rows[i].ent.size();
       }
-      std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return nq[a] > nq[b]; });
-      for (auto& v : wl) v.clear();
-      std::fill(load.begin(), load.end(), 0);
-      for (int k = 0; k < nss; k += kSlabRows) {  // quartet k / 4 = rows order[k .. k + 3], the longest first
-        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        wl[w].push_back(k);
-        load[w] += nq[order[k]] + 1;
-      }
-      for (int w = 0; w < kSlabWarps; ++w) {
-        wrp[(size_t)e * (kSlabWarps + 1) + w] = (int32_t)(squart.size() / 4);
-        for (int k : wl[w]) {
-          const int nqmax = nq[order[k]];
-          const int64_t q0 = (int64_t)squad.size() - qbase[e];
-          const size_t qa = squad.size();
-          squad.resize(qa + (size_t)kSlabRows * nqmax, 0);
-          int32_t sp4[kSlabRows] = {0xffff, 0xffff, 0xffff, 0xffff};
-          for (int g = 0; g < kSlabRows; ++g) {
-            if (k + g >= nss) continue;
-            const int i = order[k + g];
-            const int64_t r = (int64_t)sspec[i] * d + e;
-            int t = 0, pad_sp = sspec[i];
-            for (int64_t j = ip[r]; j < ip[r + 1]; ++j) {
-              if (ix[j] == r) continue;
-              if (t == 0) pad_sp = ix[j] / d;
-              const size_t q = qa + (size_t)kSlabRows * (t / 4) + g;
-              squad[q] |= (unsigned long long)((ix[j] / d) * kSlabCols * sizeof(double)) << (16 * (t % 4));
-              sslot[j] = (int32_t)(q * 4 + t % 4);
-              ++slab_nnz;
-              ++t;
-            }
-            for (; t < 4 * nqmax; ++t) {  // zero values on a mother row of the slab
-              const size_t q = qa + (size_t)kSlabRows * (t / 4) + g;
-              squad[q] |= (unsigned long long)(pad_sp * kSlabCols * sizeof(double)) << (16 * (t % 4));
-            }
-            sp4[g] = sspec[i];
-            rowslot[r] = (int32_t)(squart.size() + g);  // quartet index * 4 + row
-          }
-          if (q0 >= (1 << 30)) quads_fit = false;
-          const int32_t qd[4] = {(int32_t)((uint32_t)sp4[0] | ((uint32_t)sp4[1] << 16)),
-                                 (int32_t)((uint32_t)sp4[2] | ((uint32_t)sp4[3] << 16)), (int32_t)q0, nqmax};
-          squart.insert(squart.end(), qd, qd + 4);
-        }
-      }
-      wrp[(size_t)e * (kSlabWarps + 1) + kSlabWarps] = (int32_t)(squart.size() / 4);
-      maxbin = std::max<int32_t>(maxbin, (int32_t)(squad.size() - qbase[e]));
+      tiles.add_bin(rows, sslot, [&](int32_t sp, int32_t slot) { rowslot[(int64_t)sp * d + e] = slot; });
     }
-    qbase[d] = (int32_t)squad.size();
-    if (squad.empty()) squad.assign(4, 0);
-    if (squart.empty()) squart.assign(4, 0);
+    tiles.finish();
   }
   const size_t max_smem = 227 * 1024;
-  const size_t ssm = SlabSmem::bytes(nsp, maxbin, (nss + kSlabRows - 1) / kSlabRows);
+  const size_t ssm = SlabSmem::bytes(nsp, tiles.maxe, tiles.maxk, tiles.maxg);
   const BandInstance bi = (RT && J) ? band_kernel(RT, J) : BandInstance{nullptr, 0, 0};
   const BandInstance bi4 = (RT && J) ? band_kernel(RT, J, 4) : BandInstance{nullptr, 0, 0};
-  const bool ok = split_ok && quads_fit && ssm <= max_smem && bi.fn && bi.smem <= max_smem && (bspec.empty() || lo >= 0) &&
+  const bool ok = split_ok && nsp < 0x2000 && ssm <= max_smem && bi.fn && bi.smem <= max_smem && (bspec.empty() || lo >= 0) &&
                   (size_t)d * (kColTile + 2) * sizeof(double) <= max_smem &&
-                  (int64_t)nsp * 2 * npairs * RT * J * 32 < ((int64_t)1 << 31) && squad.size() < ((size_t)1 << 29);
+                  (int64_t)nsp * 2 * npairs * RT * J * 32 < ((int64_t)1 << 31) && tiles.nent < ((int64_t)1 << 31);
   if (!ok) return PB_OK;  // the general row kernels stay in use
   // band tiles: [species][band pair][2][RT / 2][J][32][2] DMMA A fragments per window
   std::vector<int32_t> bslot((size_t)std::max<int64_t>(R, 1), -1);
@@ -4864,12 +5030,13 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   if ((rc = upload(c, c->band_slot, bslot.data(), bslot.size()))) return rc;
   if ((rc = upload(c, c->band_spec, bspec.data(), bspec.size()))) return rc;
   if ((rc = upload(c, c->slab_spec, sspec.data(), sspec.size()))) return rc;
-  if ((rc = upload(c, c->slab_rp, qbase.data(), qbase.size()))) return rc;
-  if ((rc = upload(c, c->slab_sidx, squad.data(), squad.size()))) return rc;
-  if ((rc = upload(c, c->slab_quart, squart.data(), squart.size()))) return rc;
-  if ((rc = upload(c, c->slab_wrp, wrp.data(), wrp.size()))) return rc;
+  if ((rc = upload(c, c->slab_kbase, tiles.kbase.data(), tiles.kbase.size()))) return rc;
+  if ((rc = upload(c, c->slab_ebase, tiles.ebase.data(), tiles.ebase.size()))) return rc;
+  if ((rc = upload(c, c->slab_k, tiles.ks.data(), tiles.ks.size()))) return rc;
+  if ((rc = upload(c, c->slab_g, tiles.gs.data(), tiles.gs.size()))) return rc;
+  if ((rc = upload(c, c->slab_wrp, tiles.wrp.data(), tiles.wrp.size()))) return rc;
   if ((rc = upload(c, c->slab_rowslot, rowslot.data(), rowslot.size()))) return rc;
-  c->slab_nslots = (int64_t)squart.size();
+  c->slab_nslots = (int64_t)tiles.gs.size() * kSlabRows;
   const size_t fac_bytes = (size_t)prep_steps(n) * 3 * c->slab_nslots * sizeof(double);
   PB_CUDA(c, c->slab_fac.ensure(fac_bytes));
   PB_CUDA(c, cudaMemsetAsync(c->slab_fac.p, 0, fac_bytes, c->stream));  // slots without a row stay zero
@@ -4898,8 +5065,10 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   c->band_J = J;
   c->band_stride = (int64_t)nsp * 2 * npairs * RT * J * 32;
   c->n_slab_spec = nss;
-  c->slab_nent = (int64_t)squad.size() * 4;
-  c->slab_maxbin = maxbin;
+  c->slab_nent = tiles.nent;
+  c->slab_maxe = tiles.maxe;
+  c->slab_maxk = tiles.maxk;
+  c->slab_maxg = tiles.maxg;
   c->slab_smem = ssm;
   c->band_smem = bi.smem;
   c->band_nnz = band_nnz;
