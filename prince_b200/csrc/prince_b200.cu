@@ -2642,50 +2642,44 @@ __global__ void k_em_scale_w(EmParams e, double s) {
 }
 
 
-// w[i][k] = sum_s cw_si X[s, i][k] over the charged nuclei in species order, with
-// cw_si = A_s kappa_pair dl_step / E_i dE_i: the Bethe-Heitler pair weights of the
-// hook (propagation.py:640-661).  A warp per (bin, 32 V-column tile), each lane
-// V adjacent columns (V = 2: 16-byte loads, used when the leading dimension is
-// even; V = 1 for one-column solves, whose leading dimension is 1), so the
-// nuclear state is read by many warps at once; the species table sits in
-// shared memory and each warp loads kEmWBatch species' states ahead of the
-// (ordered) sum.
+// w[i][k] = sum_s cw_si X[s, i][k] over the charged nuclei, with cw_si = A_s
+// kappa_pair dl_step / E_i dE_i: the Bethe-Heitler pair weights of the hook
+// (propagation.py:640-661).  CTA = (bin, 32 V-column tile); its eight warps take
+// every eighth species and add their sums in warp order through shared memory.
+// A lane owns V adjacent columns (V = 2: 16-byte loads, used when the leading
+// dimension is even; V = 1 for one-column solves) and loads kEmWBatch species'
+// states ahead.  Bound by HBM: the nuclear state once.  A warp per (bin, tile)
+// that walked all 337 nuclei alone left most of the GPU idle at a few hundred
+// columns: 127 us per step at K = 300 (81 MB), this 36 us.
 constexpr int kEmWBatch = 8;
+constexpr int kEmWWarps = 8;
 
 template <int V>
-__global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
-  extern __shared__ unsigned char em_w_smem[];
+__global__ void __launch_bounds__(kEmWWarps * 32) k_em_w(EmParams e) {
+  __shared__ double red[kEmWWarps][32 * V];
   const int ncols = e.sc->ncols, w = e.sc->w;
   if ((int)blockIdx.y * (32 * V) >= ncols) return;
   const double* __restrict__ kp = e.kp + (size_t)w * e.n;
   const double dl_step = e.dl[w];
-  int64_t* soff = reinterpret_cast<int64_t*>(em_w_smem);
-  double* sA = reinterpret_cast<double*>(soff + e.n_bh);
-  for (int t = threadIdx.x; t < e.n_bh; t += blockDim.x) {
-    soff[t] = e.bh_off[t];
-    sA[t] = e.bh_A[t];
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int i = blockIdx.x * 8 + wid;
-  if (i >= e.n_cr) return;
+  const int i = blockIdx.x;
   const int k = blockIdx.y * (32 * V) + V * lane;  // columns k .. k + V - 1
-  const bool active = k < ncols;
-  const int kk = active ? k : 0;
+  const int kk = k < ncols ? k : 0;
   const double ie = e.invE[i], de = e.dE[i];
   double acc[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) acc[v] = 0.0;
-  for (int s0 = 0; s0 < e.n_bh; s0 += kEmWBatch) {
+  for (int s0 = wid; s0 < e.n_bh; s0 += kEmWWarps * kEmWBatch) {
     double xv[kEmWBatch][V];
-    double kv[kEmWBatch];
+    double cw[kEmWBatch];
 #pragma unroll
     for (int u = 0; u < kEmWBatch; ++u) {
+      const int s = s0 + u * kEmWWarps;
 #pragma unroll
       for (int v = 0; v < V; ++v) xv[u][v] = 0.0;
-      kv[u] = 0.0;
-      if (s0 + u < e.n_bh) {
-        const int64_t row = soff[s0 + u] + i;
+      cw[u] = 0.0;
+      if (s < e.n_bh) {
+        const int64_t row = __ldg(e.bh_off + s) + i;
         const double* src = e.X + (size_t)row * e.ld + kk;
         if (V == 2) {
           const double2 x2 = __ldg(reinterpret_cast<const double2*>(src));
@@ -2694,25 +2688,27 @@ __global__ void __launch_bounds__(256, 3) k_em_w(EmParams e) {
         } else {
           xv[u][0] = __ldg(src);
         }
-        kv[u] = __ldg(kp + row);
+        cw[u] = __dmul_rn(__ldg(e.bh_A + s), __ldg(kp + row));
       }
     }
 #pragma unroll
     for (int u = 0; u < kEmWBatch; ++u) {
-      const int s = s0 + u;
-      if (s < e.n_bh) {
-        const double cw = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(sA[s], kv[u]), dl_step), ie), de);
+      const double c = __dmul_rn(__dmul_rn(__dmul_rn(cw[u], dl_step), ie), de);
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const double t = __dmul_rn(cw, xv[u][v]);
-          acc[v] = (s == 0) ? t : __dadd_rn(acc[v], t);
-        }
-      }
+      for (int v = 0; v < V; ++v) acc[v] = __dadd_rn(acc[v], __dmul_rn(c, xv[u][v]));
     }
   }
 #pragma unroll
-  for (int v = 0; v < V; ++v)
-    if (k + v < ncols) e.w[(size_t)i * e.ld + k + v] = acc[v];
+  for (int v = 0; v < V; ++v) red[wid][V * lane + v] = acc[v];
+  __syncthreads();
+  for (int t = threadIdx.x; t < 32 * V; t += blockDim.x) {
+    const int col = blockIdx.y * (32 * V) + t;
+    if (col >= ncols) continue;
+    double sum = red[0][t];
+#pragma unroll
+    for (int q = 1; q < kEmWWarps; ++q) sum = __dadd_rn(sum, red[q][t]);
+    e.w[(size_t)i * e.ld + col] = sum;
+  }
 }
 
 // Adjoint of the pair weights: X[s, i][k] += cw_si lw[i][k] (e.X = lam, e.w = lw).
@@ -2755,12 +2751,11 @@ __global__ void __launch_bounds__(256) k_em_wT(EmParams e) {
 //   w = pair weights (k_em_w), es = R w, l = e- + e+ + 2 es (k_em_lep, e+- <- 0),
 //   y = Tg gamma + Te l, gamma <- y.
 void em_hook_forward(const EmParams& e, cudaStream_t st) {
-  const size_t wsm = (size_t)e.n_bh * (sizeof(int64_t) + sizeof(double));
   const long long nn = (long long)e.n_em * e.n_em, nr = (long long)e.n_em * e.n_cr;
   if (e.ld % 2 == 0)
-    k_em_w<2><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.hcols, 64)), 256, wsm, st>>>(e);
+    k_em_w<2><<<dim3((unsigned)e.n_cr, (unsigned)blocks_for(e.hcols, 64)), kEmWWarps * 32, 0, st>>>(e);
   else
-    k_em_w<1><<<dim3((unsigned)blocks_for(e.n_cr, 8), (unsigned)blocks_for(e.hcols, 32)), 256, wsm, st>>>(e);
+    k_em_w<1><<<dim3((unsigned)e.n_cr, (unsigned)blocks_for(e.hcols, 32)), kEmWWarps * 32, 0, st>>>(e);
   bgemm_step(st, e.sc, e.R, nr, e.w, nullptr, e.es, e.n_em, e.hcols, e.n_cr, e.ld);
   k_em_lep<<<(unsigned)blocks_for((int64_t)e.n_em * e.hcols, 256), 256, 0, st>>>(e);
   double* gam = e.X + (size_t)e.g_off * e.ld;
