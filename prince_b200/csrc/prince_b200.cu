@@ -204,9 +204,9 @@ struct pb_context {
   cudaEvent_t ev_hook_fork = nullptr, ev_hook_done = nullptr;
   bool tail_wait = false;           // the next tail launch waits for ev_hook_done
   int num_sms = 148;
-  DBuf tmaps;                       // [4] CUtensorMap of X and A for k_slab's and k_band_tma's TMA staging
+  DBuf tmaps;                       // [6] CUtensorMap of X and A for k_slab's and k_band_tma's TMA staging
   bool tma_ok = false;              // tmaps hold k_slab's maps of the current X / A / ld
-  bool tma_band_ok = false;         // tmaps also hold k_band_tma's maps (entries 2, 3)
+  bool tma_band_ok = false;         // tmaps also hold k_band_tma's maps (entries 2 to 5)
   bool band_tma_fits = false;       // k_band_tma's shared memory fits the layout's band tiles
   bool last_tma = false;            // the last solve staged k_slab by TMA
   const void* tma_key[3] = {nullptr, nullptr, nullptr};
@@ -760,7 +760,7 @@ struct StepParams {
   int hcols;         // host side: columns the launch grids cover (at least sc->ncols)
   const StepScal* sc;  // the step's scalars
   const CUtensorMap* tmap_src;  // k_slab: tensor map of src for the TMA staging, or null (cp.async staging)
-  const CUtensorMap* tmap_band;  // k_band_tma: tensor map of src as (64 columns x d bins) boxes, or null
+  const CUtensorMap* tmap_band;  // k_band_tma: tensor maps of src as (8 or 64 columns x d bins) boxes, or null
   long long wait_tries;         // k_slab: polls of the staging wait before it gives up (the drain keeps kWaitTries)
   int* err;          // set to a nonzero code when a bounded wait gives up
   int64_t n_steps;
@@ -1686,7 +1686,7 @@ constexpr int kFdMax = 4;           // off-diagonal FD stencil entries per row (
 constexpr int kFdHalo = 3;          // k_fd_dense: stencil offsets within +-kFdHalo bins
 constexpr int kFdDenseW = 8;        // dense weights per bin (2 kFdHalo + 1, padded to 16 bytes)
 constexpr int kFdChunk = 12;        // k_fd_dense: bins per warp pass
-constexpr int kMaxBandGroups = 64;
+constexpr int kMaxBandGroups = 148;
 
 // mbarrier and bulk-copy helpers of the TMA staging (CTA-local barrier, no cluster)
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -2350,62 +2350,107 @@ size_t band_smem_bytes() {
   return (size_t)2 * ((NW == 8 ? 2 : 1) * RT * J * 32) * sizeof(double);
 }
 
-// Band rows: add the group partials in group order, then the stage update
-// with the FD term from fdbuf.
-template <int STAGE>
-__global__ void __launch_bounds__(256) k_band_finish(StepParams p) {
+// Band rows: add the group partials, then the stage update with the FD term
+// from fdbuf.  CTA = (band row, 32-column tile): eight warps add every eighth
+// group's partials in group order and the eight sums in warp order, and one
+// warp applies the update, whose inputs it loads first.
+constexpr int kFinWarps = 8;
+constexpr int kFinSplit = 32;  // groups above which a row takes a CTA
+template <int STAGE, bool SPLIT>
+__global__ void __launch_bounds__(kFinWarps * 32) k_band_finish(StepParams p) {
+  __shared__ double red[kFinWarps][kColTile];
   const StepScalars s = load_scalars(p, p.sc);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int rb = blockIdx.x * (blockDim.x >> 5) + wid;
-  if (rb >= p.nb * p.d) return;
+  const int rb = SPLIT ? blockIdx.x : blockIdx.x * kFinWarps + wid;
+  if (rb >= p.nb * p.d || (int)blockIdx.y * kColTile >= s.ncols) return;
   const int b = rb / p.d, e = rb - b * p.d;
   const int64_t r = (int64_t)p.band_spec[b] * p.d + e;
-  const int col = blockIdx.y * kColTile + lane;
+  const int col = blockIdx.y * kColTile + lane;  // < ld
+  const size_t idx = (size_t)r * p.ld + col;
+  const bool on = (!SPLIT || wid == 0) && col < s.ncols;
+  double fd = 0.0, own = 0.0, fx = 0.0, f0 = 0.0, f1 = 0.0;
+  if (on) {
+    if (s.kap) fd = p.fdbuf[idx];
+    own = STAGE == 1 ? p.x[idx] : p.a[idx];
+    f0 = STAGE == 1 ? p.eD[r] : p.phi2[r];
+    if (STAGE == 1) f1 = p.phi1[r];
+    else fx = p.f[idx];
+  }
+  const double* part = p.band_part + ((size_t)b * p.d + e) * p.ld + col;
+  const size_t gs = (size_t)p.nb * p.d * p.ld;
+  double t = 0.0;
   if (col < s.ncols) {
-    double t = 0.0;
-    for (int g = 0; g < p.ngroups; ++g)
-      t = __dadd_rn(t, p.band_part[((size_t)(g * p.nb + b) * p.d + e) * p.ld + col]);
-    const size_t idx = (size_t)r * p.ld + col;
-    double out = t;
-    if (s.kap) out = __dadd_rn(out, p.fdbuf[idx]);
-    if (s.decay) {
-      double sL = 0.0;
-      for (int64_t j = p.l_indptr[r]; j < p.l_indptr[r + 1]; ++j)
-        sL = __dadd_rn(sL, __dmul_rn(p.l_vals[j], p.src[(size_t)p.l_indices[j] * p.ld + col]));
-      out = __dadd_rn(out, sL);
-    }
-    out = __dmul_rn(out, s.dl);
-    if (s.inj) out = __dadd_rn(out, inj_at(p, s, r, col));
-    const int64_t o = r;
-    if (p.rec_P) record_blocked<STAGE>(p, s, r, col, t, out, p.x[idx], STAGE == 2 ? p.f[idx] : 0.0);
-    if (STAGE == 1) {
-      p.a[idx] = __dadd_rn(__dmul_rn(p.eD[o], p.x[idx]), __dmul_rn(__dmul_rn(p.phi1[o], out), s.h));
-      p.f[idx] = out;
-    } else {
-      const double dF = __dmul_rn(__dadd_rn(out, -p.f[idx]), s.h);
-      p.xout[idx] = __dadd_rn(p.a[idx], __dmul_rn(dF, p.phi2[o]));
-    }
+#pragma unroll 4
+    for (int g = SPLIT ? wid : 0; g < p.ngroups; g += SPLIT ? kFinWarps : 1) t = __dadd_rn(t, part[g * gs]);
+  }
+  if (SPLIT) {
+    red[wid][lane] = t;
+    __syncthreads();
+    if (!on) return;
+    t = red[0][lane];
+#pragma unroll
+    for (int q = 1; q < kFinWarps; ++q) t = __dadd_rn(t, red[q][lane]);
+  } else if (!on) {
+    return;
+  }
+  double out = t;
+  if (s.kap) out = __dadd_rn(out, fd);
+  if (s.decay) {
+    double sL = 0.0;
+    for (int64_t j = p.l_indptr[r]; j < p.l_indptr[r + 1]; ++j)
+      sL = __dadd_rn(sL, __dmul_rn(p.l_vals[j], p.src[(size_t)p.l_indices[j] * p.ld + col]));
+    out = __dadd_rn(out, sL);
+  }
+  out = __dmul_rn(out, s.dl);
+  if (s.inj) out = __dadd_rn(out, inj_at(p, s, r, col));
+  if (p.rec_P) record_blocked<STAGE>(p, s, r, col, t, out, p.x[idx], fx);
+  if (STAGE == 1) {
+    p.a[idx] = __dadd_rn(__dmul_rn(f0, own), __dmul_rn(__dmul_rn(f1, out), s.h));
+    p.f[idx] = out;
+  } else {
+    p.xout[idx] = __dadd_rn(own, __dmul_rn(__dmul_rn(__dadd_rn(out, -fx), s.h), f0));
   }
 }
 
-// Band partial sums with TMA staging (8 warps; the same tiles and arithmetic
-// as k_band).  Per mother species one thread issues the pair's A tiles as one
-// bulk copy (double-buffered) and the species' X block (d bins x 64 columns)
-// as one tensor-map box; each warp reads its X fragments from shared memory,
-// so no register copy of the next species is held.  One CTA barrier per
-// species; every mbarrier wait is bounded: a CTA that gives up sets p.err,
-// stops issuing, waits (bounded) for the copies it issued and leaves.
+// Band partial sums with TMA staging (the same tiles and arithmetic as k_band).
+// CTA = (8 CT columns, mother-species group, band pair).  Its warps are CT
+// column tiles x RS row splits: with RS = 1 a warp multiplies all row tiles of
+// both band species, with RS = 4 half the row tiles of one, so that at eight
+// columns all four SM quarters work.  Per mother species one thread issues the
+// pair's A tiles as bulk copies (double-buffered) and the species' X block (d
+// bins x 8 CT columns) as one tensor-map box; with CT = 1 a warp reads the next
+// species' X fragments half way through this one's products.  One CTA barrier
+// per species; every mbarrier wait is bounded: a CTA that gives up sets p.err,
+// stops issuing, waits (bounded) for the copies it issued and leaves.  A warp
+// without active columns multiplies nothing.
+//
+// Bound by the FP64 tensor pipe at 64 columns (a species' 240 tiles x 8 warps x
+// 4 clocks = 7,680 of the measured 10,000), by the 80 KB of A tiles per species
+// from L2 at 8.
 constexpr int kErrBandWait = 2;  // err code: a k_band CTA's staging wait gave up
-template <int RT, int J>
-__global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
-  extern __shared__ __align__(128) double sm[];
-  constexpr int KT = 2 * RT;
-  constexpr int ABLK = 2 * RT * J * 32;  // doubles of one (species, band pair) block
-  constexpr int XS = 8 * RT * 64;        // X of one species: bins x 64 columns
+template <int RT, int J, int CT>
+struct BandTma {
+  static constexpr int RS = CT == 8 ? 1 : 4;
+  static constexpr int kWarps = CT * RS;
+  static constexpr int KT = 2 * RT;
+  static constexpr int NB = RS == 1 ? 2 : 1;            // band species of a warp
+  static constexpr int NP = RS == 1 ? RT / 2 : RT / 4;  // pairs of row tiles of a warp and band species
+  static constexpr int ABLK = 2 * RT * J * 32;          // doubles of one (species, band pair) block
+  static constexpr int XS = 8 * RT * 8 * CT;            // X of one species: bins x 8 CT columns
+  static constexpr size_t smem = (size_t)(2 * ABLK + XS) * sizeof(double) + 4 * sizeof(unsigned long long);
+};
+template <int RT, int J, int CT>
+__global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma(StepParams p) {
+  extern __shared__ __align__(16) double sm[];
+  using B = BandTma<RT, J, CT>;
+  constexpr int KT = B::KT, NB = B::NB, NP = B::NP, ABLK = B::ABLK, NCHUNK = 8;  // bulk copies of a block
+  constexpr bool AHEAD = CT < 8;  // at CT = 8 the second fragment set costs more registers than it hides
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int cb = blockIdx.x * 64, c0 = cb + wid * 8;
+  const int ct = wid % CT, rs = wid / CT;
+  const int bw = B::RS == 1 ? 0 : rs & 1, rp0 = B::RS == 1 ? 0 : (rs >> 1) * NP;  // first band species and row pair
+  const int cb = blockIdx.x * (8 * CT), c0 = cb + ct * 8;
   const int ncols = p.sc->ncols;
-  if ((int)blockIdx.x * 64 >= ncols) return;
+  if (cb >= ncols) return;
   const bool wact = c0 < ncols;  // c0 + 7 < ld: ld is a multiple of 32
   const int pair = blockIdx.z, g = blockIdx.y;
   const int s0 = g * p.spg, s1 = min(p.nsp, s0 + p.spg);
@@ -2414,8 +2459,8 @@ __global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
   const double* __restrict__ A = p.band_vals + (size_t)w * p.band_stride;
   const int npairs = gridDim.z;
   double* As = sm;             // [2][ABLK]
-  double* Xs = As + 2 * ABLK;  // [bin][64 columns]
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(Xs + XS);  // A stage 0, A stage 1, X
+  double* Xs = As + 2 * ABLK;  // [bin][8 CT columns]
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(Xs + B::XS);  // A stage 0, A stage 1, X
   int* abort_s = reinterpret_cast<int*>(bar + 3);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
@@ -2424,30 +2469,43 @@ __global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
     *abort_s = 0;
   }
   __syncthreads();
-  auto issue = [&](int sp, int stage) {  // thread 0
+  auto issue_a = [&](int sp, int stage) {  // thread 0
     mbar_expect_tx(bar + stage, (unsigned)(ABLK * sizeof(double)));
-    bulk_load(As + stage * ABLK, A + ((size_t)sp * npairs + pair) * ABLK, (unsigned)(ABLK * sizeof(double)), bar + stage);
-    mbar_expect_tx(bar + 2, (unsigned)(64 * d * sizeof(double)));
+#pragma unroll
+    for (int q = 0; q < NCHUNK; ++q)
+      bulk_load(As + stage * ABLK + q * (ABLK / NCHUNK), A + ((size_t)sp * npairs + pair) * ABLK + q * (ABLK / NCHUNK),
+                (unsigned)(ABLK / NCHUNK * sizeof(double)), bar + stage);
+  };
+  auto issue_x = [&](int sp) {  // thread 0
+    mbar_expect_tx(bar + 2, (unsigned)(8 * CT * d * sizeof(double)));
     tma_load_3d(Xs, p.tmap_band, cb, 0, sp, bar + 2);
   };
-  if (threadIdx.x == 0 && s0 < s1) issue(s0, 0);
-  double acc[2][RT][2];
+  int last_a = s0 - 1, last_x = s0 - 1;  // the last species whose copies were issued (thread 0)
+  if (threadIdx.x == 0 && s0 < s1) {
+    issue_x(s0);
+    issue_a(s0, 0);
+    last_a = last_x = s0;
+  }
+  double acc[NB][2 * NP][2];
 #pragma unroll
-  for (int b = 0; b < 2; ++b)
+  for (int b = 0; b < NB; ++b)
 #pragma unroll
-    for (int rt = 0; rt < RT; ++rt) acc[b][rt][0] = acc[b][rt][1] = 0.0;
+    for (int rt = 0; rt < 2 * NP; ++rt) acc[b][rt][0] = acc[b][rt][1] = 0.0;
   const int kr = lane & 3;
-  int last = s0 - 1;  // the last species whose copies were issued (thread 0)
-  if (s0 < s1) last = s0;
-  for (int sp = s0; sp < s1; ++sp) {
-    const int it = sp - s0, stage = it & 1;
-    bool ok = mbar_wait_bounded(bar + 2, (unsigned)(it & 1), p.wait_tries);
-    double xf[KT];
+  double xf[KT], xn[KT];
+  auto load_x = [&](int sp, double (&x)[KT]) {  // false: the copy did not land in time
+    const bool ok = mbar_wait_bounded(bar + 2, (unsigned)((sp - s0) & 1), p.wait_tries);
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt) {
       const int e = 4 * kt + kr;
-      xf[kt] = (wact && e < d) ? Xs[e * 64 + wid * 8 + (lane >> 2)] : 0.0;
+      x[kt] = (wact && e < d) ? Xs[e * (8 * CT) + ct * 8 + (lane >> 2)] : 0.0;
     }
+    return ok;
+  };
+  bool ok = AHEAD && s0 < s1 ? load_x(s0, xf) : true;
+  for (int sp = s0; sp < s1; ++sp) {
+    const int it = sp - s0, stage = it & 1;
+    if (!AHEAD) ok = load_x(sp, xf);
     ok = mbar_wait_bounded(bar + stage, (unsigned)((it >> 1) & 1), p.wait_tries) && ok;
     if (!ok) {
       atomicExch(p.err, kErrBandWait);
@@ -2455,41 +2513,59 @@ __global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
     }
     __syncthreads();  // every warp holds X(sp) and is done with A(sp - 1)
     if (*abort_s) break;
-    if (threadIdx.x == 0 && sp + 1 < s1) {
-      issue(sp + 1, stage ^ 1);
-      last = sp + 1;
+    const bool more = sp + 1 < s1;
+    if (threadIdx.x == 0 && more) {
+      issue_x(sp + 1);
+      issue_a(sp + 1, stage ^ 1);
+      last_a = last_x = sp + 1;
     }
     // a lane's fragments of row tiles 2p and 2p + 1 are one 16-byte word
     const double2* __restrict__ as = reinterpret_cast<const double2*>(As + stage * ABLK) + lane;
+    auto products = [&](int jj) {
 #pragma unroll
-    for (int jj = 0; jj < J; ++jj)
+      for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int rp = 0; rp < RT / 2; ++rp) {
-          const int kt = 4 * rp + jj;
-          if (kt >= KT) continue;
-          const double2 a2 = as[((b * (RT / 2) + rp) * J + jj) * 32];
-          dmma884(acc[b][2 * rp][0], acc[b][2 * rp][1], a2.x, xf[kt]);
-          if (kt + 2 < KT) dmma884(acc[b][2 * rp + 1][0], acc[b][2 * rp + 1][1], a2.y, xf[kt + 2]);
+        for (int rq = 0; rq < NP; ++rq) {
+          // k-tile of the row pair: 4 (rp0 + rq) + jj; xf is indexed by constants, so rp0 selects by unrolling
+          auto mul = [&](int rp) {
+            const int kt = 4 * rp + jj;
+            if (kt >= KT) return;
+            const double2 a2 = as[(((bw + b) * (RT / 2) + rp) * J + jj) * 32];
+            dmma884(acc[b][2 * rq][0], acc[b][2 * rq][1], a2.x, xf[kt]);
+            if (kt + 2 < KT) dmma884(acc[b][2 * rq + 1][0], acc[b][2 * rq + 1][1], a2.y, xf[kt + 2]);
+          };
+          if (B::RS == 1 || rp0 == 0) mul(rq);
+          else mul(NP + rq);
         }
+    };
+    if (wact)
+#pragma unroll
+      for (int jj = 0; jj < J / 2; ++jj) products(jj);
+    if (AHEAD && more) ok = load_x(sp + 1, xn);
+    if (wact)
+#pragma unroll
+      for (int jj = J / 2; jj < J; ++jj) products(jj);
+    if (AHEAD)
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) xf[kt] = xn[kt];
   }
   if (*abort_s) {  // the copies this CTA issued land before it leaves
-    if (threadIdx.x == 0 && last >= s0) {
-      const int it = last - s0;
-      mbar_wait_bounded(bar + 2, (unsigned)(it & 1), kWaitTries);
-      mbar_wait_bounded(bar + (it & 1), (unsigned)((it >> 1) & 1), kWaitTries);
+    if (threadIdx.x == 0 && last_a >= s0) {
+      mbar_wait_bounded(bar + 2, (unsigned)((last_x - s0) & 1), kWaitTries);
+      mbar_wait_bounded(bar + ((last_a - s0) & 1), (unsigned)(((last_a - s0) >> 1) & 1), kWaitTries);
+      if (last_a > s0)
+        mbar_wait_bounded(bar + ((last_a - 1 - s0) & 1), (unsigned)(((last_a - 1 - s0) >> 1) & 1), kWaitTries);
     }
     return;
   }
   if (!wact) return;
 #pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    if (2 * pair + b >= p.nb) continue;
-    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + b) * d * ld;
+  for (int b = 0; b < NB; ++b) {
+    if (2 * pair + bw + b >= p.nb) continue;
+    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + bw + b) * d * ld;
 #pragma unroll
-    for (int rt = 0; rt < RT; ++rt) {
-      const int row = 8 * rt + (lane >> 2);
+    for (int rt = 0; rt < 2 * NP; ++rt) {
+      const int row = 8 * (2 * rp0 + rt) + (lane >> 2);
       if (row >= d) continue;
       double2 o;
       o.x = acc[b][rt][0];
@@ -2497,11 +2573,6 @@ __global__ void __launch_bounds__(256, 1) k_band_tma(StepParams p) {
       *reinterpret_cast<double2*>(P + (size_t)row * ld + c0 + kr * 2) = o;
     }
   }
-}
-
-template <int RT, int J>
-size_t band_tma_smem_bytes() {
-  return (size_t)(2 * 2 * RT * J * 32 + 8 * RT * 64) * sizeof(double) + 4 * sizeof(unsigned long long);
 }
 
 // Instances of k_band: row tiles RT (d <= 8 RT) x k-tiles per row tile J
@@ -2539,23 +2610,32 @@ BandInstance band_kernel_w(int RT, int J) {
 BandInstance band_kernel(int RT, int J, int nw = 8) {
   return nw == 4 ? band_kernel_w<4>(RT, J) : band_kernel_w<8>(RT, J);
 }
-// The TMA-staged 8-warp instance.
-template <int RT>
-BandInstance band_kernel_tma_j(int J) {
-  switch (J) {
-    case 5: return {k_band_tma<RT, 5>, band_tma_smem_bytes<RT, 5>(), 8};
-    case 9: return {k_band_tma<RT, 9>, band_tma_smem_bytes<RT, 9>(), 8};
-    case 13: return {k_band_tma<RT, 13>, band_tma_smem_bytes<RT, 13>(), 8};
-    case 17: return {k_band_tma<RT, 17>, band_tma_smem_bytes<RT, 17>(), 8};
+// The TMA-staged instances: 8 or 64 columns per CTA.
+constexpr int kBandCT[2] = {1, 8};
+template <int RT, int J>
+BandInstance band_kernel_tma_ct(int ct) {
+  switch (ct) {
+    case 1: return {k_band_tma<RT, J, 1>, BandTma<RT, J, 1>::smem, BandTma<RT, J, 1>::kWarps};
+    case 8: return {k_band_tma<RT, J, 8>, BandTma<RT, J, 8>::smem, BandTma<RT, J, 8>::kWarps};
   }
   return {nullptr, 0, 0};
 }
-BandInstance band_kernel_tma(int RT, int J) {
+template <int RT>
+BandInstance band_kernel_tma_j(int J, int ct) {
+  switch (J) {
+    case 5: return band_kernel_tma_ct<RT, 5>(ct);
+    case 9: return band_kernel_tma_ct<RT, 9>(ct);
+    case 13: return band_kernel_tma_ct<RT, 13>(ct);
+    case 17: return band_kernel_tma_ct<RT, 17>(ct);
+  }
+  return {nullptr, 0, 0};
+}
+BandInstance band_kernel_tma(int RT, int J, int ct) {
   switch (RT) {
-    case 4: return band_kernel_tma_j<4>(J);
-    case 8: return band_kernel_tma_j<8>(J);
-    case 12: return band_kernel_tma_j<12>(J);
-    case 16: return band_kernel_tma_j<16>(J);
+    case 4: return band_kernel_tma_j<4>(J, ct);
+    case 8: return band_kernel_tma_j<8>(J, ct);
+    case 12: return band_kernel_tma_j<12>(J, ct);
+    case 16: return band_kernel_tma_j<16>(J, ct);
   }
   return {nullptr, 0, 0};
 }
@@ -3622,7 +3702,7 @@ EncodeTiledFn tensor_map_encoder() {
 
 // Tensor maps of X and A as (column, bin, species) for k_slab's TMA staging
 // (box = 16 columns x 1 bin x box_rows species) and for k_band_tma's (box =
-// 64 columns x d bins x 1 species).  Leaves tma_ok false (cp.async staging)
+// 8 or 64 columns x d bins x 1 species).  Leaves tma_ok false (cp.async staging)
 // when TMA is switched off, the encoder is missing or a map is refused, and
 // tma_band_ok false when only the band maps are refused.
 int ensure_tmaps(pb_context* c, bool blocked, int ld) {
@@ -3636,14 +3716,14 @@ int ensure_tmaps(pb_context* c, bool blocked, int ld) {
   const EncodeTiledFn enc = tensor_map_encoder();
   if (!enc) return PB_OK;
   const int d = c->lay_d, nsp = c->lay_nsp;
-  CUtensorMap maps[4];
+  CUtensorMap maps[6];  // k_slab's X and A, then k_band_tma's for 8 and 64 columns
   bool band_ok = d <= 256;
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < 6; ++k) {
     const bool band = k >= 2;
     if (band && !band_ok) break;
     const cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)d, (cuuint64_t)nsp};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * sizeof(double), (cuuint64_t)d * ld * sizeof(double)};
-    const cuuint32_t box[3] = {band ? 64u : (cuuint32_t)kSlabCols, band ? (cuuint32_t)d : 1u,
+    const cuuint32_t box[3] = {band ? 8u * kBandCT[k / 2 - 1] : (cuuint32_t)kSlabCols, band ? (cuuint32_t)d : 1u,
                                band ? 1u : (cuuint32_t)SlabSmem::box_rows(nsp)};
     const cuuint32_t es[3] = {1u, 1u, 1u};
     if (enc(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, k % 2 == 0 ? c->X.p : c->A.p, dims, strides, box, es,
@@ -3714,46 +3794,71 @@ const CUtensorMap* stage_tmap_band(const pb_context* c, int stage) {
                                                           : nullptr;
 }
 
-// One stage of the bin-blocked path: k_band on the second stream, k_fd then
-// k_slab on the launching stream, then k_band_finish (and the next step's row
-// factors of the bin-local rows after stage 2).
-// k_band's grid for the active columns: column blocks of 8 nw columns and
-// mother-species groups (sets p.spg, p.ngroups).  With nw = 8 the groups fill
-// at least one wave of the SMs (a CTA per SM); with nw = 4 they stay within one
-// wave, so that each SM holds at most one k_band CTA beside its k_slab CTA.
-int band_grid(const pb_context* c, StepParams& p, int nw) {
-  const int cblocks = (int)blocks_for(p.hcols, 8 * nw);
-  const int per = cblocks * std::max(c->band_npairs, 1);
-  int G;
-  if (nw == 4) {
-    G = std::max(1, std::min({c->num_sms / per, kMaxBandGroups, p.nsp}));
+// k_band's launch for the columns p.hcols: columns per CTA and mother-species
+// groups (p.spg, p.ngroups).
+//
+// Four-warp CTAs (PB_OPT_BAND_WARPS) stay within one wave, so that each SM holds
+// at most one beside its k_slab CTA.  Otherwise there is one CTA per SM and the
+// groups are those with the shortest schedule (species per SM; the fewer on
+// ties: the partial sums grow with groups x columns).  A CTA covers 64 columns,
+// or 8 when there are no more: every CTA loads 80 KB of A tiles per species
+// whatever its columns, so narrower CTAs cost more from L2 than the idle warps of
+// wide ones (A <= 56 network, us per launch with 8 / 16 / 64 columns per CTA: 7
+// columns 14.4 / 16.8 / 18.5, 32 columns 28 / 23 / 17, 128 columns 83 / 65 / 34,
+// 512 columns 314 / 243 / 101; at most 64 groups, as before: 35 us up to 32
+// columns, 39 at 128).  The cp.async kernel takes 64 columns per CTA with the
+// same groups, so that both stagings add the same partial sums.
+struct BandPlan {
+  int ct, cblocks;
+};
+BandPlan band_plan(const pb_context* c, StepParams& p) {
+  const int np = std::max(c->band_npairs, 1);
+  BandPlan plan{p.hcols <= 8 ? 1 : 8, 1};
+  int G = 1;
+  if (c->band_warps == 4) {
+    plan.cblocks = (int)blocks_for(p.hcols, 32);
+    G = std::max(1, std::min({c->num_sms / (plan.cblocks * np), kMaxBandGroups, p.nsp}));
   } else {
-    // One CTA per SM.  At least one wave of CTAs (measured best up to
-    // K = 512); with many column blocks the launch takes ceil(CTAs / SMs)
-    // waves of CTAs that each walk ceil(nsp / G) mother species, so G is
-    // raised to the one with the fewest waves x species (the smaller on ties,
-    // at most 16 beyond one wave's worth: the partial sums grow with G x
-    // columns).  At K = 2048 this takes G from 5 to 9 and k_band from 818 to
-    // 469 us per launch.
-    const int gmax = std::min({kMaxBandGroups, p.nsp, std::max(16, c->num_sms / per)});
-    int gw = 1;
+    plan.cblocks = (int)blocks_for(p.hcols, 8 * plan.ct);
     int64_t best = -1;
-    for (int g = 1; g <= gmax; ++g) {
-      const int64_t waves = ((int64_t)per * g + c->num_sms - 1) / c->num_sms;
-      const int64_t cost = waves * ((p.nsp + g - 1) / g);
+    for (int g = 1; g <= std::min(kMaxBandGroups, p.nsp); ++g) {
+      const int spg = (p.nsp + g - 1) / g;
+      if ((p.nsp + spg - 1) / spg != g) continue;
+      // full groups first, then the last group's shorter CTAs on the SMs that are free the earliest
+      const int64_t per = (int64_t)plan.cblocks * np, full = per * (g - 1), rest = p.nsp - (int64_t)(g - 1) * spg;
+      const int64_t q = full / c->num_sms, r = full % c->num_sms, layers = (per + c->num_sms - r - 1) / (c->num_sms - r);
+      const int64_t cost = std::max(r > 0 ? (q + 1) * spg : 0, q * spg + layers * rest);
       if (best < 0 || cost < best) {
         best = cost;
-        gw = g;
+        G = g;
       }
     }
-    const int fill = (c->num_sms + per - 1) / per;
-    G = std::max(1, std::min({std::max(fill, gw), kMaxBandGroups, p.nsp}));
   }
   p.spg = (p.nsp + G - 1) / G;
   p.ngroups = (p.nsp + p.spg - 1) / p.spg;
-  return cblocks;
+  return plan;
+}
+void launch_band(const pb_context* c, StepParams& p, const BandPlan& plan, cudaStream_t st) {
+  if (c->band_warps == 8 && p.tmap_band) {
+    if (plan.ct == 8) p.tmap_band += 2;  // the maps of X and A for 8 columns, then for 64
+    const BandInstance bi = band_kernel_tma(c->band_RT, c->band_J, plan.ct);
+    bi.fn<<<dim3(plan.cblocks, p.ngroups, c->band_npairs), bi.warps * 32, bi.smem, st>>>(p);
+  } else {
+    const BandInstance bi = band_kernel(c->band_RT, c->band_J, c->band_warps);
+    bi.fn<<<dim3(blocks_for(p.hcols, 8 * bi.warps), p.ngroups, c->band_npairs), bi.warps * 32, bi.smem, st>>>(p);
+  }
 }
 
+template <int STAGE>
+void launch_finish(const StepParams& p, cudaStream_t st) {
+  const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
+  const int rows = p.nb * p.d;
+  if (p.ngroups > kFinSplit) k_band_finish<STAGE, true><<<dim3((unsigned)rows, tiles), kFinWarps * 32, 0, st>>>(p);
+  else k_band_finish<STAGE, false><<<dim3(blocks_for(rows, kFinWarps), tiles), kFinWarps * 32, 0, st>>>(p);
+}
+
+// One stage of the bin-blocked path: k_band on the second stream, k_fd then
+// k_slab on the launching stream, then k_band_finish.
 template <int STAGE>
 int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   const bool photohad = (p.flags & PB_PHOTOHAD) != 0;
@@ -3762,12 +3867,10 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   p.ngroups = 0;
   p.spg = 1;
   if (photohad && p.nb > 0) {
-    const BandInstance bi = (c->band_warps == 8 && p.tmap_band) ? band_kernel_tma(c->band_RT, c->band_J)
-                                                                : band_kernel(c->band_RT, c->band_J, c->band_warps);
-    const int cblocks = band_grid(c, p, bi.warps);
+    const BandPlan plan = band_plan(c, p);
     cudaEventRecord(c->ev_fork, st);
     cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
-    bi.fn<<<dim3(cblocks, p.ngroups, c->band_npairs), bi.warps * 32, bi.smem, c->stream2>>>(p);
+    launch_band(c, p, plan, c->stream2);
     cudaEventRecord(c->ev_join, c->stream2);
     ++launches;
   }
@@ -3797,7 +3900,7 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   }
   if (p.ngroups > 0) cudaStreamWaitEvent(st, c->ev_join, 0);
   if (p.nb > 0) {
-    k_band_finish<STAGE><<<dim3(blocks_for((int64_t)p.nb * p.d, 8), tiles), 256, 0, st>>>(p);
+    launch_finish<STAGE>(p, st);
     ++launches;
   }
   return launches;
@@ -3812,7 +3915,7 @@ void launch_adj_blocked(pb_context* c, AdjBlk& q, cudaStream_t st) {
   bool forked = false;
   if (photohad && q.nb > 0) {
     const int cblocks = (int)blocks_for(q.ncols, 64);
-    const int G = std::max(1, std::min({(c->num_sms + cblocks - 1) / cblocks, kMaxBandGroups, q.nsp}));
+    const int G = std::max(1, std::min({(c->num_sms + cblocks - 1) / cblocks, 64, q.nsp}));
     q.spg = (q.nsp + G - 1) / G;
     const int ngroups = (q.nsp + q.spg - 1) / q.spg;
     cudaEventRecord(c->ev_fork, st);
@@ -4126,7 +4229,7 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
       join_hook(c, hook_pending, st);
       int cols = 0;
       for (int64_t q = k; q < k + G; ++q) cols = std::max(cols, n_active[q]);
-      cols = K == 1 ? 1 : std::min((cols + kGraphCols - 1) / kGraphCols * kGraphCols, p.ld);
+      cols = K <= kGraphCols ? K : std::min((cols + kGraphCols - 1) / kGraphCols * kGraphCols, p.ld);
       StepGraph* g = step_graph(c, p, K, G, cols, st);
       if (!g) return -1;
       p.rf_k0 = k;
@@ -5050,9 +5153,16 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   PB_CUDA(c, cudaFuncSetAttribute(bi.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi.smem));
   PB_CUDA(c, cudaFuncSetAttribute(bi4.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bi4.smem));
   {
-    const BandInstance bt = band_kernel_tma(RT, J);
-    c->band_tma_fits = bt.fn && bt.smem <= max_smem;
-    if (c->band_tma_fits) PB_CUDA(c, cudaFuncSetAttribute(bt.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt.smem));
+    c->band_tma_fits = true;
+    for (int ct : kBandCT) {
+      const BandInstance bt = band_kernel_tma(RT, J, ct);
+      c->band_tma_fits = c->band_tma_fits && bt.fn && bt.smem <= max_smem;
+    }
+    if (c->band_tma_fits)
+      for (int ct : kBandCT) {
+        const BandInstance bt = band_kernel_tma(RT, J, ct);
+        PB_CUDA(c, cudaFuncSetAttribute(bt.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt.smem));
+      }
   }
   c->band_nb = nb;
   c->band_npairs = npairs;
@@ -5206,9 +5316,8 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   set_step_factors(p, step);
   const bool photohad = (flags & PB_PHOTOHAD) != 0, kap = (flags & PB_PARTIAL_DIFF) != 0;
   const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
-  const BandInstance bi = (c->band_warps == 8 && p.tmap_band) ? band_kernel_tma(c->band_RT, c->band_J)
-                                                              : band_kernel(c->band_RT, c->band_J, c->band_warps);
-  const int cblocks = band_grid(c, p, bi.warps);
+  const BandPlan plan = band_plan(c, p);
+  const CUtensorMap* const tmap_band = p.tmap_band;
   if (!(photohad && p.nb > 0)) p.ngroups = 0;
   for (int kk = 0; kk < 4; ++kk) ms[kk] = 0.0;
   for (int kk = 0; kk < 4; ++kk) {
@@ -5225,11 +5334,13 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
         const dim3 sg(p.d, (unsigned)blocks_for(p.hcols, kSlabCols));
         slab_kernel(stage, false, c->slab_pre)<<<sg, kSlabWarps * 32, c->slab_smem, st>>>(p);
       }
-      if (kk == 2) bi.fn<<<dim3(cblocks, p.ngroups, c->band_npairs), bi.warps * 32, bi.smem, st>>>(p);
+      if (kk == 2) {
+        p.tmap_band = tmap_band;
+        launch_band(c, p, plan, st);
+      }
       if (kk == 3) {
-        const unsigned gb = (unsigned)blocks_for((int64_t)p.nb * p.d, 8);
-        if (stage == 1) k_band_finish<1><<<dim3(gb, tiles), 256, 0, st>>>(p);
-        else k_band_finish<2><<<dim3(gb, tiles), 256, 0, st>>>(p);
+        if (stage == 1) launch_finish<1>(p, st);
+        else launch_finish<2>(p, st);
       }
       PB_CUDA(c, cudaGetLastError());
       PB_CUDA(c, cudaEventRecord(c->ev1, st));
