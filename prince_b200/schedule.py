@@ -15,12 +15,12 @@ sizes, window boundaries and per-step scalars:
 
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 
 import numpy as np
 
 from . import constants as C
-from .cosmology import H, dldz
 
 
 def z_grid(initial_z, final_z, dz):
@@ -49,30 +49,31 @@ class Schedule:
 
 def make_schedule(zg, threshold):
     zg = np.asarray(zg, dtype=np.float64)
-    n_steps = zg.size - 1
-    zs = zg[:-1]
-    win = np.zeros(max(n_steps, 0), dtype=np.int32)
-    starts = []
+    n_steps = max(zg.size - 1, 0)
+    # Scalar evaluation per step: numpy's vectorised pow/sqrt paths can differ
+    # from the scalar ones by an ulp, and the reference evaluates scalars.  Plain
+    # floats give the same bits as numpy scalars (both are the C library's pow and
+    # sqrt) in a tenth of the time.
+    zs = zg[:n_steps].tolist()
+    win, starts = [], []
     cur = None
-    for k in range(n_steps):
-        z = zs[k]
+    for z in zs:
         if cur is None or abs(z - cur) > threshold:
             cur = z
             starts.append(z)
-        win[k] = len(starts) - 1
+        win.append(len(starts) - 1)
     if not starts:
         starts = [zg[0]]
-    # Scalar evaluation per step: numpy's vectorised pow/sqrt paths can differ
-    # from the scalar ones by an ulp, and the reference evaluates scalars.
-    cm2sec = C.PRINCE_UNITS.cm2sec
-    dl = np.array([dldz(z) for z in zs], dtype=np.float64)
-    hc = np.array([H(z) * cm2sec for z in zs], dtype=np.float64)
+    cm2sec = float(C.PRINCE_UNITS.cm2sec)
+    om, ol, h0 = float(C.Omega_m), float(C.Omega_Lambda), float(C.H_0s)
+    hz = [h0 * math.sqrt(om * (1 + z) ** 3 + ol) for z in zs]            # cosmology.H
+    dl = [-1.0 / ((1.0 + z) * h * cm2sec) for z, h in zip(zs, hz)]       # cosmology.dldz
     return Schedule(
         z=zg,
-        window=win,
+        window=np.array(win, dtype=np.int32),
         z_window=np.asarray(starts, dtype=np.float64),
         h=zg[1:] - zg[:-1],
-        dldz=dl,
-        hc=hc,
+        dldz=np.array(dl, dtype=np.float64),
+        hc=np.array([h * cm2sec for h in hz], dtype=np.float64),
         finj=np.array([d * 1.0 * cm2sec for d in dl], dtype=np.float64),
     )

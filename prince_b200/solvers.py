@@ -222,17 +222,15 @@ def _other_grids(run):
 
 
 def _coefficients(sources, zs):
-    """(n_steps, n_src) table of norm * evolution(z_k) per source."""
-    if not sources:
-        return np.zeros((zs.size, 0))
-    cols = []
-    for s in sources:
+    """(n_steps, n_src) table of norm * evolution(z_k) per source (the transpose of a table with a row per source)."""
+    out = np.empty((len(sources), zs.size))
+    for row, s in zip(out, sources):
         if hasattr(s, "evolution_array"):
             ev = s.evolution_array(zs)
         else:
             ev = np.array([s.evolution(z) for z in zs])
-        cols.append(s.norm * np.asarray(ev, dtype=np.float64))
-    return np.stack(cols, axis=1)
+        np.multiply(s.norm, np.asarray(ev, dtype=np.float64), out=row)
+    return out.T
 
 
 class UHECRPropagationSolverETD2:
@@ -377,7 +375,7 @@ class UHECRPropagationSolverETD2:
         srcs = [s for c in cols for s in c]
         owner = np.array([k for k, c in enumerate(cols) for _ in c], dtype=np.int64)
         zs = zg[:-1]
-        coeff = _coefficients(srcs, zs) if srcs else np.zeros((zs.size, 0))
+        coeff = _coefficients(srcs, zs).T   # a row per source
         grids = [np.asarray(s.injection_grid, dtype=np.float64) for s in srcs]
         # injected states of each source (sources of this package record them when they build their grid)
         support = [s.injection_support if getattr(s, "injection_support", None) is not None else np.flatnonzero(g)
@@ -385,11 +383,11 @@ class UHECRPropagationSolverETD2:
         use_inj = self.enable_injection_jacobian and len(srcs) > 0
         # first step at which each column receives a non-zero injection
         first = np.full(K, sched.n_steps, dtype=np.int64)
-        if use_inj:
+        if use_inj and sched.n_steps > 0:
             injects = np.array([sp.size > 0 for sp in support])
-            live = (coeff != 0.0) & injects[None, :]
-            has = live.any(axis=0)
-            first_src = np.where(has, live.argmax(axis=0), sched.n_steps)
+            live = coeff != 0.0
+            has = live.any(axis=1) & injects
+            first_src = np.where(has, live.argmax(axis=1), sched.n_steps)
             np.minimum.at(first, owner, first_src)
         perm = np.argsort(first, kind="stable")          # device column j <- user column perm[j]
         inv = np.empty(K, dtype=np.int64)
@@ -398,11 +396,17 @@ class UHECRPropagationSolverETD2:
         src_order = np.argsort(inv[owner], kind="stable") if srcs else np.zeros(0, dtype=np.int64)
         src_col = inv[owner][src_order].astype(np.int32)
         if srcs:
-            rows = np.unique(np.concatenate(support)).astype(np.int32)
-            G = np.stack([grids[si][rows] for si in src_order], axis=1)
+            injected = np.zeros(self.dim_states, dtype=bool)
+            for sp in support:
+                injected[sp] = True
+            rows = np.flatnonzero(injected).astype(np.int32)
+            G = np.empty((len(srcs), rows.size))
+            for row, si in zip(G, src_order):
+                np.take(grids[si], rows, out=row)
+            G = np.ascontiguousarray(G.T)
         else:
             rows, G = np.zeros(0, np.int32), np.zeros((0, 0))
-        return sched, K, coeff[:, src_order] if srcs else coeff, rows, G, src_col, n_active, perm, use_inj
+        return sched, K, np.ascontiguousarray(coeff[src_order].T), rows, G, src_col, n_active, perm, use_inj
 
     def solve(self, dz=1e-3, verbose=False, summary=False, progressbar=False):
         start = time.time()
