@@ -195,6 +195,19 @@ def _i64a(a):
     return np.ascontiguousarray(a, dtype=np.int64)
 
 
+def host_buffer(shape):
+    """A page-locked float64 host array for results (the device-to-host copy runs
+    at the link's rate instead of through a staging buffer); a plain array when
+    pinned memory is not available.  torch's caching host allocator reuses the
+    blocks of released results."""
+    try:
+        import torch
+
+        return torch.empty(shape, dtype=torch.float64, pin_memory=True).numpy()
+    except Exception:
+        return np.empty(shape)
+
+
 class Context:
     """One device context of the C library."""
 
@@ -278,8 +291,8 @@ class Context:
         keep = [_f64(E), _f64(zs), _f64(dl_step), _f64(eps), _f64(eps_o), _f64(mu)]
         E_, z_, dl_, eps_, epso_, mu_ = keep
         n, nz = E_.size, z_.size
-        Tg = np.empty((nz, n, n))
-        Te = np.empty((nz, n, n))
+        Tg = host_buffer((nz, n, n))
+        Te = host_buffer((nz, n, n))
         it = C.c_int32(0)
         a = EmTransferArgs()
         a.n, a.E = n, _ptr(E_, C.c_double)
@@ -300,7 +313,7 @@ class Context:
         from .constants import PRINCE_UNITS as U
 
         Ee, Ep, ep, z = _f64(E_e), _f64(E_p), _f64(eps), _f64(np.atleast_1d(zs))
-        R = np.empty((z.size, Ee.size, Ep.size))
+        R = host_buffer((z.size, Ee.size, Ep.size))
         a = BhShapeArgs()
         a.n_e, a.E_e, a.n_p, a.E_p = Ee.size, _ptr(Ee, C.c_double), Ep.size, _ptr(Ep, C.c_double)
         a.n_eps, a.eps, a.n_z, a.z = ep.size, _ptr(ep, C.c_double), z.size, _ptr(z, C.c_double)

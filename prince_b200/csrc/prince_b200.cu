@@ -64,11 +64,54 @@ struct __align__(16) StepScal {
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------
+struct DBuf;
+// Device memory of the cascade builds' temporaries, kept between calls: each call
+// hands it out from the start.  What does not fit is allocated on its own and
+// the next call starts with enough in one piece (allocating and freeing the
+// about 45 buffers of a build took a quarter of its time).
+struct Arena {
+  void* p = nullptr;
+  size_t bytes = 0, used = 0, want = 0;
+  void begin() {  // no work on the memory may be in flight
+    if (want > bytes) {
+      if (p) cudaFree(p);
+      p = nullptr;
+      bytes = 0;
+      if (cudaMalloc(&p, want) == cudaSuccess) bytes = want;
+      else cudaGetLastError();
+    }
+    used = want = 0;
+  }
+  void* take(size_t n) {
+    n = (n + 255) / 256 * 256;
+    want += n;
+    if (used + n > bytes) return nullptr;
+    void* q = static_cast<char*>(p) + used;
+    used += n;
+    return q;
+  }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    bytes = used = want = 0;
+  }
+};
 struct DBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  Arena* arena = nullptr;  // temporaries: memory comes from here while it lasts
+  bool lent = false;
   cudaError_t ensure(size_t want) {
     if (want <= bytes && p) return cudaSuccess;
+    if (arena) {
+      release();
+      if (void* q = arena->take(std::max<size_t>(want, 16))) {
+        p = q;
+        bytes = want;
+        lent = true;
+        return cudaSuccess;
+      }
+    }
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
@@ -78,9 +121,10 @@ struct DBuf {
     return e;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && !lent) cudaFree(p);
     p = nullptr;
     bytes = 0;
+    lent = false;
   }
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
@@ -237,6 +281,7 @@ struct pb_context {
   uint32_t last_flags = 0;
   double last_scale = 1.0;
 
+  Arena em_arena;                   // temporaries of pb_em_transfer and pb_bh_shape
   // captured runs of steps
   std::vector<StepGraph> step_graphs;
   uint64_t graph_clock = 0;
@@ -4518,6 +4563,7 @@ void pb_destroy(pb_context* c) {
   if (c->stream3) cudaStreamSynchronize(c->stream3);
   for (DBuf* b : all_buffers(c)) b->release();
   for (StepGraph& g : c->step_graphs) cudaGraphExecDestroy(g.exec);
+  c->em_arena.release();
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   cudaEventDestroy(c->ev2);
@@ -5573,7 +5619,13 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   std::vector<DBuf*> all{&dE_d, &E_d, &z_d, &dl_d, &eps_d, &weps_d, &epso_d, &wo_d, &mu_d, &E1_d, &w1_d, &b_d, &f_d,
                          &N, &No, &Ae, &Ap, &Bl, &Kt, &raw, &rawdN, &rawt, &emis, &pair, &P, &Sg, &cold, &De,
                          &Mic, &loss, &Pe, &epsm, &G, &e, &esc, &fin, &T1, &ec, &eh, &Gh, &Gc, &done, &Te};
-  auto cleanup = [&]() { for (DBuf* b : all) b->release(); };
+  c->em_arena.begin();
+  for (DBuf* b : all) b->arena = &c->em_arena;
+  // on every way out: the stream is idle before the memory is handed out again
+  auto cleanup = [&]() {
+    cudaStreamSynchronize(st);
+    for (DBuf* b : all) b->release();
+  };
   auto fail_cuda = [&](cudaError_t err, const char* what) {
     cleanup();
     return fail(c, PB_ERR_CUDA, "pb_em_transfer: %s: %s", what, cudaGetErrorString(err));
@@ -5624,7 +5676,9 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   }
   DBuf pe_d, pp_d;
   all.push_back(&pe_d);
+  pe_d.arena = &c->em_arena;
   all.push_back(&pp_d);
+  pp_d.arena = &c->em_arena;
   if ((rc = upload(c, pe_d, pe.data(), pe.size())) || (rc = upload(c, pp_d, pp.data(), pp.size()))) {
     cleanup();
     return rc;
@@ -5657,6 +5711,7 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   std::vector<double> pl = pe;
   DBuf pl_d;
   all.push_back(&pl_d);
+  pl_d.arena = &c->em_arena;
   if ((rc = upload(c, pl_d, pl.data(), pl.size()))) {
     cleanup();
     return rc;
@@ -5678,6 +5733,7 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   for (int i = 0; i < n; ++i) Ein[i] = a->E[i] * dE[i];
   DBuf Ein_d;
   all.push_back(&Ein_d);
+  Ein_d.arena = &c->em_arena;
   if ((rc = upload(c, Ein_d, Ein.data(), Ein.size()))) {
     cleanup();
     return rc;
@@ -5691,16 +5747,17 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   while (passes < a->max_scatter) {
     const int batch = std::min(8, a->max_scatter - passes);
     for (int q = 0; q < batch; ++q) {
+      const int* dn = done.as<int>();
       k_em_iter_a<<<gz, T, 0, st>>>(Pe.as<double>(), dE_d.as<double>(), n, nz, G.as<double>(), esc.as<double>(),
-                                    T1.as<double>());
-      bgemm(st, P.as<double>(), T1.as<double>(), e.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, true);
+                                    T1.as<double>(), dn);
+      bgemm(st, P.as<double>(), T1.as<double>(), e.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, true, dn);
       k_em_iter_b<<<gz, T, 0, st>>>(e.as<double>(), cold.as<unsigned char>(), dE_d.as<double>(), n, nz,
-                                    ec.as<double>(), eh.as<double>());
-      bgemm(st, Mic.as<double>(), ec.as<double>(), Gc.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false);
-      bgemm(st, Sg.as<double>(), eh.as<double>(), Gh.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false);
-      bgemm(st, De.as<double>(), eh.as<double>(), e.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false);
+                                    ec.as<double>(), eh.as<double>(), dn);
+      bgemm(st, Mic.as<double>(), ec.as<double>(), Gc.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false, dn);
+      bgemm(st, Sg.as<double>(), eh.as<double>(), Gh.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false, dn);
+      bgemm(st, De.as<double>(), eh.as<double>(), e.as<double>(), n, n, n, n, n, n, snn, snn, snn, nz, false, dn);
       k_em_iter_c<<<gz, T, 0, st>>>(Pe.as<double>(), n, nz, Gh.as<double>(), Gc.as<double>(), G.as<double>(),
-                                    esc.as<double>());
+                                    esc.as<double>(), dn);
       k_em_iter_conv<<<nz, 256, 0, st>>>(Ein_d.as<double>(), Pe.as<double>(), n, a->tol, G.as<double>(),
                                          e.as<double>(), esc.as<double>(), fin.as<double>(), done.as<int>());
     }
@@ -5738,7 +5795,12 @@ int pb_bh_shape(pb_context* c, const pb_bh_shape_args* a) {
   if (rc) return rc;
   cudaStream_t st = c->stream;
   DBuf Ee, Ep, eps, zs, K, neps, col, R;
-  auto cleanup = [&]() { for (DBuf* b : {&Ee, &Ep, &eps, &zs, &K, &neps, &col, &R}) b->release(); };
+  c->em_arena.begin();
+  for (DBuf* b : {&Ee, &Ep, &eps, &zs, &K, &neps, &col, &R}) b->arena = &c->em_arena;
+  auto cleanup = [&]() {
+    cudaStreamSynchronize(st);
+    for (DBuf* b : {&Ee, &Ep, &eps, &zs, &K, &neps, &col, &R}) b->release();
+  };
   if ((rc = upload(c, Ee, a->E_e, (size_t)ne)) || (rc = upload(c, Ep, a->E_p, (size_t)np)) ||
       (rc = upload(c, eps, a->eps, (size_t)nk)) || (rc = upload(c, zs, a->z, (size_t)nz))) {
     cleanup();
