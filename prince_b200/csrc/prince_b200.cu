@@ -224,12 +224,13 @@ struct pb_context {
   bool fdT_dense_ok = false;        // the transposed stencil fits k_fdT_dense's halo
   // transposed bin-blocked structures of the adjoint sweep (one band pair)
   bool blockedT_ok = false, fdT_ok = false;
-  DBuf bandT_slot, slabT_rp, slabT_offs, slabT_slot, bandT_vals, slabT_vals, fdT_cnt, fdT_off, fdT_val;
-  DBuf slabT_pairs, slabT_wrp;  // slabT_rp: quad base per bin; slabT_offs: quads
+  DBuf bandT_slot, slabT_kbase, slabT_ebase, slabT_k, slabT_g, slabT_wrp, slabT_slot, bandT_vals, slabT_vals, fdT_cnt,
+      fdT_off, fdT_val;
   DBuf vbuf, vbuf2, bTbuf, fdTbuf, outcols;
   int64_t slabT_nent = 0;
-  int32_t slabT_maxbin = 0;
+  int32_t slabT_maxe = 0, slabT_maxk = 0, slabT_maxg = 0;  // of the largest bin
   size_t slabT_smem = 0, bandT_smem = 0;
+  bool bandT_fd = false;  // k_bandT's FD instance fits
   // small networks (k_small)
   DBuf small_order;                 // rows by coupling entries, longest first
   std::vector<int32_t> small_len;   // their coupling entries
@@ -1938,19 +1939,20 @@ struct SlabSmem {
   __host__ __device__ static int nbox(int nsp) { return (nsp + 255) / 256; }
   __host__ __device__ static int box_rows(int nsp) { return ((nsp + nbox(nsp) - 1) / nbox(nsp) + 7) / 8 * 8; }
   __host__ __device__ static int rows(int nsp) { return nbox(nsp) * box_rows(nsp); }
-  __host__ __device__ static size_t bytes(int nsp, int maxe, int maxk, int maxg) {
+  // nfac: row-factor arrays (k_slabT has none)
+  __host__ __device__ static size_t bytes(int nsp, int maxe, int maxk, int maxg, int nfac = 3) {
     return 1024 + (size_t)rows(nsp) * kSlabCols * sizeof(double) + (size_t)maxe * sizeof(double) +
-           (size_t)maxk * sizeof(SlabK) + (size_t)maxg * (sizeof(SlabG) + 3 * kSlabRows * sizeof(double)) +
+           (size_t)maxk * sizeof(SlabK) + (size_t)maxg * (sizeof(SlabG) + nfac * kSlabRows * sizeof(double)) +
            sizeof(unsigned long long);
   }
-  __device__ SlabSmem(void* base, int nsp, int maxe, int maxk, int maxg) {
+  __device__ SlabSmem(void* base, int nsp, int maxe, int maxk, int maxg, int nfac = 3) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(base);
     slab = static_cast<char*>(base) + ((1024u - (a & 1023u)) & 1023u);
     vals = reinterpret_cast<double*>(slab + (size_t)rows(nsp) * kSlabCols * sizeof(double));
     ks = reinterpret_cast<SlabK*>(vals + maxe);
     grp = reinterpret_cast<SlabG*>(ks + maxk);
     fac = reinterpret_cast<double*>(grp + maxg);
-    bar = reinterpret_cast<unsigned long long*>(fac + 3 * kSlabRows * (size_t)maxg);
+    bar = reinterpret_cast<unsigned long long*>(fac + nfac * kSlabRows * (size_t)maxg);
   }
 };
 // The 16-byte chunk c (columns 2c, 2c + 1) of slab row r.
@@ -2918,8 +2920,8 @@ void em_hook_adjoint(const EmParams& e, cudaStream_t st) {
 //    fragments stay in registers for all mother species, so no reduction
 //    across species is needed (written to bT);
 //  * bin-local part: mother rows gather from the daughters of the same bin --
-//    k_slabT with the entries in bin-major, mother-grouped order.
-// D_off^T v is k_fdT (species-major, transposed per-bin stencil).  k_slabT's
+//    k_slabT with the same 8 x 4 tiles as k_slab, over mother rows.
+// D_off^T v is part of k_bandT, or k_fdT (species-major).  k_slabT's
 // epilogue combines the parts and applies the stage update of the adjoint
 // step; it also writes the next v (v2 after stage 1; after stage 2, v1 of the
 // previous step when its factors are recorded).
@@ -2933,18 +2935,19 @@ struct AdjBlk {
   uint32_t flags;
   double h, dl;
   const double* v;          // the vector A^T is applied to (n x ld)
-  double* bT;               // n x ld: band part of M_off^T v
+  double* bT;               // n x ld: band part of M_off^T v (k_bandT's FD instances: plus kappa D_off^T v)
+  bool fd_in_band;          // bT holds the FD term
   double* fdT;              // n x ld: D_off^T v
   const double* bandT;      // [W][band_stride] transposed band tiles
   int64_t band_stride;
-  const double* slabT;      // [W][slabT_stride] bin-local entries by mother row, in quads (zero padding)
+  const double* slabT;      // [W][slabT_stride] bin-local entries by mother row, in k-tile order
   int64_t slabT_stride;
-  const int* slabT_qbase;   // [d + 1] first quad of each bin (even)
-  const unsigned long long* slabT_q;  // per quad: byte offsets of the 4 daughters' rows in the v slab, 16 bits each
-  const int4* slabT_pairs;  // mother-row pairs of k_slabT's warps: species A, B (-1: none), q0 << 16 | quads of A, of B
-  const int* slabT_wrp;     // [d][kSlabTWarps + 1] first pair of each warp of a bin's CTA
-  int slabT_maxq;           // quads of the largest bin
-  int slabT_maxp;           // row pairs of a bin
+  const int* slabT_kbase;   // [d + 1] first k-tile of each bin
+  const int* slabT_ebase;   // [d + 1] first entry of each bin
+  const SlabK* slabT_k;     // k-tiles of mother-row groups (their columns: daughters)
+  const SlabG* slabT_g;     // groups of eight mother rows
+  const int* slabT_wrp;     // [d][kSlabWarps + 1] first group of each warp of a bin's CTA
+  int slabT_maxe, slabT_maxk, slabT_maxg;  // of the largest bin
   const int* fdT_cnt;       // per bin: entries of the transposed stencil, row offsets, values
   const int* fdT_off;
   const double* fdT_val;
@@ -3074,15 +3077,29 @@ __global__ void __launch_bounds__(256) k_fdT_dense(AdjBlk q) {
 
 // bT = band part of M_off^T v.  CTA = (64-column block, mother-species group),
 // 8 warps; warp = one 8-column tile.  The warp loads the v fragments of both
-// band species once (k-tiles of 4 daughter bins, shifted by J - 2 so the band
-// below each mother row tile starts at 0); per mother species the CTA copies
-// its transposed tiles into shared memory (double-buffered cp.async) and the
-// warp accumulates RT row tiles of 8 mother bins and writes them out.
-template <int RT, int J>
+// band species once (k-tiles of 4 daughter bins); per mother species the CTA
+// copies its transposed tiles into shared memory (double-buffered cp.async) and
+// the warp accumulates RT row tiles of 8 mother bins and writes them out.
+// k-tile jj of row tile mt holds the daughter bins of tile 2 mt + jj - (J - 2);
+// those below bin 0 are not multiplied.
+//
+// FD: the sums start from kappa D_off^T v instead of zero.  The species' own v
+// block comes to shared memory beside its tiles and is multiplied by the 8 x 4
+// tiles of the transposed loss stencil (four k-tiles per row tile, the same for
+// every species), so the term needs neither its own launch nor a pass of its
+// own through memory.  Where the block does not fit beside the tiles (more than
+// 96 bins at J = 13) k_fdT forms it.
+//
+// Bound by the FP64 tensor pipe (240 + 48 of the tiles of a species x 2 warps a
+// quarter x 16 clocks = 9,200 clocks at RT = 12, J = 13).  Measured at the
+// A <= 56 network, 250 columns: 67 us with all 312 tile slots multiplied and 64
+// groups at most, 48 us now, 66 us with the loss term, which took k_fdT 21 us
+// and k_slabT 25 us a launch.
+template <int RT, int J, bool FD>
 __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   constexpr int KS = J - 2;              // k-tile shift
-  constexpr int KV = 2 * RT + KS;        // v fragments per band species
+  constexpr int KV = 2 * RT;             // v fragments per band species
   constexpr int ABLK = 2 * RT * J * 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 64 + wid * 8;
@@ -3092,11 +3109,32 @@ __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
   const int d = q.d, ld = q.ld;
   const double* __restrict__ A = q.bandT + (size_t)q.w * q.band_stride;
   double* As = sm;
+  double* Ws = As + 2 * ABLK;       // FD: [RT][4][32] fragments of D_off^T, k-tiles 2 mt - 1 .. 2 mt + 2 of row tile mt
+  double* Xs = Ws + 4 * RT * 32;    // FD: the species' own v block, d bins x 64 columns
+  auto issue_x = [&](int sp) {
+    const double* src = q.v + (size_t)sp * d * ld + blockIdx.x * 64;
+    const int cw = min(64, ld - (int)blockIdx.x * 64) / 2;  // 16-byte words of a bin's row
+    for (int t = threadIdx.x; t < d * 32; t += blockDim.x) {
+      const int e = t >> 5, c = t & 31;
+      if (c < cw) cp_async16(Xs + e * 64 + 2 * c, src + (size_t)e * ld + 2 * c);
+    }
+    cp_async_commit();
+  };
   auto issue = [&](int sp, int stage) {
     const double* src = A + (size_t)sp * ABLK;
     for (int c = threadIdx.x; c < ABLK / 2; c += blockDim.x) cp_async16(As + stage * ABLK + 2 * c, src + 2 * c);
     cp_async_commit();
   };
+  if (s0 < s1) {
+    issue(s0, 0);
+    if (FD) issue_x(s0);
+  }
+  if (FD)
+    for (int t = threadIdx.x; t < 4 * RT * 32; t += blockDim.x) {
+      const int l = t & 31, mt = t >> 7, row = 8 * mt + (l >> 2), e = 4 * (2 * mt - 1 + ((t >> 5) & 3)) + (l & 3);
+      const int o = e - row + kFdHalo;
+      Ws[t] = (row < d && e >= 0 && e < d && o >= 0 && o <= 2 * kFdHalo) ? q.fdT_dense[row * kFdDenseW + o] : 0.0;
+    }
   const int kr = lane & 3;
   double vf[2][KV];
 #pragma unroll
@@ -3105,11 +3143,10 @@ __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
     const double* vs = q.v + (size_t)(on ? q.band_spec[b] : 0) * d * ld + c0 + (lane >> 2);
 #pragma unroll
     for (int t = 0; t < KV; ++t) {
-      const int e = 4 * (t - KS) + kr;
-      vf[b][t] = (on && e >= 0 && e < d) ? vs[(size_t)e * ld] : 0.0;
+      const int e = 4 * t + kr;
+      vf[b][t] = (on && e < d) ? vs[(size_t)e * ld] : 0.0;
     }
   }
-  if (s0 < s1) issue(s0, 0);
   for (int sp = s0; sp < s1; ++sp) {
     const int stage = (sp - s0) & 1;
     if (sp + 1 < s1) {
@@ -3119,19 +3156,48 @@ __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
       cp_async_wait<0>();
     }
     __syncthreads();
-    const double* __restrict__ as = As + stage * ABLK + lane;
     double acc[RT][2];
 #pragma unroll
     for (int mt = 0; mt < RT; ++mt) acc[mt][0] = acc[mt][1] = 0.0;
+    if (FD) {  // the accumulators start from kappa D_off^T v
+      if (wact) {
+        const double* kp = q.rf + 3 * q.n + (size_t)sp * d + (lane >> 2);
+        double kf[RT];
 #pragma unroll
-    for (int jj = 0; jj < J; ++jj)
+        for (int mt = 0; mt < RT; ++mt) kf[mt] = 8 * mt + (lane >> 2) < d ? kp[8 * mt] : 0.0;
+        const double* xs = Xs + wid * 8 + (lane >> 2);
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
+        for (int t = 0; t < 2 * RT; ++t) {
+          const int e = 4 * t + kr;
+          const double x = e < d ? xs[e * 64] : 0.0;
 #pragma unroll
-        for (int mt = 0; mt < RT; ++mt)
-          dmma884(acc[mt][0], acc[mt][1], as[((b * RT + mt) * J + jj) * 32], vf[b][2 * mt + jj]);
-    __syncthreads();
+          for (int mt = (t - 1) / 2; mt <= (t + 1) / 2; ++mt)  // 2 mt - 1 <= t <= 2 mt + 2
+            if (mt < RT) dmma884(acc[mt][0], acc[mt][1], Ws[(mt * 4 + t - 2 * mt + 1) * 32 + lane], x);
+        }
+#pragma unroll
+        for (int mt = 0; mt < RT; ++mt) {
+          acc[mt][0] *= kf[mt];
+          acc[mt][1] *= kf[mt];
+        }
+      }
+      __syncthreads();
+      if (sp + 1 < s1) issue_x(sp + 1);
+    }
     if (wact) {
+      // a lane's fragments of row tiles 2p and 2p + 1 are one 16-byte word
+      const double2* __restrict__ as = reinterpret_cast<const double2*>(As + stage * ABLK) + lane;
+#pragma unroll
+      for (int jj = 0; jj < J; ++jj)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int mp = 0; mp < RT / 2; ++mp) {
+            const int kt = 4 * mp + jj - KS;  // of row tile 2 mp; 2 mp + 1 has kt + 2
+            if (kt + 2 < 0) continue;
+            const double2 a2 = as[((b * (RT / 2) + mp) * J + jj) * 32];
+            if (kt >= 0) dmma884(acc[2 * mp][0], acc[2 * mp][1], a2.x, vf[b][kt]);
+            dmma884(acc[2 * mp + 1][0], acc[2 * mp + 1][1], a2.y, vf[b][kt + 2]);
+          }
       double* __restrict__ out = q.bT + (size_t)sp * d * ld + c0 + kr * 2;
 #pragma unroll
       for (int mt = 0; mt < RT; ++mt) {
@@ -3143,120 +3209,76 @@ __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
         *reinterpret_cast<double2*>(out + (size_t)row * ld) = o;
       }
     }
+    __syncthreads();
   }
 }
 
 template <int RT, int J>
-size_t bandT_smem_bytes() {
-  return (size_t)2 * (2 * RT * J * 32) * sizeof(double);
+size_t bandT_smem_bytes(bool fd) {
+  return (size_t)(2 * (2 * RT * J * 32) + (fd ? 4 * RT * 32 + 8 * RT * 64 : 0)) * sizeof(double);
 }
 
-// k_slabT's shared memory: the v slab of one bin (nsp x 16 columns), the bin's
-// entry values (4 per quad), daughter-row byte offsets (4 x 16 bits per quad)
-// and mother-row pairs.  Every block starts on a 16-byte boundary.
-constexpr int kSlabTPre = 2;        // row pairs whose inputs a warp loads ahead
-constexpr int kSlabTWarps = 12;     // two CTAs per SM (80 registers)
-struct SlabTSmem {
-  double* slab;  // rows padded to whole TMA boxes (as k_slab's)
-  unsigned long long* bar;  // the TMA staging barrier (a 16-byte slot)
-  double* vals;
-  unsigned long long* sidx;
-  int4* pairs;
-  __host__ __device__ static size_t bytes(int nsp, int maxq, int maxp) {
-    return (size_t)SlabSmem::rows(nsp) * kSlabCols * sizeof(double) + 16 +
-           (size_t)maxq * (4 * sizeof(double) + sizeof(unsigned long long)) + (size_t)maxp * sizeof(int4);
-  }
-  __device__ SlabTSmem(double* base, int nsp, int maxq) {
-    slab = base;
-    bar = reinterpret_cast<unsigned long long*>(slab + (size_t)SlabSmem::rows(nsp) * kSlabCols);
-    vals = slab + (size_t)SlabSmem::rows(nsp) * kSlabCols + 2;
-    sidx = reinterpret_cast<unsigned long long*>(vals + (size_t)maxq * 4);
-    pairs = reinterpret_cast<int4*>(sidx + maxq);
-  }
-};
-
 // Bin-local part of M_off^T v and the adjoint stage update for every row of
-// bin e.  CTA = (bin e, 16-column tile); a half-warp owns a mother row, its
-// lane c owns column col0 + c.  The v slab of bin e arrives by TMA (boxes of a
-// tensor map over v, as in k_slab), the bin's entry quads and row pairs by
-// bulk copies, all on one bounded mbarrier wait (cp.async when TMA is off);
-// each row is summed from shared
-// memory (four accumulators, one per quad position).  The row's band term, FD
-// term, lam' (stage 1) or mu (stage 2), P and Q, and its recorded factors are
-// loaded kSlabTPre pairs ahead into registers.  Stage 1 reduces the
-// photon-scale gradient of the bin's rows inside the CTA.
-template <int STAGE>
-__global__ void __launch_bounds__(kSlabTWarps * 32, 2) k_slabT(AdjBlk q) {
-  extern __shared__ __align__(128) double sm[];  // TMA boxes land at 128-byte boundaries
+// bin e.  CTA = (bin e, 16-column tile), its mother rows in groups of eight
+// whose 8 x 4 tiles over the daughters are multiplied as k_slab's are
+// (slab_tiles; a group without daughters has no tiles).  The v slab of bin e
+// arrives by TMA (swizzled boxes of a tensor map over v), the entries, k-tiles
+// and groups by bulk copies, all on one bounded mbarrier wait (cp.async when TMA
+// is off).  A lane updates four adjacent columns of a row; the rows' band term,
+// FD term and lam' (stage 1) or mu (stage 2) are loaded before the group's
+// products.  PQ (stage 1): the photon-scale gradient of the bin's rows, reduced
+// inside the CTA.
+//
+// Bound by memory: at 250 columns 5 arrays of 69 MB in 77 us (4.5 TB/s).  Rows
+// as quads of gathered entries on half-warps 111 / 102 us a launch (stage 1 / 2)
+// with the FD term as a sixth array, these tiles 102 / 107 with it and 77 / 82
+// without; prefetching the rows' inputs to L2 made no difference.
+template <int STAGE, bool PQ>
+__global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slabT(AdjBlk q) {
+  extern __shared__ __align__(128) double sm[];
   const int nsp = q.nsp, e = blockIdx.x, d = q.d, ld = q.ld;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int half = lane >> 4, c = lane & 15;
-  const int col0 = blockIdx.y * kSlabCols, col = col0 + c;  // col < ld
-  const bool active = col < q.ncols;
-  SlabTSmem L(sm, nsp, q.slabT_maxq);
-  const int qb = q.slabT_qbase[e], nqb = q.slabT_qbase[e + 1] - qb;
-  const int pb0 = q.slabT_wrp[e * (kSlabTWarps + 1)], npb = q.slabT_wrp[e * (kSlabTWarps + 1) + kSlabTWarps] - pb0;
-  const bool photohad = (q.flags & PB_PHOTOHAD) != 0, kap = (q.flags & PB_PARTIAL_DIFF) != 0;
-  const double* mv = q.slabT + (size_t)q.w * q.slabT_stride + (size_t)qb * 4;
-  if (q.tmap_v) {  // TMA: the v slab as tensor boxes, the entries and pairs as bulk copies, one barrier
+  const int g = lane >> 2, t4 = lane & 3;
+  const int col0 = blockIdx.y * kSlabCols, colA = col0 + 4 * t4;  // this lane's columns colA .. colA + 3 (< ld)
+  const int nact = min(max(q.ncols - colA, 0), 4);
+  SlabSmem L(sm, nsp, q.slabT_maxe, q.slabT_maxk, q.slabT_maxg, 0);
+  const int kb = q.slabT_kbase[e], nk = q.slabT_kbase[e + 1] - kb;
+  const int eb = q.slabT_ebase[e], ne = q.slabT_ebase[e + 1] - eb;
+  const int gb0 = q.slabT_wrp[e * (kSlabWarps + 1)], ngb = q.slabT_wrp[e * (kSlabWarps + 1) + kSlabWarps] - gb0;
+  const bool photohad = (q.flags & PB_PHOTOHAD) != 0, kap = (q.flags & PB_PARTIAL_DIFF) != 0 && !q.fd_in_band;
+  const double* mv = q.slabT + (size_t)q.w * q.slabT_stride + eb;
+  if (q.tmap_v) {
     if (threadIdx.x == 0) mbar_init(L.bar, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
       const int nb = SlabSmem::nbox(nsp), br = SlabSmem::box_rows(nsp);
-      unsigned bytes = (unsigned)(nb * br * kSlabCols * sizeof(double)) + (unsigned)(npb * sizeof(int4));
-      if (photohad) bytes += (unsigned)(nqb * (4 * sizeof(double) + sizeof(unsigned long long)));
+      unsigned bytes = (unsigned)(nb * br * kSlabCols * sizeof(double)) + (unsigned)(ngb * sizeof(SlabG));
+      if (photohad) bytes += (unsigned)(ne * sizeof(double) + nk * sizeof(SlabK));
       mbar_expect_tx(L.bar, bytes);
-      for (int b = 0; b < nb; ++b) tma_load_3d(L.slab + (size_t)b * br * kSlabCols, q.tmap_v, col0, e, b * br, L.bar);
-      if (photohad && nqb > 0) {
-        bulk_load(L.vals, mv, (unsigned)(nqb * 4 * sizeof(double)), L.bar);
-        bulk_load(L.sidx, q.slabT_q + qb, (unsigned)(nqb * sizeof(unsigned long long)), L.bar);
+      for (int b = 0; b < nb; ++b)
+        tma_load_3d(L.slab + (size_t)b * br * kSlabCols * sizeof(double), q.tmap_v, col0, e, b * br, L.bar);
+      if (photohad && nk > 0) {
+        if (ne > 0) bulk_load(L.vals, mv, (unsigned)(ne * sizeof(double)), L.bar);
+        bulk_load(L.ks, q.slabT_k + kb, (unsigned)(nk * sizeof(SlabK)), L.bar);
       }
-      if (npb > 0) bulk_load(L.pairs, q.slabT_pairs + pb0, (unsigned)(npb * sizeof(int4)), L.bar);
+      if (ngb > 0) bulk_load(L.grp, q.slabT_g + gb0, (unsigned)(ngb * sizeof(SlabG)), L.bar);
     }
   } else {
     const double* vs = q.v + (size_t)e * ld + col0;
     for (int t = threadIdx.x; t < nsp * (kSlabCols / 2); t += blockDim.x) {
-      const int sp = t / (kSlabCols / 2), cc = 2 * (t - sp * (kSlabCols / 2));
-      cp_async16(L.slab + sp * kSlabCols + cc, vs + (size_t)sp * d * ld + cc);
+      const int sp = t / (kSlabCols / 2), cc = t - sp * (kSlabCols / 2);
+      cp_async16(const_cast<double2*>(&slab_chunk(L.slab, sp, cc)), vs + (size_t)sp * d * ld + 2 * cc);
     }
     if (photohad) {
-      for (int t = threadIdx.x; t < 2 * nqb; t += blockDim.x) cp_async16(L.vals + 2 * t, mv + 2 * t);
-      const unsigned long long* mq = q.slabT_q + qb;
-      for (int t = threadIdx.x; t < nqb / 2; t += blockDim.x) cp_async16(L.sidx + 2 * t, mq + 2 * t);
+      for (int t = threadIdx.x; t < ne / 2; t += blockDim.x) cp_async16(L.vals + 2 * t, mv + 2 * t);
+      for (int t = threadIdx.x; t < nk; t += blockDim.x) cp_async16(L.ks + t, q.slabT_k + kb + t);
     }
-    for (int t = threadIdx.x; t < npb; t += blockDim.x) cp_async16(L.pairs + t, q.slabT_pairs + pb0 + t);
+    for (int t = threadIdx.x; t < 2 * ngb; t += blockDim.x)  // two 16-byte halves per group
+      cp_async16(reinterpret_cast<char*>(L.grp) + 16 * t, reinterpret_cast<const char*>(q.slabT_g + gb0) + 16 * t);
     cp_async_commit();
   }
-  const int w0 = q.slabT_wrp[e * (kSlabTWarps + 1) + wid], w1 = q.slabT_wrp[e * (kSlabTWarps + 1) + wid + 1];
+  const int w0 = q.slabT_wrp[e * (kSlabWarps + 1) + wid] - gb0, w1 = q.slabT_wrp[e * (kSlabWarps + 1) + wid + 1] - gb0;
   const double* own_src = STAGE == 1 ? q.lam : q.mu;
-  const bool want_pq = STAGE == 1 && q.gs;
-  constexpr int PRE = kSlabTPre;
-  // per pair slot: band term, FD term, own (lam' or mu), P, Q; kappa and the
-  // row factors (stage 1: phi1, phi2; stage 2: eD, phi2 of the previous step)
-  double rb[PRE], rfd[PRE], rown[PRE], rp[PRE], rq[PRE], rk[PRE], rf1[PRE], rf2[PRE];
-  int rsl[PRE];
-#define PB_SLABT_LOAD(U, PI, PR)                                                 \
-  do {                                                                           \
-    if ((PI) < w1) {                                                             \
-      const int4 pr_ = (PR);                                                     \
-      const int sp_ = half ? pr_.y : pr_.x;                                      \
-      if (sp_ >= 0) {                                                            \
-        const int r_ = sp_ * d + e;                                              \
-        const size_t ix_ = (size_t)r_ * ld + col;                                \
-        rb[U] = photohad ? q.bT[ix_] : 0.0;                                      \
-        rfd[U] = kap ? q.fdT[ix_] : 0.0;                                         \
-        rown[U] = own_src[ix_];                                                  \
-        rp[U] = want_pq ? q.P[ix_] : 0.0;                                        \
-        rq[U] = want_pq ? q.Q[ix_] : 0.0;                                        \
-        rk[U] = kap ? q.rf[3 * q.n + r_] : 0.0;                                  \
-        rf1[U] = STAGE == 1 ? q.rf[q.n + r_] : q.rf[r_];                         \
-        rf2[U] = STAGE == 1 ? q.rf[2 * q.n + r_] : (q.rf_prev ? q.rf_prev[2 * q.n + r_] : 0.0); \
-        rsl[U] = (STAGE == 1 && q.gb_inj) ? q.inj_slot[r_] : -1;                 \
-      }                                                                          \
-    }                                                                            \
-  } while (0)
-#pragma unroll
-  for (int u = 0; u < PRE; ++u) PB_SLABT_LOAD(u, w0 + u, __ldg(q.slabT_pairs + w0 + u));
   if (q.tmap_v) {
     if (!mbar_wait_bounded(L.bar, 0, q.wait_tries)) {  // the copies did not land: report and leave
       if (threadIdx.x == 0) atomicExch(q.err, kErrStagingWait);
@@ -3268,72 +3290,93 @@ __global__ void __launch_bounds__(kSlabTWarps * 32, 2) k_slabT(AdjBlk q) {
   }
   __syncthreads();
 
-  double gsa = 0.0;  // this lane's column of the photon-scale gradient over its rows
-  const char* slb = reinterpret_cast<const char*>(L.slab + c);
-  const double2* vq = reinterpret_cast<const double2*>(L.vals);
-  for (int pb = w0; pb < w1; pb += PRE) {
-#pragma unroll
-    for (int u = 0; u < PRE; ++u) {
-      const int pi = pb + u;
-      if (pi >= w1) break;
-      const int4 pr = L.pairs[pi - pb0];
-      const int sp = half ? pr.y : pr.x;
-      const int qq = half ? pr.w : pr.z;
-      const int r = sp * d + e;
-      double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-      if (sp >= 0 && photohad) {
-        const int qa = qq >> 16, qz = qa + (qq & 0xffff);
-#pragma unroll 2
-        for (int k = qa; k < qz; ++k) {
-          const double2 va = vq[2 * k], vb = vq[2 * k + 1];
-          const unsigned long long m = L.sidx[k];
-          const double x0 = *reinterpret_cast<const double*>(slb + ((unsigned)m & 0xffffu));
-          const double x1 = *reinterpret_cast<const double*>(slb + ((unsigned)(m >> 16) & 0xffffu));
-          const double x2 = *reinterpret_cast<const double*>(slb + ((unsigned)(m >> 32) & 0xffffu));
-          const double x3 = *reinterpret_cast<const double*>(slb + (unsigned)(m >> 48));
-          acc0 = __fma_rn(va.x, x0, acc0);
-          acc1 = __fma_rn(va.y, x1, acc1);
-          acc2 = __fma_rn(vb.x, x2, acc2);
-          acc3 = __fma_rn(vb.y, x3, acc3);
-        }
+  double gsa[4] = {0.0, 0.0, 0.0, 0.0};  // the photon-scale gradient of this lane's columns over its rows
+  for (int gi = w0; gi < w1; ++gi) {
+    const SlabG* G = L.grp + gi;
+    const unsigned sp = G->sp[g];
+    const bool have = sp != 0xffffu && nact > 0;
+    const int r = have ? (int)sp * d + e : e;
+    const size_t ro = (size_t)r * ld + colA;
+    double rb[4] = {0.0, 0.0, 0.0, 0.0}, rfd[4] = {0.0, 0.0, 0.0, 0.0}, own[4] = {0.0, 0.0, 0.0, 0.0};
+    double rk = 0.0, rf1 = 0.0, rf2 = 0.0;  // kappa; stage 1: phi1, phi2; stage 2: eD, phi2 of the previous step
+    int slot = -1;
+    if (have) {
+      if (photohad) load4(q.bT + ro, rb);
+      if (kap) {
+        load4(q.fdT + ro, rfd);
+        rk = q.rf[3 * q.n + r];
       }
-      if (sp >= 0 && active) {
-        double out = photohad ? ((acc0 + acc1) + (acc2 + acc3)) + rb[u] : 0.0;
-        if (kap) out += rk[u] * rfd[u];
-        if (q.lt_indptr) {
-          double sL = 0.0;
-          for (int64_t j = q.lt_indptr[r]; j < q.lt_indptr[r + 1]; ++j)
-            sL += q.lt_vals[j] * q.v[(size_t)q.lt_indices[j] * ld + col];
-          out += sL;
-        }
-        out *= q.dl;
-        const size_t idx = (size_t)r * ld + col;
-        if (STAGE == 1) {
-          const double lam = rown[u];
-          const double mu = lam + q.h * out;
-          q.mu[idx] = mu;
-          if (rsl[u] >= 0) q.gb_inj[(size_t)rsl[u] * ld + col] = q.h * rf1[u] * mu;
-          if (want_pq) gsa += mu * rp[u] + lam * rq[u];
-          q.vout[idx] = rf1[u] * mu - rf2[u] * lam;
-        } else {
-          const double lam = rf1[u] * rown[u] + q.h * out;
-          q.lam_out[idx] = lam;
-          if (q.rf_prev) q.vout[idx] = rf2[u] * lam;
-        }
-      }
-      const int pn = pi + PRE;
-      PB_SLABT_LOAD(u, pn, L.pairs[pn - pb0]);
+      load4(own_src + ro, own);
+      rf1 = STAGE == 1 ? q.rf[q.n + r] : q.rf[r];
+      rf2 = STAGE == 1 ? q.rf[2 * q.n + r] : (q.rf_prev ? q.rf_prev[2 * q.n + r] : 0.0);
+      if (STAGE == 1 && q.gb_inj) slot = q.inj_slot[r];
     }
+    double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
+    if (photohad) slab_tiles<2>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, acc0, acc1);
+    if (have) {
+      const double sM[4] = {acc0[0], acc1[0], acc0[1], acc1[1]};
+      double out[4], res[4], nv[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        out[c] = photohad ? sM[c] + rb[c] : 0.0;
+        if (kap) out[c] += rk * rfd[c];
+      }
+      if (q.lt_indptr) {
+        double sL[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int64_t j = q.lt_indptr[r]; j < q.lt_indptr[r + 1]; ++j) {
+          const double lv = q.lt_vals[j];
+          double xv[4];
+          load4(q.v + (size_t)q.lt_indices[j] * ld + colA, xv);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sL[c] += lv * xv[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) out[c] += sL[c];
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        out[c] *= q.dl;
+        if (STAGE == 1) {
+          res[c] = own[c] + q.h * out[c];
+          nv[c] = rf1 * res[c] - rf2 * own[c];
+        } else {
+          res[c] = rf1 * own[c] + q.h * out[c];
+          nv[c] = rf2 * res[c];
+        }
+      }
+      if (STAGE == 1) {
+        store4(q.mu + ro, res, nact);
+        store4(q.vout + ro, nv, nact);
+        if (slot >= 0) {
+          double gi4[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) gi4[c] = q.h * rf1 * res[c];
+          store4(q.gb_inj + (size_t)slot * ld + colA, gi4, nact);
+        }
+        if (PQ) {
+          double rp[4], rq[4];
+          load4(q.P + ro, rp);
+          load4(q.Q + ro, rq);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c < nact) gsa[c] += res[c] * rp[c] + own[c] * rq[c];
+        }
+      } else {
+        store4(q.lam_out + ro, res, nact);
+        if (q.rf_prev) store4(q.vout + ro, nv, nact);
+      }
+    }
+    __syncwarp();
   }
-#undef PB_SLABT_LOAD
-  if (want_pq) {  // the half-warps' sums for each column, added to the bin's row of gs
+  if (PQ) {  // the 8 x kSlabWarps partial sums of each column, added to the bin's row of gs
     __syncthreads();
-    double* red = L.slab;  // the slab is no longer read
-    red[threadIdx.x] = gsa;
+    double* red = reinterpret_cast<double*>(L.slab);  // the slab is no longer read
+#pragma unroll
+    for (int c = 0; c < 4; ++c) red[(wid * 8 + g) * kSlabCols + 4 * t4 + c] = gsa[c];
     __syncthreads();
     if (threadIdx.x < kSlabCols && col0 + (int)threadIdx.x < q.ncols) {
       double t = 0.0;
-      for (int h = 0; h < 2 * kSlabTWarps; ++h) t += red[h * kSlabCols + threadIdx.x];
+      for (int h = 0; h < 8 * kSlabWarps; ++h) t += red[h * kSlabCols + threadIdx.x];
       q.gs[(size_t)e * ld + col0 + threadIdx.x] += t;
     }
   }
@@ -3345,21 +3388,21 @@ struct BandTInstance {
   size_t smem;
 };
 template <int RT>
-BandTInstance bandT_kernel_j(int J) {
+BandTInstance bandT_kernel_j(int J, bool fd) {
   switch (J) {
-    case 5: return {k_bandT<RT, 5>, bandT_smem_bytes<RT, 5>()};
-    case 9: return {k_bandT<RT, 9>, bandT_smem_bytes<RT, 9>()};
-    case 13: return {k_bandT<RT, 13>, bandT_smem_bytes<RT, 13>()};
-    case 17: return {k_bandT<RT, 17>, bandT_smem_bytes<RT, 17>()};
+    case 5: return {fd ? k_bandT<RT, 5, true> : k_bandT<RT, 5, false>, bandT_smem_bytes<RT, 5>(fd)};
+    case 9: return {fd ? k_bandT<RT, 9, true> : k_bandT<RT, 9, false>, bandT_smem_bytes<RT, 9>(fd)};
+    case 13: return {fd ? k_bandT<RT, 13, true> : k_bandT<RT, 13, false>, bandT_smem_bytes<RT, 13>(fd)};
+    case 17: return {fd ? k_bandT<RT, 17, true> : k_bandT<RT, 17, false>, bandT_smem_bytes<RT, 17>(fd)};
   }
   return {nullptr, 0};
 }
-BandTInstance bandT_kernel(int RT, int J) {
+BandTInstance bandT_kernel(int RT, int J, bool fd) {
   switch (RT) {
-    case 4: return bandT_kernel_j<4>(J);
-    case 8: return bandT_kernel_j<8>(J);
-    case 12: return bandT_kernel_j<12>(J);
-    case 16: return bandT_kernel_j<16>(J);
+    case 4: return bandT_kernel_j<4>(J, fd);
+    case 8: return bandT_kernel_j<8>(J, fd);
+    case 12: return bandT_kernel_j<12>(J, fd);
+    case 16: return bandT_kernel_j<16>(J, fd);
   }
   return {nullptr, 0};
 }
@@ -3604,8 +3647,8 @@ std::vector<DBuf*> solve_buffers(pb_context* c) {
           &c->em_es, &c->em_lep, &c->em_y, &c->em_TgT, &c->em_TeT, &c->em_RT, &c->em_dlw,
           &c->band_slot, &c->band_spec, &c->slab_spec, &c->band_vals, &c->band_part, &c->slab_kbase,
           &c->slab_ebase, &c->slab_k, &c->slab_g, &c->slab_slot, &c->slab_vals, &c->slab_wrp, &c->slab_rowslot, &c->slab_fac, &c->fd_cnt, &c->fd_off, &c->fd_val, &c->fd_dense, &c->fdT_dense, &c->fdbuf,
-          &c->bandT_slot, &c->slabT_rp, &c->slabT_offs, &c->slabT_slot, &c->fdT_cnt, &c->fdT_off, &c->fdT_val,
-          &c->slabT_pairs, &c->slabT_wrp, &c->tmaps, &c->d_err, &c->tab_z, &c->tab_le, &c->tab_v};
+          &c->bandT_slot, &c->slabT_kbase, &c->slabT_ebase, &c->slabT_k, &c->slabT_g, &c->slabT_wrp, &c->slabT_slot,
+          &c->fdT_cnt, &c->fdT_off, &c->fdT_val, &c->tmaps, &c->d_err, &c->tab_z, &c->tab_le, &c->tab_v};
 }
 
 // Every device buffer: the solve's and the adjoint's scratch.
@@ -3808,7 +3851,7 @@ int ensure_tmapsT(pb_context* c, int ld) {
     const cuuint32_t box[3] = {(cuuint32_t)kSlabCols, 1u, (cuuint32_t)SlabSmem::box_rows(nsp)};
     const cuuint32_t es[3] = {1u, 1u, 1u};
     if (enc(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, k == 0 ? c->vbuf.p : c->vbuf2.p, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return PB_OK;
   }
@@ -3951,31 +3994,36 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   return launches;
 }
 
-// One stage of the bin-blocked adjoint sweep: k_bandT on the second stream,
-// k_fdT on the launching stream, then k_slabT.
+// One stage of the bin-blocked adjoint sweep: k_bandT on the second stream, with
+// the FD term where that fits and else k_fdT on the launching stream, then
+// k_slabT.
 template <int STAGE>
 void launch_adj_blocked(pb_context* c, AdjBlk& q, cudaStream_t st) {
   const bool photohad = (q.flags & PB_PHOTOHAD) != 0, kap = (q.flags & PB_PARTIAL_DIFF) != 0;
   const unsigned tiles = (unsigned)blocks_for(q.ncols, kColTile);
   bool forked = false;
+  q.fd_in_band = false;
   if (photohad && q.nb > 0) {
     const int cblocks = (int)blocks_for(q.ncols, 64);
-    const int G = std::max(1, std::min({(c->num_sms + cblocks - 1) / cblocks, 64, q.nsp}));
+    // one wave: a group writes its own species' rows, so more groups cost nothing
+    const int G = std::max(1, std::min(c->num_sms / cblocks, (int)q.nsp));
     q.spg = (q.nsp + G - 1) / G;
     const int ngroups = (q.nsp + q.spg - 1) / q.spg;
     cudaEventRecord(c->ev_fork, st);
     cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
-    const BandTInstance bi = bandT_kernel(c->band_RT, c->band_J);
+    q.fd_in_band = kap && c->fdT_dense_ok && c->bandT_fd;
+    const BandTInstance bi = bandT_kernel(c->band_RT, c->band_J, q.fd_in_band);
     bi.fn<<<dim3(cblocks, ngroups), 256, bi.smem, c->stream2>>>(q);
     cudaEventRecord(c->ev_join, c->stream2);
     forked = true;
   }
-  if (kap && c->fdT_dense_ok)
+  if (kap && !q.fd_in_band && c->fdT_dense_ok)
     k_fdT_dense<<<dim3(q.nsp, tiles), 256, (size_t)q.d * (kColTile + kFdDenseW) * sizeof(double), st>>>(q);
-  else if (kap)
+  else if (kap && !q.fd_in_band)
     k_fdT<<<dim3(q.nsp, tiles), 256, (size_t)q.d * kColTile * sizeof(double), st>>>(q);
   if (forked) cudaStreamWaitEvent(st, c->ev_join, 0);
-  k_slabT<STAGE><<<dim3(q.d, (unsigned)blocks_for(q.ncols, kSlabCols)), kSlabTWarps * 32, c->slabT_smem, st>>>(q);
+  const auto slabT = STAGE == 1 && q.gs ? k_slabT<STAGE, STAGE == 1> : k_slabT<STAGE, false>;
+  slabT<<<dim3(q.d, (unsigned)blocks_for(q.ncols, kSlabCols)), kSlabWarps * 32, c->slabT_smem, st>>>(q);
 }
 
 // The EM hook's operands for the step sc on the n x ld buffer X (a state, or the adjoint's lam).
@@ -5237,97 +5285,57 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
         const int sp = ix[j] / d, e2 = ix[j] % d;   // mother species and bin
         const int mt = e2 / 8, jj = e / 4 - 2 * mt + (J - 2);
         if (jj < 0 || jj >= J) return PB_OK;
-        const size_t tile = ((size_t)sp * 2 + b) * RT + mt;
-        btslot[j] = (int32_t)((tile * J + jj) * 32 + (e2 % 8) * 4 + (e % 4));
+        // row tiles in pairs, as the forward tiles
+        const size_t tile = ((size_t)sp * 2 + b) * (RT / 2) + mt / 2;
+        btslot[j] = (int32_t)(((tile * J + jj) * 32 + (e2 % 8) * 4 + (e % 4)) * 2 + (mt & 1));
       }
     }
-  // transposed bin-local rows (mothers), per bin: every species is a row; its
-  // daughter entries in the order (daughter species in k_slab's species order,
-  // CSR order), in quads of 4 (daughter slab byte offsets, zero values pad the
-  // last quad); rows paired for k_slabT's half-warps and the pairs spread over
-  // its warps longest-processing-time first; every bin starts on an even quad.
-  std::vector<std::vector<std::pair<int32_t, int64_t>>> bym(nsp);
-  std::vector<int32_t> tqbase((size_t)d + 1, 0), twrp((size_t)d * (kSlabTWarps + 1), 0), tpairs;
-  std::vector<unsigned long long> tquad;
+  // transposed bin-local rows (mothers), per bin: every species is a row, its
+  // columns the daughters of the same bin; groups and k-tiles as the forward rows'
   std::vector<int32_t> tslot((size_t)std::max<int64_t>(R, 1), -1);
-  int32_t tmax = 0;
-  bool tq_fit = (size_t)nsp * kSlabCols * sizeof(double) <= (1 << 16);
+  SlabTiles ttiles(d, nsp, kSlabWarps);
   {
-    std::vector<int32_t> nqm(nsp), order(nsp);
-    std::vector<std::vector<int32_t>> wl(kSlabTWarps);
-    std::vector<int64_t> load(kSlabTWarps);
+    std::vector<SlabTiles::Row> rows((size_t)nsp);
     for (int e = 0; e < d; ++e) {
-      for (auto& v : bym) v.clear();
+      for (int m = 0; m < nsp; ++m) {
+        rows[m].sp = m;
+        rows[m].ent.clear();
+      }
       for (int i = 0; i < nss; ++i) {
         const int64_t r = (int64_t)sspec[i] * d + e;
         for (int64_t j = ip[r]; j < ip[r + 1]; ++j)
-          if (ix[j] != r) bym[ix[j] / d].push_back({sspec[i], j});
+          if (ix[j] != r) rows[ix[j] / d].ent.push_back({sspec[i], j});
       }
-      tqbase[e] = (int32_t)tquad.size();
-      for (int m = 0; m < nsp; ++m) {
-        nqm[m] = (int32_t)((bym[m].size() + 3) / 4);
-        order[m] = m;
-      }
-      std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return nqm[a] > nqm[b]; });
-      for (auto& v : wl) v.clear();
-      std::fill(load.begin(), load.end(), 0);
-      for (int k = 0; k < nsp; k += 2) {
-        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        wl[w].push_back(k);
-        load[w] += nqm[order[k]] + 1;
-      }
-      for (int w = 0; w < kSlabTWarps; ++w) {
-        twrp[(size_t)e * (kSlabTWarps + 1) + w] = (int32_t)(tpairs.size() / 4);
-        for (int k : wl[w]) {
-          int32_t pr[4] = {-1, -1, 0, 0};
-          for (int hf = 0; hf < 2; ++hf) {
-            if (k + hf >= nsp) continue;
-            const int m = order[k + hf];
-            const int64_t q0 = (int64_t)tquad.size() - tqbase[e];
-            int t = 0;
-            const unsigned long long pad = bym[m].empty() ? 0ull : (unsigned long long)bym[m][0].first * kSlabCols * sizeof(double);
-            for (auto& dj : bym[m]) {
-              if (t % 4 == 0) tquad.push_back(0);
-              tquad.back() |= ((unsigned long long)dj.first * kSlabCols * sizeof(double)) << (16 * (t % 4));
-              tslot[dj.second] = (int32_t)((tquad.size() - 1) * 4 + t % 4);
-              ++t;
-            }
-            for (; t % 4; ++t) tquad.back() |= pad << (16 * (t % 4));
-            if (q0 >= (1 << 15) || nqm[m] >= (1 << 16)) tq_fit = false;
-            pr[hf] = m;
-            pr[2 + hf] = (int32_t)((q0 << 16) | nqm[m]);
-          }
-          tpairs.insert(tpairs.end(), pr, pr + 4);
-        }
-      }
-      twrp[(size_t)e * (kSlabTWarps + 1) + kSlabTWarps] = (int32_t)(tpairs.size() / 4);
-      if ((tquad.size() - tqbase[e]) % 2) tquad.push_back(0);
-      tmax = std::max<int32_t>(tmax, (int32_t)(tquad.size() - tqbase[e]));
+      ttiles.add_bin(rows, tslot, [](int32_t, int32_t) {});
     }
-    tqbase[d] = (int32_t)tquad.size();
-    if (tquad.empty()) tquad.assign(2, 0);
+    ttiles.finish();
   }
-  if (!tq_fit) return PB_OK;
-  // at least one double per thread: stage 1 reduces the gradient over the slab's space
-  const size_t tsm = std::max(SlabTSmem::bytes(nsp, tmax, (nsp + 1) / 2), (size_t)kSlabTWarps * 32 * sizeof(double));
-  const BandTInstance bti = bandT_kernel(RT, J);
+  // k_slabT reduces the photon-scale gradient over the slab's space
+  const size_t tsm = std::max(SlabSmem::bytes(nsp, ttiles.maxe, ttiles.maxk, ttiles.maxg, 0),
+                              1024 + (size_t)kSlabWarps * 8 * kSlabCols * sizeof(double));
+  const BandTInstance bti = bandT_kernel(RT, J, false), btf = bandT_kernel(RT, J, true);
   if (tsm > max_smem || !bti.fn || bti.smem > max_smem || (size_t)d * kColTile * sizeof(double) > max_smem) return PB_OK;
   if ((rc = upload(c, c->bandT_slot, btslot.data(), btslot.size()))) return rc;
-  if ((rc = upload(c, c->slabT_rp, tqbase.data(), tqbase.size()))) return rc;
-  if ((rc = upload(c, c->slabT_offs, tquad.data(), tquad.size()))) return rc;
-  if ((rc = upload(c, c->slabT_pairs, tpairs.data(), tpairs.size()))) return rc;
-  if ((rc = upload(c, c->slabT_wrp, twrp.data(), twrp.size()))) return rc;
+  if ((rc = upload(c, c->slabT_kbase, ttiles.kbase.data(), ttiles.kbase.size()))) return rc;
+  if ((rc = upload(c, c->slabT_ebase, ttiles.ebase.data(), ttiles.ebase.size()))) return rc;
+  if ((rc = upload(c, c->slabT_k, ttiles.ks.data(), ttiles.ks.size()))) return rc;
+  if ((rc = upload(c, c->slabT_g, ttiles.gs.data(), ttiles.gs.size()))) return rc;
+  if ((rc = upload(c, c->slabT_wrp, ttiles.wrp.data(), ttiles.wrp.size()))) return rc;
   if ((rc = upload(c, c->slabT_slot, tslot.data(), tslot.size()))) return rc;
   PB_CUDA(c, cudaStreamSynchronize(c->stream));
-  for (const void* fn : {(const void*)k_slabT<1>, (const void*)k_slabT<2>}) {
+  for (const void* fn : {(const void*)k_slabT<1, false>, (const void*)k_slabT<1, true>, (const void*)k_slabT<2, false>}) {
     PB_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));  // per kernel
     PB_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
   }
   PB_CUDA(c, cudaFuncSetAttribute(bti.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bti.smem));
-  c->slabT_nent = (int64_t)tquad.size() * 4;
-  c->slabT_maxbin = tmax;
+  c->slabT_nent = ttiles.nent;
+  c->slabT_maxe = ttiles.maxe;
+  c->slabT_maxk = ttiles.maxk;
+  c->slabT_maxg = ttiles.maxg;
   c->slabT_smem = tsm;
   c->bandT_smem = bti.smem;
+  c->bandT_fd = btf.fn && btf.smem <= max_smem;
+  if (c->bandT_fd) PB_CUDA(c, cudaFuncSetAttribute(btf.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)btf.smem));
   c->blockedT_ok = true;
   return PB_OK;
 }
@@ -6286,12 +6294,14 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
         q.band_stride = c->band_stride;
         q.slabT = c->slabT_vals.as<double>();
         q.slabT_stride = c->slabT_nent;
-        q.slabT_qbase = c->slabT_rp.as<int>();
-        q.slabT_q = c->slabT_offs.as<unsigned long long>();
-        q.slabT_pairs = c->slabT_pairs.as<int4>();
+        q.slabT_kbase = c->slabT_kbase.as<int>();
+        q.slabT_ebase = c->slabT_ebase.as<int>();
+        q.slabT_k = c->slabT_k.as<SlabK>();
+        q.slabT_g = c->slabT_g.as<SlabG>();
         q.slabT_wrp = c->slabT_wrp.as<int>();
-        q.slabT_maxq = c->slabT_maxbin;
-        q.slabT_maxp = (c->lay_nsp + 1) / 2;
+        q.slabT_maxe = c->slabT_maxe;
+        q.slabT_maxk = c->slabT_maxk;
+        q.slabT_maxg = c->slabT_maxg;
         q.fdT_cnt = c->fdT_cnt.as<int>();
         q.fdT_off = c->fdT_off.as<int>();
         q.fdT_val = c->fdT_val.as<double>();
