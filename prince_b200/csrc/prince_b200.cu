@@ -896,6 +896,7 @@ struct StepParams {
   const double* fd_val;
   const double* fd_dense;   // [d][kFdDenseW] stencil weights of offsets -kFdHalo..kFdHalo (k_fd_dense)
   double* fdbuf;            // n x ld: D_off (kappa v) of the stage
+  bool fd_band;             // k_band_tma forms fdbuf (k_fd_dense is not launched)
   double* fdkp;             // n x ld: D_off (kappa_pair v), adjoint record pass with the photon scale, or null
   const int* band_spec;     // species with cross-bin coupling rows
   int nb;
@@ -1817,6 +1818,20 @@ __global__ void __launch_bounds__(256) k_fd(StepParams p) {
   }
 }
 
+// One row of the dense loss stencil: w the row's weights in shared memory, u
+// kappa x of the bins from kFdHalo below.
+__device__ __forceinline__ double fd_row(const double* w, const double* u) {
+  const double2* w2 = reinterpret_cast<const double2*>(w);
+  const double2 wa = w2[0], wb = w2[1], wc = w2[2], wd = w2[3];
+  double sD = __dmul_rn(wa.x, u[0]);
+  sD = __dadd_rn(sD, __dmul_rn(wa.y, u[1]));
+  sD = __dadd_rn(sD, __dmul_rn(wb.x, u[2]));
+  sD = __dadd_rn(sD, __dmul_rn(wb.y, u[3]));
+  sD = __dadd_rn(sD, __dmul_rn(wc.x, u[4]));
+  sD = __dadd_rn(sD, __dmul_rn(wc.y, u[5]));
+  return __dadd_rn(sD, __dmul_rn(wd.x, u[6]));
+}
+
 // fdbuf = D_off (kappa v), register-blocked.  CTA = (species block, 32-column
 // tile), lane = column: the block's d x 32 states, its kappa and the dense
 // stencil weights go to shared memory; a warp then takes kFdChunk consecutive
@@ -1864,16 +1879,7 @@ __global__ void __launch_bounds__(256) k_fd_dense(StepParams p) {
       for (int i = 0; i < kFdChunk; ++i) {
         const int e = c0 + i;
         if (e >= d) break;
-        const double2* w2 = reinterpret_cast<const double2*>(wt + e * kFdDenseW);
-        const double2 wa = w2[0], wb = w2[1], wc = w2[2], wd = w2[3];
-        double sD = __dmul_rn(wa.x, u[i]);
-        sD = __dadd_rn(sD, __dmul_rn(wa.y, u[i + 1]));
-        sD = __dadd_rn(sD, __dmul_rn(wb.x, u[i + 2]));
-        sD = __dadd_rn(sD, __dmul_rn(wb.y, u[i + 3]));
-        sD = __dadd_rn(sD, __dmul_rn(wc.x, u[i + 4]));
-        sD = __dadd_rn(sD, __dmul_rn(wc.y, u[i + 5]));
-        sD = __dadd_rn(sD, __dmul_rn(wd.x, u[i + 6]));
-        out[(size_t)e * ld] = sD;
+        out[(size_t)e * ld] = fd_row(wt + e * kFdDenseW, u + i);
       }
     }
   }
@@ -2460,6 +2466,8 @@ __global__ void __launch_bounds__(kFinWarps * 32) k_band_finish(StepParams p) {
 }
 
 // Band partial sums with TMA staging (the same tiles and arithmetic as k_band).
+// With CT = 1 the CTAs of band pair 0 also form the loss term of their species
+// and columns (fdbuf, as k_fd_dense) from the X block.
 // CTA = (8 CT columns, mother-species group, band pair).  Its warps are CT
 // column tiles x RS row splits: with RS = 1 a warp multiplies all row tiles of
 // both band species, with RS = 4 half the row tiles of one, so that at eight
@@ -2484,7 +2492,8 @@ struct BandTma {
   static constexpr int NP = RS == 1 ? RT / 2 : RT / 4;  // pairs of row tiles of a warp and band species
   static constexpr int ABLK = 2 * RT * J * 32;          // doubles of one (species, band pair) block
   static constexpr int XS = 8 * RT * 8 * CT;            // X of one species: bins x 8 CT columns
-  static constexpr size_t smem = (size_t)(2 * ABLK + XS) * sizeof(double) + 4 * sizeof(unsigned long long);
+  static constexpr int FDS = CT == 1 ? 8 * RT * (kFdDenseW + 1) : 0;  // the loss stencil and the species' kappa
+  static constexpr size_t smem = (size_t)(2 * ABLK + XS + FDS) * sizeof(double) + 4 * sizeof(unsigned long long);
 };
 template <int RT, int J, int CT>
 __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma(StepParams p) {
@@ -2507,7 +2516,9 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
   const int npairs = gridDim.z;
   double* As = sm;             // [2][ABLK]
   double* Xs = As + 2 * ABLK;  // [bin][8 CT columns]
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(Xs + B::XS);  // A stage 0, A stage 1, X
+  double* Ws = Xs + B::XS;     // CT = 1: [bin][kFdDenseW] loss stencil
+  double* Ks = Ws + 8 * RT * kFdDenseW;  // CT = 1: kappa of the species
+  unsigned long long* bar = reinterpret_cast<unsigned long long*>(Xs + B::XS + B::FDS);  // A stage 0, A stage 1, X
   int* abort_s = reinterpret_cast<int*>(bar + 3);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
@@ -2515,6 +2526,10 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
     mbar_init(bar + 2, 1);
     *abort_s = 0;
   }
+  const bool fd = CT == 1 && p.fd_band && pair == 0;  // this CTA forms the loss term of its species and columns
+  if (fd)
+    for (int t = threadIdx.x; t < d * kFdDenseW; t += blockDim.x) Ws[t] = p.fd_dense[t];
+  double kap = fd && s0 < s1 && (int)threadIdx.x < d ? p.kap[(size_t)s0 * d + threadIdx.x] : 0.0;  // of bin threadIdx.x
   __syncthreads();
   auto issue_a = [&](int sp, int stage) {  // thread 0
     mbar_expect_tx(bar + stage, (unsigned)(ABLK * sizeof(double)));
@@ -2558,13 +2573,39 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
       atomicExch(p.err, kErrBandWait);
       *abort_s = 1;
     }
+    const bool more = sp + 1 < s1;
+    if (fd) {
+      if ((int)threadIdx.x < d) Ks[threadIdx.x] = kap;
+      if (more && (int)threadIdx.x < d) kap = p.kap[(size_t)(sp + 1) * d + threadIdx.x];
+    }
     __syncthreads();  // every warp holds X(sp) and is done with A(sp - 1)
     if (*abort_s) break;
-    const bool more = sp + 1 < s1;
+    if (threadIdx.x == 0 && more) {
+      issue_a(sp + 1, stage ^ 1);
+      last_a = sp + 1;
+    }
+    if (fd) {  // k_fd_dense's sums from the X block, a thread one column and FCH bins at a time
+      constexpr int CW = 8 * CT, FCH = 6;
+      const int c = threadIdx.x % CW;
+      for (int e0 = threadIdx.x / CW * FCH; e0 < d; e0 += (int)blockDim.x / CW * FCH) {
+        double u[FCH + 2 * kFdHalo];
+#pragma unroll
+        for (int i = 0; i < FCH + 2 * kFdHalo; ++i) {
+          const int e = e0 - kFdHalo + i;
+          u[i] = (e >= 0 && e < d) ? __dmul_rn(Ks[e], Xs[e * CW + c]) : 0.0;
+        }
+        double* __restrict__ out = p.fdbuf + ((size_t)sp * d + e0) * ld + cb + c;
+#pragma unroll
+        for (int i = 0; i < FCH; ++i) {
+          if (e0 + i >= d) break;
+          out[(size_t)i * ld] = fd_row(Ws + (e0 + i) * kFdDenseW, u + i);
+        }
+      }
+      __syncthreads();  // X(sp) is read
+    }
     if (threadIdx.x == 0 && more) {
       issue_x(sp + 1);
-      issue_a(sp + 1, stage ^ 1);
-      last_a = last_x = sp + 1;
+      last_x = sp + 1;
     }
     // a lane's fragments of row tiles 2p and 2p + 1 are one 16-byte word
     const double2* __restrict__ as = reinterpret_cast<const double2*>(As + stage * ABLK) + lane;
@@ -2596,7 +2637,7 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
 #pragma unroll
       for (int kt = 0; kt < KT; ++kt) xf[kt] = xn[kt];
   }
-  if (*abort_s) {  // the copies this CTA issued land before it leaves
+  if (*abort_s) {  // the copies this CTA issued land before it leaves (X and A of the same last species)
     if (threadIdx.x == 0 && last_a >= s0) {
       mbar_wait_bounded(bar + 2, (unsigned)((last_x - s0) & 1), kWaitTries);
       mbar_wait_bounded(bar + ((last_a - s0) & 1), (unsigned)(((last_a - s0) >> 1) & 1), kWaitTries);
@@ -3946,7 +3987,8 @@ void launch_finish(const StepParams& p, cudaStream_t st) {
 }
 
 // One stage of the bin-blocked path: k_band on the second stream, k_fd then
-// k_slab on the launching stream, then k_band_finish.
+// k_slab on the launching stream, then k_band_finish; or k_band with the loss
+// term, k_slab and k_band_finish in a line.
 template <int STAGE>
 int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   const bool photohad = (p.flags & PB_PHOTOHAD) != 0;
@@ -3954,16 +3996,25 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   int64_t launches = 0;
   p.ngroups = 0;
   p.spg = 1;
+  bool forked = false;
+  p.fd_band = false;
   if (photohad && p.nb > 0) {
     const BandPlan plan = band_plan(c, p);
-    cudaEventRecord(c->ev_fork, st);
-    cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
-    launch_band(c, p, plan, c->stream2);
-    cudaEventRecord(c->ev_join, c->stream2);
+    // the loss term with the band tiles where a CTA covers the columns alone: at 64 columns a CTA the two
+    // kernels beside each other are faster (A <= 56 network, 512 columns: 139 us for both, 145 us in one; 7
+    // columns: 13 + 9 us in parallel, 12 us in one, without the fork)
+    p.fd_band = kap && c->fd_dense_ok && !p.fdkp && c->band_warps == 8 && p.tmap_band && plan.ct == 1;
+    forked = !p.fd_band;
+    if (forked) {
+      cudaEventRecord(c->ev_fork, st);
+      cudaStreamWaitEvent(c->stream2, c->ev_fork, 0);
+    }
+    launch_band(c, p, plan, forked ? c->stream2 : st);
+    if (forked) cudaEventRecord(c->ev_join, c->stream2);
     ++launches;
   }
   const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
-  if (kap) {
+  if (kap && !p.fd_band) {
     const size_t fsmem = (size_t)p.d * (kColTile + kFdDenseW + 2) * sizeof(double);
     if (c->fd_dense_ok && p.fdkp) k_fd_dense<true><<<dim3(p.nsp, tiles), 256, fsmem, st>>>(p);
     else if (c->fd_dense_ok) k_fd_dense<false><<<dim3(p.nsp, tiles), 256, fsmem, st>>>(p);
@@ -3986,7 +4037,7 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
     k_step_multi<STAGE><<<dim3((unsigned)q.nsb, tiles), 256, 0, st>>>(q);
     ++launches;
   }
-  if (p.ngroups > 0) cudaStreamWaitEvent(st, c->ev_join, 0);
+  if (forked) cudaStreamWaitEvent(st, c->ev_join, 0);
   if (p.nb > 0) {
     launch_finish<STAGE>(p, st);
     ++launches;
