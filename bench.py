@@ -338,9 +338,9 @@ def kernel_rooflines(solver, run, sched, n_active, n_inj):
     n states, ns bin-local rows, E entries of the bin-local rows:
       k_fd_dense    read v and kappa, write D_off (kappa v):  16 n K + 8 n
                     (k_fd, the table-driven form, where the stencil does not fit)
-      k_slab        read v (all rows), entries (12 E), FD term, row factors;
+      k_slab        read v (all rows), entries (8 E), FD term, row factors;
                     stage 1 writes a and F(x), stage 2 reads F(x), writes x:
-                    8 n K + 12 E + 24 ns K + 24 ns
+                    8 n K + 8 E + 24 ns K + 24 ns
       k_band        useful flops 2 nnz_band K on the FP64 tensor pipe (DMMA)
       k_band_finish read the group partials and the band rows' inputs.
     """
@@ -363,7 +363,7 @@ def kernel_rooflines(solver, run, sched, n_active, n_inj):
     fd_name = "k_fd_dense" if ctx.info(_lib.PB_INFO_FD_DENSE) else "k_fd"
     kb = {
         fd_name: 16.0 * n * K + 8.0 * n,
-        "k_slab": 8.0 * n * K + 12.0 * nent + 24.0 * ns * K + 24.0 * ns,
+        "k_slab": 8.0 * n * K + 8.0 * nent + 24.0 * ns * K + 24.0 * ns,
     }
     traffic = ncu_traffic() if K == 512 else {}
     kernels = []

@@ -54,7 +54,7 @@ extern "C" {
 #define PB_OPT_BAND_WARPS 12       /* warps of a band-tile CTA: 8 (default, 64 columns, one CTA per SM) or 4
                                      (32 columns in half the registers and shared memory, so the band
                                      tiles run on the tensor pipe beside the bin-local gather on each SM) */
-#define PB_OPT_SLAB_PREFETCH 13    /* row quartets whose FD term and F(x) a bin-local warp loads ahead: 1, 2 (default), 3 */
+#define PB_OPT_SLAB_PREFETCH 13    /* pairs of k-tile descriptors that a bin-local warp holds: 1 (none ahead), 2 (default), 3 */
 #define PB_OPT_STAGING_WAIT_TRIES 11 /* polls of k_slab's bounded staging wait before it gives up and the solve
                                      returns PB_ERR_DEVICE (default 2^24; < 0 restores it; 0 gives up at
                                      once, which tests the error path). The CTA still drains its copies. */
@@ -352,7 +352,7 @@ int pb_solve(pb_context* ctx, const pb_solve_args* args);
 /* Autotuner of the batched bin-blocked stage: runs the solve described by
  * `args` (normally a short schedule with every column active, on the live
  * operator, injection and photon field) `reps` + 1 times for each candidate
- * (band-tile CTA warps 8 / 4, k_slab prefetch depth 2 / 3 / 4, k_slab staging
+ * (band-tile CTA warps 8 / 4, k_slab prefetch depth 1 / 2 / 3, k_slab staging
  * by TMA / cp.async), scores each by its fastest step loop, and leaves the
  * fastest set on the context (the PB_OPT_BAND_WARPS, PB_OPT_SLAB_PREFETCH and
  * PB_OPT_TMA_STAGING options).  Writes up to max_out candidates to out, the
@@ -420,7 +420,7 @@ int pb_integrate_const(pb_context* ctx, int64_t n, const double* d, int64_t nnz,
  * The buffers themselves must hold the sizes above: the library cannot check
  * a device allocation's extent.
  *
- * The call allocates and frees nothing: its scratch (about 6 MB) is one static
+ * The call allocates and frees nothing: its scratch (about 7 MB) is one static
  * device array sized for at most PB_NOALLOC_MAX_STATES states and
  * PB_NOALLOC_MAX_STEPS steps; larger sizes are rejected with PB_ERR_ARG.  Every
  * GPU that loads the library holds that array until the process exits.

@@ -9,9 +9,13 @@
 //      diagonal/off-diagonal split -> prefix sum -> M_off CSR pattern
 //   4. fold GEMM over all windows on the FP64 tensor pipe (DMMA), written
 //      straight into M_off values [w][nnz] and the diagonal [w][n]
-//   5. ETD2 steps: two fused kernels per step (stage 1 -> a, F(x);
-//      stage 2 -> x), each an SpMV/SpMM of M_off with the FD loss stencil,
-//      the explicit-decay term, the injection and the phi-function epilogue.
+//   5. ETD2 steps, two stages each (stage 1 -> a, F(x); stage 2 -> x): an
+//      SpMV/SpMM of M_off with the FD loss stencil, the explicit-decay term,
+//      the injection and the phi-function epilogue.  One column: a kernel per
+//      stage; a batch: band tiles, FD stencil, bin-local tiles and a finish per
+//      stage; a small network: all steps in one launch.  The factors of a run
+//      of steps come from one launch, and captured runs of 16 steps are
+//      replayed for any schedule.
 //
 // The algorithm follows the reference CPU solver of PriNCe:
 //   src/prince_cr/solvers/etd2.py:329-439 (phi functions, step),
@@ -132,7 +136,7 @@ struct DBuf {
 }  // namespace
 
 constexpr long long kWaitTries = 1ll << 24;  // polls of a bounded wait (well above any staging time)
-constexpr int kSlabPreDefault = 2;           // k_slab's default prefetch depth (row quartets)
+constexpr int kSlabPreDefault = 2;           // k_slab's default prefetch depth (pairs of k-tile descriptors)
 struct StepGraph {  // a captured run of steps and the parameters it was captured for
   std::vector<uint64_t> key;
   cudaGraphExec_t exec = nullptr;
@@ -207,13 +211,13 @@ struct pb_context {
   int32_t band_nb = 0, band_RT = 0, band_J = 0, n_slab_spec = 0;
   int64_t band_stride = 0;          // band-tile doubles per window
   int32_t band_npairs = 0;
-  DBuf band_slot, band_spec, slab_spec, band_vals, band_part;
+  DBuf band_slot, band_spec, band_vals, band_part;
   // bin-local rows: coupling entries in bin-major order
   DBuf slab_kbase, slab_ebase, slab_k, slab_g, slab_wrp, slab_slot, slab_vals, slab_rowslot, slab_fac;
   int64_t slab_nslots = 0;          // group slots over all bins (eight per group)
   int64_t slab_nent = 0;            // entries per window (every bin's count rounded up to even)
   int32_t slab_maxe = 0, slab_maxk = 0, slab_maxg = 0;  // of the largest bin
-  size_t slab_smem = 0, band_smem = 0;
+  size_t slab_smem = 0;
   // FD stencil per bin (same in every species block): host copy of D and the table
   std::vector<int64_t> h_d_indptr;
   std::vector<int32_t> h_d_indices;
@@ -229,7 +233,7 @@ struct pb_context {
   DBuf vbuf, vbuf2, bTbuf, fdTbuf, outcols;
   int64_t slabT_nent = 0;
   int32_t slabT_maxe = 0, slabT_maxk = 0, slabT_maxg = 0;  // of the largest bin
-  size_t slabT_smem = 0, bandT_smem = 0;
+  size_t slabT_smem = 0;
   bool bandT_fd = false;  // k_bandT's FD instance fits
   // small networks (k_small)
   DBuf small_order;                 // rows by coupling entries, longest first
@@ -240,7 +244,7 @@ struct pb_context {
   int32_t tma_mode = 1;             // 1: k_slab stages by TMA when tensor maps can be encoded; 0: cp.async
   long long staging_wait_tries = kWaitTries;  // k_slab's first staging wait (PB_OPT_STAGING_WAIT_TRIES)
   int32_t band_warps = 8;           // warps of a k_band CTA (PB_OPT_BAND_WARPS: 8 or 4)
-  int32_t slab_pre = kSlabPreDefault;  // k_slab prefetch depth in row quartets (PB_OPT_SLAB_PREFETCH: 1..3)
+  int32_t slab_pre = kSlabPreDefault;  // k_slab: pairs of k-tile descriptors held (PB_OPT_SLAB_PREFETCH: 1..3)
   bool last_blocked = false;
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -876,8 +880,6 @@ struct StepParams {
   // bin-blocked batched path
   int d;                    // bins per species block
   int nsp;                  // species blocks
-  const int* slab_spec;     // species whose coupling rows are bin-local
-  int n_slab_spec;
   const int* slab_kbase;    // [d + 1] first k-tile of each bin
   const int* slab_ebase;    // [d + 1] first entry of each bin (even)
   const SlabK* slab_k;      // k-tiles of k_slab
@@ -3686,7 +3688,7 @@ std::vector<DBuf*> solve_buffers(pb_context* c) {
           &c->lt_indptr, &c->lt_indices, &c->lt_vals, &c->inj_rows, &c->src_col_d, &c->ckpt,
           &c->em_bh_off, &c->em_bh_A, &c->em_invE, &c->em_dE, &c->em_Tg, &c->em_Te, &c->em_R, &c->em_wbuf,
           &c->em_es, &c->em_lep, &c->em_y, &c->em_TgT, &c->em_TeT, &c->em_RT, &c->em_dlw,
-          &c->band_slot, &c->band_spec, &c->slab_spec, &c->band_vals, &c->band_part, &c->slab_kbase,
+          &c->band_slot, &c->band_spec, &c->band_vals, &c->band_part, &c->slab_kbase,
           &c->slab_ebase, &c->slab_k, &c->slab_g, &c->slab_slot, &c->slab_vals, &c->slab_wrp, &c->slab_rowslot, &c->slab_fac, &c->fd_cnt, &c->fd_off, &c->fd_val, &c->fd_dense, &c->fdT_dense, &c->fdbuf,
           &c->bandT_slot, &c->slabT_kbase, &c->slabT_ebase, &c->slabT_k, &c->slabT_g, &c->slabT_wrp, &c->slabT_slot,
           &c->fdT_cnt, &c->fdT_off, &c->fdT_val, &c->tmaps, &c->d_err, &c->tab_z, &c->tab_le, &c->tab_v};
@@ -3785,8 +3787,6 @@ void fill_step_params(pb_context* c, StepParams& p, int K, int ld, uint32_t flag
   p.ctiles = ctiles;
   p.d = c->lay_d;
   p.nsp = c->lay_nsp;
-  p.slab_spec = c->slab_spec.as<int>();
-  p.n_slab_spec = c->n_slab_spec;
   p.slab_kbase = c->slab_kbase.as<int>();
   p.slab_ebase = c->slab_ebase.as<int>();
   p.slab_k = c->slab_k.as<SlabK>();
@@ -5272,7 +5272,6 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
     }
   if ((rc = upload(c, c->band_slot, bslot.data(), bslot.size()))) return rc;
   if ((rc = upload(c, c->band_spec, bspec.data(), bspec.size()))) return rc;
-  if ((rc = upload(c, c->slab_spec, sspec.data(), sspec.size()))) return rc;
   if ((rc = upload(c, c->slab_kbase, tiles.kbase.data(), tiles.kbase.size()))) return rc;
   if ((rc = upload(c, c->slab_ebase, tiles.ebase.data(), tiles.ebase.size()))) return rc;
   if ((rc = upload(c, c->slab_k, tiles.ks.data(), tiles.ks.size()))) return rc;
@@ -5320,7 +5319,6 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   c->slab_maxk = tiles.maxk;
   c->slab_maxg = tiles.maxg;
   c->slab_smem = ssm;
-  c->band_smem = bi.smem;
   c->band_nnz = band_nnz;
   c->slab_nnz = slab_nnz;
   c->blocked_ok = true;
@@ -5384,7 +5382,6 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   c->slabT_maxk = ttiles.maxk;
   c->slabT_maxg = ttiles.maxg;
   c->slabT_smem = tsm;
-  c->bandT_smem = bti.smem;
   c->bandT_fd = btf.fn && btf.smem <= max_smem;
   if (c->bandT_fd) PB_CUDA(c, cudaFuncSetAttribute(btf.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)btf.smem));
   c->blockedT_ok = true;
