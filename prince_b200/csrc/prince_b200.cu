@@ -5227,6 +5227,15 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   int RT = 0, J = 0;
   for (int v : kBandRT) if (!RT && v >= RTr) RT = v;
   for (int v : kBandJ) if (!J && v >= Jr) J = v;
+  // What no layout fits is turned down before the tiles are built: SlabTiles indexes by mother species, so every
+  // block row's columns have to be block rows, and its grouping takes about species^2 / 64 words per distinct bin.
+  const size_t max_smem = 227 * 1024;
+  const BandInstance bi = (RT && J) ? band_kernel(RT, J) : BandInstance{nullptr, 0, 0};
+  const BandInstance bi4 = (RT && J) ? band_kernel(RT, J, 4) : BandInstance{nullptr, 0, 0};
+  if (!split_ok || nsp >= 0x2000 || SlabSmem::bytes(nsp, 0, 0, 0) > max_smem || !bi.fn || bi.smem > max_smem ||
+      (!bspec.empty() && lo < 0) || (size_t)d * (kColTile + 2) * sizeof(double) > max_smem ||
+      (int64_t)nsp * 2 * npairs * RT * J * 32 >= ((int64_t)1 << 31))
+    return PB_OK;  // the general row kernels stay in use
   // bin-local rows, per bin, as DMMA row groups and k-tiles (SlabTiles)
   int64_t band_nnz = 0, slab_nnz = 0;
   std::vector<int32_t> sslot((size_t)std::max<int64_t>(R, 1), -1), rowslot((size_t)n, -1);
@@ -5246,14 +5255,8 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
     }
     tiles.finish();
   }
-  const size_t max_smem = 227 * 1024;
   const size_t ssm = SlabSmem::bytes(nsp, tiles.maxe, tiles.maxk, tiles.maxg);
-  const BandInstance bi = (RT && J) ? band_kernel(RT, J) : BandInstance{nullptr, 0, 0};
-  const BandInstance bi4 = (RT && J) ? band_kernel(RT, J, 4) : BandInstance{nullptr, 0, 0};
-  const bool ok = split_ok && nsp < 0x2000 && ssm <= max_smem && bi.fn && bi.smem <= max_smem && (bspec.empty() || lo >= 0) &&
-                  (size_t)d * (kColTile + 2) * sizeof(double) <= max_smem &&
-                  (int64_t)nsp * 2 * npairs * RT * J * 32 < ((int64_t)1 << 31) && tiles.nent < ((int64_t)1 << 31);
-  if (!ok) return PB_OK;  // the general row kernels stay in use
+  if (ssm > max_smem || tiles.nent >= ((int64_t)1 << 31)) return PB_OK;  // as above
   // band tiles: [species][band pair][2][RT / 2][J][32][2] DMMA A fragments per window
   std::vector<int32_t> bslot((size_t)std::max<int64_t>(R, 1), -1);
   for (int b = 0; b < nb; ++b)
