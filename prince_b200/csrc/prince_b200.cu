@@ -143,6 +143,12 @@ struct StepGraph {  // a captured run of steps and the parameters it was capture
   int64_t launches = 0;
   uint64_t used = 0;
 };
+struct TmaKey {  // what a pair of (column, bin, species) tensor maps was encoded for
+  const void* p0 = nullptr;
+  const void* p1 = nullptr;
+  int ld = 0, d = 0, nsp = 0;
+  bool operator==(const TmaKey& o) const { return p0 == o.p0 && p1 == o.p1 && ld == o.ld && d == o.d && nsp == o.nsp; }
+};
 struct pb_context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -254,14 +260,14 @@ struct pb_context {
   bool tail_wait = false;           // the next tail launch waits for ev_hook_done
   int num_sms = 148;
   DBuf tmaps;                       // [6] CUtensorMap of X and A for k_slab's and k_band_tma's TMA staging
-  bool tma_ok = false;              // tmaps hold k_slab's maps of the current X / A / ld
+  bool tma_ok = false;              // tmaps hold k_slab's maps of tma_key
   bool tma_band_ok = false;         // tmaps also hold k_band_tma's maps (entries 2 to 5)
   bool band_tma_fits = false;       // k_band_tma's shared memory fits the layout's band tiles
   bool last_tma = false;            // the last solve staged k_slab by TMA
-  const void* tma_key[3] = {nullptr, nullptr, nullptr};
+  TmaKey tma_key;
   DBuf tmapsT;                      // [2] CUtensorMap of the adjoint's v buffers for k_slabT's TMA staging
-  bool tmaT_ok = false;             // tmapsT hold maps of the current vbuf / vbuf2 / ld
-  const void* tmaT_key[3] = {nullptr, nullptr, nullptr};
+  bool tmaT_ok = false;             // tmapsT hold maps of tmaT_key
+  TmaKey tmaT_key;
   DBuf d_err;                       // int: a bounded wait of a kernel gave up
   // caller's row order: device row i holds the caller's row row_map[i] (none: identity)
   bool have_row_map = false;
@@ -3836,9 +3842,9 @@ EncodeTiledFn tensor_map_encoder() {
 // tma_band_ok false when only the band maps are refused.
 int ensure_tmaps(pb_context* c, bool blocked, int ld) {
   const bool want = blocked && c->tma_mode == 1 && ld % kSlabCols == 0;
-  if (want && c->tma_ok && c->tma_key[0] == c->X.p && c->tma_key[1] == c->A.p &&
-      c->tma_key[2] == reinterpret_cast<const void*>((intptr_t)ld))
-    return PB_OK;
+  // the buffers keep their addresses when another layout's states fit them, so the layout is part of the key
+  const TmaKey key{c->X.p, c->A.p, ld, c->lay_d, c->lay_nsp};
+  if (want && c->tma_ok && c->tma_key == key) return PB_OK;
   c->tma_ok = false;
   c->tma_band_ok = false;
   if (!want) return PB_OK;
@@ -3864,9 +3870,7 @@ int ensure_tmaps(pb_context* c, bool blocked, int ld) {
   }
   PB_CUDA(c, c->tmaps.ensure(sizeof(maps)));
   PB_CUDA(c, cudaMemcpy(c->tmaps.p, maps, sizeof(maps), cudaMemcpyHostToDevice));
-  c->tma_key[0] = c->X.p;
-  c->tma_key[1] = c->A.p;
-  c->tma_key[2] = reinterpret_cast<const void*>((intptr_t)ld);
+  c->tma_key = key;
   c->tma_ok = true;
   c->tma_band_ok = band_ok;
   return PB_OK;
@@ -3877,9 +3881,8 @@ int ensure_tmaps(pb_context* c, bool blocked, int ld) {
 // (cp.async staging) when TMA is switched off or a map is refused.
 int ensure_tmapsT(pb_context* c, int ld) {
   const bool want = c->tma_mode == 1 && ld % kSlabCols == 0;
-  if (want && c->tmaT_ok && c->tmaT_key[0] == c->vbuf.p && c->tmaT_key[1] == c->vbuf2.p &&
-      c->tmaT_key[2] == reinterpret_cast<const void*>((intptr_t)ld))
-    return PB_OK;
+  const TmaKey key{c->vbuf.p, c->vbuf2.p, ld, c->lay_d, c->lay_nsp};
+  if (want && c->tmaT_ok && c->tmaT_key == key) return PB_OK;
   c->tmaT_ok = false;
   if (!want) return PB_OK;
   const EncodeTiledFn enc = tensor_map_encoder();
@@ -3898,9 +3901,7 @@ int ensure_tmapsT(pb_context* c, int ld) {
   }
   PB_CUDA(c, c->tmapsT.ensure(sizeof(maps)));
   PB_CUDA(c, cudaMemcpy(c->tmapsT.p, maps, sizeof(maps), cudaMemcpyHostToDevice));
-  c->tmaT_key[0] = c->vbuf.p;
-  c->tmaT_key[1] = c->vbuf2.p;
-  c->tmaT_key[2] = reinterpret_cast<const void*>((intptr_t)ld);
+  c->tmaT_key = key;
   c->tmaT_ok = true;
   return PB_OK;
 }
