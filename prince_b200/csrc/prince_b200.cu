@@ -4329,8 +4329,10 @@ StepGraph* step_graph(pb_context* c, StepParams p, int K, int G, int cols, cudaS
     g.launches += launch_step(c, p, K, run + j, hook, st);
   }
   join_hook(c, hook, st);
+  const bool refused = cudaPeekAtLastError() != cudaSuccess;  // a launch is missing from the run: it must not be kept
   cudaGraph_t graph = nullptr;
-  if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) {
+  if (cudaStreamEndCapture(st, &graph) != cudaSuccess || refused ||
+      cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     return nullptr;
   }

@@ -1,0 +1,51 @@
+"""Captured runs of steps: what is kept, what is replayed, and the same bits wherever a step falls (needs a B200)."""
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+def _bare_context(n):
+    """A context with ``n`` states that only lose energy: no coupling entries, no stencil neighbours."""
+    from prince_b200 import _lib
+    ctx = _lib.Context(0)
+    empty = sp.csr_matrix((n, n))
+    ctx.set_coupling(n, empty.indptr, empty.indices)
+    ctx.set_photon_grid(np.logspace(-15, -6, 8))
+    ctx.set_photon_field([(0, 1.0, 1e-13, 0.0)])
+    ctx.set_fd_operator(empty, np.ones(n))
+    ctx.set_losses(np.ones(n), np.zeros(n), np.full(n, -1), np.linspace(1.0, 2.0, 4), np.ones(4), np.ones((1, 4)))
+    return ctx
+
+
+class _Sched:
+    def __init__(self, n_steps):
+        self.n_steps = n_steps
+        self.z_window = np.array([0.5])
+        self.window = np.zeros(n_steps, dtype=np.int32)
+        self.h = np.full(n_steps, -1e-3)
+        self.dldz = np.full(n_steps, -1.0)
+        self.hc = np.full(n_steps, 1.0)
+        self.finj = np.zeros(n_steps)
+
+
+def test_run_with_a_refused_launch_is_not_kept():
+    """More columns than a grid has column tiles: the launch is refused on the host.  Every solve has to say so, the
+    second as the first: a run kept without its kernels would return the initial state as the answer."""
+    from prince_b200 import _lib
+    ctx = _bare_context(2)
+    K = 65535 * 32 + 1
+    sched = _Sched(16)
+    state = np.ones((2, K))
+    n_active = np.full(16, K, dtype=np.int32)
+    for _ in range(2):
+        with pytest.raises(RuntimeError):
+            ctx.solve(sched, _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, K, None, n_active, state, init_state=True)
+    # the context still solves what fits
+    K = 4
+    state = np.ones((2, K))
+    ctx.solve(sched, _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, K, None, np.full(16, K, dtype=np.int32), state,
+              init_state=True)
+    np.testing.assert_allclose(state, np.exp(16e-3), rtol=1e-12)
