@@ -1299,6 +1299,7 @@ template <int STAGE>
 __global__ void __launch_bounds__(kPlainThreads, 2) k_step_plain(StepParams p) {
   __shared__ double red[kPlainThreads / 32];
   const StepScalars s = load_scalars(p, p.sc);
+  if (s.ncols == 0) return;  // a step of a captured run that the column sits out
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double* __restrict__ v = p.src;
   const double* __restrict__ mv = p.m_vals + (size_t)s.w * p.m_wstride;

@@ -49,3 +49,16 @@ def test_run_with_a_refused_launch_is_not_kept():
     ctx.solve(sched, _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, K, None, np.full(16, K, dtype=np.int32), state,
               init_state=True)
     np.testing.assert_allclose(state, np.exp(16e-3), rtol=1e-12)
+
+
+@pytest.mark.parametrize("n", [600, 1500])
+def test_one_column_sits_out_the_steps_without_active_columns(n):
+    """Steps without active columns leave the state alone, inside a captured run (n above the small networks') as
+    in one launch of all steps and step by step: sixteen steps of which twelve are taken, then two more."""
+    from prince_b200 import _lib
+    ctx = _bare_context(n)
+    active = np.ones(18, dtype=np.int32)
+    active[[3, 4, 9, 15]] = 0
+    state = np.ones((n, 1))
+    ctx.solve(_Sched(18), _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, 1, None, active, state, init_state=True)
+    np.testing.assert_allclose(state, np.exp(14e-3), rtol=1e-12)
