@@ -1299,7 +1299,6 @@ template <int STAGE>
 __global__ void __launch_bounds__(kPlainThreads, 2) k_step_plain(StepParams p) {
   __shared__ double red[kPlainThreads / 32];
   const StepScalars s = load_scalars(p, p.sc);
-  if (s.ncols == 0) return;  // a step of a captured run that the column sits out
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double* __restrict__ v = p.src;
   const double* __restrict__ mv = p.m_vals + (size_t)s.w * p.m_wstride;
@@ -3730,6 +3729,18 @@ void csr_transpose(int64_t n, int64_t nnz, const int64_t* ip, const int32_t* ix,
 }
 
 
+constexpr int kGraphCols = 64;  // column granularity of a step's launches
+// The columns that the launches of a step with `active` columns of a K-column solve are laid out for.  The band
+// tiles' groups, and so the order of their partial sums, follow from it: it depends on the step alone, not on the
+// run or the pass that the step is launched in, so that a solve's states are the same bits with any checkpoints
+// and in the record pass.
+int launch_cols(int K, int active) {
+  if (active == 0) return 0;
+  if (K <= kGraphCols) return K;
+  const int ld = (K + kColTile - 1) / kColTile * kColTile;
+  return std::min((active + kGraphCols - 1) / kGraphCols * kGraphCols, ld);
+}
+
 // Whether a solve with K columns runs the bin-blocked kernels.
 bool use_blocked(const pb_context* c, int K) {
   const int64_t ld = ((K + kColTile - 1) / kColTile) * kColTile;
@@ -4273,7 +4284,6 @@ int64_t launch_small(pb_context* c, StepParams& p, const SmallPlan& pl, int K, i
 }
 
 constexpr size_t kMaxStepGraphs = 24;
-constexpr int kGraphCols = 64;  // column granularity of a captured run's grids
 
 // The captured run of `G` steps on the context's step-scalar buffer s_run for
 // up to `cols` active columns, or null when it cannot be captured.  The steps
@@ -4348,8 +4358,11 @@ StepGraph* step_graph(pb_context* c, StepParams p, int K, int G, int cols, cudaS
 // advanced at step k; a step without active columns is skipped (every column
 // is still exactly zero).  With `ckpt`, the state before every step k with
 // k % every == 0 is copied to checkpoint k / every.  Runs of steps between
-// checkpoints replay a captured graph; what is left, and the record pass, is
-// launched step by step.  Returns the kernel count, or -1 on a failure.
+// checkpoints that are laid out for the same columns replay a captured graph,
+// half a run or more of them (a step that is switched off in a run costs its
+// empty launches, about 17 us in the blocked form; one launched alone about 40 us
+// of host time); what is left, and the record pass, is launched step by step.
+// Returns the kernel count, or -1 on a failure.
 int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_active, int64_t k0, int64_t k1,
                      cudaStream_t st, double* ckpt, int every) {
   const int64_t n = c->n;
@@ -4361,6 +4374,7 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
   const bool record = p.rec_P != nullptr;  // the factors of the segment stay in p.rf for the sweep
   const int G = (int)std::min<int64_t>(kGraphSteps, prep_steps(n));
   static const bool no_graph = getenv("PRINCE_B200_NO_GRAPH") != nullptr;
+  const bool runs = !no_graph && !record;
   bool hook_pending = false;
   for (int64_t k = k0; k < k1;) {
     const bool copy = ckpt && every > 0;
@@ -4372,31 +4386,35 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
       ++k;
       continue;
     }
-    const int64_t stop = copy ? std::min<int64_t>(k1, (k / every + 1) * every) : k1;  // the next checkpoint
-    if (!no_graph && !record && k >= prepared && stop - k >= G) {
-      join_hook(c, hook_pending, st);
-      int cols = 0;
-      for (int64_t q = k; q < k + G; ++q) cols = std::max(cols, n_active[q]);
-      cols = K <= kGraphCols ? K : std::min((cols + kGraphCols - 1) / kGraphCols * kGraphCols, p.ld);
-      StepGraph* g = step_graph(c, p, K, G, cols, st);
-      if (!g) return -1;
-      p.rf_k0 = k;
-      launch_prep(p, scal, k, G, st);
-      cudaMemcpyAsync(c->s_run.p, scal + k, G * sizeof(StepScal), cudaMemcpyDeviceToDevice, st);
-      if (cudaGraphLaunch(g->exec, st) != cudaSuccess) return -1;
-      launches += 1 + g->launches;
-      k += G;
-      continue;
-    }
+    p.hcols = launch_cols(K, n_active[k]);
     if (k >= prepared) {
-      const int64_t count = std::min<int64_t>(prep_steps(n), (stop - k >= G ? k1 : stop) - k);
+      const int64_t stop = copy ? std::min<int64_t>(k1, (k / every + 1) * every) : k1;  // the next checkpoint
+      int64_t same = k + 1;  // end of the steps up to there that are laid out alike (at most a run of them)
+      while (same < stop && same < k + G && launch_cols(K, n_active[same]) == p.hcols) ++same;
+      const int64_t m = same - k;
+      // The run's other steps, if any, have no active columns.  One column takes whole runs: k_step_plain does not
+      // read the active columns (a check ahead of its loads cost 2% of a solve, one at its end 8%).
+      if (runs && (K == 1 ? m == G : 2 * m >= G)) {
+        join_hook(c, hook_pending, st);
+        StepGraph* g = step_graph(c, p, K, G, p.hcols, st);
+        if (!g) return -1;
+        p.rf_k0 = k;
+        launch_prep(p, scal, k, m, st);
+        StepScal* run = c->s_run.as<StepScal>();
+        cudaMemcpyAsync(run, scal + k, m * sizeof(StepScal), cudaMemcpyDeviceToDevice, st);
+        if (m < G) cudaMemsetAsync(run + m, 0, (G - m) * sizeof(StepScal), st);
+        if (cudaGraphLaunch(g->exec, st) != cudaSuccess) return -1;
+        launches += 1 + g->launches;
+        k = same;
+        continue;
+      }
+      const int64_t count = std::min(prep_steps(n), (runs ? same : k1) - k);
       if (!record) p.rf_k0 = k;
       launch_prep(p, scal, k, count, st);
       ++launches;
       prepared = k + count;
     }
     set_step_factors(p, k);
-    p.hcols = n_active[k];
     launches += launch_step(c, p, K, scal + k, hook_pending, st);
     ++k;
   }
@@ -5411,7 +5429,7 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   StepParams p;
   memset(&p, 0, sizeof(p));
   fill_step_params(c, p, K, ld, flags, pair, inj, c->last_S, ld / kColTile);
-  p.hcols = c->h_nact[step];
+  p.hcols = launch_cols(K, c->h_nact[step]);
   p.src = stage == 1 ? c->X.as<double>() : c->A.as<double>();
   p.x = c->X.as<double>();
   p.xout = c->X.as<double>();

@@ -62,3 +62,38 @@ def test_one_column_sits_out_the_steps_without_active_columns(n):
     state = np.ones((n, 1))
     ctx.solve(_Sched(18), _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, 1, None, active, state, init_state=True)
     np.testing.assert_allclose(state, np.exp(14e-3), rtol=1e-12)
+
+
+@pytest.fixture(scope="module")
+def medium_run():
+    from workloads import network_run
+    return network_run(max_mass=16, n_species=60, seed=5)
+
+
+@pytest.mark.parametrize("K,band_warps", [(20, 8), (70, 8), (203, 8), (203, 4)])
+def test_states_do_not_depend_on_the_checkpoints(medium_run, K, band_warps):
+    """Columns that switch on step by step, across multiples of 64: with checkpoints every step, every five (all
+    steps launched alone), every 32 and none (runs at other places), the states are the same bits."""
+    import torch
+    from prince_b200 import _lib
+    from prince_b200 import adjoint as AD
+    run = medium_run
+    rng = np.random.default_rng(K)
+    species = [2212, 1000020040, 1000070140]
+    sb = AD.SourceBatch(run, species, z_max=list(rng.uniform(0.005, 0.08, K)), initial_z=0.08)
+    G = sb.grids(torch.tensor(rng.uniform(0.5, 2.2, K)), torch.tensor(rng.uniform(9.3, 10.5, K)),
+                 torch.tensor(rng.dirichlet(np.ones(3), K)))
+    coeff = sb.coefficients(torch.tensor(rng.uniform(-2, 4, K)))
+    out = []
+    for every in (1, 5, 32, 0):
+        plan = sb.plan(0.08, ckpt_every=every)
+        ctx = plan.dev.ctx
+        ctx.set_option(_lib.PB_OPT_BAND_WARPS, band_warps)
+        try:
+            X = AD.PropagateFunction.apply(G, coeff, torch.tensor(1.0, dtype=torch.float64), plan)
+        finally:
+            ctx.set_option(_lib.PB_OPT_BAND_WARPS, 8)
+        assert ctx.info(_lib.PB_INFO_LAST_BLOCKED) == 1
+        out.append(X.cpu().numpy())
+    for other in out[1:]:
+        assert np.array_equal(out[0], other)
