@@ -27,6 +27,7 @@ PB_OPT_TMA_STAGING, PB_INFO_LAST_TMA = 9, 10
 PB_OPT_STAGING_WAIT_TRIES = 11
 PB_OPT_BAND_WARPS = 12
 PB_OPT_SLAB_PREFETCH = 13
+PB_INFO_STEP_CAPTURES = 14
 
 _d = C.POINTER(C.c_double)
 _i32 = C.POINTER(C.c_int32)

@@ -295,6 +295,7 @@ struct pb_context {
   Arena em_arena;                   // temporaries of pb_em_transfer and pb_bh_shape
   // captured runs of steps
   std::vector<StepGraph> step_graphs;
+  int64_t captures = 0;             // runs captured so far
   uint64_t graph_clock = 0;
 
   // timing
@@ -3729,7 +3730,8 @@ void csr_transpose(int64_t n, int64_t nnz, const int64_t* ip, const int32_t* ix,
 }
 
 
-constexpr int kGraphCols = 64;  // column granularity of a step's launches
+constexpr int kGraphCols = 64;    // column granularity of a step's launches, at least
+constexpr int kGraphSizes = 12;   // column counts of a solve's launches, at most: half the captured runs kept
 // The columns that the launches of a step with `active` columns of a K-column solve are laid out for.  The band
 // tiles' groups, and so the order of their partial sums, follow from it: it depends on the step alone, not on the
 // run or the pass that the step is launched in, so that a solve's states are the same bits with any checkpoints
@@ -3738,7 +3740,8 @@ int launch_cols(int K, int active) {
   if (active == 0) return 0;
   if (K <= kGraphCols) return K;
   const int ld = (K + kColTile - 1) / kColTile * kColTile;
-  return std::min((active + kGraphCols - 1) / kGraphCols * kGraphCols, ld);
+  const int gran = (ld + kGraphCols * kGraphSizes - 1) / (kGraphCols * kGraphSizes) * kGraphCols;
+  return std::min((active + gran - 1) / gran * gran, ld);
 }
 
 // Whether a solve with K columns runs the bin-blocked kernels.
@@ -4350,6 +4353,7 @@ StepGraph* step_graph(pb_context* c, StepParams p, int K, int G, int cols, cudaS
   cudaGraphDestroy(graph);
   g.key = std::move(key);
   g.used = c->graph_clock;
+  ++c->captures;
   c->step_graphs.push_back(std::move(g));
   return &c->step_graphs.back();
 }
@@ -5562,6 +5566,7 @@ int pb_get_info(pb_context* c, int32_t key, int64_t* value) {
     case PB_INFO_BAND_ENTRIES: *value = c->band_nnz; return PB_OK;
     case PB_INFO_SLAB_ENTRIES: *value = c->slab_nnz; return PB_OK;
     case PB_INFO_SLAB_ROWS: *value = (int64_t)c->n_slab_spec * c->lay_d; return PB_OK;
+    case PB_INFO_STEP_CAPTURES: *value = c->captures; return PB_OK;
     case PB_INFO_FD_DENSE: *value = c->fd_dense_ok ? 1 : 0; return PB_OK;
   }
   return fail(c, PB_ERR_ARG, "pb_get_info: unknown key %d", key);

@@ -97,3 +97,52 @@ def test_states_do_not_depend_on_the_checkpoints(medium_run, K, band_warps):
         out.append(X.cpu().numpy())
     for other in out[1:]:
         assert np.array_equal(out[0], other)
+
+
+def _batch(run, K, z_range, initial_z, seed):
+    from prince_b200.solvers import MultiRHSPropagationSolverETD2
+    from workloads import draw_points, point_source
+    m = MultiRHSPropagationSolverETD2(initial_z=initial_z, final_z=0.0, prince_run=run, K=K)
+    for k, p in enumerate(draw_points(run, K, seed=seed, z_range=z_range)):
+        m[k].add_source_class(point_source(run, p))
+    return m
+
+
+def test_wide_ragged_batch_captures_once(medium_run):
+    """2,048 columns that switch on over 800 steps: every column count of the launches is captured by the first
+    solve and found by the second."""
+    from prince_b200 import _lib
+    m = _batch(medium_run, 2048, (0.01, 0.4), 0.4, seed=1)
+    m.solve(dz=5e-4)
+    ctx = m._dev.ctx
+    first, state = ctx.info(_lib.PB_INFO_STEP_CAPTURES), m.state.copy()
+    m.solve(dz=5e-4)
+    assert ctx.info(_lib.PB_INFO_STEP_CAPTURES) == first
+    assert np.array_equal(m.state, state)
+
+
+def test_runs_are_dropped_and_captured_again(medium_run):
+    """More batch sizes than runs are kept: the first size's run has gone when it is solved again, with another
+    schedule and then the first one, and the states are the same bits as before, and as with the other staging."""
+    from prince_b200 import _lib
+    run = medium_run
+    first = _batch(run, 9, (0.01, 0.04), 0.04, seed=2)
+    ctx = first._dev.ctx
+    first.solve(dz=1e-3)
+    state = first.state.copy()
+    for K in range(10, 40):
+        _batch(run, K, (0.01, 0.02), 0.02, seed=K).solve(dz=1e-3)
+    before = ctx.info(_lib.PB_INFO_STEP_CAPTURES)
+    other = _batch(run, 9, (0.01, 0.03), 0.03, seed=3)
+    other.solve(dz=1e-3)
+    assert ctx.info(_lib.PB_INFO_STEP_CAPTURES) == before + 1
+    first.solve(dz=1e-3)
+    assert ctx.info(_lib.PB_INFO_STEP_CAPTURES) == before + 1   # the same run, for another schedule
+    assert np.array_equal(first.state, state)
+    again = other.state.copy()
+    ctx.set_option(_lib.PB_OPT_TMA_STAGING, 0)                  # other kernels, the same sums
+    try:
+        other.solve(dz=1e-3)
+    finally:
+        ctx.set_option(_lib.PB_OPT_TMA_STAGING, 1)
+    assert np.array_equal(other.state, again)
