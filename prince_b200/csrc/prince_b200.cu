@@ -2061,6 +2061,57 @@ __device__ __forceinline__ void slab_tiles(unsigned ks, int nkt, unsigned slab, 
   }
 }
 
+// NaN if any of a lane's sums is one (or at least 2^1017 in magnitude): their high words as floats, times zero.  An
+// instruction a sum on a pipe that is idle beside the products; comparing the words took two on the integer pipe.
+template <int N>
+__device__ __forceinline__ float nan_mark(const double (&v)[N]) {
+  float m = 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) m = __fmaf_rn(__int_as_float(__double2hiint(v[i])), 0.0f, m);
+  return m;
+}
+
+// The sums of a group entry by entry, a lane its row's columns 4 t .. 4 t + 3.  slab_tiles multiplies a mother's
+// state by zero for the rows that do not couple to it, which is a NaN where the state is not finite; only then does
+// a warp come here, so that such a state reaches the rows that couple to it and no others.
+__device__ __noinline__ double4 slab_entries(unsigned ks, int nkt, unsigned slab, int lane) {
+  const unsigned g4 = lane & 28u, c = 2 * (lane & 3);
+  double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int k = 0; k < nkt; ++k, ks += 16) {
+    const uint4 kd = lds_u4(ks);
+    unsigned row = kd.x >> g4 & 15u, at = slab + kd.y + 8 * __popc(kd.x & ((1u << g4) - 1u));
+    for (; row; row &= row - 1u, at += 8) {
+      const unsigned kk = __ffs((int)row) - 1;
+      const unsigned r = ((kk & 2 ? kd.w : kd.z) >> (16 * (kk & 1))) & 0xffffu;
+      const double v = lds_d(at);
+      const double2 x = lds_d2(slab + ((r ^ c) << 4)), y = lds_d2(slab + ((r ^ (c + 1)) << 4));
+      s.x = __fma_rn(v, x.x, s.x);
+      s.y = __fma_rn(v, x.y, s.y);
+      s.z = __fma_rn(v, y.x, s.z);
+      s.w = __fma_rn(v, y.y, s.w);
+    }
+  }
+  return s;
+}
+
+// The group's sums of a lane's row and columns 4 t .. 4 t + 3.
+template <int PREF>
+__device__ __forceinline__ void slab_sums(unsigned ks, int nkt, unsigned slab, int lane, double (&sM)[4]) {
+  double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
+  slab_tiles<PREF>(ks, nkt, slab, lane, acc0, acc1);
+  sM[0] = acc0[0];
+  sM[1] = acc1[0];
+  sM[2] = acc0[1];
+  sM[3] = acc1[1];
+  if (__any_sync(0xffffffffu, isnan(nan_mark(sM)))) {
+    const double4 s = slab_entries(ks, nkt, slab, lane);
+    sM[0] = s.x;
+    sM[1] = s.y;
+    sM[2] = s.z;
+    sM[3] = s.w;
+  }
+}
+
 // Bin-local rows.  CTA = (bin e, 16-column tile); the state slab of bin e, the
 // bin's entries, k-tiles, row groups and row factors arrive in shared memory by
 // asynchronous copies; a warp then walks its row groups (balanced over the
@@ -2068,9 +2119,7 @@ __device__ __forceinline__ void slab_tiles(unsigned ks, int nkt, unsigned slab, 
 // applies the stage update to its eight rows, a lane four adjacent columns of a
 // row.  The rows' FD term (fdbuf), F(x) in stage 2 and injection slots are
 // loaded before the group's products.
-// REC: the adjoint's record pass (P / Q sensitivities).  A mother's state
-// multiplies the zeros of the rows that do not couple to it, so a non-finite
-// state of one species reaches the other rows of its tiles too.
+// REC: the adjoint's record pass (P / Q sensitivities).
 //
 // Bound by HBM by bytes.  One row per quarter-warp with the entries' states
 // gathered one by one was bound by shared-memory wavefronts (28M per launch at
@@ -2180,10 +2229,9 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slab(StepParams p) {
         if (STAGE == 2) load4(p.rec_sx + ro, rsx);
       }
     }
-    double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
-    if (s.photohad) slab_tiles<PREF>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, acc0, acc1);
+    double sM[4] = {0.0, 0.0, 0.0, 0.0};
+    if (s.photohad) slab_sums<PREF>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, sM);
     if (have) {
-      const double sM[4] = {acc0[0], acc1[0], acc0[1], acc1[1]};
       double own[4];
       {
         const double2 oa = slab_chunk(L.slab, sp, 2 * t4), ob = slab_chunk(L.slab, sp, 2 * t4 + 1);
@@ -3125,6 +3173,36 @@ __global__ void __launch_bounds__(256) k_fdT_dense(AdjBlk q) {
   }
 }
 
+// One warp's rows and columns of k_bandT<.., FD> term by term.  The stencil's tiles multiply the bins outside it by
+// zero, which is a NaN where v is not finite; a warp that finds one in its sums comes here and writes them again.
+template <int RT, int J>
+__device__ __noinline__ void bandT_rows(const double* v, const double* fdT_dense, const double* kap, const int* band_spec,
+                                        int nb, const double* A, int sp, int d, int ld, int c0, double* bT) {
+  const int lane = threadIdx.x & 31;
+  for (int row = lane >> 2; row < d; row += 8) {
+    double2 t = make_double2(0.0, 0.0);
+    auto add = [&](double w, int species, int e) {
+      const double* x = v + ((size_t)species * d + e) * ld + c0 + (lane & 3) * 2;
+      t.x += w * x[0];
+      t.y += w * x[1];
+    };
+    for (int e = max(row - kFdHalo, 0); e <= min(row + kFdHalo, d - 1); ++e)
+      add(fdT_dense[row * kFdDenseW + e - row + kFdHalo], sp, e);
+    t.x *= kap[row];
+    t.y *= kap[row];
+    for (int b = 0; b < nb; ++b)
+      for (int jj = 0; jj < J; ++jj)
+        for (int u = 0; u < 4; ++u) {
+          const int e = 4 * (row / 8 * 2 + jj - (J - 2)) + u;
+          if (e >= 0 && e < d)
+            add(A[(((b * (RT / 2) + row / 16) * J + jj) * 32 + row % 8 * 4 + u) * 2 + (row >> 3 & 1)], band_spec[b], e);
+        }
+    double* o = bT + ((size_t)sp * d + row) * ld + c0 + (lane & 3) * 2;
+    o[0] = t.x;
+    o[1] = t.y;
+  }
+}
+
 // bT = band part of M_off^T v.  CTA = (64-column block, mother-species group),
 // 8 warps; warp = one 8-column tile.  The warp loads the v fragments of both
 // band species once (k-tiles of 4 daughter bins); per mother species the CTA
@@ -3258,6 +3336,14 @@ __global__ void __launch_bounds__(256, 1) k_bandT(AdjBlk q) {
         o.y = acc[mt][1];
         *reinterpret_cast<double2*>(out + (size_t)row * ld) = o;
       }
+      if (FD) {
+        float mark = 0.0f;
+#pragma unroll
+        for (int mt = 0; mt < RT; ++mt) mark += nan_mark(acc[mt]);
+        if (__any_sync(0xffffffffu, isnan(mark)))
+          bandT_rows<RT, J>(q.v, q.fdT_dense, q.rf + 3 * q.n + (size_t)sp * d, q.band_spec, q.nb, As + stage * ABLK, sp, d, ld,
+                            c0, q.bT);
+      }
     }
     __syncthreads();
   }
@@ -3361,10 +3447,9 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 2) k_slabT(AdjBlk q) {
       rf2 = STAGE == 1 ? q.rf[2 * q.n + r] : (q.rf_prev ? q.rf_prev[2 * q.n + r] : 0.0);
       if (STAGE == 1 && q.gb_inj) slot = q.inj_slot[r];
     }
-    double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
-    if (photohad) slab_tiles<2>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, acc0, acc1);
+    double sM[4] = {0.0, 0.0, 0.0, 0.0};
+    if (photohad) slab_sums<2>(smem_u32(L.ks + G->kt0), G->nkt, smem_u32(L.slab), lane, sM);
     if (have) {
-      const double sM[4] = {acc0[0], acc1[0], acc0[1], acc1[1]};
       double out[4], res[4], nv[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
