@@ -40,7 +40,9 @@ extern "C" {
 #define PB_EM_CASCADE 64u   /* co-evolved EM cascade (run.enable_em_cascade) */
 
 /* pb_set_option / pb_get_info keys */
-#define PB_OPT_BATCHED_KERNELS 1 /* 1 (default): bin-blocked kernels for K > 1 when the layout allows; 0: row kernels */
+#define PB_OPT_BATCHED_KERNELS 1 /* 1 (default): for K > 1 all steps in one launch on networks of up to 1,024 states
+                                    (no checkpoints or EM cascade, one wave of clusters), else the bin-blocked
+                                    kernels when the layout allows; 0: row kernels */
 #define PB_INFO_BLOCKED_LAYOUT 2 /* 1 if pb_set_layout found a pattern the bin-blocked kernels handle */
 #define PB_INFO_LAST_BLOCKED 3   /* 1 if the last pb_solve ran the bin-blocked kernels */
 #define PB_INFO_BAND_SPECIES 4   /* species whose coupling rows leave their energy bin */
@@ -218,8 +220,9 @@ int pb_get_info(pb_context* ctx, int32_t key, int64_t* value);
 
 /* Measurement aid: re-runs the bin-blocked kernels of one stage (1 or 2) of
  * step `step` of the last solve, each kernel alone between CUDA events on the
- * context's stream, and returns the mean of `reps` launches in milliseconds:
- * ms[0] FD term, ms[1] bin-local rows, ms[2] band partial sums, ms[3] band
+ * context's stream (after a small network's solve in one launch too, whose
+ * operator it first folds into those kernels' form), and returns the mean of
+ * `reps` launches in milliseconds: ms[0] FD term, ms[1] bin-local rows, ms[2] band partial sums, ms[3] band
  * rows (0 for a kernel the stage does not run).  Overwrites the stage's
  * output buffers.  No reference counterpart. */
 int pb_profile_stage(pb_context* ctx, int64_t step, int32_t stage, int32_t reps, double* ms);
@@ -354,8 +357,9 @@ int pb_solve(pb_context* ctx, const pb_solve_args* args);
  * `args` (normally a short schedule with every column active, on the live
  * operator, injection and photon field) `reps` + 1 times for each candidate
  * (band-tile CTA warps 8 / 4, k_slab prefetch depth 1 / 2 / 3, k_slab staging
- * by TMA / cp.async), scores each by its fastest step loop, and leaves the
- * fastest set on the context (the PB_OPT_BAND_WARPS, PB_OPT_SLAB_PREFETCH and
+ * by TMA / cp.async), scores each by its fastest step loop (of the bin-blocked
+ * kernels also where a plain solve of the network takes one launch: its
+ * gradients run them), and leaves the fastest set on the context (the PB_OPT_BAND_WARPS, PB_OPT_SLAB_PREFETCH and
  * PB_OPT_TMA_STAGING options).  Writes up to max_out candidates to out, the
  * chosen one first, and their count to n_out.  `args->state` receives the
  * short solve's states.  Replaces: the fixed K-dependent multi-RHS tile

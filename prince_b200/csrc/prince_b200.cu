@@ -200,7 +200,7 @@ struct pb_context {
   DBuf X, A, F, rowf;
   DBuf scan_tmp;
   size_t scan_tmp_bytes = 0;
-  int32_t last_W = 0;
+  int32_t last_W = 0, last_dph = 0;  // windows and photon bins of the last solve
   bool have_solution = false;
   std::vector<StepScal> h_scal;  // step scalars of the current solve (host copy)
   std::vector<int32_t> h_nact;  // active columns of each step of the last solve (host copy)
@@ -252,6 +252,7 @@ struct pb_context {
   int32_t band_warps = 8;           // warps of a k_band CTA (PB_OPT_BAND_WARPS: 8 or 4)
   int32_t slab_pre = kSlabPreDefault;  // k_slab: pairs of k-tile descriptors held (PB_OPT_SLAB_PREFETCH: 1..3)
   bool last_blocked = false;
+  bool op_blocked = false;          // band_vals and slab_vals hold the last solve's operator in the current layout
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // the EM hook of a step beside the next step's nuclear stage (decoupled EM grid)
@@ -4275,6 +4276,38 @@ void join_hook(pb_context* c, bool& hook_pending, cudaStream_t st) {
   hook_pending = false;
 }
 
+// Buffers of the bin-blocked kernels for W windows and leading dimension ld.
+int ensure_blocked(pb_context* c, int W, int ld) {
+  PB_CUDA(c, c->slab_vals.ensure((size_t)W * std::max<int64_t>(c->slab_nent, 1) * sizeof(double)));
+  PB_CUDA(c, c->fdbuf.ensure((size_t)c->n * ld * sizeof(double)));
+  PB_CUDA(c, c->band_vals.ensure((size_t)W * std::max<int64_t>(c->band_stride, 1) * sizeof(double)));
+  PB_CUDA(c, c->band_part.ensure((size_t)kMaxBandGroups * std::max(c->band_nb, 1) * c->lay_d * ld * sizeof(double)));
+  return PB_OK;
+}
+
+// Zeros the band tiles and the bins' entries: the fold writes the entries that the first window keeps.
+int clear_blocked(pb_context* c, int W, cudaStream_t st) {
+  if (c->band_stride > 0) PB_CUDA(c, cudaMemsetAsync(c->band_vals.p, 0, (size_t)W * c->band_stride * sizeof(double), st));
+  if (c->slab_nent > 0) PB_CUDA(c, cudaMemsetAsync(c->slab_vals.p, 0, (size_t)W * c->slab_nent * sizeof(double), st));
+  return PB_OK;
+}
+
+// The coupling entries of W windows: the fold kernel times the windows' photon vectors, into the rows' values and
+// diagonal and, for the bin-blocked kernels, into the band tiles and the bins' entries.
+void launch_fold(pb_context* c, int W, bool blocked, cudaStream_t st) {
+  const int64_t R = c->R, mstride = std::max<int64_t>(R, 1);
+  const int* dest = c->dest.as<int>();
+  const FoldTile ft = fold_tile(c->dph, W);
+  const FoldArgs fa{c->kernel.as<double>(), R, c->dph, (c->dph + 3) / 4 * 4, W, c->PT.as<double>(), dest, dest + mstride,
+                    c->m_vals.as<double>(), mstride, c->m_diag.as<double>(), c->n,
+                    blocked ? c->band_slot.as<int>() : nullptr, blocked ? c->band_vals.as<double>() : nullptr,
+                    c->band_stride, blocked ? c->slab_slot.as<int>() : nullptr,
+                    blocked ? c->slab_vals.as<double>() : nullptr, c->slab_nent, ft.wm, ft.wn, ft.stages};
+  const int64_t ftiles = (R + 32 * ft.wm - 1) / (32 * ft.wm);
+  const unsigned fcols = blocks_for(W, 16 * ft.wn);
+  k_fold_gemm<<<dim3((unsigned)std::min<int64_t>(ftiles, c->num_sms), fcols), 32 * ft.wm * ft.wn, ft.smem, st>>>(fa);
+}
+
 // Whether a solve runs k_small, and how: one wave of clusters must hold all
 // columns (beyond it the bin-blocked kernels read the operator fewer times).
 // One column per cluster and the largest cluster that leaves the columns in
@@ -5327,6 +5360,7 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
     std::stable_sort(sspec.begin(), sspec.end(), [&](int32_t a, int32_t b) { return cnt[a] > cnt[b]; });
   }
   c->blocked_ok = false;
+  c->op_blocked = false;
   c->band_tma_fits = false;
   c->lay_d = d;
   c->lay_nsp = nsp;
@@ -5507,7 +5541,9 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   if (!ms || reps < 1 || (stage != 1 && stage != 2)) return fail(c, PB_ERR_ARG, "pb_profile_stage: bad arguments");
   if (!c->have_solution) return fail(c, PB_ERR_STATE, "pb_profile_stage: run pb_solve first");
   const int K = c->last_K;
-  if (!use_blocked(c, K) || !c->last_blocked) return fail(c, PB_ERR_STATE, "pb_profile_stage: the last solve did not run the bin-blocked kernels");
+  if (!use_blocked(c, K)) return fail(c, PB_ERR_STATE, "pb_profile_stage: the last solve's columns do not run the bin-blocked kernels");
+  if (!c->op_blocked && (!c->have_kernel || c->dph != c->last_dph))
+    return fail(c, PB_ERR_STATE, "pb_profile_stage: the photon grid has changed since the last solve");
   if (step < 0 || step >= c->last_S || c->h_nact[step] == 0) return fail(c, PB_ERR_ARG, "pb_profile_stage: step without active columns");
   int rc = set_device(c);
   if (rc) return rc;
@@ -5515,6 +5551,17 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   const uint32_t flags = c->last_flags;
   const bool pair = (flags & PB_PAIRPROD) && (flags & PB_PARTIAL_DIFF);
   const bool inj = (flags & PB_INJECTION) && c->n_src > 0;
+  const bool photohad = (flags & PB_PHOTOHAD) != 0, kap = (flags & PB_PARTIAL_DIFF) != 0;
+  cudaStream_t st = c->stream;
+  PB_CUDA(c, c->d_err.ensure(sizeof(int)));
+  if (!c->op_blocked) {  // a small network's solve in one launch, or another layout's: its operator in these kernels' form
+    if ((rc = ensure_blocked(c, c->last_W, ld)) || (rc = ensure_tmaps(c, true, ld)) || (rc = clear_blocked(c, c->last_W, st)))
+      return rc;
+    if (photohad && c->R > 0) launch_fold(c, c->last_W, true, st);
+    PB_CUDA(c, cudaMemcpyAsync(c->A.p, c->X.p, (size_t)c->n * ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    PB_CUDA(c, cudaMemcpyAsync(c->F.p, c->X.p, (size_t)c->n * ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    c->op_blocked = true;
+  }
   StepParams p;
   memset(&p, 0, sizeof(p));
   fill_step_params(c, p, K, ld, flags, pair, inj, c->last_S, ld / kColTile);
@@ -5524,13 +5571,10 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   p.xout = c->X.as<double>();
   p.tmap_src = stage_tmap(c, stage);
   p.tmap_band = stage_tmap_band(c, stage);
-  PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   p.err = c->d_err.as<int>();
-  cudaStream_t st = c->stream;
   p.rf_k0 = step;
   launch_prep(p, c->s_scal.as<StepScal>(), step, 1, st);
   set_step_factors(p, step);
-  const bool photohad = (flags & PB_PHOTOHAD) != 0, kap = (flags & PB_PARTIAL_DIFF) != 0;
   const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
   const BandPlan plan = band_plan(c, p);
   const CUtensorMap* const tmap_band = p.tmap_band;
@@ -6081,13 +6125,8 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
     PB_CUDA(c, c->ckpt.ensure((size_t)((S + a->ckpt_every - 1) / a->ckpt_every + 1) * n * ld * sizeof(double)));
   const SmallPlan small = small_plan(c, K, flags, a->ckpt_every);
   const bool blocked = !small.cc && use_blocked(c, K);
-  if (blocked) {
-    PB_CUDA(c, c->slab_vals.ensure((size_t)W * std::max<int64_t>(c->slab_nent, 1) * sizeof(double)));
-    PB_CUDA(c, c->fdbuf.ensure(sbytes));
-    PB_CUDA(c, c->band_vals.ensure((size_t)W * std::max<int64_t>(c->band_stride, 1) * sizeof(double)));
-    PB_CUDA(c, c->band_part.ensure((size_t)kMaxBandGroups * std::max(c->band_nb, 1) * c->lay_d * ld * sizeof(double)));
-  }
-  c->last_blocked = blocked;
+  if (blocked && (rc = ensure_blocked(c, W, ld))) return rc;
+  c->last_blocked = c->op_blocked = blocked;
   PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   if ((rc = ensure_tmaps(c, blocked, ld))) return rc;
   c->last_tma = blocked && c->tma_ok;
@@ -6141,10 +6180,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   int* dest = c->dest.as<int>();
   int* diag_row = dest + mstride;
   PB_CUDA(c, cudaMemsetAsync(c->m_diag.p, 0, (size_t)W * n * sizeof(double), st));
-  if (blocked && c->band_stride > 0)
-    PB_CUDA(c, cudaMemsetAsync(c->band_vals.p, 0, (size_t)W * c->band_stride * sizeof(double), st));
-  if (blocked && c->slab_nent > 0)
-    PB_CUDA(c, cudaMemsetAsync(c->slab_vals.p, 0, (size_t)W * c->slab_nent * sizeof(double), st));
+  if (blocked && (rc = clear_blocked(c, W, st))) return rc;
   if ((flags & PB_PHOTOHAD) && R > 0) {
     k_fold_first<<<blocks_for(R + 1, 8), 256, 0, st>>>(c->kernel.as<double>(), R, c->dph, c->PT.as<double>(),
                                                        c->cpl_is_diag.as<int>(), c->keep.as<int>());
@@ -6161,15 +6197,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
                                                            c->seg_me.as<int64_t>());
       ++launches;
     }
-    const FoldTile ft = fold_tile(c->dph, W);
-    const FoldArgs fa{c->kernel.as<double>(), R, c->dph, (c->dph + 3) / 4 * 4, W, c->PT.as<double>(), dest, diag_row,
-                      c->m_vals.as<double>(), mstride, c->m_diag.as<double>(), n,
-                      blocked ? c->band_slot.as<int>() : nullptr, blocked ? c->band_vals.as<double>() : nullptr,
-                      c->band_stride, blocked ? c->slab_slot.as<int>() : nullptr,
-                      blocked ? c->slab_vals.as<double>() : nullptr, c->slab_nent, ft.wm, ft.wn, ft.stages};
-    const int64_t ftiles = (R + 32 * ft.wm - 1) / (32 * ft.wm);
-    const unsigned fcols = blocks_for(W, 16 * ft.wn);
-    k_fold_gemm<<<dim3((unsigned)std::min<int64_t>(ftiles, c->num_sms), fcols), 32 * ft.wm * ft.wn, ft.smem, st>>>(fa);
+    launch_fold(c, W, blocked, st);
     launches += 5;
   } else {
     PB_CUDA(c, cudaMemsetAsync(c->m_indptr.p, 0, ((size_t)n + 1) * sizeof(int64_t), st));
@@ -6219,6 +6247,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   PB_CUDA(c, cudaEventElapsedTime(&c->last_steps_ms, c->ev2, c->ev3));
   c->last_launches = launches;
   c->last_W = W;
+  c->last_dph = c->dph;
   c->have_solution = true;
   c->last_ckpt = a->ckpt_every;
   c->last_S = S;

@@ -69,3 +69,23 @@ def test_small_network_with_more_than_512_rows(K):
     assert worst <= TOL, (worst, above, total)
     assert above <= 1e-4 * total, (above, total)
 
+
+
+def test_stage_profile_after_a_solve_in_one_launch(light):
+    """The bin-blocked kernels of a small network's batch can be timed after a solve that ran in one launch, as
+    after one that ran them; the states that the solve left are those of before, and the next solve's too."""
+    import numpy as np
+    from prince_b200 import _lib
+    from prince_b200.solvers import MultiRHSPropagationSolverETD2
+    from workloads import draw_points, point_source
+    m = MultiRHSPropagationSolverETD2(initial_z=0.05, final_z=0.0, prince_run=light, K=19)
+    for k, p in enumerate(draw_points(light, 19, seed=19, z_range=(0.05, 0.06))):
+        m[k].add_source_class(point_source(light, p))
+    m.solve(dz=1e-3)
+    ctx, state = m._dev.ctx, m.state.copy()
+    assert ctx.info(_lib.PB_INFO_LAST_BLOCKED) == 0
+    for stage in (1, 2):
+        times = ctx.profile_stage(10, stage, reps=2)
+        assert all(t > 0.0 for t in times), times
+    m.solve(dz=1e-3)
+    assert np.array_equal(m.state, state)
