@@ -222,9 +222,9 @@ int pb_get_info(pb_context* ctx, int32_t key, int64_t* value);
  * step `step` of the last solve, each kernel alone between CUDA events on the
  * context's stream (after a small network's solve in one launch too, whose
  * operator it first folds into those kernels' form), and returns the mean of
- * `reps` launches in milliseconds: ms[0] FD term, ms[1] bin-local rows, ms[2] band partial sums, ms[3] band
- * rows (0 for a kernel the stage does not run).  Overwrites the stage's
- * output buffers.  No reference counterpart. */
+ * `reps` launches in milliseconds: ms[0] FD term, ms[1] bin-local rows, ms[2]
+ * band partial sums, ms[3] band rows (0 for a kernel the stage does not run).
+ * Overwrites the stage's output buffers.  No reference counterpart. */
 int pb_profile_stage(pb_context* ctx, int64_t step, int32_t stage, int32_t reps, double* ms);
 
 /* Measured FP64 tensor-pipe (DMMA) throughput of the device in TFLOP/s, from a

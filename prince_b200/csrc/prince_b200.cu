@@ -72,20 +72,24 @@ struct DBuf;
 // Device memory of the cascade builds' temporaries, kept between calls: each call
 // hands it out from the start.  What does not fit is allocated on its own and
 // the next call starts with enough in one piece (allocating and freeing the
-// about 45 buffers of a build took a quarter of its time).
+// about 45 buffers of a build took a quarter of its time), up to kArenaMax (700
+// windows of 128 bins; beyond it the rest is allocated and freed by each call).
+// An idle arena is given up when an allocation of its context fails.
+constexpr size_t kArenaMax = (size_t)2 << 30;
 struct Arena {
   void* p = nullptr;
   size_t bytes = 0, used = 0, want = 0;
+  bool busy = false;
   void begin() {  // no work on the memory may be in flight
-    if (want > bytes) {
-      if (p) cudaFree(p);
-      p = nullptr;
-      bytes = 0;
-      if (cudaMalloc(&p, want) == cudaSuccess) bytes = want;
+    if (std::min(want, kArenaMax) > bytes) {
+      release();
+      if (cudaMalloc(&p, std::min(want, kArenaMax)) == cudaSuccess) bytes = std::min(want, kArenaMax);
       else cudaGetLastError();
     }
     used = want = 0;
+    busy = true;
   }
+  void end() { busy = false; }
   void* take(size_t n) {
     n = (n + 255) / 256 * 256;
     want += n;
@@ -94,12 +98,16 @@ struct Arena {
     used += n;
     return q;
   }
-  void release() {
+  // Frees the memory, not the size that the next call starts with; whether there was any.
+  bool release() {
+    const bool had = p != nullptr;
     if (p) cudaFree(p);
     p = nullptr;
-    bytes = used = want = 0;
+    bytes = used = 0;
+    return had;
   }
 };
+thread_local Arena* t_arena = nullptr;  // the arena of the context that this thread's call works on (set_device)
 struct DBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -121,6 +129,11 @@ struct DBuf {
     bytes = 0;
     if (want == 0) want = 16;
     cudaError_t e = cudaMalloc(&p, want);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // the caller reports it; a later launch must not find it
+      if (t_arena && !t_arena->busy && t_arena->release()) e = cudaMalloc(&p, want);
+      if (e != cudaSuccess) cudaGetLastError();
+    }
     if (e == cudaSuccess) bytes = want;
     return e;
   }
@@ -3746,6 +3759,7 @@ int upload(pb_context* c, DBuf& b, const T* src, size_t count) {
 }
 
 int set_device(pb_context* c) {
+  t_arena = &c->em_arena;
   PB_CUDA(c, cudaSetDevice(c->device));
   return PB_OK;
 }
@@ -4806,6 +4820,7 @@ void pb_destroy(pb_context* c) {
   if (c->stream3) cudaStreamSynchronize(c->stream3);
   for (DBuf* b : all_buffers(c)) b->release();
   for (StepGraph& g : c->step_graphs) cudaGraphExecDestroy(g.exec);
+  if (t_arena == &c->em_arena) t_arena = nullptr;
   c->em_arena.release();
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
@@ -5840,6 +5855,7 @@ int pb_em_transfer(pb_context* c, const pb_em_transfer_args* a) {
   auto cleanup = [&]() {
     cudaStreamSynchronize(st);
     for (DBuf* b : all) b->release();
+    c->em_arena.end();
   };
   auto fail_cuda = [&](cudaError_t err, const char* what) {
     cleanup();
@@ -6015,6 +6031,7 @@ int pb_bh_shape(pb_context* c, const pb_bh_shape_args* a) {
   auto cleanup = [&]() {
     cudaStreamSynchronize(st);
     for (DBuf* b : {&Ee, &Ep, &eps, &zs, &K, &neps, &col, &R}) b->release();
+    c->em_arena.end();
   };
   if ((rc = upload(c, Ee, a->E_e, (size_t)ne)) || (rc = upload(c, Ep, a->E_p, (size_t)np)) ||
       (rc = upload(c, eps, a->eps, (size_t)nk)) || (rc = upload(c, zs, a->z, (size_t)nz))) {
