@@ -12,7 +12,10 @@ else -> ``RuntimeError``, with the library's message.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
+import threading
+import weakref
 
 import numpy as np
 
@@ -209,6 +212,30 @@ def host_buffer(shape):
         return np.empty(shape)
 
 
+_LOCKED_MAX = 256 << 20  # bytes of page-locked cascade results alive at a time (700 windows of 128 bins)
+_locked = 0
+_locked_guard = threading.RLock()  # a finalizer may run inside the guarded lines
+
+
+def _locked_add(nbytes):
+    global _locked
+    with _locked_guard:
+        _locked += nbytes
+
+
+def bounded_host_buffer(shape):
+    """``host_buffer`` for results that a caller may keep for long (a view of one window keeps its whole block):
+    page-locked while the living ones stay within ``_LOCKED_MAX``, else a plain array."""
+    nbytes = 8 * math.prod(shape)
+    with _locked_guard:
+        if _locked + nbytes > _LOCKED_MAX:
+            return np.empty(shape)
+        _locked_add(nbytes)
+    a = host_buffer(shape)
+    weakref.finalize(a, _locked_add, -nbytes).atexit = False
+    return a
+
+
 class Context:
     """One device context of the C library."""
 
@@ -292,8 +319,8 @@ class Context:
         keep = [_f64(E), _f64(zs), _f64(dl_step), _f64(eps), _f64(eps_o), _f64(mu)]
         E_, z_, dl_, eps_, epso_, mu_ = keep
         n, nz = E_.size, z_.size
-        Tg = host_buffer((nz, n, n))
-        Te = host_buffer((nz, n, n))
+        Tg = bounded_host_buffer((nz, n, n))
+        Te = bounded_host_buffer((nz, n, n))
         it = C.c_int32(0)
         a = EmTransferArgs()
         a.n, a.E = n, _ptr(E_, C.c_double)
@@ -314,7 +341,7 @@ class Context:
         from .constants import PRINCE_UNITS as U
 
         Ee, Ep, ep, z = _f64(E_e), _f64(E_p), _f64(eps), _f64(np.atleast_1d(zs))
-        R = host_buffer((z.size, Ee.size, Ep.size))
+        R = bounded_host_buffer((z.size, Ee.size, Ep.size))
         a = BhShapeArgs()
         a.n_e, a.E_e, a.n_p, a.E_p = Ee.size, _ptr(Ee, C.c_double), Ep.size, _ptr(Ep, C.c_double)
         a.n_eps, a.eps, a.n_z, a.z = ep.size, _ptr(ep, C.c_double), z.size, _ptr(z, C.c_double)

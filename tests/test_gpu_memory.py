@@ -62,3 +62,26 @@ def test_solve_takes_the_idle_temporaries_when_memory_runs_out(em_run):
         del hog
     assert np.isfinite(x).all() and (x != 1.0).any()
     _build(em_run, 3)
+
+
+def test_page_locked_cascade_results_are_bounded(em_run):
+    """Results that are kept are page-locked up to a bound and plain beyond it, the same values; one window kept
+    counts as its block, and what is released counts no more."""
+    from prince_b200 import _lib
+
+    def locked(a):
+        return torch.from_numpy(a).is_pinned()
+
+    Tg, Te = _build(em_run, 100)
+    assert locked(Tg) and locked(Te)
+    kept, total = [], 0
+    while total <= 2 * _lib._LOCKED_MAX:
+        g, e = _build(em_run, 100)
+        kept.append(g[0])   # views: each keeps its build's block alive
+        kept.append(e[0])
+        total += g.nbytes + e.nbytes
+        assert np.array_equal(g, Tg) and np.array_equal(e, Te)
+    assert sum(Tg.nbytes for a in kept if locked(a)) <= _lib._LOCKED_MAX
+    assert not locked(kept[-1])
+    del kept, g, e
+    assert all(locked(a) for a in _build(em_run, 100))
