@@ -923,9 +923,10 @@ struct StepParams {
   double* fdkp;             // n x ld: D_off (kappa_pair v), adjoint record pass with the photon scale, or null
   const int* band_spec;     // species with cross-bin coupling rows
   int nb;
+  int part_ld;              // band_part's columns: the step's (hcols), padded to column tiles
   const double* band_vals;  // [W][nsp][band pair][2][RT][J][32] DMMA A fragments
   int64_t band_stride;
-  double* band_part;        // [G][nb][d][ld] partial sums of the band rows
+  double* band_part;        // [G][nb][d][part_ld] partial sums of the band rows
   int ngroups;              // mother-species groups of the band launch
   int spg;                  // species per group
 };
@@ -2456,7 +2457,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_band(StepParams p) {
 #pragma unroll
   for (int b = 0; b < 2; ++b) {
     if (2 * pair + b >= p.nb) continue;
-    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + b) * d * ld;
+    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + b) * d * p.part_ld;
 #pragma unroll
     for (int rt = 0; rt < RT; ++rt) {
       const int row = 8 * rt + (lane >> 2);
@@ -2464,7 +2465,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_band(StepParams p) {
       double2 o;
       o.x = acc[b][rt][0];
       o.y = acc[b][rt][1];
-      *reinterpret_cast<double2*>(P + (size_t)row * ld + c0 + kr * 2) = o;
+      *reinterpret_cast<double2*>(P + (size_t)row * p.part_ld + c0 + kr * 2) = o;
     }
   }
 }
@@ -2500,8 +2501,8 @@ __global__ void __launch_bounds__(kFinWarps * 32) k_band_finish(StepParams p) {
     if (STAGE == 1) f1 = p.phi1[r];
     else fx = p.f[idx];
   }
-  const double* part = p.band_part + ((size_t)b * p.d + e) * p.ld + col;
-  const size_t gs = (size_t)p.nb * p.d * p.ld;
+  const double* part = p.band_part + ((size_t)b * p.d + e) * p.part_ld + col;
+  const size_t gs = (size_t)p.nb * p.d * p.part_ld;
   double t = 0.0;
   if (col < s.ncols) {
 #pragma unroll 4
@@ -2721,7 +2722,7 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
     if (2 * pair + bw + b >= p.nb) continue;
-    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + bw + b) * d * ld;
+    double* __restrict__ P = p.band_part + (size_t)(g * p.nb + 2 * pair + bw + b) * d * p.part_ld;
 #pragma unroll
     for (int rt = 0; rt < 2 * NP; ++rt) {
       const int row = 8 * (2 * rp0 + rt) + (lane >> 2);
@@ -2729,7 +2730,7 @@ __global__ void __launch_bounds__(32 * BandTma<RT, J, CT>::kWarps, 1) k_band_tma
       double2 o;
       o.x = acc[b][rt][0];
       o.y = acc[b][rt][1];
-      *reinterpret_cast<double2*>(P + (size_t)row * ld + c0 + kr * 2) = o;
+      *reinterpret_cast<double2*>(P + (size_t)row * p.part_ld + c0 + kr * 2) = o;
     }
   }
 }
@@ -4040,7 +4041,7 @@ const CUtensorMap* stage_tmap_band(const pb_context* c, int stage) {
 }
 
 // k_band's launch for the columns p.hcols: columns per CTA and mother-species
-// groups (p.spg, p.ngroups).
+// groups.
 //
 // Four-warp CTAs (PB_OPT_BAND_WARPS) stay within one wave, so that each SM holds
 // at most one beside its k_slab CTA.  Otherwise there is one CTA per SM and the
@@ -4054,23 +4055,23 @@ const CUtensorMap* stage_tmap_band(const pb_context* c, int stage) {
 // columns, 39 at 128).  The cp.async kernel takes 64 columns per CTA with the
 // same groups, so that both stagings add the same partial sums.
 struct BandPlan {
-  int ct, cblocks;
+  int ct, cblocks, spg, groups, part_ld;
 };
-BandPlan band_plan(const pb_context* c, StepParams& p) {
-  const int np = std::max(c->band_npairs, 1);
-  BandPlan plan{p.hcols <= 8 ? 1 : 8, 1};
+BandPlan band_plan(const pb_context* c, int hcols) {
+  const int np = std::max(c->band_npairs, 1), nsp = c->lay_nsp;
+  BandPlan plan{hcols <= 8 ? 1 : 8, 1, 1, 1, (int)blocks_for(hcols, kColTile) * kColTile};
   int G = 1;
   if (c->band_warps == 4) {
-    plan.cblocks = (int)blocks_for(p.hcols, 32);
-    G = std::max(1, std::min({c->num_sms / (plan.cblocks * np), kMaxBandGroups, p.nsp}));
+    plan.cblocks = (int)blocks_for(hcols, 32);
+    G = std::max(1, std::min({c->num_sms / (plan.cblocks * np), kMaxBandGroups, nsp}));
   } else {
-    plan.cblocks = (int)blocks_for(p.hcols, 8 * plan.ct);
+    plan.cblocks = (int)blocks_for(hcols, 8 * plan.ct);
     int64_t best = -1;
-    for (int g = 1; g <= std::min(kMaxBandGroups, p.nsp); ++g) {
-      const int spg = (p.nsp + g - 1) / g;
-      if ((p.nsp + spg - 1) / spg != g) continue;
+    for (int g = 1; g <= std::min(kMaxBandGroups, nsp); ++g) {
+      const int spg = (nsp + g - 1) / g;
+      if ((nsp + spg - 1) / spg != g) continue;
       // full groups first, then the last group's shorter CTAs on the SMs that are free the earliest
-      const int64_t per = (int64_t)plan.cblocks * np, full = per * (g - 1), rest = p.nsp - (int64_t)(g - 1) * spg;
+      const int64_t per = (int64_t)plan.cblocks * np, full = per * (g - 1), rest = nsp - (int64_t)(g - 1) * spg;
       const int64_t q = full / c->num_sms, r = full % c->num_sms, layers = (per + c->num_sms - r - 1) / (c->num_sms - r);
       const int64_t cost = std::max(r > 0 ? (q + 1) * spg : 0, q * spg + layers * rest);
       if (best < 0 || cost < best) {
@@ -4079,9 +4080,26 @@ BandPlan band_plan(const pb_context* c, StepParams& p) {
       }
     }
   }
-  p.spg = (p.nsp + G - 1) / G;
-  p.ngroups = (p.nsp + p.spg - 1) / p.spg;
+  plan.spg = (nsp + G - 1) / G;
+  plan.groups = (nsp + plan.spg - 1) / plan.spg;
   return plan;
+}
+void apply_plan(StepParams& p, const BandPlan& plan) {
+  p.spg = plan.spg;
+  p.ngroups = plan.groups;
+  p.part_ld = plan.part_ld;
+}
+// The partial sums of every layout that the launches of a K-column solve take.  Many groups go with few columns:
+// 512 columns of the A <= 56 network take 15 MB (148 groups of all columns would take 116).
+int ensure_band_part(pb_context* c, int K) {
+  size_t most = 0;
+  for (int a = 1, h; a <= K; a = h + 1) {
+    h = launch_cols(K, a);
+    const BandPlan plan = band_plan(c, h);
+    most = std::max(most, (size_t)plan.groups * plan.part_ld);
+  }
+  PB_CUDA(c, c->band_part.ensure(most * std::max(c->band_nb, 1) * c->lay_d * sizeof(double)));
+  return PB_OK;
 }
 void launch_band(const pb_context* c, StepParams& p, const BandPlan& plan, cudaStream_t st) {
   if (c->band_warps == 8 && p.tmap_band) {
@@ -4115,7 +4133,8 @@ int64_t launch_blocked_stage(pb_context* c, StepParams& p, cudaStream_t st) {
   bool forked = false;
   p.fd_band = false;
   if (photohad && p.nb > 0) {
-    const BandPlan plan = band_plan(c, p);
+    const BandPlan plan = band_plan(c, p.hcols);
+    apply_plan(p, plan);
     // the loss term with the band tiles where a CTA covers the columns alone: at 64 columns a CTA the two
     // kernels beside each other are faster (A <= 56 network, 512 columns: 139 us for both, 145 us in one; 7
     // columns: 13 + 9 us in parallel, 12 us in one, without the fork)
@@ -4290,13 +4309,12 @@ void join_hook(pb_context* c, bool& hook_pending, cudaStream_t st) {
   hook_pending = false;
 }
 
-// Buffers of the bin-blocked kernels for W windows and leading dimension ld.
-int ensure_blocked(pb_context* c, int W, int ld) {
+// Buffers of the bin-blocked kernels for W windows and K columns (leading dimension ld).
+int ensure_blocked(pb_context* c, int W, int K, int ld) {
   PB_CUDA(c, c->slab_vals.ensure((size_t)W * std::max<int64_t>(c->slab_nent, 1) * sizeof(double)));
   PB_CUDA(c, c->fdbuf.ensure((size_t)c->n * ld * sizeof(double)));
   PB_CUDA(c, c->band_vals.ensure((size_t)W * std::max<int64_t>(c->band_stride, 1) * sizeof(double)));
-  PB_CUDA(c, c->band_part.ensure((size_t)kMaxBandGroups * std::max(c->band_nb, 1) * c->lay_d * ld * sizeof(double)));
-  return PB_OK;
+  return ensure_band_part(c, K);
 }
 
 // Zeros the band tiles and the bins' entries: the fold writes the entries that the first window keeps.
@@ -4436,7 +4454,7 @@ StepGraph* step_graph(pb_context* c, StepParams p, int K, int G, int cols, cudaS
   p.xout = nullptr;
   p.tmap_src = p.tmap_band = nullptr;
   p.err = nullptr;
-  p.ngroups = p.spg = 0;
+  p.ngroups = p.spg = p.part_ld = 0;
   p.n_steps = 0;
   std::vector<uint64_t> key;
   auto put_bytes = [&](const void* q, size_t bytes) {
@@ -5570,13 +5588,14 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   cudaStream_t st = c->stream;
   PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   if (!c->op_blocked) {  // a small network's solve in one launch, or another layout's: its operator in these kernels' form
-    if ((rc = ensure_blocked(c, c->last_W, ld)) || (rc = ensure_tmaps(c, true, ld)) || (rc = clear_blocked(c, c->last_W, st)))
+    if ((rc = ensure_blocked(c, c->last_W, K, ld)) || (rc = ensure_tmaps(c, true, ld)) || (rc = clear_blocked(c, c->last_W, st)))
       return rc;
     if (photohad && c->R > 0) launch_fold(c, c->last_W, true, st);
     PB_CUDA(c, cudaMemcpyAsync(c->A.p, c->X.p, (size_t)c->n * ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
     PB_CUDA(c, cudaMemcpyAsync(c->F.p, c->X.p, (size_t)c->n * ld * sizeof(double), cudaMemcpyDeviceToDevice, st));
     c->op_blocked = true;
   }
+  if ((rc = ensure_band_part(c, K))) return rc;  // the options may have changed since the solve
   StepParams p;
   memset(&p, 0, sizeof(p));
   fill_step_params(c, p, K, ld, flags, pair, inj, c->last_S, ld / kColTile);
@@ -5591,7 +5610,8 @@ int pb_profile_stage(pb_context* c, int64_t step, int32_t stage, int32_t reps, d
   launch_prep(p, c->s_scal.as<StepScal>(), step, 1, st);
   set_step_factors(p, step);
   const unsigned tiles = (unsigned)blocks_for(p.hcols, kColTile);
-  const BandPlan plan = band_plan(c, p);
+  const BandPlan plan = band_plan(c, p.hcols);
+  apply_plan(p, plan);
   const CUtensorMap* const tmap_band = p.tmap_band;
   if (!(photohad && p.nb > 0)) p.ngroups = 0;
   for (int kk = 0; kk < 4; ++kk) ms[kk] = 0.0;
@@ -6142,7 +6162,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
     PB_CUDA(c, c->ckpt.ensure((size_t)((S + a->ckpt_every - 1) / a->ckpt_every + 1) * n * ld * sizeof(double)));
   const SmallPlan small = small_plan(c, K, flags, a->ckpt_every);
   const bool blocked = !small.cc && use_blocked(c, K);
-  if (blocked && (rc = ensure_blocked(c, W, ld))) return rc;
+  if (blocked && (rc = ensure_blocked(c, W, K, ld))) return rc;
   c->last_blocked = c->op_blocked = blocked;
   PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   if ((rc = ensure_tmaps(c, blocked, ld))) return rc;
@@ -6429,6 +6449,7 @@ int pb_adjoint(pb_context* c, const pb_solve_args* a, const double* seed, int32_
   StepParams p;
   memset(&p, 0, sizeof(p));
   const int ctiles = ld / (K == 1 ? 1 : kColTile);
+  if (use_blocked(c, K) && (rc = ensure_band_part(c, K))) return rc;  // the options may have changed since the solve
   fill_step_params(c, p, K, ld, flags, pair, inj, S, ctiles);
   p.inv_scale = 1.0 / a->photon_scale;
   p.rf = c->rec_rf.as<double>();

@@ -85,3 +85,32 @@ def test_page_locked_cascade_results_are_bounded(em_run):
     assert not locked(kept[-1])
     del kept, g, e
     assert all(locked(a) for a in _build(em_run, 100))
+
+
+def test_band_partial_sums_take_the_launches_size():
+    """2,048 columns: a solve allocates its states (four arrays), its operator, and partial sums of the groups that
+    its launches take: a group has a species at least, so no more than 60 groups of the 192 band rows (189 MB), not
+    the 148 of the largest launch (466 MB)."""
+    from prince_b200 import _lib
+    from prince_b200.photonfields import device_components, device_table
+    from prince_b200.schedule import make_schedule, z_grid
+    from prince_b200.solvers import DeviceRun
+    from workloads import network_run
+    run = network_run(max_mass=16, n_species=60, seed=5)
+    ctx = DeviceRun.of(run, 0).ctx
+    ctx.set_photon_field(device_components(run.photon_field), table=device_table(run.photon_field))
+    n, K = run.dim_states, 2048
+    sched = make_schedule(z_grid(2e-3, 0.0, 1e-3), run.backend.update_rates_z_threshold)
+    x = np.ones((n, K))
+
+    def solve(cols):
+        ctx.solve(sched, _lib.PB_ADIABATIC | _lib.PB_PARTIAL_DIFF, cols, None,
+                  np.full(sched.n_steps, cols, dtype=np.int32), np.ascontiguousarray(x[:, :cols]), init_state=True)
+
+    solve(2)
+    before = _free()
+    solve(K)
+    assert ctx.info(_lib.PB_INFO_LAST_BLOCKED) == 1
+    taken = before - _free()
+    partial = run.spec_man.nspec * 192 * K * 8
+    assert taken <= 4 * x.nbytes + partial + (64 << 20), (taken, x.nbytes)
