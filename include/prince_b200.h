@@ -53,6 +53,8 @@ extern "C" {
 #define PB_OPT_TMA_STAGING 9     /* 1 (default): the bin-local and band-tile kernels stage by TMA (tensor maps,
                                     bulk copies); 0: cp.async */
 #define PB_INFO_STEP_CAPTURES 14 /* runs of steps captured by this context so far (a solve replays those it finds) */
+#define PB_INFO_LAST_SMALL 15    /* the last pb_solve in one launch of all steps: columns x 256 + CTAs of a cluster;
+                                    0 if it ran other kernels */
 #define PB_INFO_LAST_TMA 10      /* 1 if the last pb_solve staged the bin-local kernel by TMA */
 #define PB_OPT_BAND_WARPS 12       /* warps of a band-tile CTA: 8 (default, 64 columns, one CTA per SM) or 4
                                      (32 columns in half the registers and shared memory, so the band

@@ -31,6 +31,7 @@ PB_OPT_STAGING_WAIT_TRIES = 11
 PB_OPT_BAND_WARPS = 12
 PB_OPT_SLAB_PREFETCH = 13
 PB_INFO_STEP_CAPTURES = 14
+PB_INFO_LAST_SMALL = 15
 
 _d = C.POINTER(C.c_double)
 _i32 = C.POINTER(C.c_int32)

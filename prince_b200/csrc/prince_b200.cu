@@ -259,6 +259,7 @@ struct pb_context {
   std::vector<int32_t> small_len;   // their coupling entries
   int64_t fd_row_max = 0;           // off-diagonal FD entries of a row (at most)
   bool small_off = false;           // the tuner measures the bin-blocked kernels
+  int32_t last_small = 0;           // PB_INFO_LAST_SMALL
   int32_t batched_mode = 1;         // 0: general row kernels; 1: bin-blocked kernels when the layout allows
   int32_t tma_mode = 1;             // 1: k_slab stages by TMA when tensor maps can be encoded; 0: cp.async
   long long staging_wait_tries = kWaitTries;  // k_slab's first staging wait (PB_OPT_STAGING_WAIT_TRIES)
@@ -4391,9 +4392,9 @@ SmallPlan small_plan(pb_context* c, int K, uint32_t flags, int ckpt_every) {
       cfg.dynamicSmemBytes = smem;
       cfg.attrs = &at;
       cfg.numAttrs = 1;
-      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024) != cudaSuccess) continue;
       int fit = 0;
-      if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess || fit < clusters) {
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess || fit < clusters) {
         cudaGetLastError();
         continue;
       }
@@ -5730,6 +5731,7 @@ int pb_get_info(pb_context* c, int32_t key, int64_t* value) {
     case PB_INFO_BAND_ENTRIES: *value = c->band_nnz; return PB_OK;
     case PB_INFO_SLAB_ENTRIES: *value = c->slab_nnz; return PB_OK;
     case PB_INFO_SLAB_ROWS: *value = (int64_t)c->n_slab_spec * c->lay_d; return PB_OK;
+    case PB_INFO_LAST_SMALL: *value = c->last_small; return PB_OK;
     case PB_INFO_STEP_CAPTURES: *value = c->captures; return PB_OK;
     case PB_INFO_FD_DENSE: *value = c->fd_dense_ok ? 1 : 0; return PB_OK;
   }
@@ -6164,6 +6166,7 @@ int pb_solve(pb_context* c, const pb_solve_args* a) {
   const bool blocked = !small.cc && use_blocked(c, K);
   if (blocked && (rc = ensure_blocked(c, W, K, ld))) return rc;
   c->last_blocked = c->op_blocked = blocked;
+  c->last_small = small.cc * 256 + small.cs;
   PB_CUDA(c, c->d_err.ensure(sizeof(int)));
   if ((rc = ensure_tmaps(c, blocked, ld))) return rc;
   c->last_tma = blocked && c->tma_ok;

@@ -89,3 +89,41 @@ def test_stage_profile_after_a_solve_in_one_launch(light):
         assert all(t > 0.0 for t in times), times
     m.solve(dz=1e-3)
     assert np.array_equal(m.state, state)
+
+
+def _small_batch(run, K):
+    """A batch of K points over 50 steps: (solver after the solve, columns and CTAs of a cluster, sources)."""
+    from prince_b200 import _lib
+    from prince_b200.solvers import MultiRHSPropagationSolverETD2
+    from workloads import draw_points, point_source
+    srcs = [point_source(run, p) for p in draw_points(run, K, seed=K, z_range=(0.01, 0.06))]
+    m = MultiRHSPropagationSolverETD2(initial_z=0.05, final_z=0.0, prince_run=run, K=K)
+    for k, s in enumerate(srcs):
+        m[k].add_source_class(s)
+    m.solve(dz=1e-3)
+    return m, divmod(m._dev.ctx.info(_lib.PB_INFO_LAST_SMALL), 256), srcs
+
+
+@pytest.mark.parametrize("K,columns", [(2, 1), (17, 1), (75, 1), (149, 2), (296, 2), (297, 0)])
+def test_small_network_batches_take_one_launch(light, K, columns):
+    """The batch sizes of the oracle test above run the kernel that they are there for: a column per cluster up to
+    the SMs, then two, and beyond one wave the bin-blocked kernels."""
+    _, (cc, cs), _ = _small_batch(light, K)
+    assert cc == columns and (cs >= 1) == (columns > 0), (cc, cs)
+    if K == 2:
+        assert cs == 8
+
+
+def test_four_columns_per_cluster_match_the_oracle():
+    """576 states: 75 columns do not fit a CTA each, and take four per cluster of several CTAs."""
+    from prince_b200 import photonfields as pf, synth
+    from prince_b200.run import PriNCeRun
+    from workloads import A56_GRID, A56_PHOTON
+    model = synth.SyntheticPhotoNuclear(synth.light_network_species(), seed=1)
+    run = PriNCeRun(model, pf.CMBPhotonSpectrum(), cosmic_ray_grid=A56_GRID, photon_grid=A56_PHOTON)
+    m, (cc, cs), srcs = _small_batch(run, 75)
+    assert cc == 4 and cs > 1, (cc, cs)
+    ref = O.OracleSolver(run, 0.05, 0.0, K=75, exp="cr").solve([[s] for s in srcs], dz=1e-3)
+    worst, above, total = local_scale_check(m.state, ref, [s.sl for s in run.spec_man.species_refs], tol=TOL)
+    assert worst <= TOL, (worst, above, total)
+    assert above <= 1e-4 * total, (above, total)
