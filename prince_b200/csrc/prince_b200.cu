@@ -1940,6 +1940,10 @@ __device__ __forceinline__ void record_blocked(const StepParams& p, const StepSc
 // A k-tile's entries are stored without its zeros: `mask` has bit 4 g + kk set
 // where row g couples to mother kk, and the entries follow one another from
 // `base` in the order of those bits.
+// A group whose rows share few mothers is gathered instead (nkt < 0: -nkt
+// passes of one entry per row): its first record holds the rows' entry counts
+// (eight bytes) and the first entry's offset, and record 1 + t the eight rows'
+// mothers of pass t as slab rows; the entries lie pass by pass, eight places each.
 struct __align__(16) SlabK {
   unsigned mask;
   unsigned base;           // byte offset of the first entry from the slab's start
@@ -1947,7 +1951,7 @@ struct __align__(16) SlabK {
 };
 struct __align__(16) SlabG {
   unsigned short sp[8];    // species of the eight rows, 0xffff: none
-  int kt0, nkt;            // k-tiles, from the bin's first; an even count
+  int kt0, nkt;            // k-tiles, from the bin's first; an even count (a gathered group: see above)
   int pad[2];
 };
 
@@ -2026,6 +2030,11 @@ __device__ __forceinline__ uint4 lds_u4(unsigned a) {
 __device__ __forceinline__ double2 lds_d2(unsigned a) {
   double2 v;
   asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ unsigned lds_u16(unsigned a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return v;
 }
 __device__ __forceinline__ double lds_d(unsigned a) {
@@ -2110,9 +2119,47 @@ __device__ __noinline__ double4 slab_entries(unsigned ks, int nkt, unsigned slab
   return s;
 }
 
+// The sums of a gathered group in n passes: the quarter-warp of row g loads an entry and its mother's columns, four
+// passes in flight.
+__device__ __forceinline__ void slab_gather(unsigned ks, int n, unsigned slab, int lane, double (&s)[4]) {
+  const uint4 h = lds_u4(ks);
+  const unsigned g = lane >> 2, c = 2 * (lane & 3);
+  const int len = (g < 4 ? h.x : h.y) >> (8 * (g & 3)) & 255u;
+  unsigned at = slab + h.z + 8 * g, kr = ks + 16 + 2 * g;
+  s[0] = s[1] = s[2] = s[3] = 0.0;
+  for (int t = 0; t < n; t += 4, at += 4 * 64, kr += 4 * 16) {
+    unsigned r[4];
+    double v[4];
+    double2 x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool on = t + u < len;
+      r[u] = on ? lds_u16(kr + 16 * u) : 0u;
+      v[u] = on ? lds_d(at + 64 * u) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = lds_d2(slab + ((r[u] ^ c) << 4));
+      y[u] = lds_d2(slab + ((r[u] ^ (c + 1)) << 4));
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (t + u < len) {
+        s[0] = __fma_rn(v[u], x[u].x, s[0]);
+        s[1] = __fma_rn(v[u], x[u].y, s[1]);
+        s[2] = __fma_rn(v[u], y[u].x, s[2]);
+        s[3] = __fma_rn(v[u], y[u].y, s[3]);
+      }
+  }
+}
+
 // The group's sums of a lane's row and columns 4 t .. 4 t + 3.
 template <int PREF>
 __device__ __forceinline__ void slab_sums(unsigned ks, int nkt, unsigned slab, int lane, double (&sM)[4]) {
+  if (nkt < 0) {
+    slab_gather(ks, -nkt, slab, lane, sM);
+    return;
+  }
   double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};
   slab_tiles<PREF>(ks, nkt, slab, lane, acc0, acc1);
   sM[0] = acc0[0];
@@ -4602,6 +4649,13 @@ void const_steps(StepParams& p, const StepScal* scal, int64_t per_prep, double* 
 // its columns from the four classes of ((column / 2) mod 4) where it can: the
 // slab rows of distinct classes lie in distinct shared-memory banks.  A bin with
 // the previous bin's columns keeps its groups.
+// A group with no fewer k-tiles than its longest row has entries is gathered
+// (slab_gather): a pass of eight entries costs about a k-tile of up to 32, and the
+// tiles' zeros are work for nothing.  350 species with 16 random mothers each,
+// 512 columns: 245 us a launch in tiles, 180 gathered, 163 by the former row
+// quartets; 8 mothers 152, 149, 138; 4 or fewer 141 either way (130).  The A <= 56
+// network, whose rows share their mothers: 160 in tiles, 190 gathered, and 162
+// with the line at 7 / 8 of the longest row.
 struct SlabTiles {
   struct Row {
     int32_t sp;
@@ -4611,8 +4665,10 @@ struct SlabTiles {
     std::vector<int> rows;      // indices into the bin's rows
     std::vector<int32_t> cols;  // in k-tile order, four per tile (-1: none)
     bool pad = false;           // the last tile holds no entries
+    int gather = 0;             // passes of a gathered group, 0: tiles
   };
   int d, nsp, nwarps;
+  bool gathers;                 // false: tiles only (they take less shared memory)
   unsigned entry_offset;        // of the bin's entries from the slab's start in shared memory
   std::vector<int32_t> kbase, ebase, wrp;
   std::vector<SlabK> ks;
@@ -4622,8 +4678,9 @@ struct SlabTiles {
   std::vector<std::vector<int32_t>> last_cols;
   std::vector<Group> groups;
 
-  SlabTiles(int d_, int nsp_, int nwarps_)
-      : d(d_), nsp(nsp_), nwarps(nwarps_), entry_offset((unsigned)SlabSmem::rows(nsp_) * kSlabCols * sizeof(double)) {}
+  SlabTiles(int d_, int nsp_, int nwarps_, bool gathers_)
+      : d(d_), nsp(nsp_), nwarps(nwarps_), gathers(gathers_),
+        entry_offset((unsigned)SlabSmem::rows(nsp_) * kSlabCols * sizeof(double)) {}
 
   void make_groups(const std::vector<Row>& rows) {
     groups.clear();
@@ -4695,6 +4752,9 @@ struct SlabTiles {
         for (int q = 0; q < 3; ++q) gr.cols.push_back(-1);
         gr.pad = true;
       }
+      size_t longest = 0;
+      for (int i : gr.rows) longest = std::max(longest, rows[i].ent.size());
+      if (gathers && longest > 0 && longest < 256 && gr.cols.size() / 4 >= longest) gr.gather = (int)longest;
       groups.push_back(std::move(gr));
     }
   }
@@ -4721,7 +4781,8 @@ struct SlabTiles {
     for (int i : order) {
       const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
       wl[w].push_back(i);
-      load[w] += (int64_t)groups[i].cols.size() / 4 + 4;  // the update costs about four k-tiles
+      // the update costs about four k-tiles
+      load[w] += (groups[i].gather ? (int64_t)groups[i].gather : (int64_t)groups[i].cols.size() / 4) + 4;
     }
     unsigned ent = 0;
     std::vector<std::vector<int64_t>> at((size_t)kSlabRows, std::vector<int64_t>((size_t)nsp, -1));
@@ -4732,12 +4793,34 @@ struct SlabTiles {
         SlabG G;
         memset(&G, 0, sizeof(G));
         G.kt0 = (int)ks.size() - kb;
-        G.nkt = (int)gr.cols.size() / 4;
+        G.nkt = gr.gather ? -gr.gather : (int)gr.cols.size() / 4;
         for (int g = 0; g < kSlabRows; ++g) {
           G.sp[g] = g < (int)gr.rows.size() ? (unsigned short)rows[gr.rows[g]].sp : 0xffff;
           if (g >= (int)gr.rows.size()) continue;
           row_slot(rows[gr.rows[g]].sp, (int32_t)(gs.size() * kSlabRows + g));
+          if (gr.gather) continue;
           for (const auto& q : rows[gr.rows[g]].ent) at[g][q.first] = q.second;
+        }
+        if (gr.gather) {
+          SlabK h;
+          memset(&h, 0, sizeof(h));
+          std::vector<SlabK> pass((size_t)gr.gather, h);
+          unsigned char len[kSlabRows] = {};
+          for (int g = 0; g < (int)gr.rows.size(); ++g)
+            for (const auto& q : rows[gr.rows[g]].ent) {
+              const unsigned short r = (unsigned short)(8 * q.first + (q.first & 7));
+              memcpy(reinterpret_cast<char*>(&pass[len[g]]) + g * sizeof(r), &r, sizeof(r));
+              slot[q.second] = (int32_t)(nent + ent + len[g] * kSlabRows + g);
+              ++len[g];
+            }
+          memcpy(&h, len, sizeof(len));
+          const unsigned at0 = entry_offset + ent * (unsigned)sizeof(double);
+          memcpy(reinterpret_cast<char*>(&h) + 8, &at0, sizeof(at0));
+          ks.push_back(h);
+          ks.insert(ks.end(), pass.begin(), pass.end());
+          ent += (unsigned)(gr.gather * kSlabRows);
+          gs.push_back(G);
+          continue;
         }
         for (int k = 0; k < G.nkt; ++k) {
           SlabK K;
@@ -5418,9 +5501,10 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   // bin-local rows, per bin, as DMMA row groups and k-tiles (SlabTiles)
   int64_t band_nnz = 0, slab_nnz = 0;
   std::vector<int32_t> sslot((size_t)std::max<int64_t>(R, 1), -1), rowslot((size_t)n, -1);
-  SlabTiles tiles(d, nsp, kSlabWarps);
-  {
+  auto build_tiles = [&](bool gathers) {
+    SlabTiles t(d, nsp, kSlabWarps, gathers);
     std::vector<SlabTiles::Row> rows((size_t)nss);
+    slab_nnz = 0;
     for (int e = 0; e < d; ++e) {
       for (int i = 0; i < nss; ++i) {
         const int64_t r = (int64_t)sspec[i] * d + e;
@@ -5430,10 +5514,13 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
           if (ix[j] != r) rows[i].ent.push_back({ix[j] / d, j});
         slab_nnz += (int64_t)rows[i].ent.size();
       }
-      tiles.add_bin(rows, sslot, [&](int32_t sp, int32_t slot) { rowslot[(int64_t)sp * d + e] = slot; });
+      t.add_bin(rows, sslot, [&](int32_t sp, int32_t slot) { rowslot[(int64_t)sp * d + e] = slot; });
     }
-    tiles.finish();
-  }
+    t.finish();
+    return t;
+  };
+  SlabTiles tiles = build_tiles(true);
+  if (SlabSmem::bytes(nsp, tiles.maxe, tiles.maxk, tiles.maxg) > max_smem) tiles = build_tiles(false);
   const size_t ssm = SlabSmem::bytes(nsp, tiles.maxe, tiles.maxk, tiles.maxg);
   if (ssm > max_smem || tiles.nent >= ((int64_t)1 << 31)) return PB_OK;  // as above
   // band tiles: [species][band pair][2][RT / 2][J][32][2] DMMA A fragments per window
@@ -5524,8 +5611,8 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
   // transposed bin-local rows (mothers), per bin: every species is a row, its
   // columns the daughters of the same bin; groups and k-tiles as the forward rows'
   std::vector<int32_t> tslot((size_t)std::max<int64_t>(R, 1), -1);
-  SlabTiles ttiles(d, nsp, kSlabWarps);
-  {
+  auto build_ttiles = [&](bool gathers) {
+    SlabTiles t(d, nsp, kSlabWarps, gathers);
     std::vector<SlabTiles::Row> rows((size_t)nsp);
     for (int e = 0; e < d; ++e) {
       for (int m = 0; m < nsp; ++m) {
@@ -5537,10 +5624,13 @@ int pb_set_layout_rows(pb_context* c, int32_t d, int64_t n_blocks) {
         for (int64_t j = ip[r]; j < ip[r + 1]; ++j)
           if (ix[j] != r) rows[ix[j] / d].ent.push_back({sspec[i], j});
       }
-      ttiles.add_bin(rows, tslot, [](int32_t, int32_t) {});
+      t.add_bin(rows, tslot, [](int32_t, int32_t) {});
     }
-    ttiles.finish();
-  }
+    t.finish();
+    return t;
+  };
+  SlabTiles ttiles = build_ttiles(true);
+  if (SlabSmem::bytes(nsp, ttiles.maxe, ttiles.maxk, ttiles.maxg, 0) > max_smem) ttiles = build_ttiles(false);
   // k_slabT reduces the photon-scale gradient over the slab's space
   const size_t tsm = std::max(SlabSmem::bytes(nsp, ttiles.maxe, ttiles.maxk, ttiles.maxg, 0),
                               1024 + (size_t)kSlabWarps * 8 * kSlabCols * sizeof(double));
