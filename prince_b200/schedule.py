@@ -66,8 +66,9 @@ def make_schedule(zg, threshold):
         starts = [zg[0]]
     cm2sec = float(C.PRINCE_UNITS.cm2sec)
     om, ol, h0 = float(C.Omega_m), float(C.Omega_Lambda), float(C.H_0s)
-    hz = [h0 * math.sqrt(om * (1 + z) ** 3 + ol) for z in zs]            # cosmology.H
-    dl = [-1.0 / ((1.0 + z) * h * cm2sec) for z, h in zip(zs, hz)]       # cosmology.dldz
+    # the expressions of cosmology.H and cosmology.dldz (tests/test_schedule.py holds them together)
+    hz = [h0 * math.sqrt(om * (1 + z) ** 3 + ol) for z in zs]
+    dl = [-1.0 / ((1.0 + z) * h * cm2sec) for z, h in zip(zs, hz)]
     return Schedule(
         z=zg,
         window=np.array(win, dtype=np.int32),
