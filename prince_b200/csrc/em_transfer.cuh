@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(128) k_bgemm(BGemm g) {
 
 void launch_bgemm(cudaStream_t st, const BGemm& g, int batch) {
   const long long ctas64 = (long long)((g.N + 63) / 64) * ((g.M + 63) / 64) * batch;
-  if (ctas64 >= 148)
+  if (ctas64 >= kSMs)
     k_bgemm<4, 4, 16><<<dim3((g.N + 63) / 64, (g.M + 63) / 64, batch), 128, 0, st>>>(g);
   else
     k_bgemm<2, 1, 32><<<dim3((g.N + 15) / 16, (g.M + 31) / 32, batch), 128, 0, st>>>(g);

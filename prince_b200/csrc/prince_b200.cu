@@ -14,7 +14,7 @@
 //      the injection and the phi-function epilogue.  One column: a kernel per
 //      stage; a batch: band tiles, FD stencil, bin-local tiles and a finish per
 //      stage; a small network: all steps in one launch.  The factors of a run
-//      of steps come from one launch, and captured runs of 16 steps are
+//      of steps come from one launch, and captured runs of up to 16 steps are
 //      replayed for any schedule.
 //
 // The algorithm follows the reference CPU solver of PriNCe:
@@ -47,8 +47,9 @@
 namespace {
 
 constexpr int kAbiVersion = 2;
+constexpr int kSMs = 148;          // of a B200, in rules and sizes without a context
 constexpr int kLongRow = 256;      // rows with more coupling entries are cut into segments
-constexpr int kMaxPhoton = 200;    // photon bins held in shared memory by the fold (208 KB tile)
+constexpr int kMaxPhoton = 200;    // photon bins held in shared memory by the fold (157 KB at the most bins)
 constexpr int kColTile = 32;       // state columns per warp in the batched step
 constexpr int kSegLen = 256;       // coupling entries per long-row segment
 constexpr int kMaxEmBins = 1024;   // EM / nucleon bins of the cascade hook (as the transfer build)
@@ -562,8 +563,8 @@ __global__ void k_seg_map(const int64_t* __restrict__ cb, const int64_t* __restr
 
 // ---------------------------------------------------------------------------
 // fold GEMM on the FP64 tensor pipe: out[w][r] = sum_j K[r][j] * PT[w][j]
-// mma.sync m8n8k4 f64 (DMMA).  CTA tile 64 entries x 64 windows, whole photon
-// axis in shared memory; the epilogue scatters into M_off values / diagonal.
+// mma.sync m8n8k4 f64 (DMMA), whole photon axis in shared memory; the epilogue
+// scatters into M_off values / diagonal.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -816,13 +817,15 @@ __global__ void k_eval_exp(const double* __restrict__ x, double* __restrict__ y,
 // ---------------------------------------------------------------------------
 // ETD2 step kernels
 //
-// Per step, two launches (stage 1 and 2) over the rows; short rows get a warp,
-// rows with more than kLongRow coupling entries a whole CTA.  The per-row
-// factors of a step (kappa, eD, phi1, phi2) depend on z alone: k_prep computes
-// them for a run of steps in one launch (kPrepRows rows x steps), so that the
-// serial double-double exp of a row is never on a step's critical path.  One
-// launch per step (as part of the stage-2 kernels and a kernel of its own) cost
-// 5 us of latency each; a run of 16 steps of the A <= 56 network takes 15 us.
+// Per step, two launches (stage 1 and 2) over the rows: k_step_plain for one
+// column; k_step_multi, the general form for several, with a warp per short row
+// and a warp per segment of a row of more than kLongRow coupling entries; or the
+// bin-blocked kernels below.  The per-row factors of a step (kappa, eD, phi1,
+// phi2) depend on z alone: k_prep computes them for a run of steps in one launch
+// (kPrepRows rows x steps), so that the serial double-double exp of a row is
+// never on a step's critical path.  One launch per step (as part of the stage-2
+// kernels and a kernel of its own) cost 5 us of latency each; a run of 15 steps
+// of the A <= 56 network takes 15 us.
 // ---------------------------------------------------------------------------
 struct SlabK;
 struct SlabG;
@@ -1043,9 +1046,9 @@ __global__ void __launch_bounds__(128) k_prep(StepParams p) {
 }
 
 constexpr int64_t kPrepRows = 1 << 19;  // rows x steps of one k_prep launch (about 30 MB of factors)
-// Steps whose factors one launch prepares.
-constexpr int64_t kGraphSteps = 16;     // steps of a captured run
+constexpr int64_t kGraphSteps = 16;     // steps of a captured run, at most (15 at 33,600 rows: one launch prepares them)
 constexpr int64_t kPrepMaxSteps = 1024;
+// Steps whose factors one launch prepares.
 inline int64_t prep_steps(int64_t n) {
   return std::max<int64_t>(4, std::min<int64_t>(kPrepMaxSteps, kPrepRows / std::max<int64_t>(n, 1)));
 }
@@ -1741,9 +1744,10 @@ __global__ void __launch_bounds__(T, 1) k_small(StepParams p, SmallArgs q) {
 //  * bin-local rows: every M_off entry couples bin e to bin e of another
 //    species (boost-conserving fragments).  Their entries are stored
 //    bin-major (all rows of bin e contiguous).  k_slab stages the state slab
-//    of one bin -- all species x 32 columns -- and the bin's entries in shared
-//    memory and sums each row from there, so a state value is read from DRAM
-//    once per stage instead of once per coupling entry.
+//    of one bin -- all species x 16 columns -- and the bin's entries in shared
+//    memory and multiplies its rows from there in groups of eight (8 x 4 tiles,
+//    or entry by entry where they share few mothers), so a state value is read
+//    from DRAM once per stage instead of once per coupling entry.
 //  * band rows (species with cross-bin entries: the redistributed nucleons):
 //    their block rows against each mother species form a band of d x d tiles.
 //    k_band multiplies them on the FP64 tensor pipe (DMMA m8n8k4) with the
@@ -1752,13 +1756,14 @@ __global__ void __launch_bounds__(T, 1) k_small(StepParams p, SmallArgs q) {
 // The FD loss term D_off (kappa v) couples neighbouring bins of one species;
 // k_fd evaluates it species-major (one species block per CTA, in shared
 // memory) into fdbuf before the row kernels read it.  A stage is
-// k_band (second stream) || k_fd -> k_slab, then k_band_finish.
+// k_band (second stream) || k_fd -> k_slab, then k_band_finish; for up to eight
+// columns k_band with the loss term, k_slab, k_band_finish in a line.
 // ---------------------------------------------------------------------------
 constexpr int kFdMax = 4;           // off-diagonal FD stencil entries per row (bin-blocked path)
 constexpr int kFdHalo = 3;          // k_fd_dense: stencil offsets within +-kFdHalo bins
 constexpr int kFdDenseW = 8;        // dense weights per bin (2 kFdHalo + 1, padded to 16 bytes)
 constexpr int kFdChunk = 12;        // k_fd_dense: bins per warp pass
-constexpr int kMaxBandGroups = 148;
+constexpr int kMaxBandGroups = kSMs;
 
 // mbarrier and bulk-copy helpers of the TMA staging (CTA-local barrier, no cluster)
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -1995,9 +2000,6 @@ __device__ __forceinline__ const double2& slab_chunk(const char* slab, unsigned 
   return *reinterpret_cast<const double2*>(slab + r * 128u + ((c ^ (r & 7u)) << 4));
 }
 
-__device__ __forceinline__ double2 dadd2(double2 a, double2 b) {
-  return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
-}
 // The injection of one column (rows of injected species only).
 __device__ __forceinline__ double slab_inj(const StepParams& p, int64_t step, int slot, int src0, int src1) {
   const double* cf = p.coeff + (size_t)step * p.n_src;
