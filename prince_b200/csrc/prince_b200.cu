@@ -4626,18 +4626,64 @@ int64_t launch_steps(pb_context* c, StepParams& p, int K, const int32_t* n_activ
   return launches;
 }
 
-// All steps of a constant operator (one column), state x in place.
-void const_steps(StepParams& p, const StepScal* scal, int64_t per_prep, double* x, cudaStream_t st) {
+// One stage of a constant operator whose rows are short: a thread per row, the sum in CSR order without contraction
+// (as the host CSR product does).  Stage 2 forms the row's factors of the next step too (`next`, null at the last),
+// whose exp would take a launch of its own.
+template <int STAGE>
+__global__ void __launch_bounds__(256) k_const(StepParams p, double* next) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= p.n) return;
+  const double h = p.sc->h, own = p.src[r];
+  double F = 0.0;
+  const int64_t j1 = p.m_indptr[r + 1];
+#pragma unroll 4
+  for (int64_t j = p.m_indptr[r]; j < j1; ++j) F = __dadd_rn(F, __dmul_rn(p.m_vals[j], p.src[p.m_indices[j]]));
+  if (STAGE == 1) {  // a = eD x + (phi1 F(x)) h
+    p.a[r] = __dadd_rn(__dmul_rn(p.eD[r], own), __dmul_rn(__dmul_rn(p.phi1[r], F), h));
+    p.f[r] = F;
+    return;
+  }
+  // x = a + ((F(a) - F(x)) h) phi2
+  p.xout[r] = __dadd_rn(own, __dmul_rn(__dmul_rn(__dadd_rn(F, -p.f[r]), h), p.phi2[r]));
+  if (next) {
+    double e, f1, f2;
+    phi_of(p.sc[1].h, p.m_diag[r], e, f1, f2);
+    next[r] = e;
+    next[p.n + r] = f1;
+    next[2 * p.n + r] = f2;
+  }
+}
+
+// All steps of a constant operator (one column, dl/dz = 1), state x in place.  Up to four entries a row on average a
+// thread takes a row: with k_step_plain's four lanes a row, which fill four times the blocks, and k_prep's launches
+// 400 steps of 40,000 rows took 6.6 ms with one entry a row and with four (now 4.3 and 5.4), of 3,000 rows 4.5
+// (4.1).  Longer rows take the lanes: eight entries 4.6 ms against 5.6 for 3,000 rows, sixteen 8.2 against 11.5 for
+// 40,000.
+constexpr int64_t kConstEntries = 4;
+void const_steps(StepParams& p, const StepScal* scal, int64_t nnz, int64_t per_prep, double* x, cudaStream_t st) {
   p.x = x;
   p.xout = x;
+  const bool rows = nnz <= kConstEntries * p.n;
+  const int64_t slot = 4 * p.n;  // row factors of one step; two fit the smallest scratch
+  if (rows && p.n_steps > 0) launch_prep(p, scal, 0, 1, st);
   for (int64_t k = 0; k < p.n_steps; ++k) {
+    p.sc = scal + k;
+    p.src = x;
+    if (rows) {
+      p.eD = p.rf + (k & 1) * slot;
+      p.phi1 = p.eD + p.n;
+      p.phi2 = p.phi1 + p.n;
+      k_const<1><<<blocks_for(p.n, 256), 256, 0, st>>>(p, nullptr);
+      p.src = p.a;
+      k_const<2><<<blocks_for(p.n, 256), 256, 0, st>>>(p, k + 1 < p.n_steps ? p.rf + ((k + 1) & 1) * slot : nullptr);
+      continue;
+    }
     if (k % per_prep == 0) {
       p.rf_k0 = k;
       launch_prep(p, scal, k, std::min(per_prep, p.n_steps - k), st);
+      p.sc = scal + k;
     }
     set_step_factors(p, k);
-    p.sc = scal + k;
-    p.src = x;
     k_step_plain<1><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
     p.src = p.a;
     k_step_plain<2><<<plain_blocks(p), kPlainThreads, 0, st>>>(p);
@@ -6849,7 +6895,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
     return rc;
   }
   if (A.ensure((size_t)n * sizeof(double)) != cudaSuccess || F.ensure((size_t)n * sizeof(double)) != cudaSuccess ||
-      rowf.ensure((size_t)prep_steps(n) * 4 * n * sizeof(double)) != cudaSuccess) {
+      rowf.ensure((size_t)(nnz <= kConstEntries * n ? 2 : prep_steps(n)) * 4 * n * sizeof(double)) != cudaSuccess) {
     cleanup();
     return fail(c, PB_ERR_CUDA, "pb_integrate_const: allocation failed");
   }
@@ -6869,7 +6915,7 @@ int pb_integrate_const(pb_context* c, int64_t n, const double* d, int64_t nnz, c
   p.n_prows = (int)n;
   p.n_steps = n_steps;
   p.rf = rowf.as<double>();
-  const_steps(p, hs.as<StepScal>(), prep_steps(n), X.as<double>(), st);
+  const_steps(p, hs.as<StepScal>(), nnz, prep_steps(n), X.as<double>(), st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(state, X.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -6959,7 +7005,7 @@ int pb_integrate_const_noalloc(pb_context* c, int64_t n, const double* d, int64_
   p.n_prows = (int)n;
   p.n_steps = n_steps;
   p.rf = rowf;
-  const_steps(p, scal, kNaPrepSteps, state, st);
+  const_steps(p, scal, nnz, kNaPrepSteps, state, st);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(c, PB_ERR_CUDA, "pb_integrate_const_noalloc: %s", cudaGetErrorString(e));
