@@ -2191,7 +2191,7 @@ __device__ __forceinline__ void slab_sums(unsigned ks, int nkt, unsigned slab, i
 // K = 512, 84 per 16-column group of 16 entries); an 8 x 4 tile reads its four
 // mothers' rows once for eight daughters: at the A <= 56 network 458 k-tiles of
 // 35% fill per bin instead of 1,476 entry quads, 8 wavefronts and 8 tensor
-// clocks each.  Measured per launch at K = 512: 165 / 170 us before, 160 / 154 us
+// clocks each.  Measured per launch at K = 512: 165 / 170 us before, 160 / 156 us
 // now; what is left is the latency of a CTA's phases (staging, products, update)
 // at two CTAs per SM: 2 x 12 warps, three teams of eight warps sharing the
 // tables, and entries read from L2 at four CTAs per SM were slower (163 / 170,
